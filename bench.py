@@ -99,8 +99,14 @@ KERNEL_FLOPS = {
 }
 
 
+def n_planes(S):
+    """Digit planes per operand of split code S (six digits are five nine-bit planes)."""
+    return 5 if S == 6 else S
+
+
 def n_products(S):
-    """bf16 slice products per FP64 product: pairs (s, t) with s + t <= S + 1."""
+    """bf16 slice products per FP64 product: pairs (s, t) with s + t <= planes + 1."""
+    S = n_planes(S)
     return S * (S + 1) // 2
 
 
@@ -427,7 +433,7 @@ def run_ours(args):
         # digit planes once + T written; part of T's writes still sit in L2 at
         # the end of the launch); the same ratio applied to this workload's bytes
         kpad = -(-N // 16) * 16
-        alg_bytes = float(N) * Q * kpad * 2 * S + 8.0 * P * N * Q
+        alg_bytes = float(N) * Q * kpad * 2 * n_planes(S) + 8.0 * P * N * Q
         traffic = 0.9883 * alg_bytes
     if name.startswith("ozaki_tc"):
         tensor_fl = n_products(S) * fl
@@ -698,8 +704,8 @@ def mo_kernel_bytes(N, P, Q, S):
     """Algorithmic DRAM bytes per call of each bandwidth-bound kernel of
     computeJKH_MO ("jkh") and computeLagrange2 ("lag2"): every input read once
     and every output written once (float64 = 8 B; a digit slicing reads 8 B and
-    writes 2S B per element, its exponent pass reads the 8 B once more)."""
-    dig = 8 + 2 * S
+    writes 2 B per plane and element, its exponent pass reads the 8 B once more)."""
+    dig = 8 + 2 * n_planes(S)
     jkh = {
         "slice_digits": (P * N + P * N * Q) * dig,
         "slice_rowexp": (P * N + P * N * Q) * 8,

@@ -320,12 +320,13 @@ int gb_graph_destroy(gb_graph* graph);
 /* ========================================================================
  * Split-product ("mixed") path on the tcgen05 tensor cores.
  *
- * FP64 operands are cut into nslices (1..6) balanced base-128 bf16 digit
- * slices with a power-of-two exponent per row; the slice products with
- * s + t <= nslices + 1 run as bf16 tcgen05 MMAs with FP32 accumulation in
- * TMEM, the leading product groups accumulated exactly.  nslices = 6 agrees
- * with FP64 to ~1e-12 normwise; nslices = 2 is the three-product bf16x3 split
- * (~1e-4).  nslices = GB_SPLIT_TF32X3 selects the three-product TF32 split
+ * FP64 operands are cut into bf16 digit slices with a power-of-two exponent
+ * per row: nslices = 1..5 asks for that many balanced 7-bit digits, nslices = 6
+ * for five 9-bit ones (45 bits, more than six 7-bit digits hold).  The products
+ * of slices s and t with s + t <= number of slices + 1 run as bf16 tcgen05 MMAs
+ * with FP32 accumulation in TMEM, the leading product groups accumulated
+ * exactly.  nslices = 6 agrees with FP64 to ~1e-12 normwise; nslices = 2 is the
+ * three-product bf16x3 split (~1e-4).  nslices = GB_SPLIT_TF32X3 selects the three-product TF32 split
  * instead (hi = tf32(x), lo = tf32(x - hi); hi hi + hi lo + lo hi as tf32
  * tcgen05 MMAs, FP32 accumulation; ~1e-6).  Device status of these kernels:
  * gb_device_status.

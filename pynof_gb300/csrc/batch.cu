@@ -133,10 +133,10 @@ extern "C" int gb_jkj_batch_create_mixed(int nmol, const double* const* C, const
   }
   // phases whose outputs store rows along their unit stride (orbitals on the
   // 128-wide N tile, and K) run as persistent grouped launches
-  bool persT = false, persJ = false, persK = false;
-  GB_TRY(ozaki_group_upload(pt.data(), nmol, tabT, &persT));
-  GB_TRY(ozaki_group_upload(pj.data(), nmol, tabJ, &persJ));
-  GB_TRY(ozaki_group_upload(pk.data(), nmol, tabK, &persK));
+  bool persT = false, persJ = false, persK = false, fdT = false, fdJ = false, fdK = false;
+  GB_TRY(ozaki_group_upload(pt.data(), nmol, tabT, &persT, &fdT));
+  GB_TRY(ozaki_group_upload(pj.data(), nmol, tabJ, &persJ, &fdJ));
+  GB_TRY(ozaki_group_upload(pk.data(), nmol, tabK, &persK, &fdK));
 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // The per-molecule kernels between the grouped GEMMs (slicing, the diagonal
@@ -187,16 +187,16 @@ extern "C" int gb_jkj_batch_create_mixed(int nmol, const double* const* C, const
     GB_TRY(branches([&](int i, cudaStream_t b) {
       return slice_operand(SliceSrc{C[i], 0, lin(1), lin(nbf[i]), false}, ws[i].A, b);
     }));
-    GB_TRY(ozaki_gemm_grouped(tabT, nmol, tilesT, S, pt[0].g.bn, s, "ozaki_tc:batch_half_transform", persT));
+    GB_TRY(ozaki_gemm_grouped(tabT, nmol, tilesT, S, pt[0].g.bn, s, "ozaki_tc:batch_half_transform", persT, fdT));
     GB_TRY(branches([&](int i, cudaStream_t b) {
       GB_TRY(launch_contract_diag(C[i], ws[i].Tf, ws[i].dv, nbf[i], nbf5[i], naux[i], b));
       return slice_operand(SliceSrc{ws[i].dv, 0, lin(naux[i]), lin(1), true}, ws[i].d, b);
     }));
-    GB_TRY(ozaki_gemm_grouped(tabJ, nmol, tilesJ, S, pj[0].g.bn, s, "ozaki_tc:batch_J", persJ));
+    GB_TRY(ozaki_gemm_grouped(tabJ, nmol, tilesJ, S, pj[0].g.bn, s, "ozaki_tc:batch_J", persJ, fdJ));
     GB_TRY(branches([&](int i, cudaStream_t b) {
       return slice_operand(SliceSrc{ws[i].Tf, (long long)nbf[i] * naux[i], lin(naux[i]), lin(1), true}, ws[i].T, b);
     }));
-    GB_TRY(ozaki_gemm_grouped(tabK, nmol, tilesK, S, 128, s, "ozaki_tc:batch_K", persK));
+    GB_TRY(ozaki_gemm_grouped(tabK, nmol, tilesK, S, 128, s, "ozaki_tc:batch_K", persK, fdK));
     return GB_OK;
   };
   st = body();

@@ -49,8 +49,15 @@ enum SymMode { SYM_NONE = 0, SYM_ROWCOL = 1, SYM_PAIRCOL = 2, SYM_TRIROW = 4, SY
 // Packed upper-triangle index r = m N - m (m - 1) / 2 + (n - m), 0 <= m <= n < N,
 // back to (m, n) (rows of the triangle in order, each from its diagonal on).
 __host__ __device__ __forceinline__ void tri_pair(long long r, int N, int& m, int& n) {
+#ifdef __CUDA_ARCH__
+  // an FP32 estimate, a step or two off at most (a double square root takes ~700 clocks here)
+  const float b = 2.0f * (float)N + 1.0f;
+  const unsigned long long left = (unsigned long long)(2ll * N + 1) * (unsigned long long)(2ll * N + 1) - 8ull * (unsigned long long)r;
+  long long x = (long long)((b - sqrtf((float)left)) * 0.5f);
+#else
   const double b = 2.0 * N + 1.0;
   long long x = (long long)((b - sqrt(b * b - 8.0 * (double)r)) * 0.5);
+#endif
   x = x < 0 ? 0 : (x > N - 1 ? N - 1 : x);
   while (x > 0 && x * N - x * (x - 1) / 2 > r) --x;
   while (x + 1 < N && (x + 1) * N - (x + 1) * x / 2 <= r) ++x;

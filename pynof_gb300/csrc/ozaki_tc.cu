@@ -1,18 +1,19 @@
 // tcgen05 split-product FP64 GEMM (see ozaki_tc.cuh).
 //
 // CTA tile: 128 rows of A (M) x BN rows of B (N), BN in {32, 64, 128}.
-// 18 warps.  warp 0 lane 0 is the producer: a 4-stage ring in which every
-// stage holds the S slices of a 128 x 16 block of A (one contiguous
+// 18 warps.  warp 0 lane 0 is the producer: a ring of STAGES stages in which
+// every stage holds the S slices of a 128 x 16 block of A (one contiguous
 // cp.async.bulk copy -- the slicer stores the digits in the tensor-core
 // core-matrix order, slice.cuh) and of a BN x 16 block of B (one copy, or two
 // per slice when BN < 128).  warp 1 allocates TMEM (4 BN columns) and its
-// lane 0 issues tcgen05.mma (M=128, N=BN, K=16, bf16 -> f32).  warps 2..17
+// lane 0 issues tcgen05.mma (M=128, K=16, bf16 -> f32; N=BN, or a multiple of
+// it where consecutive B slices go to consecutive accumulators).  warps 2..17
 // drain and finish: warp w reads TMEM lanes 32 (w % 4) .. +31 (tile rows) and
 // BN/4 columns from (w - 2) / 4 * BN/4 of every accumulator.
 //
 // TMEM columns: [0,BN) group 2, [BN,2BN) group 3, [2BN,3BN) group 4 (exact,
-// drained every 12 stages = 192 k), [3BN,4BN) groups 5.. (whole K, or per
-// chunk with fdrain).
+// drained after every chunk, chunk_blocks), [3BN,4BN) groups 5.. (whole K, or
+// per chunk with fdrain).
 //
 // One launch covers one GEMM (optionally batched), or -- the grouped kernel --
 // a table of GEMMs of different shapes (e.g. one per molecule of a batch).
@@ -37,7 +38,15 @@ static __device__ int g_tc_status;
 namespace gb {
 namespace {
 
-constexpr int BM = 128, BK = SL_K, STAGES = 4, CH = 12;
+constexpr int BM = 128, BK = SL_K, STAGES = 5;
+constexpr int CH_TF32 = 12;  // stages per chunk of the TF32x3 form (96 k)
+constexpr int CH_W7 = 12;    // and of seven-bit digits (192 k: groups 2 and 4 below 2^22 units whatever the digits are)
+// Nine-bit digits: stages per chunk that are exact whatever the digits are: 48 k, where group 2
+// stays below 2^16 * 48 < 2^22 - 2^16 units and groups 3 and 4 below
+// 3 * 2^16 * 48 < 2^24 - 2^16 (see drain_exact for the limits).
+constexpr int CH_MIN = 3;
+constexpr float LIM_G2 = 4194304.0f - 65536.0f, LIM_G34 = 16777216.0f - 65536.0f;
+constexpr int CH_RUNS_MAX = 32;  // runs of 128 k per chunk at most (the FP32 group's own range)
 constexpr int NUM_EPI_WARPS = 16, THREADS = 32 * (2 + NUM_EPI_WARPS);
 // 18 warps put 5 warps on two of the four SM sub-partitions, whose register
 // files hold 16K registers each: 5 * 32 * 96 <= 16384 caps the kernel at 96.
@@ -64,6 +73,8 @@ struct TileCfg {
 __host__ __device__ constexpr uint32_t epi_table_bytes(int BN) { return 20u * (uint32_t)(BM + BN); }
 constexpr float MAGIC = 12582912.0f;                          // 1.5 * 2^23
 constexpr int MAGIC_BITS = 0x4B400000;
+constexpr int FDRAIN_K = 4096;  // K above which the FP32 group is drained per chunk (OzGemm::fdrain)
+constexpr int PAIR_FRAC = 9;    // fraction bits of the assembly up to FDRAIN_K (fold_pair)
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -87,12 +98,16 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 
+// A waiting thread may sleep this long per try: 17 warps that poll take issue
+// slots and shared-memory cycles from the MMA warp.
+constexpr uint32_t WAIT_HINT_NS = 20000;
+
 __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   uint32_t done;
   asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}\n"
       : "=r"(done)
-      : "r"(bar), "r"(parity)
+      : "r"(bar), "r"(parity), "r"(WAIT_HINT_NS)
       : "memory");
   return done != 0;
 }
@@ -136,9 +151,10 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                : "memory");
 }
 
-// UMMA shared-memory descriptor of one slice tile of `rows` rows x 16 k:
-// K-major, no swizzle; core matrices (8 rows x 16 B) rows*16 B apart along K
-// (leading byte offset) and 128 B apart along the rows (stride byte offset).
+// UMMA shared-memory descriptor of the first slice of a stage's operand, whose
+// k groups hold `rows` rows in all (S slices one after another): K-major, no
+// swizzle; core matrices (8 rows x 16 B) rows*16 B apart along K (leading byte
+// offset) and 128 B apart along the rows (stride byte offset).
 __device__ __forceinline__ uint64_t desc_tile(uint32_t saddr, uint32_t rows) {
   uint64_t d = (uint64_t)((saddr >> 4) & 0x3FFFu);
   d |= (uint64_t)((rows * 16u) >> 4) << 16;  // leading byte offset
@@ -203,35 +219,96 @@ __device__ __forceinline__ long long split_round(float t, int frac, float two_fr
   return (long long)((unsigned long long)(long long)ti << frac) + fi;
 }
 
-// Drain of the exact groups g = 2..gE of CW columns of this warp's TMEM lanes
-// into R: group g holds FP32 integer multiples of 2^-7g below 2^22 units, taken
-// out with magic_int and combined as sum_g i_g 2^(7 (gE - g)) (units of
-// 2^-7gE; groups 3 and 4 fit one int32, < 2^30), scaled by 2^fr.
-template <int BN, int gE, int CW>
+// Exponent of group g's unit 2^-(e_s + e_t), s + t = g.
+__host__ __device__ constexpr int group_exp(int W, int g) { return W == 9 ? 9 * g - 2 : W * g; }
+
+// One element's exact groups, as FP32 values x2, x3, x4 (integers u_g over the
+// unit U_g): from the last group up, the nearest multiple of 2^W units is
+// carried into the group above (exact in FP32 while |u_3|, |u_4| stay below
+// 2^24 - 2^16).  Leaves the top group with its carry (below 2^22 units) in x2 and
+// returns the remainders, an FP32 value below 2^(2 W - 1) + 2^(W - 1) units of the last
+// group.
+template <int W, int gE>
+__device__ __forceinline__ float carry_groups(float& x2, float x3, float x4) {
+  constexpr float B = (float)(1 << W);
+  constexpr float U2 = (float)(1ll << group_exp(W, 2)), U3 = U2 * B, U4 = U3 * B;  // units per 1.0
+  float low = 0.0f;
+  if (gE >= 4) {
+    const float h4 = fmaf(x4, U4 / B, MAGIC) - MAGIC;  // rint(u_4 / 2^W), in units of group 3
+    low = fmaf(h4, -1.0f / U3, x4);
+    x3 = fmaf(h4, 1.0f / U3, x3);
+  }
+  if (gE >= 3) {
+    const float h3 = fmaf(x3, U3 / B, MAGIC) - MAGIC;
+    const float l3 = fmaf(h3, -1.0f / U2, x3);
+    low = gE >= 4 ? low + l3 : l3;
+    x2 = fmaf(h3, 1.0f / U2, x2);
+  }
+  return low;
+}
+
+// Drain of the exact groups g = 2..gE of CW columns of this warp's TMEM lanes.
+//
+// Up to FDRAIN_K of K (fdrain off) an element's sum is a pair of 32-bit parts
+// held in the two halves of its R: the top group's units as an integer (the
+// magic number's bits are added as they are; their bias comes off in
+// fold_pair) and the remainders as an FP32 number, exact below 2^24 units, i.e.
+// for FDRAIN_K / 48 = 86 chunks of at most 2^17.1 units.  That is 11 single-issue
+// instructions an element; 64-bit sums take about twice that, and at one
+// instruction a clock and sub-partition a drain took 3.8 to 4.3 K clocks of
+// which the MMAs waited for most (1.8 K now).
+// With fdrain R is a 64-bit integer in units of the last group, scaled by 2^fr.
+template <int BN, int W, int gE, bool PAIR, int CW>
 __device__ __forceinline__ void drain_exact(uint32_t lbase, long long (&R)[CW], int fr) {
+  constexpr float U2 = (float)(1ll << group_exp(W, 2)), UE = (float)(1ll << group_exp(W, gE));
 #pragma unroll
   for (int h = 0; h < CW / 4; ++h) {
-    uint32_t v2[4], v3[4], v4[4];
+    uint32_t v2[4], v3[4] = {}, v4[4] = {};
     tmem_ld4_async(lbase + (uint32_t)(h * 4), v2);
     if (gE >= 3) tmem_ld4_async(lbase + (uint32_t)(BN + h * 4), v3);
     if (gE >= 4) tmem_ld4_async(lbase + (uint32_t)(2 * BN + h * 4), v4);
     tmem_wait_ld();
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int i2 = magic_int(__uint_as_float(v2[j]), 16384.0f);  // 2^14
-      long long acc;
-      if (gE == 2) {
-        acc = i2;
-      } else if (gE == 3) {
-        acc = (long long)i2 * 128 + magic_int(__uint_as_float(v3[j]), 2097152.0f);  // 2^21
+      float x2 = __uint_as_float(v2[j]);
+      const float low = carry_groups<W, gE>(x2, __uint_as_float(v3[j]), __uint_as_float(v4[j]));
+      long long& r = R[h * 4 + j];
+      if constexpr (PAIR) {
+        const uint32_t top = (uint32_t)r + __float_as_uint(fmaf(x2, U2, MAGIC));
+        const float rest = __uint_as_float((uint32_t)((unsigned long long)r >> 32)) + low;
+        r = (long long)(((unsigned long long)__float_as_uint(rest) << 32) | top);
       } else {
-        const int i34 = magic_int(__uint_as_float(v3[j]), 2097152.0f) * 128 +
-                        magic_int(__uint_as_float(v4[j]), 268435456.0f);  // 2^28
-        acc = (long long)i2 * 16384 + i34;
+        asm volatile("" : "+l"(r));
+        const long long acc = (long long)magic_int(x2, U2) * (1 << (group_exp(W, gE) - group_exp(W, 2))) +
+                              (gE >= 3 ? magic_int(low, UE) : 0);
+        r += (long long)((unsigned long long)acc << fr);
       }
-      R[h * 4 + j] += (long long)((unsigned long long)acc << fr);
     }
   }
+}
+
+// An element's pair (see drain_exact) after `chunks` drains with the FP32 group's
+// value f (|f| < 2^21 units of the last exact group) added: the top part keeps
+// its unit, the other half becomes an integer in units of the last exact
+// group's 2^-PAIR_FRAC, |rest| < 2^17 + 2^21 of them.  wide_pair makes one 64-bit
+// integer of the two.
+template <int W, int gE, bool HAS_F>
+__device__ __forceinline__ long long fold_pair(long long r, float f, uint32_t bias) {
+  constexpr float U2 = (float)(1ll << group_exp(W, 2)), UE = (float)(1ll << group_exp(W, gE));
+  uint32_t top = (uint32_t)r - bias, rest = 0;
+  if (gE > 2) {
+    const float low = __uint_as_float((uint32_t)((unsigned long long)r >> 32));
+    const float h = fmaf(low, U2, MAGIC);  // carry of the summed remainders
+    top += __float_as_uint(h) - (uint32_t)MAGIC_BITS;
+    rest = (uint32_t)magic_int(fmaf(h - MAGIC, -1.0f / U2, low), UE) << PAIR_FRAC;
+    if (HAS_F) rest += (uint32_t)__float2int_rn(f * (UE * (float)(1 << PAIR_FRAC)));
+  }
+  return (long long)(((unsigned long long)rest << 32) | top);
+}
+template <int W, int gE>
+__device__ __forceinline__ long long wide_pair(long long r) {
+  constexpr int A = group_exp(W, gE) - group_exp(W, 2) + PAIR_FRAC;
+  return (long long)(int)(uint32_t)r * (1ll << A) + (long long)(int)(uint32_t)((unsigned long long)r >> 32);
 }
 
 // int64 fixed point z * 2^scale -> double, round to nearest even, integer ops
@@ -254,16 +331,28 @@ __device__ __forceinline__ double fixed_to_double(long long z, int scale, int ne
   return __longlong_as_double((long long)(sign | ((((unsigned long long)(ef - 1)) << 52) + mant + up)));
 }
 
-// z * 2^scale as a double, negated when `negate`: the hardware int64 -> double
-// conversion (round to nearest even, as fixed_to_double) with the scale added
-// to the exponent field; results outside the normal range take the integer path.
-__device__ __forceinline__ double scaled_to_double(long long z, int scale, int negate) {
-  const long long b0 = __double_as_longlong(__ll2double_rn(z));
-  const int e0 = (int)((b0 >> 52) & 0x7FF) + scale;
-  if (z != 0 && e0 >= 1 && e0 <= 2046)
-    return __longlong_as_double((long long)(((unsigned long long)b0 + ((unsigned long long)(long long)scale << 52)) ^
-                                            ((unsigned long long)(negate != 0) << 63)));
-  return fixed_to_double(z, scale, negate);
+// z * 2^scale as a double, with the sign flipped where `flip` has its top bit: the
+// hardware int64 -> double conversion with the scale added to the exponent
+// field (shifting the leading one into place with integer instructions instead
+// made a tile's stores 18 K clocks long, this way 12 K).  False for results
+// outside the normal range, which are for fixed_to_double.
+__device__ __forceinline__ bool scaled_to_double(long long z, int scale, uint32_t flip, double& out) {
+  const double d = __ll2double_rn(z);
+  const uint32_t h = (uint32_t)__double2hiint(d);
+  const uint32_t e0 = ((h >> 20) & 0x7FFu) + (uint32_t)scale - 1u;
+  const bool zero = h == 0;
+  out = zero ? 0.0 : __hiloint2double((int)((h + ((uint32_t)scale << 20)) ^ flip), __double2loint(d));
+  return zero || e0 < 2046u;
+}
+
+// Widest store (in doubles) that p's alignment allows, and a store of four.
+__device__ __forceinline__ int store_width(const double* p) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+  return (a & 31) == 0 ? 4 : (a & 15) == 0 ? 2 : 1;
+}
+__device__ __forceinline__ void store4(double* p, const double (&v)[4]) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3])
+               : "memory");
 }
 
 struct KArgs {
@@ -303,60 +392,119 @@ __device__ __forceinline__ void mma_bf16_c(uint32_t d_tmem, uint64_t a, uint64_t
         : "memory");
 }
 
+// Stages per chunk of a tile: the longest multiple of the slicer's 128-k runs
+// whose exact groups' partial sums provably stay within the drain's limits, from
+// the norms of the two row blocks (a run's sum of products of digits s and t is
+// at most 2 sqrt(norm_s norm_t)); CH_MIN where not even one run is.  Digits of
+// the path's operands (Gaussian-like rows) allow 2 to 3 runs, 256 to 384 k; the
+// worst case alone would allow 48 k, and the 192-k chunks of seven-bit digits
+// took 21 products instead of 15.
+template <int W>
+__device__ __forceinline__ int chunk_blocks(const SlicedDesc& A, const SlicedDesc& B, int bz, int m0, int n0,
+                                            int nkb) {
+  if (W != 9) return CH_W7;
+  if (nkb <= CH_MIN) return CH_MIN;
+  const int* na = A.norms + ((long long)(A.batch == 1 ? 0 : bz) * A.rblocks() + m0 / SL_ROWS) * SL_NORMS;
+  const int* nb = B.norms + ((long long)(B.batch == 1 ? 0 : bz) * B.rblocks() + n0 / SL_ROWS) * SL_NORMS;
+  float a[SL_NORMS], b[SL_NORMS];
+#pragma unroll
+  for (int i = 0; i < SL_NORMS; ++i) {
+    a[i] = sqrtf(__int_as_float(__ldg(na + i)));
+    b[i] = sqrtf(__int_as_float(__ldg(nb + i)));
+  }
+  const float up = 2.002f;  // the bound's 2, and room for the roundings of the norms
+  const float g2 = up * a[0] * b[0], g3 = up * (a[0] * b[1] + a[1] * b[0]),
+              g4 = up * (a[0] * b[2] + a[2] * b[0] + a[1] * b[1]);
+  const float most = fminf(LIM_G2 / fmaxf(g2, 1.0f), LIM_G34 / fmaxf(fmaxf(g3, g4), 1.0f));
+  if (!(most >= 1.0f)) return CH_MIN;
+  return SL_KPC * (most < (float)CH_RUNS_MAX ? (int)most : CH_RUNS_MAX);
+}
+
 // Products of one stage (S digit slices; product (s, t) of A slice s and B
 // slice t goes to group g = s + t, kept only for g <= S + 1), fully unrolled
 // and ordered by A slice: the products of one A slice run back to back and
 // take A from the collector after the first, so each A slice tile is read
-// from shared memory once per stage (6 reads instead of 21 at S = 6; B is
-// read per product).  The slice tiles' descriptors differ from the stage's
-// first ones only in the start-address field.
+// from shared memory once per stage (5 reads instead of 15 at S = 5; B is
+// read per product).  The slices' descriptors differ from the stage's first
+// ones only in the start-address field.
 //   SEL 0: every product; 1: the FP32 group only (g >= 5); 2: the exact
 //   groups only (g <= 4, accumulator columns (g - 2) BN).
+//   WIDE: consecutive B slices whose groups' accumulators are consecutive (g,
+//   g + 1, .. <= 5) go into one MMA of up to 256 columns (11 MMAs instead of
+//   15 at BN = 128); otherwise one MMA per product, as wide as idesc says.
 //   restart_exact: the exact groups start from zero (their first product,
-//   s = 1, overwrites); restart_f: the FP32 group (at 3 BN) starts from zero.
-template <int S, int BN, int SEL>
+//   s = 1, overwrites); restart_f: the FP32 group (at 3 BN) starts from zero
+//   (equal to restart_exact when SEL == 0).
+template <int S, int BN, int SEL, bool WIDE>
 __device__ __forceinline__ void issue_products(uint32_t tmem, uint64_t da, uint64_t db, uint32_t idesc,
                                                bool restart_exact, bool restart_f) {
   using T = TileCfg<BN, 0>;
   bool f_first = true;
 #pragma unroll
   for (int s = 1; s <= S; ++s) {
-    const uint64_t das = da + (uint64_t)((s - 1) * (TILE_BYTES >> 4));
+    const uint64_t das = da + (uint64_t)((s - 1) * (SL_SLICE_STEP >> 4));
     // this slice's products under SEL: t in [t0, t1]
     const int t0 = SEL == 1 ? (5 - s > 1 ? 5 - s : 1) : 1;
     const int t1 = SEL == 2 ? (4 - s < S + 1 - s ? 4 - s : S + 1 - s) : S + 1 - s;
+    int t = t0;
 #pragma unroll
-    for (int t = t0; t <= t1; ++t) {
+    for (int it = 0; it < S; ++it) {
+      if (t > t1) break;
       const int gg = s + t;
       const bool exact = gg <= 4;
+      int w = 1;  // products in this MMA
+      if (WIDE && exact) {
+        w = 256 / BN;
+        w = w < t1 - t + 1 ? w : t1 - t + 1;
+        w = w < 6 - gg ? w : 6 - gg;
+      }
       const uint32_t d = tmem + (uint32_t)((exact ? gg - 2 : 3) * BN);
-      const uint64_t dbt = db + (uint64_t)((t - 1) * (T::B_TILE >> 4));
+      const uint64_t dbt = db + (uint64_t)((t - 1) * BN);
+      const uint32_t id = WIDE ? (T::IDESC & ~(0x3Fu << 17)) | ((uint32_t)((w * BN) >> 3) << 17) : idesc;
       bool acc;
       if (exact) {
         acc = !(restart_exact && s == 1);
       } else {
         acc = !(restart_f && f_first);
-        f_first = false;
       }
-      if (t0 == t1)
-        mma_bf16_c<0>(d, das, dbt, idesc, acc);
-      else if (t == t0)
-        mma_bf16_c<1>(d, das, dbt, idesc, acc);
-      else if (t == t1)
-        mma_bf16_c<3>(d, das, dbt, idesc, acc);
+      if (gg + w - 1 >= 5) f_first = false;
+      const bool head = t == t0, tail = t + w > t1;
+      if (head && tail)
+        mma_bf16_c<0>(d, das, dbt, id, acc);
+      else if (head)
+        mma_bf16_c<1>(d, das, dbt, id, acc);
+      else if (tail)
+        mma_bf16_c<3>(d, das, dbt, id, acc);
       else
-        mma_bf16_c<2>(d, das, dbt, idesc, acc);
+        mma_bf16_c<2>(d, das, dbt, id, acc);
+      t += w;
     }
   }
+}
+
+// The same with the width chosen at run time: a tile whose last columns are
+// missing runs one MMA per product, only as wide as it needs, when that is
+// cheaper (below ~104 columns an MMA takes 53 clocks whatever its width, a
+// 128-column one 65).
+template <int S, int BN, int SEL>
+__device__ __forceinline__ void issue_stage(bool wide, uint32_t tmem, uint64_t da, uint64_t db, uint32_t idesc,
+                                            bool restart_exact, bool restart_f) {
+  if (wide)
+    issue_products<S, BN, SEL, true>(tmem, da, db, idesc, restart_exact, restart_f);
+  else
+    issue_products<S, BN, SEL, false>(tmem, da, db, idesc, restart_exact, restart_f);
+}
+template <int BN>
+__device__ __forceinline__ bool wide_tile(int n_mma) {
+  return BN < 128 || n_mma > 104;
 }
 
 // TF32x3 products of one stage: hi hi + hi lo + lo hi into the one accumulator.
 template <int BN>
 __device__ __forceinline__ void issue_tf32(uint32_t tmem, uint64_t da, uint64_t db, uint32_t idesc, bool& started) {
-  using T = TileCfg<BN, 1>;
   mma_tf32(tmem, da, db, idesc, started);
-  mma_tf32(tmem, da, db + (uint64_t)(T::B_TILE >> 4), idesc, true);
-  mma_tf32(tmem, da + (uint64_t)(TILE_BYTES >> 4), db, idesc, true);
+  mma_tf32(tmem, da, db + (uint64_t)BN, idesc, true);
+  mma_tf32(tmem, da + (uint64_t)(SL_SLICE_STEP >> 4), db, idesc, true);
   started = true;
 }
 
@@ -402,8 +550,9 @@ __device__ __forceinline__ bool decode_tile(const OzGemm& g, long long t, int& b
 }
 
 // One output tile, all roles.
-template <int S, int BN, int KIND>
+template <int CODE, int BN>
 __device__ __forceinline__ void cta_tile(const KArgs& a, int bz, int m0, int n0, unsigned char* smem_raw) {
+  constexpr int S = form_of(CODE).S, KIND = form_of(CODE).kind, W = form_of(CODE).W;
   using T = TileCfg<BN, KIND>;
   const OzGemm& g = a.g;
   constexpr int gE = (S + 1) < 4 ? (S + 1) : 4;
@@ -464,7 +613,8 @@ __device__ __forceinline__ void cta_tile(const KArgs& a, int bz, int m0, int n0,
   const uint32_t tmem = *tmem_slot;
 
   const int nkb = (g.K + T::KPER - 1) / T::KPER;
-  const int nchunks = (nkb + CH - 1) / CH;
+  const int ch = KIND ? CH_TF32 : chunk_blocks<W>(a.A, a.B, bz, m0, n0, nkb);  // stages per chunk
+  const int nchunks = (nkb + ch - 1) / ch;
   // A ragged last column tile runs its MMAs only as wide as it needs (N a
   // multiple of 16 for M = 128); the idle epilogue warps skip their columns.
   const int n_valid = min(BN, g.N - n0);
@@ -500,12 +650,12 @@ __device__ __forceinline__ void cta_tile(const KArgs& a, int bz, int m0, int n0,
         if (BN == SL_ROWS) {
           bulk_load(sa + a_bytes, gblk, b_bytes, full_bar(st));
         } else {
-          // BN rows of each k group of each slice tile: two runs of BN * 16 bytes
+          // BN rows of each slice of each k group: two runs of BN * 16 bytes per slice
 #pragma unroll
-          for (int s = 0; s < S; ++s)
+          for (int kg = 0; kg < 2; ++kg)
 #pragma unroll
-            for (int kg = 0; kg < 2; ++kg)
-              bulk_load(sa + a_bytes + s * T::B_TILE + kg * (BN * 16), gblk + s * TILE_BYTES + kg * 2048, BN * 16,
+            for (int s = 0; s < S; ++s)
+              bulk_load(sa + a_bytes + (kg * S + s) * (BN * 16), gblk + (kg * S + s) * SL_SLICE_STEP, BN * 16,
                         full_bar(st));
         }
         ++issued;
@@ -515,20 +665,25 @@ __device__ __forceinline__ void cta_tile(const KArgs& a, int bz, int m0, int n0,
     // ---------------- MMA issuer ----------------
     if (lane == 0) {
       bool f_started = false;
-      for (int kb = 0; kb < nkb; ++kb) {
+      int c = 0, kc = 0;  // chunk, stage in the chunk
+      for (int kb = 0; kb < nkb; ++kb, ++kc) {
         const int st = kb % STAGES;
+        if (kc == ch) {
+          kc = 0;
+          ++c;
+        }
         if (!mbar_wait(full_bar(st), (kb / STAGES) & 1, abort_flag, a.wait_ns)) {
           signal_abort(abort_flag);
           break;
         }
         tc_fence_after();
         const uint32_t sa = sbase + st * stage_bytes;
-        const uint64_t da = desc_tile(sa, BM), db = desc_tile(sa + a_bytes, BN);
+        const uint64_t da = desc_tile(sa, S * BM), db = desc_tile(sa + a_bytes, S * BN);
         if constexpr (KIND == 1) {
           // chunk c accumulates in buffer c & 1, drained by the epilogue while
           // chunk c + 1 runs; before reusing a buffer wait for its last drain
-          const int c = kb / CH, bsel = c & 1;
-          if ((kb % CH) == 0) {
+          const int bsel = c & 1;
+          if (kc == 0) {
             if (c >= 2) {
               if (!mbar_wait(bsel ? accempty1_bar : accempty_bar, ((c >> 1) - 1) & 1, abort_flag, a.wait_ns)) {
                 signal_abort(abort_flag);
@@ -539,16 +694,15 @@ __device__ __forceinline__ void cta_tile(const KArgs& a, int bz, int m0, int n0,
             f_started = false;
           }
           issue_tf32<BN>(tmem + (uint32_t)(bsel * BN), da, db, idesc, f_started);
-          if ((kb % CH) == CH - 1 || kb == nkb - 1) mma_commit(bsel ? accfull1_bar : accfull_bar);
+          if (kc == ch - 1 || kb == nkb - 1) mma_commit(bsel ? accfull1_bar : accfull_bar);
           mma_commit(empty_bar(st));
           continue;
         }
-        const int c = kb / CH;
-        const bool first = (kb % CH) == 0;
-        if (!first) {
-          issue_products<S, BN, 0>(tmem, da, db, idesc, false, false);
+        const bool wide = wide_tile<BN>(n_mma);
+        if (kc != 0) {
+          issue_stage<S, BN, 0>(wide, tmem, da, db, idesc, false, false);
         } else if (c == 0) {
-          issue_products<S, BN, 0>(tmem, da, db, idesc, true, true);
+          issue_stage<S, BN, 0>(wide, tmem, da, db, idesc, true, true);
         } else if (g.fdrain) {
           // the FP32 accumulator is drained with the exact groups: it restarts
           // every chunk, after the drain
@@ -557,18 +711,18 @@ __device__ __forceinline__ void cta_tile(const KArgs& a, int bz, int m0, int n0,
             break;
           }
           tc_fence_after();
-          issue_products<S, BN, 0>(tmem, da, db, idesc, true, true);
+          issue_stage<S, BN, 0>(wide, tmem, da, db, idesc, true, true);
         } else {
           // the FP32 group runs ahead while the exact groups drain
-          issue_products<S, BN, 1>(tmem, da, db, idesc, false, false);
+          issue_stage<S, BN, 1>(wide, tmem, da, db, idesc, false, false);
           if (!mbar_wait(accempty_bar, (c - 1) & 1, abort_flag, a.wait_ns)) {
             signal_abort(abort_flag);
             break;
           }
           tc_fence_after();
-          issue_products<S, BN, 2>(tmem, da, db, idesc, true, false);
+          issue_stage<S, BN, 2>(wide, tmem, da, db, idesc, true, false);
         }
-        if ((kb % CH) == CH - 1 || kb == nkb - 1) mma_commit(accfull_bar);
+        if (kc == ch - 1 || kb == nkb - 1) mma_commit(accfull_bar);
         mma_commit(empty_bar(st));
       }
       mma_commit(done_bar);
@@ -614,14 +768,14 @@ __device__ __forceinline__ void cta_tile(const KArgs& a, int bz, int m0, int n0,
         }
         e_coff[c] = in ? g.c_c.at(cj) : 0;
         e_mc[c] = mc;
-        e_scol[c] = in ? a.B.exps[bbz * g.N + jj] - (KIND ? 31 : 7 * gE + a.frac) : 0;
+        e_scol[c] = in ? a.B.exps[bbz * g.N + jj] - (KIND ? 31 : group_exp(W, gE) + a.frac) : 0;
       }
     }
     long long R[CW];
 #pragma unroll
     for (int j = 0; j < CW; ++j) R[j] = 0;
     const float two_frac = __int_as_float((127 + a.frac) << 23);  // 2^frac
-    const float upE = __int_as_float((127 + 7 * gE) << 23);       // 2^(7 gE)
+    const float upE = __int_as_float((127 + (KIND ? 0 : group_exp(W, gE))) << 23);  // units of group gE per 1.0
     bool ok = true;
     for (int c = 0; c < nchunks; ++c) {
       if constexpr (KIND == 1) {
@@ -657,8 +811,12 @@ __device__ __forceinline__ void cta_tile(const KArgs& a, int bz, int m0, int n0,
         break;
       }
       tc_fence_after();
-      const int fr = g.fdrain ? a.frac : 0;  // fraction bits carried by R from the start
-      if (cols_live) drain_exact<BN, gE, CW>(lbase, R, fr);
+      if (cols_live) {
+        if (g.fdrain)
+          drain_exact<BN, W, gE, false>(lbase, R, a.frac);
+        else
+          drain_exact<BN, W, gE, true>(lbase, R, 0);
+      }
       if (has_inexact && g.fdrain && cols_live) {
 #pragma unroll
         for (int h = 0; h < CW / 8; ++h) {
@@ -688,7 +846,8 @@ __device__ __forceinline__ void cta_tile(const KArgs& a, int bz, int m0, int n0,
       const int rlim = min(BM, g.M - m0), clim = min(BN, g.N - n0);
       // one output element: convert and store (plus its mirror)
       auto put = [&](long long z, int scale, long long ro, long long co, long long mr, long long mc) {
-        const double val = scaled_to_double(z, scale, g.negate);
+        double val;
+        if (!scaled_to_double(z, scale, g.negate ? 0x80000000u : 0u, val)) val = fixed_to_double(z, scale, g.negate);
         Cb[ro + co] = val;
         if (mirror_rc) {
           Cb[mc + mr] = val;
@@ -726,8 +885,8 @@ __device__ __forceinline__ void cta_tile(const KArgs& a, int bz, int m0, int n0,
             for (int j = 0; j < 8; ++j) {
               long long z = R[h * 8 + j];
               if (!g.fdrain)
-                z = (long long)((unsigned long long)z << a.frac) +
-                    split_round(__uint_as_float(v[j]) * upE, a.frac, two_frac);
+                z = wide_pair<W, gE>(fold_pair<W, gE, has_inexact>(z, __uint_as_float(v[j]),
+                                                                   (uint32_t)nchunks * (uint32_t)MAGIC_BITS));
               sink(cg * CW + h * 8 + j, z);
             }
           }
@@ -807,10 +966,11 @@ __device__ __forceinline__ void cta_tile(const KArgs& a, int bz, int m0, int n0,
 // releases TMEM as soon as the last chunk is folded into registers, so the
 // next tile's MMAs overlap the conversion and stores.  Pipeline phases
 // (stages, chunks) count on across tiles.
-template <int S, int BN, bool GROUPED>
+template <int CODE, int BN, bool GROUPED, bool FD>
 __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __restrict__ probs,
                                                const long long* __restrict__ starts, int nprob, int ntiles,
                                                unsigned int* counter, unsigned char* smem_raw) {
+  constexpr int S = form_of(CODE).S, W = form_of(CODE).W;
   using T = TileCfg<BN, 0>;
   constexpr int gE = (S + 1) < 4 ? (S + 1) : 4;
   constexpr bool has_inexact = (S + 1) > 4;
@@ -829,12 +989,13 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * STAGES + 5);
   // tile hand-off from the producer to the MMA issuer and the epilogue: a
-  // ring of (problem, tile) indices (tile -1 ends the walk) behind full /
-  // empty barriers
+  // ring of (problem, tile, stages per chunk) (tile -1 ends the walk) behind
+  // full / empty barriers
   constexpr int RING = 4;
-  static_assert(2 * STAGES + 6 <= 16 && (24 + RING) * 8 <= 256, "barrier block of smem_bytes");
+  static_assert(2 * STAGES + 6 <= 16 && 24 * 8 + 3 * RING * 4 <= 256, "barrier block of smem_bytes");
   volatile int* ring = reinterpret_cast<volatile int*>(bars + 24);
   volatile int* ringp = ring + RING;
+  volatile int* ringc = ringp + RING;
   const uint32_t ringbar0 = smem_u32(bars + 16);
   auto ring_full = [&](int r) { return ringbar0 + 8u * r; };
   auto ring_empty = [&](int r) { return ringbar0 + 8u * (RING + r); };
@@ -843,7 +1004,7 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
   auto full_bar = [&](int st) { return bar0 + 8u * st; };
   auto empty_bar = [&](int st) { return bar0 + 8u * (STAGES + st); };
   const uint32_t accfull_bar = bar0 + 8u * (2 * STAGES), accempty_bar = bar0 + 8u * (2 * STAGES + 1),
-                 done_bar = bar0 + 8u * (2 * STAGES + 2);
+                 done_bar = bar0 + 8u * (2 * STAGES + 2), fempty_bar = bar0 + 8u * (2 * STAGES + 3);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
@@ -855,6 +1016,7 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
     mbar_init(accfull_bar, 1);
     mbar_init(accempty_bar, NUM_EPI_WARPS);
     mbar_init(done_bar, 1);
+    mbar_init(fempty_bar, NUM_EPI_WARPS);
     for (int r = 0; r < RING; ++r) {
       mbar_init(ring_full(r), 1);
       mbar_init(ring_empty(r), 1 + NUM_EPI_WARPS);
@@ -910,12 +1072,13 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
           }
           if (decode_tile<BN>(prob_ref<GROUPED>(a0, probs, p).g, t, bz, m0, n0)) break;
         }
-        ring[slot] = t;
-        ringp[slot] = p;
-        mbar_arrive(ring_full(slot));
-        if (t < 0) break;
         const KArgs& a = prob_ref<GROUPED>(a0, probs, p);
         const int nkb = (a.g.K + BK - 1) / BK;
+        ring[slot] = t;
+        ringp[slot] = p;
+        if (t >= 0) ringc[slot] = chunk_blocks<W>(a.A, a.B, bz, m0, n0, nkb);
+        mbar_arrive(ring_full(slot));
+        if (t < 0) break;
         const long long abz = a.A.batch == 1 ? 0 : bz, bbz = a.B.batch == 1 ? 0 : bz;
         const unsigned char* ga = reinterpret_cast<const unsigned char*>(a.A.planes) + abz * a.A.batch_bytes() +
                                   (long long)(m0 / BM) * a.A.kblocks() * a_bytes;
@@ -942,10 +1105,10 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
             bulk_load(sa + a_bytes, gblk, b_bytes, full_bar(st));
           } else {
 #pragma unroll
-            for (int s2 = 0; s2 < S; ++s2)
+            for (int kg = 0; kg < 2; ++kg)
 #pragma unroll
-              for (int kg = 0; kg < 2; ++kg)
-                bulk_load(sa + a_bytes + s2 * T::B_TILE + kg * (BN * 16), gblk + s2 * TILE_BYTES + kg * 2048, BN * 16,
+              for (int s2 = 0; s2 < S; ++s2)
+                bulk_load(sa + a_bytes + (kg * S + s2) * (BN * 16), gblk + (kg * S + s2) * SL_SLICE_STEP, BN * 16,
                           full_bar(st));
           }
           ++gkb;
@@ -963,7 +1126,7 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
           signal_abort(abort_flag);
           break;
         }
-        const int t = ring[slot], p = ringp[slot];
+        const int t = ring[slot], p = ringp[slot], ch = ringc[slot];  // ch: stages per chunk
         mbar_arrive(ring_empty(slot));
         if (t < 0) break;
         const OzGemm& g = prob_ref<GROUPED>(a0, probs, p).g;
@@ -973,51 +1136,58 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
         const int n_valid = min(BN, g.N - n0);
         const int n_mma = (n_valid + 15) & ~15;
         const uint32_t idesc = (T::IDESC & ~(0x3Fu << 17)) | ((uint32_t)(n_mma >> 3) << 17);
+        const bool wide = wide_tile<BN>(n_mma);
+        // wait until the epilogue has read an accumulator
+        auto drained = [&](uint32_t bar, uint32_t parity) {
+          if (!mbar_wait(bar, parity, abort_flag, a0.wait_ns)) return false;
+          tc_fence_after();
+          return true;
+        };
+        int kc = 0;  // stage of the chunk
         for (int kb = 0; kb < nkb; ++kb) {
           const int st = gkb % STAGES;
-          if (!mbar_wait(full_bar(st), (uint32_t)((gkb / STAGES) & 1), abort_flag, a0.wait_ns)) {
+          bool ok = mbar_wait(full_bar(st), (uint32_t)((gkb / STAGES) & 1), abort_flag, a0.wait_ns);
+          if (ok) {
+            tc_fence_after();
+            const uint32_t sa = sbase + st * stage_bytes;
+            const uint64_t da = desc_tile(sa, S * BM), db = desc_tile(sa + a_bytes, S * BN);
+            const uint32_t last_chunk = (uint32_t)((gch - 1) & 1), last_tile = (uint32_t)((i - 1) & 1);
+            if (kc > 0 || gch == 0) {
+              issue_stage<S, BN, 0>(wide, tmem, da, db, idesc, kb == 0, kb == 0);
+            } else if (FD || !has_inexact) {
+              // a chunk's first stage: everything is drained after every chunk
+              ok = drained(accempty_bar, last_chunk) && (FD || kb > 0 || drained(fempty_bar, last_tile));
+              if (ok) issue_stage<S, BN, 0>(wide, tmem, da, db, idesc, true, true);
+            } else if (kb == 0) {
+              // a tile's first stage: the exact groups are drained before the
+              // FP32 group is folded in
+              ok = drained(accempty_bar, last_chunk);
+              if (ok) issue_stage<S, BN, 2>(wide, tmem, da, db, idesc, true, false);
+              ok = ok && drained(fempty_bar, last_tile);
+              if (ok) issue_stage<S, BN, 1>(wide, tmem, da, db, idesc, false, true);
+            } else {
+              // a later chunk's: the FP32 group goes on while the exact groups
+              // drain (one stage of it: taking several stages of one kind first
+              // hides the drain but splits the merged MMAs, 8 reads of A slices a
+              // stage instead of 5, and shared memory bounds the MMAs: 1592 clocks
+              // a stage with four, 1541 with one)
+              issue_stage<S, BN, 1>(wide, tmem, da, db, idesc, false, false);
+              ok = drained(accempty_bar, last_chunk);
+              if (ok) issue_stage<S, BN, 2>(wide, tmem, da, db, idesc, true, false);
+            }
+          }
+          if (!ok) {
             signal_abort(abort_flag);
             aborted = true;
             break;
           }
-          tc_fence_after();
-          const uint32_t sa = sbase + st * stage_bytes;
-          const uint64_t da = desc_tile(sa, BM), db = desc_tile(sa + a_bytes, BN);
-          const int c = kb / CH;
-          const bool first = (kb % CH) == 0;
-          const bool chunk_last = (kb % CH) == CH - 1 || kb == nkb - 1;
-          // a new tile (or, with fdrain, every chunk) must wait until the
-          // epilogue has taken everything out of TMEM; inside a tile the FP32
-          // group may run ahead while the exact groups drain
-          if (first && gch > 0 && (c == 0 || g.fdrain)) {
-            if (!mbar_wait(accempty_bar, (uint32_t)((gch - 1) & 1), abort_flag, a0.wait_ns)) {
-              signal_abort(abort_flag);
-              aborted = true;
-              break;
-            }
-            tc_fence_after();
-          }
-          if (first && c > 0 && !g.fdrain) {
-            // the FP32 group runs ahead while the exact groups drain
-            issue_products<S, BN, 1>(tmem, da, db, idesc, false, false);
-            if (!mbar_wait(accempty_bar, (uint32_t)((gch - 1) & 1), abort_flag, a0.wait_ns)) {
-              signal_abort(abort_flag);
-              aborted = true;
-              break;
-            }
-            tc_fence_after();
-            issue_products<S, BN, 2>(tmem, da, db, idesc, true, false);
-          } else {
-            // the tile's first stage restarts every accumulator (with fdrain,
-            // every chunk's first stage does)
-            issue_products<S, BN, 0>(tmem, da, db, idesc, first, first && (c == 0 || g.fdrain));
-          }
           mma_commit(empty_bar(st));
-          if (chunk_last) {
+          ++gkb;
+          if (++kc == ch || kb == nkb - 1) {
             mma_commit(accfull_bar);
             ++gch;
+            kc = 0;
           }
-          ++gkb;
         }
       }
       mma_commit(done_bar);
@@ -1029,7 +1199,7 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
     const int cg = (warp - 2) >> 2;
     const int et = threadIdx.x - 64;
     const uint32_t lbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(cg * CW);
-    const float upE = __int_as_float((127 + 7 * gE) << 23);
+    const float upE = __int_as_float((127 + group_exp(W, gE)) << 23);
     const int row = q * 32 + lane;
     int gch = 0;
     for (int i = 0;; ++i) {
@@ -1037,7 +1207,7 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
       const bool got = mbar_wait(ring_full(slot), (uint32_t)((i / RING) & 1), abort_flag, a0.wait_ns);
       if (!got) signal_abort(abort_flag);
       const int t = got ? ring[slot] : -1;
-      const int p = got ? ringp[slot] : 0;
+      const int p = got ? ringp[slot] : 0, ch = got ? (int)ringc[slot] : (int)CH_MIN;
       __syncwarp();
       if (lane == 0) mbar_arrive(ring_empty(slot));
       // every epilogue warp is done with the previous tile's tables, and all
@@ -1046,10 +1216,11 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
       if (t < 0) break;
       const KArgs& a = prob_ref<GROUPED>(a0, probs, p);
       const OzGemm& g = a.g;
-      const int nchunks = ((g.K + BK - 1) / BK + CH - 1) / CH;
       const float two_frac = __int_as_float((127 + a.frac) << 23);  // 2^frac
       int bz, m0, n0;
       decode_tile<BN>(g, t, bz, m0, n0);
+      const int nkb = (g.K + BK - 1) / BK;
+      const int nchunks = (nkb + ch - 1) / ch;
       {
         const long long abz = a.A.batch == 1 ? 0 : bz, bbz = a.B.batch == 1 ? 0 : bz;
         if (et < BM) {
@@ -1072,16 +1243,9 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
           const bool in = jj < g.N;
           long long mc = -1;
           if (in && g.sym == SYM_ROWCOL) mc = g.c_r.at(jj);
-          long long cj = jj;
-          if (in && g.sym == SYM_TRICOL) {
-            int mm, nn;
-            tri_pair(jj, g.pair_n, mm, nn);
-            cj = (long long)mm * g.pair_n + nn;
-            if (nn > mm) mc = g.c_c.at((long long)nn * g.pair_n + mm);
-          }
-          e_coff[c] = in ? g.c_c.at(cj) : 0;
+          e_coff[c] = in ? g.c_c.at(jj) : 0;
           e_mc[c] = mc;
-          e_scol[c] = in ? a.B.exps[bbz * g.N + jj] - 7 * gE - a.frac : 0;
+          e_scol[c] = in ? a.B.exps[bbz * g.N + jj] - group_exp(W, gE) - a.frac : 0;
         }
       }
       epi_barrier_any(false);  // tables visible
@@ -1099,53 +1263,107 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
           break;
         }
         tc_fence_after();
-        const int fr = g.fdrain ? a.frac : 0;
-        if (cols_live) drain_exact<BN, gE, CW>(lbase, R, fr);
-        const bool last = c == nchunks - 1;
-        if (has_inexact && cols_live && (g.fdrain || last)) {
-          // the FP32 group: drained every chunk (fdrain) or folded in at the end
+        if (FD && cols_live) {
+          // the FP32 group is drained every chunk too
+          drain_exact<BN, W, gE, false>(lbase, R, a.frac);
+          if (has_inexact) {
 #pragma unroll
-          for (int h = 0; h < CW / 8; ++h) {
-            uint32_t v[8];
-            tmem_ld8_async(lbase + (uint32_t)(3 * BN + h * 8), v);
-            tmem_wait_ld();
+            for (int h = 0; h < CW / 8; ++h) {
+              uint32_t v[8];
+              tmem_ld8_async(lbase + (uint32_t)(3 * BN + h * 8), v);
+              tmem_wait_ld();
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const long long f = split_round(__uint_as_float(v[j]) * upE, a.frac, two_frac);
-              R[h * 8 + j] = g.fdrain ? R[h * 8 + j] + f : (long long)((unsigned long long)R[h * 8 + j] << a.frac) + f;
+              for (int j = 0; j < 8; ++j)
+                R[h * 8 + j] += split_round(__uint_as_float(v[j]) * upE, a.frac, two_frac);
             }
           }
-        } else if (last && !g.fdrain) {
-#pragma unroll
-          for (int j = 0; j < CW; ++j) R[j] = (long long)((unsigned long long)R[j] << a.frac);
+        } else if (cols_live) {
+          drain_exact<BN, W, gE, true>(lbase, R, 0);
         }
+        ++gch;
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(accempty_bar);  // TMEM free for the next chunk / tile
-        ++gch;
+        if (lane == 0) mbar_arrive(accempty_bar);  // the exact groups (FD: all of TMEM) are free
       }
       if (!ok) continue;  // the next tile's barrier sees the abort flag in every warp
+      if (!FD && cols_live) {
+        // fold the FP32 group in, so that nothing is left in TMEM
+        const uint32_t bias = (uint32_t)nchunks * (uint32_t)MAGIC_BITS;
+#pragma unroll
+        for (int h = 0; h < CW / 4; ++h) {
+          uint32_t v[4] = {};
+          if (has_inexact) {
+            tmem_ld4_async(lbase + (uint32_t)(3 * BN + h * 4), v);
+            tmem_wait_ld();
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            asm volatile("" : "+l"(R[h * 4 + j]), "+r"(v[j]));  // in order: few live temporaries
+            R[h * 4 + j] = fold_pair<W, gE, has_inexact>(R[h * 4 + j], __uint_as_float(v[j]), bias);
+            asm volatile("" : "+l"(R[h * 4 + j]));
+          }
+        }
+      }
+      if (!FD) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(fempty_bar);  // the FP32 group is free
+      }
       // convert and store from registers (rows are the output's unit stride)
       double* Cb = g.C + (long long)bz * g.c_sb;
-      const bool mirror_rc = (g.sym == SYM_ROWCOL) && (m0 != n0);
-      const int rlim = min(BM, g.M - m0), clim = min(BN, g.N - n0);
-      if (row < rlim) {
-        const int srow = e_srow[row];
-        const long long ro = e_roff[row], mr = e_mr[row];
+      const int rlim = min(BM, g.M - m0), cw = min(CW, g.N - n0 - cg * CW);  // this warp's columns
+      if (row < rlim && cw > 0) {
+        const uint32_t flip = g.negate ? 0x80000000u : 0u;
+        const int c0 = cg * CW, srow = e_srow[row];
+        // a mirror image: none, of an off-diagonal tile (SYM_ROWCOL; the row's
+        // columns are consecutive there), or of a pair (SYM_TRIROW)
+        const bool mirror_rc = g.sym == SYM_ROWCOL && m0 != n0;
+        const long long ro = e_roff[row], mr = g.sym == SYM_TRIROW || mirror_rc ? e_mr[row] : -1;
+        double* mir = mirror_rc ? Cb + mr + e_mc[c0] : nullptr;
+        const int vec = !mirror_rc || cw < CW ? 1 : store_width(mir);
+        bool fine = true;
 #pragma unroll
-        for (int j = 0; j < CW; ++j) {
-          const int c = cg * CW + j;
-          if (c >= clim) continue;
-          const double val = scaled_to_double(R[j], srow + e_scol[c], g.negate);
-          const long long co = e_coff[c];
-          Cb[ro + co] = val;
+        for (int j = 0; j < CW; j += 4) {
+          double v[4];
+          const int4 sc = *reinterpret_cast<const int4*>(e_scol + c0 + j);
+          const int scs[4] = {sc.x, sc.y, sc.z, sc.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            fine &= scaled_to_double(FD ? R[j + u] : wide_pair<W, gE>(R[j + u]), srow + scs[u], flip, v[u]) ||
+                    j + u >= cw;
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (j + u < cw) {
+              const long long co = e_coff[c0 + j + u];
+              Cb[ro + co] = v[u];
+              if (mr >= 0 && !mirror_rc) Cb[mr + co] = v[u];
+            }
           if (mirror_rc) {
-            Cb[e_mc[c] + mr] = val;
-          } else if (g.sym == SYM_TRICOL) {
-            const long long mc = e_mc[c];
-            if (mc >= 0) Cb[ro + mc] = val;
-          } else if (g.sym == SYM_TRIROW) {
-            if (mr >= 0) Cb[mr + co] = val;
+            if (vec == 4) {
+              store4(mir + j, v);
+            } else if (vec == 2) {
+              *reinterpret_cast<double2*>(mir + j) = make_double2(v[0], v[1]);
+              *reinterpret_cast<double2*>(mir + j + 2) = make_double2(v[2], v[3]);
+            } else {
+#pragma unroll
+              for (int u = 0; u < 4; ++u)
+                if (j + u < cw) mir[j + u] = v[u];
+            }
+          }
+          asm volatile("" ::: "memory");  // four columns at a time: 64 of the 96 registers hold R
+        }
+        if (!fine) {  // a result outside the normal range: the general conversion for the row, from local memory
+          long long z[CW];
+#pragma unroll
+          for (int j = 0; j < CW; ++j) z[j] = R[j];
+#pragma unroll 1
+          for (int j = 0; j < cw; ++j) {
+            const double val =
+                fixed_to_double(FD ? z[j] : wide_pair<W, gE>(z[j]), srow + e_scol[c0 + j], g.negate);
+            const long long co = e_coff[c0 + j];
+            Cb[ro + co] = val;
+            if (mirror_rc) mir[j] = val;
+            else if (mr >= 0) Cb[mr + co] = val;
           }
         }
       }
@@ -1165,37 +1383,37 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
   }
 }
 
-template <int S, int BN>
+template <int CODE, int BN, bool FD>
 __global__ void __maxnreg__(MAX_REGS) ozaki_persistent_kernel(const __grid_constant__ KArgs a, int ntiles) {
   extern __shared__ unsigned char smem_raw[];
   if (*(volatile int*)&g_tc_status != 0) return;
-  cta_persistent<S, BN, false>(a, nullptr, nullptr, 1, ntiles, a.g.tile_counter, smem_raw);
+  cta_persistent<CODE, BN, false, FD>(a, nullptr, nullptr, 1, ntiles, a.g.tile_counter, smem_raw);
 }
 
 // Grouped persistent launch: problem p owns the tiles [starts[p], starts[p + 1])
 // of one tile space walked in order through `counter` (caller memory, zeroed
 // before the launch), one CTA per SM.
-template <int S, int BN>
+template <int CODE, int BN, bool FD>
 __global__ void __maxnreg__(MAX_REGS)
     ozaki_persistent_grouped_kernel(const KArgs* __restrict__ probs, const long long* __restrict__ starts, int nprob,
                                     int ntiles, unsigned int* counter) {
   extern __shared__ unsigned char smem_raw[];
   if (*(volatile int*)&g_tc_status != 0) return;
-  cta_persistent<S, BN, true>(probs[0], probs, starts, nprob, ntiles, counter, smem_raw);
+  cta_persistent<CODE, BN, true, FD>(probs[0], probs, starts, nprob, ntiles, counter, smem_raw);
 }
 
-template <int S, int BN, int KIND>
+template <int CODE, int BN>
 __global__ void __maxnreg__(MAX_REGS) ozaki_kernel(const __grid_constant__ KArgs a) {
   extern __shared__ unsigned char smem_raw[];
   // a CTA of this or an earlier launch gave up: do not start (the host sees the status word)
   if (*(volatile int*)&g_tc_status != 0) return;
   int bz, m0, n0;
   if (!decode_tile<BN>(a.g, (long long)blockIdx.x + (long long)blockIdx.y * gridDim.x, bz, m0, n0)) return;
-  cta_tile<S, BN, KIND>(a, bz, m0, n0, smem_raw);
+  cta_tile<CODE, BN>(a, bz, m0, n0, smem_raw);
 }
 
 // Grouped launch: problem p owns the tiles [starts[p], starts[p + 1]).
-template <int S, int BN, int KIND>
+template <int CODE, int BN>
 __global__ void __maxnreg__(MAX_REGS)
     ozaki_grouped_kernel(const KArgs* __restrict__ probs, const long long* __restrict__ starts, int nprob) {
   extern __shared__ unsigned char smem_raw[];
@@ -1210,7 +1428,7 @@ __global__ void __maxnreg__(MAX_REGS)
   const KArgs& a = probs[lo];
   int bz, m0, n0;
   if (!decode_tile<BN>(a.g, t - starts[lo], bz, m0, n0)) return;
-  cta_tile<S, BN, KIND>(a, bz, m0, n0, smem_raw);
+  cta_tile<CODE, BN>(a, bz, m0, n0, smem_raw);
 }
 
 // ---------------------------------------------------------------------------
@@ -1230,51 +1448,58 @@ using GroupedFn = void (*)(const KArgs*, const long long*, int);
 template <int BN>
 KernelFn single_for(int S) {
   switch (S) {
-    case 1: return ozaki_kernel<1, BN, 0>;
-    case 2: return ozaki_kernel<2, BN, 0>;
-    case 3: return ozaki_kernel<3, BN, 0>;
-    case 4: return ozaki_kernel<4, BN, 0>;
-    case 5: return ozaki_kernel<5, BN, 0>;
-    case SPLIT_TF32X3: return ozaki_kernel<2, BN, 1>;
-    default: return ozaki_kernel<6, BN, 0>;
+    case 1: return ozaki_kernel<1, BN>;
+    case 2: return ozaki_kernel<2, BN>;
+    case 3: return ozaki_kernel<3, BN>;
+    case 4: return ozaki_kernel<4, BN>;
+    case 5: return ozaki_kernel<5, BN>;
+    case SPLIT_TF32X3: return ozaki_kernel<SPLIT_TF32X3, BN>;
+    default: return ozaki_kernel<6, BN>;
   }
 }
 
 template <int BN>
 GroupedFn grouped_for(int S) {
   switch (S) {
-    case 1: return ozaki_grouped_kernel<1, BN, 0>;
-    case 2: return ozaki_grouped_kernel<2, BN, 0>;
-    case 3: return ozaki_grouped_kernel<3, BN, 0>;
-    case 4: return ozaki_grouped_kernel<4, BN, 0>;
-    case 5: return ozaki_grouped_kernel<5, BN, 0>;
-    case SPLIT_TF32X3: return ozaki_grouped_kernel<2, BN, 1>;
-    default: return ozaki_grouped_kernel<6, BN, 0>;
+    case 1: return ozaki_grouped_kernel<1, BN>;
+    case 2: return ozaki_grouped_kernel<2, BN>;
+    case 3: return ozaki_grouped_kernel<3, BN>;
+    case 4: return ozaki_grouped_kernel<4, BN>;
+    case 5: return ozaki_grouped_kernel<5, BN>;
+    case SPLIT_TF32X3: return ozaki_grouped_kernel<SPLIT_TF32X3, BN>;
+    default: return ozaki_grouped_kernel<6, BN>;
   }
 }
 
+// fd: the FP32 group is drained per chunk (K > FDRAIN_K)
 using PersistFn = void (*)(KArgs, int);
-PersistFn persistent_for(int S) {
+template <bool FD>
+PersistFn persistent_of(int S) {
   switch (S) {
-    case 1: return ozaki_persistent_kernel<1, 128>;
-    case 2: return ozaki_persistent_kernel<2, 128>;
-    case 3: return ozaki_persistent_kernel<3, 128>;
-    case 4: return ozaki_persistent_kernel<4, 128>;
-    case 5: return ozaki_persistent_kernel<5, 128>;
-    default: return ozaki_persistent_kernel<6, 128>;
+    case 1: return ozaki_persistent_kernel<1, 128, FD>;
+    case 2: return ozaki_persistent_kernel<2, 128, FD>;
+    case 3: return ozaki_persistent_kernel<3, 128, FD>;
+    case 4: return ozaki_persistent_kernel<4, 128, FD>;
+    case 5: return ozaki_persistent_kernel<5, 128, FD>;
+    default: return ozaki_persistent_kernel<6, 128, FD>;
   }
 }
+PersistFn persistent_for(int S, bool fd) { return fd ? persistent_of<true>(S) : persistent_of<false>(S); }
 
 using PersistGroupedFn = void (*)(const KArgs*, const long long*, int, int, unsigned int*);
-PersistGroupedFn persistent_grouped_for(int S) {
+template <bool FD>
+PersistGroupedFn persistent_grouped_of(int S) {
   switch (S) {
-    case 1: return ozaki_persistent_grouped_kernel<1, 128>;
-    case 2: return ozaki_persistent_grouped_kernel<2, 128>;
-    case 3: return ozaki_persistent_grouped_kernel<3, 128>;
-    case 4: return ozaki_persistent_grouped_kernel<4, 128>;
-    case 5: return ozaki_persistent_grouped_kernel<5, 128>;
-    default: return ozaki_persistent_grouped_kernel<6, 128>;
+    case 1: return ozaki_persistent_grouped_kernel<1, 128, FD>;
+    case 2: return ozaki_persistent_grouped_kernel<2, 128, FD>;
+    case 3: return ozaki_persistent_grouped_kernel<3, 128, FD>;
+    case 4: return ozaki_persistent_grouped_kernel<4, 128, FD>;
+    case 5: return ozaki_persistent_grouped_kernel<5, 128, FD>;
+    default: return ozaki_persistent_grouped_kernel<6, 128, FD>;
   }
+}
+PersistGroupedFn persistent_grouped_for(int S, bool fd) {
+  return fd ? persistent_grouped_of<true>(S) : persistent_grouped_of<false>(S);
 }
 
 KernelFn kernel_for(int S, int BN) {
@@ -1305,29 +1530,31 @@ int configure_device() {
           cudaFuncSetAttribute(grouped_kernel_for(sl, bn), cudaFuncAttributeMaxDynamicSharedMemorySize, sm),
           "cudaFuncSetAttribute"));
     }
-  for (int sl = 1; sl <= 6; ++sl) {
-    GB_TRY(cuda_status(cudaFuncSetAttribute(persistent_for(sl), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem_bytes(sl, 128)),
-                       "cudaFuncSetAttribute"));
-    GB_TRY(cuda_status(cudaFuncSetAttribute(persistent_grouped_for(sl), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)smem_bytes(sl, 128)),
-                       "cudaFuncSetAttribute"));
-  }
+  for (int sl = 1; sl <= 6; ++sl)
+    for (bool fd : {false, true}) {
+      const int sm = (int)smem_bytes(sl, 128);
+      GB_TRY(cuda_status(cudaFuncSetAttribute(persistent_for(sl, fd), cudaFuncAttributeMaxDynamicSharedMemorySize, sm),
+                         "cudaFuncSetAttribute"));
+      GB_TRY(cuda_status(
+          cudaFuncSetAttribute(persistent_grouped_for(sl, fd), cudaFuncAttributeMaxDynamicSharedMemorySize, sm),
+          "cudaFuncSetAttribute"));
+    }
   GB_TRY(cuda_status(cudaDeviceGetAttribute(&g_num_sms[dev], cudaDevAttrMultiProcessorCount, dev),
                      "cudaDeviceGetAttribute"));
   configured[dev] = current_context_id();
   return GB_OK;
 }
 
-// Fraction bits of the fixed-point assembly: keep |z| < 2^62.
-int frac_bits(int S, int K) {
-  if (S == SPLIT_TF32X3) return 0;
-  const int nkb = (K + BK - 1) / BK;
-  const int nchunks = (nkb + CH - 1) / CH;
-  const int gE = S + 1 < 4 ? S + 1 : 4;
+// Fraction bits of the fixed-point assembly: keep |z| < 2^62 (|z| 2^-frac is
+// below 1.01 K units of 1.0, each 2^group_exp units of the last exact group).
+int frac_bits(int code, int K) {
+  if (code == SPLIT_TF32X3) return 0;
+  if (K <= FDRAIN_K) return PAIR_FRAC;
+  const SliceForm f = form_of(code);
+  const int gE = f.S + 1 < 4 ? f.S + 1 : 4;
   int lg = 0;
-  while ((1 << lg) < nchunks) ++lg;
-  const int rbits = lg + 22 + 7 * (gE - 2) + 2;
+  while (lg < 31 && (1ll << lg) < K) ++lg;
+  const int rbits = lg + 1 + group_exp(f.W, gE);
   int frac = 62 - rbits;
   if (frac > 16) frac = 16;
   if (frac < 0) frac = 0;
@@ -1336,7 +1563,8 @@ int frac_bits(int S, int K) {
 
 int check_problem(const SlicedDesc& A, const SlicedDesc& B, const OzGemm& g) {
   const SliceForm f = form_of(g.S);
-  GB_REQUIRE(valid_split(g.S) && A.S == f.S && B.S == f.S && A.kind == f.kind && B.kind == f.kind,
+  GB_REQUIRE(valid_split(g.S) && A.S == f.S && B.S == f.S && A.kind == f.kind && B.kind == f.kind && A.W == f.W &&
+                 B.W == f.W,
              GB_ERR_INVALID_ARG, "ozaki_gemm: split form mismatch (code %d)", g.S);
   GB_REQUIRE(g.bn == 32 || g.bn == 64 || g.bn == 128, GB_ERR_INVALID_ARG, "ozaki_gemm: N tile %d not in {32,64,128}",
              g.bn);
@@ -1363,7 +1591,7 @@ std::atomic<int> g_withhold_stage{-1};
 
 KArgs make_args(const SlicedDesc& A, const SlicedDesc& B, const OzGemm& g) {
   KArgs ka{g, A, B, frac_bits(g.S, g.K), g_wait_limit_ns.load(), g_withhold_stage.load()};
-  if (g.K > 4096 && g.S != SPLIT_TF32X3) ka.g.fdrain = 1;
+  if (g.K > FDRAIN_K && g.S != SPLIT_TF32X3) ka.g.fdrain = 1;
   return ka;
 }
 
@@ -1407,7 +1635,7 @@ int ozaki_gemm(const SlicedDesc& A, const SlicedDesc& B, const OzGemm& g, cudaSt
       kp.g.tile_counter = nullptr;  // one tile per CTA, or the static walk
     }
     const int pi = prof_begin(g.tag, stream);
-    persistent_for(g.S)<<<(unsigned)grid, THREADS, smem_bytes(g.S, 128), stream>>>(kp, (int)tiles);
+    persistent_for(g.S, ka.g.fdrain)<<<(unsigned)grid, THREADS, smem_bytes(g.S, 128), stream>>>(kp, (int)tiles);
     prof_end(pi, stream);
   } else {
     const int pi = prof_begin(g.tag, stream);
@@ -1424,20 +1652,25 @@ size_t ozaki_group_table_bytes(int nprob) {
   return align256((size_t)nprob * sizeof(KArgs)) + align256((size_t)(nprob + 1) * sizeof(long long)) + 256;
 }
 
-int ozaki_group_upload(const OzProblem* probs, int nprob, void* table, bool* persistent) {
+int ozaki_group_upload(const OzProblem* probs, int nprob, void* table, bool* persistent, bool* group_fdrain) {
   GB_REQUIRE(nprob >= 1 && probs && table, GB_ERR_INVALID_ARG, "ozaki_group_upload: empty group");
   std::vector<KArgs> args;
   std::vector<long long> starts(1, 0);
   bool all_rows_fast = true;
+  int fdrain = 0;
   for (int i = 0; i < nprob; ++i) {
     GB_TRY(check_problem(probs[i].A, probs[i].B, probs[i].g));
     GB_REQUIRE(probs[i].g.S == probs[0].g.S && probs[i].g.bn == probs[0].g.bn, GB_ERR_INVALID_ARG,
                "ozaki_group_upload: a group shares one slice count and tile width");
     args.push_back(make_args(probs[i].A, probs[i].B, probs[i].g));
+    fdrain |= args.back().g.fdrain;
     starts.push_back(starts.back() + ozaki_tiles(probs[i].g));
     const OzGemm& g = probs[i].g;
     all_rows_fast = all_rows_fast && !(g.c_c.div == 0 && g.c_c.s0 == 1) && (g.c_r.div == 0 && g.c_r.s0 == 1);
   }
+  // one drain form for the group (the fraction bits suit both)
+  for (KArgs& ka : args) ka.g.fdrain = fdrain;
+  if (group_fdrain) *group_fdrain = fdrain != 0;
   // the persistent form stores from the epilogue's registers: every output's
   // tile rows must be its unit stride; bf16 digits and 128-wide tiles
   if (persistent)
@@ -1452,7 +1685,7 @@ int ozaki_group_upload(const OzProblem* probs, int nprob, void* table, bool* per
 }
 
 int ozaki_gemm_grouped(const void* table, int nprob, long long total_tiles, int S, int bn, cudaStream_t stream,
-                       const char* tag, bool persistent) {
+                       const char* tag, bool persistent, bool fdrain) {
   if (total_tiles <= 0) return GB_OK;
   GB_TRY(configure_device());
   const char* t = static_cast<const char*>(table);
@@ -1469,7 +1702,7 @@ int ozaki_gemm_grouped(const void* table, int nprob, long long total_tiles, int 
     const long long grid = total_tiles < nsm ? total_tiles : nsm;
     GB_TRY(cuda_status(cudaMemsetAsync(counter, 0, sizeof(unsigned int), stream), "grouped tile counter"));
     const int pi = prof_begin(tag, stream);
-    persistent_grouped_for(S)<<<(unsigned)grid, THREADS, smem_bytes(S, 128), stream>>>(probs, starts, nprob,
+    persistent_grouped_for(S, fdrain)<<<(unsigned)grid, THREADS, smem_bytes(S, 128), stream>>>(probs, starts, nprob,
                                                                                       (int)total_tiles, counter);
     prof_end(pi, stream);
     const cudaError_t le = cudaGetLastError();

@@ -191,10 +191,11 @@ inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) /
 }  // namespace
 
 int launch_contract_diag(const double* C, const double* T, double* d, int N, int P, int Q, cudaStream_t s,
-                         int* texps) {
+                         int* texps, size_t texps_ints) {
   if (texps) {
-    // every entry below any exponent folded in (0x80808080 < -1021)
-    GB_TRY(cuda_status(cudaMemsetAsync(texps, 0x80, sizeof(int) * (size_t)P * N, s), "contract_diag exponents"));
+    // every entry below any exponent folded in (0x80808080 < -1021), and below
+    // any norm's bits
+    GB_TRY(cuda_status(cudaMemsetAsync(texps, 0x80, sizeof(int) * texps_ints, s), "contract_diag exponents"));
     GB_LAUNCH("contract_diag", s,
               contract_diag_exps_kernel<<<dim3(cdiv(Q, 128), P), 128, 0, s>>>(C, T, d, texps, N, P, Q,
                                                                                device_status_word()));

@@ -6,11 +6,11 @@
 
 namespace gb {
 
-// d[q][l] = sum_n C[n][q] T[q][n][l]
 // d[q][l] = sum_n C[n][q] T[q][n][l]; with texps also the row exponents of
-// T's digit slicing with rows (q, n) and K = l (texps[q N + n]).
+// T's digit slicing with rows (q, n) and K = l (texps[q N + n]); the texps_ints
+// int32 from texps on (the exponents and the norms behind them) are preset.
 int launch_contract_diag(const double* C, const double* T, double* d, int N, int P, int Q, cudaStream_t s,
-                         int* texps = nullptr);
+                         int* texps = nullptr, size_t texps_ints = 0);
 // d[p][l] = src[p * stride_pp + l]
 int launch_gather_diag(const double* src, double* d, int P, int Q, long long stride_pp, cudaStream_t s);
 // out[r] = sum_l src[r][l]^2

@@ -23,7 +23,7 @@ bool orbitals_on_n(long long P, long long rows) {
   const long long rows128 = (rows + 127) / 128 * 128;
   const long long normal = (P + 127) / 128 * 128 * rows128;
   const long long swapped = rows128 * (P / 128 * 128 + ((P % 128) + 15) / 16 * 16);
-  return swapped < normal;
+  return swapped <= normal;  // equal: the rows-fast form, which runs persistent
 }
 
 // T[q][(n,l)] = sum_m C[m][q] b[m][(n,l)] from the sliced C^T (A, rows q) and b (bT)
@@ -133,7 +133,8 @@ int jkj_mixed_t(const double* C, const Prepared& pr, const JkjMixedWs& w, int N,
   // T[q][(n,l)] = sum_m C[m][q] b[m][(n,l)]
   GB_TRY(half_transform_gemm(w.A, pr.bT, N, P, Q, w.Tf, w.ctr, s));
   // the contraction also records the row exponents of T's slicing (jkj_mixed_k)
-  GB_TRY(launch_contract_diag(C, w.Tf, w.dv, N, P, Q, s, w.T.kind == 0 ? w.T.exps : nullptr));
+  GB_TRY(launch_contract_diag(C, w.Tf, w.dv, N, P, Q, s, w.T.kind == 0 ? w.T.exps : nullptr,
+                              sliced_meta_ints(P, N)));
   return slice_operand(SliceSrc{w.dv, 0, lin(Q), lin(1), true}, w.d, s);
 }
 
@@ -147,6 +148,7 @@ int jkj_mixed_jr(const Prepared& pr, const JkjMixedWs& w, int N, int P, int Q, i
   d.planes = reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<unsigned char*>(w.d.planes) +
                                               (size_t)(q0 / SL_ROWS) * (size_t)w.d.kblocks() * w.d.block_bytes());
   d.exps = w.d.exps + q0;
+  d.norms = w.d.norms + (size_t)(q0 / SL_ROWS) * SL_NORMS;
   d.rows = q1 - q0;
   OzGemm gj{};
   gj.K = Q; gj.batch = 1; gj.S = S; gj.C = J + (size_t)q0 * N * N; gj.c_sb = 0; gj.pair_n = N; gj.tag = "ozaki_tc:J";
@@ -175,6 +177,7 @@ int jkj_mixed_k(const JkjMixedWs& w, int N, int Q, int S, int q0, int q1, double
   T.planes = reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<unsigned char*>(w.T.planes) +
                                               (size_t)q0 * (size_t)w.T.batch_bytes());
   T.exps = w.T.exps + (size_t)q0 * N;
+  T.norms = w.T.norms + (size_t)q0 * w.T.rblocks() * SL_NORMS;
   T.batch = q1 - q0;
   GB_TRY(slice_operand(SliceSrc{w.Tf + (size_t)q0 * N * Q, (long long)N * Q, lin(Q), lin(1), true}, T, s,
                        T.kind == 0));
@@ -440,36 +443,45 @@ struct Lag2MixedWs {
   SlicedDesc dS, dT, cjS, Ct, Zt;  // the small GEMMs' operands (w, J_MO, elag = -C^T Z)
   double *Tf, *bMO, *Y, *X, *d, *w, *cjm;
   double* part;  // ns partial exchange products (ns > 1)
-  double* Z;     // Z[m][b] = sum_(q,l) T[q][m][l] Y[b][q][l]
+  double* Z;     // Z^T: Z[b][m] = sum_(q,l) T[q][m][l] Y[b][q][l]
   int ns, kc;    // K splits of the exchange GEMM (whole ranges of orbitals q) and K per split
   unsigned int* ctr;  // tile counter of the persistent GEMMs
 };
 
-// K splits of the exchange GEMM (M = nbf5, N = nbf, K = nbf5 naux): with few
+// K splits of the exchange GEMM (M = nbf, N = nbf5, K = nbf5 naux): with few
 // output tiles the long K would run on a few CTAs, so it is cut into ranges
 // of >= 768 that run as a batch; the partial products are summed in a fixed
 // order (deterministic).  Each split covers whole orbitals q (nbf5 divisible
-// by the split count), so its part of T is one strided block.
+// by the split count), so its part of T is one strided block.  A range is also
+// kept within 4096 where whole orbitals allow it: the kernel then drains 32-bit
+// pairs instead of 64-bit sums and the FP32 group once instead of per chunk (at
+// nbf=600 300 ranges of 2400, against 10 of 72000; the partial products are
+// 0.43 GB more to write and read).
 int exchange_splits(int N, int P, int Q) {
   const long long tiles = (long long)((N + 127) / 128) * ((P + 127) / 128);
   const long long K = (long long)P * Q;
-  if (tiles >= 76 || K < 2 * 768) return 1;
-  long long s = (152 + tiles - 1) / tiles;
-  s = s < K / 768 ? s : K / 768;
-  s = s < 64 ? s : 64;
-  while (s > 1 && P % s != 0) --s;  // equal ranges of whole orbitals
+  long long s = 1;
+  if (tiles < 76 && K >= 2 * 768) {
+    s = (152 + tiles - 1) / tiles;
+    s = s < K / 768 ? s : K / 768;
+    s = s < 64 ? s : 64;
+    while (s > 1 && P % s != 0) --s;  // equal ranges of whole orbitals
+  }
+  while (s < P && (P / s) * (long long)Q > 4096) {
+    do ++s;
+    while (s < P && P % s != 0);
+  }
   return (int)s;
 }
 
-// out[r][c] (row stride ld) = sum_s part[s][r][c], r < rows, c < cols
-__global__ void sum_splits_kernel(const double* __restrict__ part, int ns, int rows, int cols,
-                                  double* __restrict__ out, int ld) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)rows * cols) return;
-  const long long RC = (long long)rows * cols;
+// out[i] = sum_s part[s][i], i < n
+__global__ void sum_splits_kernel(const double* __restrict__ part, int ns, long long n, double* __restrict__ out) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
   double v = 0.0;
-  for (int s = 0; s < ns; ++s) v += part[s * RC + idx];
-  out[(idx / cols) * ld + idx % cols] = v;
+#pragma unroll 4
+  for (int s = 0; s < ns; ++s) v += part[s * n + i];
+  out[i] = v;
 }
 
 template <class Cv>
@@ -577,24 +589,22 @@ int lagrange2_mixed_body(const double* C, const double* H, const void* prep, con
   OzGemm ge{};
   ge.M = N; ge.N = P; ge.K = w.kc; ge.batch = w.ns; ge.S = S;
   ge.sym = SYM_NONE; ge.tag = "ozaki_tc:ck_exchange"; ge.tile_counter = w.ctr;
+  // stored transposed, [b][m]: the tile rows are then the unit stride (the persistent kernel)
+  ge.C = w.ns > 1 ? w.part : w.Z; ge.c_sb = (long long)N * P; ge.c_r = lin(1); ge.c_c = lin(N);
+  GB_TRY(ozaki_gemm(w.Sx, w.Sy, ge, s));
   if (w.ns > 1) {
-    ge.C = w.part; ge.c_sb = (long long)N * P; ge.c_r = lin(P); ge.c_c = lin(1);
-    GB_TRY(ozaki_gemm(w.Sx, w.Sy, ge, s));
     const long long np = (long long)N * P;
     GB_LAUNCH("sum_splits", s,
-              sum_splits_kernel<<<(unsigned)((np + 255) / 256), 256, 0, s>>>(w.part, w.ns, N, P, w.Z, P));
-  } else {
-    ge.C = w.Z; ge.c_sb = 0; ge.c_r = lin(P); ge.c_c = lin(1);
-    GB_TRY(ozaki_gemm(w.Sx, w.Sy, ge, s));
+              sum_splits_kernel<<<(unsigned)((np + 127) / 128), 128, 0, s>>>(w.part, w.ns, np, w.Z));
   }
-  // elag[a][b] = -sum_m C[m][a] Z[m][b] (b < nbf5), then the n_b Hmat term
+  // elag[a][b] = -sum_m C[m][a] Z[m][b] (b < nbf5), then the n_b Hmat term; rows b are the unit stride
   GB_TRY(slice_operand(SliceSrc{C, 0, lin(1), lin(N), false}, w.Ct, s));
-  GB_TRY(slice_operand(SliceSrc{w.Z, 0, lin(1), lin(P), false}, w.Zt, s));
+  GB_TRY(slice_operand(SliceSrc{w.Z, 0, lin(N), lin(1), true}, w.Zt, s));
   OzGemm gz{};
-  gz.M = N; gz.N = P; gz.K = N; gz.batch = 1; gz.S = S; gz.negate = 1;
-  gz.C = elag; gz.c_sb = 0; gz.c_r = lin(N); gz.c_c = lin(1);
+  gz.M = P; gz.N = N; gz.K = N; gz.batch = 1; gz.S = S; gz.negate = 1;
+  gz.C = elag; gz.c_sb = 0; gz.c_r = lin(1); gz.c_c = lin(N);
   gz.sym = SYM_NONE; gz.tag = "ozaki_tc:elag"; gz.tile_counter = w.ctr;
-  GB_TRY(ozaki_gemm(w.Ct, w.Zt, gz, s));
+  GB_TRY(ozaki_gemm(w.Zt, w.Ct, gz, s));
   return launch_lagrange2_hterm(Hmat, n, elag, N, P, s);
 }
 

@@ -14,44 +14,43 @@ __device__ __forceinline__ int exponent_of(unsigned long long maxbits) {
   return (ex == 0 ? 1 : ex) - 1022;
 }
 
-// Balanced base-128 digits of round(x 2^(7S - E)), pre-weighted: digit s as
-// the FP32 bits of d 2^(-7 s) (|d| <= 128, exact in bf16, so the upper half of
-// those bits is the bf16 pattern; the lower half is zero).  The 64-bit integer
-// xi = H 2^(7 NL) + L (0 <= L < 2^(7 NL)) is taken apart in 32-bit pieces: the
-// NL lowest digits come from L (its carry, 0 or 1, goes to H), the others from
-// H.  Each digit's FP32 value comes from the 1.5 * 2^23 magic number (exact for
-// |d| < 2^22), scaled by 2^(-7 s) in the same (exact) fused multiply-add.
-template <int S>
+// Balanced W-bit digits of round(x 2^(e_S - E)), pre-weighted: digit s as the
+// FP32 bits of d 2^-e_s (exact in bf16, so the upper half of those bits is the
+// bf16 pattern; the lower half is zero).  The 64-bit integer xi = H 2^(W NL) + L
+// (0 <= L < 2^(W NL)) is taken apart in 32-bit pieces: the NL lowest digits come
+// from L (its carry, 0 or 1, goes to H), the others from H.  Each digit's FP32
+// value comes from the 1.5 * 2^23 magic number (exact for |d| < 2^22), scaled
+// by its weight in the same (exact) fused multiply-add.
+template <int S, int W>
 __device__ __forceinline__ void make_digits(double x, int E, uint32_t* out) {
   const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
   int ex = (int)((bits >> 52) & 0x7FF);
   unsigned long long m = bits & 0xFFFFFFFFFFFFFull;
   if (ex) m |= 1ull << 52; else ex = 1;
-  const int r = 1075 + E - ex - 7 * S;  // right shift of the 53-bit mantissa (>= 11 for S <= 6)
+  const int r = 1075 + E - ex - digit_exp(W, S);  // right shift of the 53-bit mantissa (>= 9 for e_S <= 44)
   long long xi;
-  if (r <= 0) xi = (long long)(m << (-r));
-  else if (r >= 64) xi = 0;
+  if (r >= 64) xi = 0;
   else xi = (long long)((m + (1ull << (r - 1))) >> r);
   if (bits >> 63) xi = -xi;
-  constexpr int NL = S - 1 < 3 ? S - 1 : 3;
-  int L = (int)(xi & ((1ll << (7 * NL)) - 1));
-  int H = (int)(xi >> (7 * NL));
+  constexpr int NL = S - 1 < 3 ? S - 1 : 3, HALF = 1 << (W - 1), MASK = (1 << W) - 1;
+  int L = (int)(xi & ((1ll << (W * NL)) - 1));
+  int H = (int)(xi >> (W * NL));
 #pragma unroll
   for (int s = S; s > S - NL; --s) {
-    const int d = ((L + 64) & 127) - 64;
-    L = (L - d) >> 7;
-    const float w = __int_as_float((127 - 7 * s) << 23);
+    const int d = ((L + HALF) & MASK) - HALF;
+    L = (L - d) >> W;
+    const float w = __int_as_float((127 - digit_exp(W, s)) << 23);
     out[s - 1] = __float_as_uint(fmaf(__int_as_float(0x4B400000 + d), w, -12582912.0f * w));
   }
   H += L;
 #pragma unroll
   for (int s = S - NL; s >= 2; --s) {
-    const int d = ((H + 64) & 127) - 64;
-    H = (H - d) >> 7;
-    const float w = __int_as_float((127 - 7 * s) << 23);
+    const int d = ((H + HALF) & MASK) - HALF;
+    H = (H - d) >> W;
+    const float w = __int_as_float((127 - digit_exp(W, s)) << 23);
     out[s - 1] = __float_as_uint(fmaf(__int_as_float(0x4B400000 + d), w, -12582912.0f * w));
   }
-  const float w1 = __int_as_float((127 - 7) << 23);
+  const float w1 = __int_as_float((127 - digit_exp(W, 1)) << 23);
   out[0] = __float_as_uint(fmaf(__int_as_float(0x4B400000 + H), w1, -12582912.0f * w1));
 }
 
@@ -62,12 +61,21 @@ __device__ __forceinline__ void note_nonfinite(unsigned long long maxbits, int* 
   if (maxbits >= 0x7FF0000000000000ull && status) atomicCAS(status, 0, GB_ERR_NONFINITE);
 }
 
+// The warp (all 32 lanes, `row` its first row) that meets the first row of a
+// 128-row block clears the block's norms for the digit kernel.
+__device__ __forceinline__ void clear_norms(int* norms, long long b, long long row, int rows, int lane) {
+  if (norms && row % SL_ROWS == 0 && lane < SL_NORMS)
+    norms[(b * ((rows + SL_ROWS - 1) / SL_ROWS) + row / SL_ROWS) * SL_NORMS + lane] = 0;
+}
+
 // One warp per row; K is the unit-stride index.
-__global__ void rowexp_kfast_kernel(SliceSrc src, int rows, int K, int* __restrict__ exps, int* status) {
+__global__ void rowexp_kfast_kernel(SliceSrc src, int rows, int K, int* __restrict__ exps, int* __restrict__ norms,
+                                    int* status) {
   const long long b = blockIdx.y;
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
+  clear_norms(norms, b, row, rows, lane);
   const double* base = src.p + b * src.sb + src.row_at(row);
   unsigned long long mx = 0;
   if (src.k.div == 0) {
@@ -102,11 +110,12 @@ __global__ void rowexp_kfast_kernel(SliceSrc src, int rows, int K, int* __restri
 // each warp reads 256 contiguous bytes per k) and its 8 warps split K; the
 // partial maxima meet in shared memory.
 __global__ void __launch_bounds__(256) rowexp_rfast_kernel(SliceSrc src, int rows, int K, int* __restrict__ exps,
-                                                           int* status) {
+                                                           int* __restrict__ norms, int* status) {
   __shared__ unsigned long long part[8][32];
   const long long b = blockIdx.y;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long long row = (long long)blockIdx.x * 32 + lane;
+  if (w == 0) clear_norms(norms, b, (long long)blockIdx.x * 32, rows, lane);
   unsigned long long mx = 0;
   if (row < rows) {
     const double* base = src.p + b * src.sb + src.row_at(row);
@@ -124,9 +133,6 @@ __global__ void __launch_bounds__(256) rowexp_rfast_kernel(SliceSrc src, int row
     note_nonfinite(mx, status);
   }
 }
-
-// k blocks per CTA of the digit slicer
-constexpr int SL_KPC = 8;
 
 // The 8 source values of thread (row r, k group at k0) of one k block.
 __device__ __forceinline__ void load_group(const SliceSrc& src, const double* base, bool rok, int k0, int K,
@@ -152,22 +158,29 @@ __device__ __forceinline__ void load_group(const SliceSrc& src, const double* ba
   }
 }
 
-// Digits of the 8 values, packed per slice as 8 bf16 (one 16-byte store each).
-template <int S>
-__device__ __forceinline__ void store_group(const double (&xs)[8], int e, unsigned char* out) {
+// Digits of the 8 values, packed per slice as 8 bf16 (one 16-byte store each);
+// nq[s] += the sum of the squares of the weighted digits of slice s < SL_NORMS
+// (nine-bit digits).
+template <int S, int W>
+__device__ __forceinline__ void store_group(const double (&xs)[8], int e, unsigned char* out, float (&nq)[SL_NORMS]) {
   uint32_t pk[S][4];
 #pragma unroll
   for (int u = 0; u < 8; u += 2) {
     uint32_t d0[S], d1[S];
-    make_digits<S>(xs[u], e, d0);
-    make_digits<S>(xs[u + 1], e, d1);
+    make_digits<S, W>(xs[u], e, d0);
+    make_digits<S, W>(xs[u + 1], e, d1);
     // the two bf16 patterns (upper halves) side by side
 #pragma unroll
     for (int s = 0; s < S; ++s) pk[s][u >> 1] = __byte_perm(d0[s], d1[s], 0x7632);
+#pragma unroll
+    for (int s = 0; s < (W == 9 ? SL_NORMS : 0); ++s) {
+      const float a = __uint_as_float(d0[s]), b = __uint_as_float(d1[s]);
+      nq[s] = fmaf(a, a, fmaf(b, b, nq[s]));
+    }
   }
 #pragma unroll
   for (int s = 0; s < S; ++s)
-    *reinterpret_cast<uint4*>(out + (long long)s * SL_TILE_BYTES) = make_uint4(pk[s][0], pk[s][1], pk[s][2], pk[s][3]);
+    *reinterpret_cast<uint4*>(out + s * SL_SLICE_STEP) = make_uint4(pk[s][0], pk[s][1], pk[s][2], pk[s][3]);
 }
 
 // One CTA of 256 threads per (row block, run of SL_KPC consecutive k blocks):
@@ -180,7 +193,7 @@ __device__ __forceinline__ void store_group(const double (&xs)[8], int e, unsign
 // CTAs per SM): occupancy keeps more loads in flight than prefetching the next
 // k block into registers did (measured: 1.62 ms against 1.87-1.93 ms for the
 // T of one nbf=600 build, 8.64 GB).
-template <int S>
+template <int S, int W>
 __global__ void __launch_bounds__(256, 4) digits_blocked_kernel(SliceSrc src, SlicedDesc dst) {
   const long long b = blockIdx.y;
   const int kbn = dst.kblocks();
@@ -194,11 +207,22 @@ __global__ void __launch_bounds__(256, 4) digits_blocked_kernel(SliceSrc src, Sl
   const double* base = src.p + b * src.sb + (rok ? src.row_at(r) : 0);
   const int e = rok ? dst.exps[b * dst.rows + r] : 0;
   unsigned char* out0 = reinterpret_cast<unsigned char*>(dst.planes) + b * dst.batch_bytes() +
-                        ((long long)rb * kbn * S) * SL_TILE_BYTES + (kg * 16 + rg) * 128 + ri * 16;
+                        ((long long)rb * kbn * S) * SL_TILE_BYTES + (kg * S * 16 + rg) * 128 + ri * 16;
   double xa[8];
+  float nq[SL_NORMS] = {};
   for (int kb = kb0; kb < kb1; ++kb) {
     load_group(src, base, rok, kb * SL_K + kg * 8, dst.K, xa);
-    store_group<S>(xa, e, out0 + (long long)kb * S * SL_TILE_BYTES);
+    store_group<S, W>(xa, e, out0 + (long long)kb * S * SL_TILE_BYTES, nq);
+  }
+  if constexpr (W == 9) {
+    // non-negative floats order as their bits
+    int* nb = dst.norms + (b * dst.rblocks() + rb) * SL_NORMS;
+#pragma unroll
+    for (int s = 0; s < SL_NORMS; ++s) {
+      const float scale = __int_as_float((127 + 2 * digit_exp(W, s + 1)) << 23);  // back to squares of the digits
+      const unsigned int mx = __reduce_max_sync(0xffffffffu, __float_as_uint(nq[s] * scale));
+      if (lane == 0) atomicMax(nb + s, (int)mx);
+    }
   }
 }
 
@@ -266,9 +290,9 @@ __global__ void __launch_bounds__(256) tf32_blocked_kernel(SliceSrc src, SlicedD
     tf32_split((rok && k < dst.K) ? base[src.k.at(k)] : 0.0, e, hi[u], lo[u]);
   }
   unsigned char* out = reinterpret_cast<unsigned char*>(dst.planes) + b * dst.batch_bytes() +
-                       ((long long)blockIdx.x * 2) * SL_TILE_BYTES + (kg * 16 + rg) * 128 + ri * 16;
+                       ((long long)blockIdx.x * 2) * SL_TILE_BYTES + (kg * 2 * 16 + rg) * 128 + ri * 16;
   *reinterpret_cast<uint4*>(out) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-  *reinterpret_cast<uint4*>(out + SL_TILE_BYTES) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  *reinterpret_cast<uint4*>(out + SL_SLICE_STEP) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
 }
 
 inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
@@ -276,24 +300,26 @@ inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) /
 }  // namespace
 
 int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bool exps_ready) {
-  GB_REQUIRE((dst.kind == 0 && dst.S >= 1 && dst.S <= 6) || (dst.kind == 1 && dst.S == 2), GB_ERR_INVALID_ARG,
+  GB_REQUIRE((dst.kind == 0 && dst.S >= 1 && dst.S <= 5) || (dst.kind == 1 && dst.S == 2), GB_ERR_INVALID_ARG,
              "slice_operand: bad split form (planes %d, kind %d)", dst.S, dst.kind);
   GB_REQUIRE(dst.batch >= 1 && dst.batch <= 65535 && dst.rows >= 0, GB_ERR_BAD_SHAPE, "slice_operand: bad batch");
   GB_REQUIRE((reinterpret_cast<uintptr_t>(dst.planes) & 15) == 0, GB_ERR_INVALID_ARG,
              "slice_operand: planes not 16-byte aligned");
   if (dst.rows == 0 || dst.K == 0) return GB_OK;
+  int* norms = dst.kind == 0 ? dst.norms : nullptr;
+  GB_REQUIRE(dst.kind != 0 || norms, GB_ERR_INVALID_ARG, "slice_operand: no norms");
   if (exps_ready) {
     GB_REQUIRE(dst.kind == 0, GB_ERR_INVALID_ARG, "slice_operand: recorded exponents are for digit slices");
   } else if (src.kfast) {
     int* st = device_status_word();
     GB_LAUNCH("slice_rowexp", s,
               rowexp_kfast_kernel<<<dim3(cdiv(dst.rows, 8), dst.batch), 256, 0, s>>>(src, dst.rows, dst.K, dst.exps,
-                                                                                    st));
+                                                                                    norms, st));
   } else {
     int* st = device_status_word();
     GB_LAUNCH("slice_rowexp", s,
               rowexp_rfast_kernel<<<dim3(cdiv(dst.rows, 32), dst.batch), 256, 0, s>>>(src, dst.rows, dst.K,
-                                                                                     dst.exps, st));
+                                                                                     dst.exps, norms, st));
   }
   const long long blocks = (long long)dst.rblocks() * dst.kblocks();
   GB_REQUIRE(blocks <= 2147483647LL, GB_ERR_BAD_SHAPE, "slice_operand: too many blocks");
@@ -302,13 +328,17 @@ int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bo
     return GB_OK;
   }
   const dim3 grid((unsigned)((long long)dst.rblocks() * ((dst.kblocks() + SL_KPC - 1) / SL_KPC)), dst.batch);
+  if (dst.W == 9) {
+    GB_REQUIRE(dst.S == 5, GB_ERR_INVALID_ARG, "slice_operand: nine-bit digits come in five planes");
+    GB_LAUNCH("slice_digits", s, digits_blocked_kernel<5, 9><<<grid, 256, 0, s>>>(src, dst));
+    return GB_OK;
+  }
   switch (dst.S) {
-    case 1: GB_LAUNCH("slice_digits", s, digits_blocked_kernel<1><<<grid, 256, 0, s>>>(src, dst)); break;
-    case 2: GB_LAUNCH("slice_digits", s, digits_blocked_kernel<2><<<grid, 256, 0, s>>>(src, dst)); break;
-    case 3: GB_LAUNCH("slice_digits", s, digits_blocked_kernel<3><<<grid, 256, 0, s>>>(src, dst)); break;
-    case 4: GB_LAUNCH("slice_digits", s, digits_blocked_kernel<4><<<grid, 256, 0, s>>>(src, dst)); break;
-    case 5: GB_LAUNCH("slice_digits", s, digits_blocked_kernel<5><<<grid, 256, 0, s>>>(src, dst)); break;
-    default: GB_LAUNCH("slice_digits", s, digits_blocked_kernel<6><<<grid, 256, 0, s>>>(src, dst)); break;
+    case 1: GB_LAUNCH("slice_digits", s, digits_blocked_kernel<1, 7><<<grid, 256, 0, s>>>(src, dst)); break;
+    case 2: GB_LAUNCH("slice_digits", s, digits_blocked_kernel<2, 7><<<grid, 256, 0, s>>>(src, dst)); break;
+    case 3: GB_LAUNCH("slice_digits", s, digits_blocked_kernel<3, 7><<<grid, 256, 0, s>>>(src, dst)); break;
+    case 4: GB_LAUNCH("slice_digits", s, digits_blocked_kernel<4, 7><<<grid, 256, 0, s>>>(src, dst)); break;
+    default: GB_LAUNCH("slice_digits", s, digits_blocked_kernel<5, 7><<<grid, 256, 0, s>>>(src, dst)); break;
   }
   return GB_OK;
 }

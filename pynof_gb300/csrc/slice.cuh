@@ -1,14 +1,18 @@
 // Digit slicing of FP64 operands for the split-product tensor-core path.
 //
 // A row x[0..K) of an FP64 operand is written as
-//     x[k] = 2^E * sum_{s=1..S} d_s[k] 2^(-7 s)   (+ rounding error < 2^(E - 7S - 1))
+//     x[k] = 2^E * sum_{s=1..S} d_s[k] 2^-e_s   (+ rounding error <= 2^(E - 1 - e_S))
 // with E the row's power-of-two exponent (|x[k]| < 2^E for the whole row) and
-// d_s balanced base-128 digits: |d_1| <= 128, |d_s| <= 64 for s >= 2.  Every
-// digit is stored pre-weighted as the bf16 value d_s 2^(-7 s), which is exact
-// (at most 8 significant bits).  Products of two slices then carry their
-// positional weight, and a sum of slice products over a K-chunk is an integer
-// multiple of 2^(-7 g) (g = s + t) that FP32 holds exactly while it stays below
-// 2^24 units -- the property the tensor-core kernel relies on.
+// d_s balanced digits of W bits: W = 9, |d_s| <= 256, e_s = 9 s - 1 for the
+// six-digit code, W = 7, |d_1| <= 128, |d_s| <= 64, e_s = 7 s for the codes
+// below it.  Nine bits is what bf16 holds of a signed integer (every integer up
+// to 256 is exact), so each digit is stored pre-weighted as the bf16 value
+// d_s 2^-e_s.  Products of two slices then carry their positional weight, and a
+// sum of slice products over a K-chunk is an integer multiple of 2^-(e_s + e_t),
+// the same for equal s + t = g, that FP32 holds exactly while it stays within
+// 2^24 units -- the property the tensor-core kernel relies on.  How long such a
+// chunk of nine-bit digits may be depends on their sizes, so the slicer also
+// records a bound of them per 128-row block (norms below).
 //
 // The digits are computed from the FP64 bit pattern with integer arithmetic
 // only (GB300's FP64 ALU rate is ~1/64 of FP32).
@@ -16,13 +20,19 @@
 // Memory layout ("blocked"): the slices are stored in exactly the order the
 // tensor-core kernel's shared memory wants them, so that one pipeline stage of
 // one operand is a single contiguous bulk copy.  Rows are cut into blocks of
-// 128 and K into blocks of 16; block (rb, kb) holds the S slice tiles of
-// 128 x 16 bf16 back to back (4 KB each).  Inside a tile the 8 x 8 "core
-// matrices" (8 rows of 16 bytes) are ordered k group major, row group minor,
-// so the 16 core matrices of one k group are 2 KB of consecutive bytes:
-//   byte(r, k) = ((k / 8) * 16 + r / 8) * 128 + (r % 8) * 16 + (k % 8) * 2.
+// 128 and K into blocks of 16; block (rb, kb) holds the S slices of 128 x 16
+// bf16 (4 KB each) as 8 x 8 "core matrices" (8 rows of 16 bytes), k group
+// major, then slice, then row group:
+//   byte(s, r, k) = (((k / 8) * S + s) * 16 + r / 8) * 128 + (r % 8) * 16 + (k % 8) * 2.
+// The rows of consecutive slices thus follow each other inside a k group, and
+// one MMA can take several slices of B as one wider operand.
 // Blocks are ordered [batch][rb][kb].  Rows and K are zero-padded to whole
 // blocks.  Exponents: exps[b][r] (int32).
+//
+// Norms: norms[b][rb][s - 1], s <= 3, is the FP32 bit pattern of an upper bound
+// of sum d_s^2 over one k group parity (8 of every 16 k) of any run of 128 k of
+// any row of the block; a run's sum of products of two digits is then at most
+// 2 sqrt(norm_a norm_b) (Cauchy-Schwarz).
 //
 // TF32x3 form (split code SPLIT_TF32X3): two planes, hi = tf32(x 2^-E) and
 // lo = tf32(x 2^-E - hi) (each rounded to nearest even, 11 significant bits,
@@ -30,7 +40,7 @@
 // lo hi with FP32 accumulation).  A block is then 128 rows x 8 k of 32-bit
 // elements, the same 4 KB tiles and core-matrix order with 4 elements per
 // 16-byte core-matrix row:
-//   byte(r, k) = ((k / 4) * 16 + r / 8) * 128 + (r % 8) * 16 + (k % 4) * 4.
+//   byte(s, r, k) = (((k / 4) * 2 + s) * 16 + r / 8) * 128 + (r % 8) * 16 + (k % 4) * 4.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -43,15 +53,23 @@ constexpr int SL_ROWS = 128;               // rows per block
 constexpr int SL_K = 16;                   // K per block
 constexpr int SL_TILE_BYTES = SL_ROWS * SL_K * 2;  // one slice of one block: 4 KB
 
-// Split codes ("nslices" in the C ABI): 1..6 bf16 digit slices, or the TF32x3 split.
+constexpr int SL_SLICE_STEP = SL_ROWS * 16;  // from one slice of a k group to the next
+constexpr int SL_KPC = 8;                  // k blocks per slicer CTA, and per run of the norms
+constexpr int SL_NORMS = 3;                // digits whose norms are recorded
+
+// Split codes ("nslices" in the C ABI): 1..5 seven-bit digit slices, 6 (42 bits,
+// 21 products of s + t <= 7 if they were seven-bit ones) is five nine-bit slices
+// (45 bits, 15 products of s + t <= 6), or the TF32x3 split.
 constexpr int SPLIT_TF32X3 = 32;
 struct SliceForm {
-  int S, kind;  // planes; 0 = bf16 digits, 1 = tf32 hi/lo
+  int S, kind, W;  // planes; 0 = bf16 digits, 1 = tf32 hi/lo; bits per digit
 };
-__host__ __device__ inline bool valid_split(int code) { return (code >= 1 && code <= 6) || code == SPLIT_TF32X3; }
-__host__ __device__ inline SliceForm form_of(int code) {
-  return code == SPLIT_TF32X3 ? SliceForm{2, 1} : SliceForm{code, 0};
+__host__ __device__ constexpr bool valid_split(int code) { return (code >= 1 && code <= 6) || code == SPLIT_TF32X3; }
+__host__ __device__ constexpr SliceForm form_of(int code) {
+  return code == SPLIT_TF32X3 ? SliceForm{2, 1, 0} : code == 6 ? SliceForm{5, 0, 9} : SliceForm{code, 0, 7};
 }
+// e_s of W-bit digits
+__host__ __device__ constexpr int digit_exp(int W, int s) { return W == 9 ? 9 * s - 1 : W * s; }
 
 struct SliceSrc {
   const double* p;
@@ -74,8 +92,10 @@ struct SlicedDesc {
   int* exps;              // [batch][rows]
   int batch, rows, K, S;
   int kind = 0;  // 0: bf16 digits, 16 k per block; 1: tf32 hi/lo, 8 k per block
+  int W = 7;     // bits per digit (kind 0)
+  int* norms = nullptr;  // [batch][row block][SL_NORMS], directly behind exps where it is carved (kind 0)
   __host__ __device__ int kper() const { return kind ? SL_K / 2 : SL_K; }
-  __host__ __device__ int code() const { return kind ? SPLIT_TF32X3 : S; }  // the split code it was cut with
+  __host__ __device__ int code() const { return kind ? SPLIT_TF32X3 : W == 9 ? 6 : S; }  // the split code it was cut with
   __host__ __device__ int rblocks() const { return (rows + SL_ROWS - 1) / SL_ROWS; }
   __host__ __device__ int kblocks() const { return (K + kper() - 1) / kper(); }
   __host__ __device__ long long block_bytes() const { return (long long)S * SL_TILE_BYTES; }
@@ -85,23 +105,28 @@ struct SlicedDesc {
 // `code` is a split code (1..6 or SPLIT_TF32X3).
 inline size_t sliced_plane_bytes(int batch, int rows, int K, int code) {
   const SliceForm f = form_of(code);
-  SlicedDesc d{nullptr, nullptr, batch, rows, K, f.S, f.kind};
+  SlicedDesc d{nullptr, nullptr, batch, rows, K, f.S, f.kind, f.W};
   return (size_t)batch * d.batch_bytes();
 }
-inline size_t sliced_exp_bytes(int batch, int rows) { return (size_t)batch * rows * sizeof(int); }
+// Exponents and, behind them, the norms (int32 each).
+inline size_t sliced_meta_ints(int batch, int rows) {
+  return (size_t)batch * rows + (size_t)batch * ((rows + SL_ROWS - 1) / SL_ROWS) * SL_NORMS;
+}
 
 // Carve a sliced operand (planes + exponents) out of a workspace or buffer.
 template <class Cv>
 SlicedDesc take_sliced(Cv& c, int batch, int rows, int K, int code) {
   auto* p = c.template take<unsigned char>(sliced_plane_bytes(batch, rows, K, code));
-  auto* e = c.template take<int>((size_t)batch * rows);
+  auto* e = c.template take<int>(sliced_meta_ints(batch, rows));
   const SliceForm f = form_of(code);
-  return SlicedDesc{reinterpret_cast<__nv_bfloat16*>(p), e, batch, rows, K, f.S, f.kind};
+  return SlicedDesc{reinterpret_cast<__nv_bfloat16*>(p), e, batch, rows, K, f.S, f.kind, f.W,
+                    e ? e + (size_t)batch * rows : nullptr};
 }
 
 // Exponents then digits; both kernels read the source once.  With
 // exps_ready the row exponents are already in dst.exps (recorded by the
-// kernel that wrote the source) and only the digits are formed.
+// kernel that read the source before) and only the digits are formed; the
+// norms then hold a value below every float's bits (memset with 0x80 bytes).
 int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bool exps_ready = false);
 
 }  // namespace gb

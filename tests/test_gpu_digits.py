@@ -1,0 +1,71 @@
+"""Nine-bit digit slices (split code 6): chunks, carries and tile edges.
+
+The leading digit groups are exact sums in FP32 chunks whose length the kernel
+takes from the digits' norms.  Operands whose digits are all as large as they
+get (equal rows, one sign) make every chunk as full as it can be: a chunk too
+long, or a carry lost between groups, would show as an error of 2^-24 and more.
+
+Tolerance, relative to the largest |C| (which is K 2^(Ea + Eb) up to a factor of
+4 for these operands): the dropped products s + t > 6 are at most
+4 * 2^16 * 2^-61 * 1.01 < 2^-42.9 per k, the slicing error 2 * 2^-45, and the FP32
+group, at most 2^-25 per k, loses at most 2^-24 of itself in each of its
+9 K / 16 additions: 2^-49.8 K.  For K <= 1300 that is below
+4 (2^-42.9 + 2^-44 + 2^-39.4) < 2^-37 = 7.3e-12.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+TOL = 2.0 ** -37
+
+
+@pytest.fixture(scope="module")
+def ops():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from pynof_gb300 import ops as o
+
+    return o
+
+
+def _operands(kind, M, N, K):
+    rng = np.random.default_rng(M + 3 * N + 7 * K)
+    if kind == "full":  # every digit 255 or 256 of one sign: x just below 1
+        x = 1.0 - 2.0 ** -40 * rng.integers(1, 3, K)
+        return np.tile(x, (M, 1)), np.tile(x, (N, 1))
+    if kind == "halves":  # balanced digits at their bound: +-256 in every place
+        x = sum(256.0 * 2.0 ** -(9 * s - 1) * (1 if s == 1 else 0.5) for s in range(1, 6)) * 0.5
+        sg = np.where(rng.random(K) < 0.5, -1.0, 1.0)
+        return np.tile(x * sg, (M, 1)), np.tile(x * sg, (N, 1))
+    a = rng.standard_normal((max(M, N), K))  # equal rows of A and B: sums of squares
+    return a[:M].copy(), a[:N].copy()
+
+
+@pytest.mark.parametrize("kind", ["full", "halves", "gauss"])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (128, 128, 47), (129, 127, 48), (130, 104, 49), (127, 105, 128),
+                                   (200, 260, 129), (64, 300, 257), (257, 48, 400), (128, 176, 1300)])
+def test_full_chunks_and_tile_edges(ops, kind, M, N, K):
+    A, B = _operands(kind, M, N, K)
+    ref = A @ B.T
+    C = ops.dgemm_mixed(ops.to_device(A), ops.to_device(B), 6).cpu().numpy()
+    ops.check_device_status()
+    err = np.max(np.abs(C - ref)) / np.max(np.abs(ref))
+    assert err < TOL, err
+
+
+@pytest.mark.parametrize("nbf,naux,nbf5", [(3, 5, 2), (24, 116, 24), (70, 129, 33), (150, 500, 70)])
+def test_build_with_equal_orbitals(ops, nbf, naux, nbf5):
+    """The JK build (persistent kernel, symmetric tiles) on a factor and
+    orbitals of one sign and nearly one size, against float64."""
+    rng = np.random.default_rng(nbf)
+    b = 1.0 - 2.0 ** -30 * rng.random((nbf, nbf, naux))
+    b = 0.5 * (b + b.transpose(1, 0, 2))
+    C = 1.0 - 2.0 ** -30 * rng.random((nbf, nbf))
+    T = np.einsum("mq,mnl->qnl", C[:, :nbf5], b)
+    d = np.einsum("nq,qnl->ql", C[:, :nbf5], T)
+    J, K = np.einsum("ql,mnl->qmn", d, b), np.einsum("qml,qnl->qmn", T, T)
+    dJ, dK = ops.jkj_ri_mixed(ops.to_device(C), ops.PreparedRI(ops.to_device(b), 6), nbf5)
+    ops.check_device_status()
+    for got, ref in ((dJ, J), (dK, K)):
+        assert np.max(np.abs(got.cpu().numpy() - ref)) / np.max(np.abs(ref)) < 3 * TOL
