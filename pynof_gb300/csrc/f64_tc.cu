@@ -1,0 +1,702 @@
+// FP64-accurate GEMM on the tensor cores: see f64_tc.cuh.
+//
+// One persistent CTA per SM, 18 warps as in ozaki_tc.cu: a producer (one bulk
+// copy of A's slices and two per slice of B's per 16-k stage, five stages), the
+// MMA issuer, and 16 epilogue warps.  CTA tile 128 x 64: five exact accumulators
+// and the FP32 one take 384 TMEM columns (a 128-wide tile's six would need 768),
+// and an epilogue thread keeps 16 elements, each as a 64-bit integer and an FP64
+// sum, in registers.
+//
+// What bounds it: per 16-k stage 28 products of 128 x 64, of which the exact ones
+// run as MMAs up to 256 columns wide (consecutive B slices into consecutive
+// accumulators); a 64-column MMA takes 53 clocks, 83 % of a 128-column one, so a
+// stage is ~1100 clocks of MMAs.
+#include "f64_tc.cuh"
+
+#include <algorithm>
+#include <mutex>
+
+#include "tc_prims.cuh"
+
+namespace gb {
+namespace {
+
+constexpr int S = 7, GE = 6, GMAX = 8;
+constexpr int BM = TC_BM, BN = 64, STAGES = 5, CW = BN / 4;
+constexpr int THREADS = 32 * (2 + NUM_EPI_WARPS), MAX_REGS = 96;
+constexpr uint32_t A_BYTES = S * SL_TILE_BYTES, B_BYTES = S * BN * SL_K * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+constexpr uint32_t TMEM_COLS = 512;
+constexpr uint32_t TABLE_BYTES = 20u * (BM + BN);
+constexpr size_t SMEM_BYTES = (size_t)STAGES * STAGE_BYTES + TABLE_BYTES + 256 + 1024;
+constexpr int SUPER = 64;   // stages (1024 k) an element's 64-bit sum covers: |sum| < 1024 * 1.01 * 2^52 < 2^63
+constexpr int CH_MIN = 3;   // stages per chunk whatever the digits are: 5 * 2^16 * 48 < 2^24 - 2^16 units of group 6
+constexpr float LIM_TOP = 4194304.0f - 65536.0f, LIM = 16777216.0f - 65536.0f;
+
+struct DArgs {
+  SlicedDesc A, B;  // A: rows of the tile (M), B: columns (N)
+  int M, N, K, batch;
+  int m_off, n_off;  // the output indices of row / column 0 (panels)
+  double* C;
+  long long c_sb;
+  Index2 c_r, c_c;
+  int sym, pair_n;  // SYM_NONE, SYM_ROWCOL, SYM_TRIROW, SYM_TRICOL
+  double alpha, beta;
+  int nsplit, kbs;  // K splits and stages per split; partial sums go to part
+  double* part;     // [split][batch][j][i]
+  const int* nonfinite;
+  int* status;  // the device's status word (timeouts)
+  unsigned int* counter;
+  unsigned long long wait_ns;
+  int ntiles;
+};
+
+__device__ __forceinline__ void give_up(volatile int* abort_flag, int* status) {
+  *abort_flag = 1;
+  if (status) atomicCAS(status, 0, GB_ERR_TIMEOUT);
+}
+
+// Tile -> (split, batch, m0, n0); false for tiles a symmetric output does not
+// need.  The dimension with fewer tiles runs fastest (CTAs that share a block of
+// the other operand run together).
+__device__ __forceinline__ bool decode(const DArgs& a, int t, int& sp, int& bz, int& m0, int& n0) {
+  const int mt = (a.M + BM - 1) / BM, nt = (a.N + BN - 1) / BN;
+  const int per = mt * nt;
+  const int z = t / per, r = t % per;
+  sp = z / a.batch;
+  bz = z % a.batch;
+  if (mt <= nt) {
+    m0 = (r % mt) * BM;
+    n0 = (r / mt) * BN;
+  } else {
+    n0 = (r % nt) * BN;
+    m0 = (r / nt) * BM;
+  }
+  return !(a.sym == SYM_ROWCOL && n0 + BN - 1 < m0);
+}
+
+// Stages per chunk: see chunk_blocks in ozaki_tc.cu; here groups 2..6.
+__device__ __forceinline__ int chunk_stages(const DArgs& a, int bz, int m0, int n0, int nkb) {
+  if (nkb <= CH_MIN) return CH_MIN;
+  float x[GE - 1], y[GE - 1];
+  block_norms(a.A, bz, m0, x);
+  block_norms(a.B, bz, n0, y);
+  const float up = 2.002f;
+  float most = LIM_TOP / fmaxf(up * x[0] * y[0], 1.0f);
+#pragma unroll
+  for (int g = 3; g <= GE; ++g) {
+    float sum = 0.0f;
+#pragma unroll
+    for (int s = 1; s < g; ++s) sum = fmaf(x[s - 1], y[g - s - 1], sum);
+    most = fminf(most, LIM / fmaxf(up * sum, 1.0f));
+  }
+  if (!(most >= 1.0f)) return CH_MIN;
+  return most < (float)(SUPER / SL_KPC) ? SL_KPC * (int)most : SUPER;
+}
+
+// value * 2^scale (scale any sum of two row exponents)
+__device__ __forceinline__ double scaled(double v, int scale) {
+  const uint32_t h = (uint32_t)__double2hiint(v);
+  const uint32_t e0 = ((h >> 20) & 0x7FFu) + (uint32_t)scale - 1u;
+  if (e0 < 2046u && h != 0) return __hiloint2double((int)(h + ((uint32_t)scale << 20)), __double2loint(v));
+  return v == 0.0 ? 0.0 : scalbn(v, scale);
+}
+
+// Where element (i, j) of a finished result goes, with its mirror image.
+__device__ __forceinline__ void put(const DArgs& a, double* C, long long off, long long moff, double v) {
+  if (a.alpha != 1.0) v *= a.alpha;
+  double* p = C + off;
+  if (a.beta != 0.0) v = fma(a.beta, *p, v);
+  *p = v;
+  if (moff >= 0) C[moff] = v;
+}
+
+// One element's exact groups in units of group 6 (2^-52): carries of 512 units
+// upwards, exact in FP32 while |u_3..6| < 2^24 - 2^16; the remainders of groups 6, 5
+// and of 4, 3 are summed (below 2^18 units) and the three integers come from the
+// magic number.
+__device__ __forceinline__ long long exact_sum(float x2, float x3, float x4, float x5, float x6) {
+  constexpr float U2 = 65536.0f, U3 = U2 * 512.0f, U4 = U3 * 512.0f, U5 = U4 * 512.0f, U6 = U5 * 512.0f;
+  const float h6 = fmaf(x6, U6 / 512.0f, MAGIC) - MAGIC;
+  float low = fmaf(h6, -1.0f / U5, x6);
+  x5 = fmaf(h6, 1.0f / U5, x5);
+  const float h5 = fmaf(x5, U5 / 512.0f, MAGIC) - MAGIC;
+  low += fmaf(h5, -1.0f / U4, x5);
+  x4 = fmaf(h5, 1.0f / U4, x4);
+  const float h4 = fmaf(x4, U4 / 512.0f, MAGIC) - MAGIC;
+  float mid = fmaf(h4, -1.0f / U3, x4);
+  x3 = fmaf(h4, 1.0f / U3, x3);
+  const float h3 = fmaf(x3, U3 / 512.0f, MAGIC) - MAGIC;
+  mid += fmaf(h3, -1.0f / U2, x3);
+  x2 = fmaf(h3, 1.0f / U2, x2);
+  return (long long)magic_int(x2, U2) * (1ll << 36) + (long long)magic_int(mid, U4) * (1ll << 18) + magic_int(low, U6);
+}
+
+__global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArgs a) {
+  extern __shared__ unsigned char smem_raw[];
+  if (*a.nonfinite != 0) return;  // gemm_f64's kernel does this one
+  unsigned char* smem =
+      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  long long* e_roff = reinterpret_cast<long long*>(smem + STAGES * STAGE_BYTES);
+  long long* e_mr = e_roff + BM;
+  long long* e_coff = e_mr + BM;
+  long long* e_mc = e_coff + BN;
+  int* e_srow = reinterpret_cast<int*>(e_mc + BN);
+  int* e_scol = e_srow + BM;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES + TABLE_BYTES);
+  // bars: full[5], empty[5], accfull, accempty, done, fempty, (slot, flag), ring full[4], ring empty[4], ring
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 14);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 15);
+  constexpr int RING = 4;
+  static_assert(2 * STAGES + 4 <= 14 && 24 * 8 + 2 * RING * 4 <= 256, "barrier block");
+  volatile int* ring = reinterpret_cast<volatile int*>(bars + 24);
+  volatile int* ringc = ring + RING;
+  const uint32_t sbase = smem_u32(smem), bar0 = smem_u32(bars);
+  auto full_bar = [&](int st) { return bar0 + 8u * st; };
+  auto empty_bar = [&](int st) { return bar0 + 8u * (STAGES + st); };
+  const uint32_t accfull_bar = bar0 + 80, accempty_bar = bar0 + 88, done_bar = bar0 + 96, fempty_bar = bar0 + 104;
+  auto ring_full = [&](int r) { return bar0 + 128u + 8u * r; };
+  auto ring_empty = [&](int r) { return bar0 + 160u + 8u * r; };
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < STAGES; ++i) {
+      mbar_init(full_bar(i), 1);
+      mbar_init(empty_bar(i), 1);
+    }
+    mbar_init(accfull_bar, 1);
+    mbar_init(accempty_bar, NUM_EPI_WARPS);
+    mbar_init(done_bar, 1);
+    mbar_init(fempty_bar, NUM_EPI_WARPS);
+    for (int r = 0; r < RING; ++r) {
+      mbar_init(ring_full(r), 1);
+      mbar_init(ring_empty(r), 1 + NUM_EPI_WARPS);
+    }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(const_cast<uint32_t*>(tmem_slot))),
+                 "r"(TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    tc_fence_before();
+  }
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const int nkb = (a.K + SL_K - 1) / SL_K;
+
+  int gkb_issued = 0;
+  if (warp == 0) {
+    // ---------------- producer ----------------
+    if (lane == 0) {
+      int& gkb = gkb_issued;
+      bool aborted = false;
+      for (int i = 0; !aborted; ++i) {
+        const int slot = i % RING;
+        if (!mbar_wait(ring_empty(slot), (uint32_t)(((i / RING) & 1) ^ 1), abort_flag, a.wait_ns)) {
+          give_up(abort_flag, a.status);
+          break;
+        }
+        int t, sp = 0, bz = 0, m0 = 0, n0 = 0;
+        for (;;) {
+          const unsigned int u = atomicAdd(a.counter, 1u);
+          t = u >= (unsigned int)a.ntiles ? -1 : (int)u;
+          if (t < 0 || decode(a, t, sp, bz, m0, n0)) break;
+        }
+        const int kb0 = sp * a.kbs, kb1 = min(kb0 + a.kbs, nkb);
+        ring[slot] = t;
+        if (t >= 0) ringc[slot] = chunk_stages(a, bz, m0, n0, kb1 - kb0);
+        mbar_arrive(ring_full(slot));
+        if (t < 0) break;
+        const long long abz = a.A.batch == 1 ? 0 : bz, bbz = a.B.batch == 1 ? 0 : bz;
+        const unsigned char* ga = reinterpret_cast<const unsigned char*>(a.A.planes) + abz * a.A.batch_bytes() +
+                                  (long long)(m0 / BM) * nkb * A_BYTES;
+        const unsigned char* gbp = reinterpret_cast<const unsigned char*>(a.B.planes) + bbz * a.B.batch_bytes() +
+                                   (long long)(n0 / SL_ROWS) * nkb * (S * SL_TILE_BYTES) + ((n0 % SL_ROWS) / 8) * 128;
+        for (int kb = kb0; kb < kb1; ++kb) {
+          const int st = gkb % STAGES;
+          if (!mbar_wait(empty_bar(st), (uint32_t)(((gkb / STAGES) & 1) ^ 1), abort_flag, a.wait_ns)) {
+            give_up(abort_flag, a.status);
+            aborted = true;
+            break;
+          }
+          mbar_expect_tx(full_bar(st), STAGE_BYTES);
+          const uint32_t sa = sbase + st * STAGE_BYTES;
+          bulk_load(sa, ga + (long long)kb * A_BYTES, A_BYTES, full_bar(st));
+          const unsigned char* gblk = gbp + (long long)kb * (S * SL_TILE_BYTES);
+#pragma unroll
+          for (int x = 0; x < 2 * S; ++x)  // 64 rows of each slice of each k group
+            bulk_load(sa + A_BYTES + x * (BN * 16), gblk + x * SL_SLICE_STEP, BN * 16, full_bar(st));
+          ++gkb;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ---------------- MMA issuer ----------------
+    if (lane == 0) {
+      int gkb = 0, gch = 0, gsc = 0;  // stages, chunks, 64-bit sums so far
+      bool aborted = false;
+      for (int i = 0; !aborted; ++i) {
+        const int slot = i % RING;
+        if (!mbar_wait(ring_full(slot), (uint32_t)((i / RING) & 1), abort_flag, a.wait_ns)) {
+          give_up(abort_flag, a.status);
+          break;
+        }
+        const int t = ring[slot], ch = ringc[slot];
+        mbar_arrive(ring_empty(slot));
+        if (t < 0) break;
+        int sp, bz, m0, n0;
+        decode(a, t, sp, bz, m0, n0);
+        const int kb0 = sp * a.kbs, kb1 = min(kb0 + a.kbs, nkb);
+        auto drained = [&](uint32_t bar, int n) {
+          if (!mbar_wait(bar, (uint32_t)((n - 1) & 1), abort_flag, a.wait_ns)) return false;
+          tc_fence_after();
+          return true;
+        };
+        int kc = 0, ks = 0;  // stage of the chunk, of the 64-bit sum
+        for (int kb = kb0; kb < kb1; ++kb) {
+          const int st = gkb % STAGES;
+          bool ok = mbar_wait(full_bar(st), (uint32_t)((gkb / STAGES) & 1), abort_flag, a.wait_ns);
+          if (ok) {
+            tc_fence_after();
+            const uint32_t sa = sbase + st * STAGE_BYTES;
+            const uint64_t da = desc_tile(sa, S * BM), db = desc_tile(sa + A_BYTES, S * BN);
+            if (kc > 0 || gch == 0) {
+              issue_products<S, GE, GMAX, BN, 0, true>(tmem, da, db, 0, kc == 0, kc == 0);
+            } else if (ks == 0) {
+              // a sum's first stage: the exact groups are drained before the FP32 group
+              ok = drained(accempty_bar, gch);
+              if (ok) issue_products<S, GE, GMAX, BN, 2, true>(tmem, da, db, 0, true, false);
+              ok = ok && drained(fempty_bar, gsc);
+              if (ok) issue_products<S, GE, GMAX, BN, 1, true>(tmem, da, db, 0, false, true);
+            } else {
+              issue_products<S, GE, GMAX, BN, 1, true>(tmem, da, db, 0, false, false);
+              ok = drained(accempty_bar, gch);
+              if (ok) issue_products<S, GE, GMAX, BN, 2, true>(tmem, da, db, 0, true, false);
+            }
+          }
+          if (!ok) {
+            give_up(abort_flag, a.status);
+            aborted = true;
+            break;
+          }
+          mma_commit(empty_bar(st));
+          ++gkb;
+          ++kc;
+          ++ks;
+          const bool sum_end = ks == SUPER || kb == kb1 - 1;
+          if (kc == ch || sum_end) {
+            mma_commit(accfull_bar);
+            ++gch;
+            kc = 0;
+          }
+          if (sum_end) {
+            ++gsc;
+            ks = 0;
+          }
+        }
+      }
+      mma_commit(done_bar);
+    }
+  } else {
+    // ---------------- epilogue ----------------
+    const int q = warp & 3, cg = (warp - 2) >> 2, et = threadIdx.x - 64;
+    const uint32_t lbase = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(cg * CW);
+    const int row = q * 32 + lane;
+    int gch = 0;
+    for (int i = 0;; ++i) {
+      const int slot = i % RING;
+      const bool got = mbar_wait(ring_full(slot), (uint32_t)((i / RING) & 1), abort_flag, a.wait_ns);
+      if (!got) give_up(abort_flag, a.status);
+      const int t = got ? ring[slot] : -1, ch = got ? (int)ringc[slot] : (int)CH_MIN;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ring_empty(slot));
+      if (epi_barrier_any(!got || *abort_flag != 0)) break;
+      if (t < 0) break;
+      int sp, bz, m0, n0;
+      decode(a, t, sp, bz, m0, n0);
+      const int kb0 = sp * a.kbs, kb1 = min(kb0 + a.kbs, nkb);
+      const bool parts = a.nsplit > 1;
+      {
+        const long long abz = a.A.batch == 1 ? 0 : bz, bbz = a.B.batch == 1 ? 0 : bz;
+        if (et < BM) {
+          const int li = m0 + et;
+          const bool in = li < a.M;
+          const long long gi = (long long)a.m_off + li;
+          long long ro = li, mr = -1;
+          if (in && !parts) {
+            ro = a.c_r.at(gi);
+            if (a.sym == SYM_ROWCOL) mr = a.c_c.at(gi);
+            if (a.sym == SYM_TRIROW) {
+              int mm, nn;
+              tri_pair(gi, a.pair_n, mm, nn);
+              ro = a.c_r.at((long long)mm * a.pair_n + nn);
+              if (nn > mm) mr = a.c_r.at((long long)nn * a.pair_n + mm);
+            }
+          }
+          e_roff[et] = ro;
+          e_mr[et] = mr;
+          e_srow[et] = in ? a.A.exps[abz * a.M + li] : 0;
+        } else if (et < BM + BN) {
+          const int c = et - BM, lj = n0 + c;
+          const bool in = lj < a.N;
+          const long long gj = (long long)a.n_off + lj;
+          long long co = (long long)lj * a.M, mc = -1;
+          if (in && !parts) {
+            co = a.c_c.at(gj);
+            if (a.sym == SYM_ROWCOL) mc = a.c_r.at(gj);
+            if (a.sym == SYM_TRICOL) {
+              int mm, nn;
+              tri_pair(gj, a.pair_n, mm, nn);
+              co = a.c_c.at((long long)mm * a.pair_n + nn);
+              if (nn > mm) mc = a.c_c.at((long long)nn * a.pair_n + mm);
+            }
+          }
+          e_coff[c] = co;
+          e_mc[c] = mc;
+          e_scol[c] = in ? a.B.exps[bbz * a.N + lj] : 0;
+        }
+      }
+      epi_barrier_any(false);  // tables visible
+      double acc[CW];
+      long long R[CW];
+      bool ok = true;
+      for (int s0 = kb0; s0 < kb1 && ok; s0 += SUPER) {
+        const int s1 = min(s0 + SUPER, kb1);
+#pragma unroll
+        for (int j = 0; j < CW; ++j) R[j] = 0;
+        for (int c0 = s0; c0 < s1; c0 += ch) {
+          const bool have = mbar_wait(accfull_bar, (uint32_t)(gch & 1), abort_flag, a.wait_ns);
+          if (!__all_sync(0xffffffffu, have)) {
+            give_up(abort_flag, a.status);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+#pragma unroll
+          for (int h = 0; h < CW / 4; ++h) {
+            uint32_t v[GE - 1][4];
+#pragma unroll
+            for (int g = 0; g < GE - 1; ++g) tmem_ld4_async(lbase + (uint32_t)(g * BN + h * 4), v[g]);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              R[h * 4 + j] += exact_sum(__uint_as_float(v[0][j]), __uint_as_float(v[1][j]), __uint_as_float(v[2][j]),
+                                        __uint_as_float(v[3][j]), __uint_as_float(v[4][j]));
+          }
+          ++gch;
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(accempty_bar);
+        }
+        if (!ok) break;
+        // the FP32 group's whole units (below 2^20; what is below half a unit, 2^-53
+        // of the row bounds, is less than FP64 arithmetic loses from ~50 k on)
+#pragma unroll
+        for (int h = 0; h < CW / 4; ++h) {
+          uint32_t f[4];
+          tmem_ld4_async(lbase + (uint32_t)((GE - 1) * BN + h * 4), f);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 4; ++j) R[h * 4 + j] += magic_int(__uint_as_float(f[j]), 0x1p52f);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(fempty_bar);
+        // into FP64: one conversion an element (the FP64 pipe takes ~2 a clock and
+        // SM), one addition more from the second 1024 k on
+        if (s0 == kb0) {
+#pragma unroll
+          for (int j = 0; j < CW; ++j) acc[j] = __ll2double_rn(R[j]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < CW; ++j) acc[j] += __ll2double_rn(R[j]);
+        }
+      }
+      if (!ok) continue;  // the next tile's barrier sees the abort flag in every warp
+      const int gi = m0 + row;
+      if (gi < a.M) {
+        double* Cb = parts ? a.part + ((long long)sp * a.batch + bz) * (long long)a.M * a.N : a.C + (long long)bz * a.c_sb;
+        const long long ro = e_roff[row], mr = e_mr[row];
+        const int srow = e_srow[row];
+#pragma unroll
+        for (int j = 0; j < CW; ++j) {
+          const int c = cg * CW + j, gj = n0 + c;
+          if (gj < a.N) {
+            const double v = scaled(acc[j], srow + e_scol[c] - 52);
+            const long long co = e_coff[c];
+            if (parts) {
+              Cb[ro + co] = v;
+            } else if (a.sym == SYM_ROWCOL) {
+              if (gj >= gi) put(a, Cb, ro + co, gj > gi ? mr + e_mc[c] : -1, v);
+            } else if (a.sym == SYM_TRIROW) {
+              put(a, Cb, ro + co, mr >= 0 ? mr + co : -1, v);
+            } else if (a.sym == SYM_TRICOL) {
+              const long long mc = e_mc[c];
+              put(a, Cb, ro + co, mc >= 0 ? ro + mc : -1, v);
+            } else {
+              put(a, Cb, ro + co, -1, v);
+            }
+          }
+          asm volatile("" ::: "memory");
+        }
+      }
+    }
+  }
+
+  __syncthreads();
+  if (warp == 0 && lane == 0 && *abort_flag) {
+    for (int k = gkb_issued > STAGES ? gkb_issued - STAGES : 0; k < gkb_issued; ++k)
+      mbar_wait(full_bar(k % STAGES), (uint32_t)((k / STAGES) & 1), nullptr, a.wait_ns);
+  }
+  if (warp == 1) {
+    if (*abort_flag) mbar_wait(done_bar, 0, nullptr, a.wait_ns);
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+  }
+}
+
+// Partial sums of the K splits, in order, into the output.
+__global__ void __launch_bounds__(256) sum_parts_kernel(const __grid_constant__ DArgs a) {
+  if (*a.nonfinite != 0) return;
+  const long long MN = (long long)a.M * a.N, all = MN * a.batch;
+  const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (idx >= all) return;
+  const int bz = (int)(idx / MN);
+  const long long r = idx % MN;
+  const int i = (int)(r % a.M), j = (int)(r / a.M);
+  if (a.sym == SYM_ROWCOL && j < i) return;
+  double v = 0.0;
+  for (int s = 0; s < a.nsplit; ++s) v += a.part[s * all + idx];
+  const long long gi = (long long)a.m_off + i, gj = (long long)a.n_off + j;
+  long long off, moff = -1;
+  int mm, nn;
+  if (a.sym == SYM_TRIROW) {
+    tri_pair(gi, a.pair_n, mm, nn);
+    off = a.c_r.at((long long)mm * a.pair_n + nn) + a.c_c.at(gj);
+    if (nn > mm) moff = a.c_r.at((long long)nn * a.pair_n + mm) + a.c_c.at(gj);
+  } else if (a.sym == SYM_TRICOL) {
+    tri_pair(gj, a.pair_n, mm, nn);
+    off = a.c_r.at(gi) + a.c_c.at((long long)mm * a.pair_n + nn);
+    if (nn > mm) moff = a.c_r.at(gi) + a.c_c.at((long long)nn * a.pair_n + mm);
+  } else {
+    off = a.c_r.at(gi) + a.c_c.at(gj);
+    if (a.sym == SYM_ROWCOL && j > i) moff = a.c_r.at(gj) + a.c_c.at(gi);
+  }
+  put(a, a.C + (long long)bz * a.c_sb, off, moff, v);
+}
+
+// ---------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------
+constexpr size_t PANEL_BYTES = (size_t)3 << 30;  // slices held at a time, where an operand is cut into panels
+
+long long up128(long long x) { return (x + 127) / 128 * 128; }
+size_t slice_bytes(long long batch, long long rows, long long K) {
+  return align256(sliced_plane_bytes((int)batch, (int)rows, (int)K, SPLIT_F64)) +
+         align256(sliced_meta_ints((int)batch, (int)rows) * sizeof(int));
+}
+
+// How a GEMM is run: X is the operand on the tile rows, Y on its columns.
+struct Plan {
+  bool use = false;
+  bool swap = false;         // X is B
+  bool tri = false;          // the pair operand (B) is packed to its upper triangle
+  long long xr = 0, yr = 0;  // rows of X and Y
+  int pb = 1;                // batch entries per panel
+  long long px = 0, py = 0;  // rows of X, Y per panel
+  int nsplit = 1, kbs = 0;   // K splits per panel, stages each
+  size_t xb = 0, yb = 0, partb = 0;
+  size_t bytes() const { return 256 + xb + yb + partb; }
+};
+
+Plan make_plan(long long M, long long N, long long K, int batch, bool a_shared, bool b_shared, int sym, int pair_n) {
+  Plan p;
+  if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return p;
+  p.tri = sym == SYM_PAIRCOL;
+  const long long n = p.tri ? (long long)pair_n * (pair_n + 1) / 2 : N;
+  // orientation: less padding of the 128 x 64 tiles
+  auto tiles = [](long long x, long long y) { return ((x + BM - 1) / BM) * ((y + BN - 1) / BN); };
+  p.swap = tiles(n, M) < tiles(M, n);
+  p.xr = p.swap ? n : M;
+  p.yr = p.swap ? M : n;
+  const bool xs = batch == 1 || (p.swap ? b_shared : a_shared), ys = batch == 1 || (p.swap ? a_shared : b_shared);
+  const long long nkb = (K + SL_K - 1) / SL_K;
+  if (p.xr > (1 << 30) || p.yr > (1 << 30) || K > (1 << 30) || K >= (1ll << 31) - 16) return p;
+  const double all_tiles = (double)tiles(p.xr, p.yr) * batch * (sym == SYM_ROWCOL ? 0.55 : 1.0);
+  // Rule: the estimated time against gemm_f64's.  Measured on GB300: a stage of a
+  // tile takes ~1300 clocks at ~2 GHz, slicing moves 30 bytes an element at ~5 TB/s,
+  // the seven launches of a GEMM ~60 us (at 300^3, 62 us of FP64 arithmetic, this took 85); the FP64 pipe gives 1.0 TFLOP/s when its
+  // 64 x 64 tiles fill the SMs (gemm_f64's other kernel less).
+  const double el = (double)M * K * (a_shared ? 1 : batch) + (double)n * K * (b_shared ? 1 : batch);
+  const double ctas = std::min(152.0, all_tiles * (double)std::max(1ll, nkb / 16));
+  const double t_tc = 60e-6 + el * 30.0 / 5e12 + all_tiles * nkb * 1300.0 / 2e9 / ctas;
+  const double t_f64 = 2.0 * M * N * K * batch * (sym == SYM_NONE ? 1.0 : 0.5) / 1.0e12;
+  p.use = t_tc < 0.7 * t_f64;
+  if (!p.use) return p;
+  // panels: over the batch, or over the rows of the operand with more of them
+  p.px = p.xr;
+  p.py = p.yr;
+  p.pb = batch;
+  auto size = [&]() {
+    p.xb = slice_bytes(xs ? 1 : p.pb, p.px, K);
+    p.yb = slice_bytes(ys ? 1 : p.pb, p.py, K);
+  };
+  size();
+  if (p.xb + p.yb > PANEL_BYTES) {
+    if (batch > 1) {
+      while (p.pb > 1 && p.xb + p.yb > PANEL_BYTES) {
+        p.pb = (p.pb + 1) / 2;
+        size();
+      }
+    } else {
+      long long& big = p.px >= p.py ? p.px : p.py;
+      while (big > 128 && p.xb + p.yb > PANEL_BYTES) {
+        big = up128((big + 1) / 2);
+        size();
+      }
+    }
+  }
+  // the symmetric tiles of a panel would need its offsets
+  if (sym == SYM_ROWCOL && (p.px < p.xr || p.py < p.yr)) {
+    p.use = false;
+    return p;
+  }
+  // K splits of at least 16 stages, whole norm runs: the split count whose tiles
+  // take the fewest stages in a row on 152 SMs (a tile more costs an SM its
+  // epilogue, ~12 stages' time)
+  const long long pt = tiles(p.px, p.py) * p.pb;
+  long long kbs = nkb;
+  double best = 1e300;
+  for (long long ns = 1; ns <= 64 && (ns == 1 || nkb / ns >= 16) && (ns == 1 || pt * ns <= 152 * 8); ++ns) {
+    long long k = (nkb + ns - 1) / ns;
+    if (ns > 1) k = (k + SL_KPC - 1) / SL_KPC * SL_KPC;
+    const double cost = (double)((pt * ((nkb + k - 1) / k) + 151) / 152) * (double)(k + 12);
+    if (cost < best) {
+      best = cost;
+      kbs = k;
+    }
+  }
+  p.kbs = (int)kbs;
+  p.nsplit = (int)((nkb + kbs - 1) / kbs);
+  p.partb = p.nsplit > 1 ? align256(sizeof(double) * (size_t)p.nsplit * p.pb * p.px * p.py) : 0;
+  return p;
+}
+
+int configure() {
+  static std::mutex mu;
+  static unsigned long long done[64] = {0};
+  int dev = 0;
+  GB_TRY(cuda_status(cudaGetDevice(&dev), "cudaGetDevice"));
+  const unsigned long long ctx = current_context_id();
+  std::lock_guard<std::mutex> lk(mu);
+  if (dev < 0 || dev >= 64 || (ctx != 0 && done[dev] == ctx)) return GB_OK;
+  GB_TRY(cuda_status(
+      cudaFuncSetAttribute(f64_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES),
+      "f64_tc: cudaFuncSetAttribute"));
+  done[dev] = current_context_id();
+  return GB_OK;
+}
+
+bool same_index(const Index2& a, const Index2& b) { return a.div == b.div && a.s1 == b.s1 && a.s0 == b.s0; }
+
+}  // namespace
+
+size_t gemm_f64_tc_bytes(long long M, long long N, long long K, int batch, bool a_shared, bool b_shared, int sym,
+                         int pair_n) {
+  const Plan p = make_plan(M, N, K, batch, a_shared, b_shared, sym, pair_n);
+  return p.use ? p.bytes() : 0;
+}
+
+int gemm_f64_tc(const GemmF64& g, const TcWork& w, cudaStream_t s) {
+  const bool a_shared = g.batch == 1 || g.A.sb == 0, b_shared = g.batch == 1 || g.B.sb == 0;
+  const Plan p = make_plan(g.M, g.N, g.K, g.batch, a_shared, b_shared, g.sym, g.pair_n);
+  // a second panel cannot follow a first that already added into the output
+  // (a NaN in its rows would have gemm_f64 add again)
+  const bool panels = p.use && (p.pb < g.batch || p.px < p.xr || p.py < p.yr);
+  if (!p.use || !w.p || w.bytes < p.bytes() || (g.beta != 0.0 && panels)) return gemm_f64(g, s);
+  GB_TRY(configure());
+  Carve cv(w.p, w.bytes);
+  int* words = cv.take<int>(2);  // [0] non-finite operand, [1] tile counter
+  auto sliced = [&](long long batch, long long rows) { return take_sliced(cv, (int)batch, (int)rows, g.K, SPLIT_F64); };
+  const bool xs = p.swap ? b_shared : a_shared, ys = p.swap ? a_shared : b_shared;
+  // the sources: A's rows are the M index, B's the N index
+  const SliceSrc sa{g.A.p, g.A.sb, g.A.r, g.A.c, g.a_kfast};
+  SliceSrc sb{g.B.p, g.B.sb, g.B.c, g.B.r, g.b_kfast};
+  if (p.tri) sb.tri_n = g.pair_n;
+  const bool one = !p.tri && g.M == g.N && g.A.p == g.B.p && g.A.sb == g.B.sb && same_index(g.A.r, g.B.c) &&
+                   same_index(g.A.c, g.B.r) && p.px == p.xr && p.py == p.yr;
+  SlicedDesc X = sliced(xs ? 1 : p.pb, p.px), Y = one ? X : sliced(ys ? 1 : p.pb, p.py);
+  double* part = p.nsplit > 1 ? cv.take<double>((size_t)p.nsplit * p.pb * p.px * p.py) : nullptr;
+  int* status = device_status_word();
+  GB_TRY(cuda_status(cudaMemsetAsync(words, 0, 2 * sizeof(int), s), "f64_tc: words"));
+  bool first = true;
+  for (int b0 = 0; b0 < g.batch; b0 += p.pb) {
+    const int nb = std::min(p.pb, g.batch - b0);
+    for (long long x0 = 0; x0 < p.xr; x0 += p.px) {
+      for (long long y0 = 0; y0 < p.yr; y0 += p.py) {
+        const int xn = (int)std::min(p.px, p.xr - x0), yn = (int)std::min(p.py, p.yr - y0);
+        auto cut = [&](SlicedDesc d, SliceSrc src, bool shared, long long r0, int rows, SlicedDesc& out, bool fresh) -> int {
+          d.rows = rows;
+          d.batch = shared ? 1 : nb;
+          d.norms = d.exps + (size_t)d.batch * rows;
+          out = d;
+          if (!fresh) return GB_OK;
+          src.row0 = r0;
+          if (!shared) src.p += (long long)b0 * src.sb;
+          return slice_operand(src, d, s, false, words);
+        };
+        // an operand that this panel shares with the one before is there already
+        SlicedDesc x, y;
+        const bool fx = first || !xs || p.px < p.xr, fy = first || !ys || p.py < p.yr;
+        GB_TRY(cut(X, p.swap ? sb : sa, xs, x0, xn, x, fx));
+        if (one)
+          y = x;
+        else
+          GB_TRY(cut(Y, p.swap ? sa : sb, ys, y0, yn, y, fy));
+        if (!first) GB_TRY(cuda_status(cudaMemsetAsync(words + 1, 0, sizeof(int), s), "f64_tc: tile counter"));
+        first = false;
+        DArgs a{};
+        a.A = x;
+        a.B = y;
+        a.M = xn;
+        a.N = yn;
+        a.K = g.K;
+        a.batch = nb;
+        a.m_off = (int)x0;
+        a.n_off = (int)y0;
+        a.C = g.C.p + (long long)b0 * g.C.sb;
+        a.c_sb = g.C.sb;
+        a.c_r = p.swap ? g.C.c : g.C.r;
+        a.c_c = p.swap ? g.C.r : g.C.c;
+        a.sym = p.tri ? (p.swap ? SYM_TRIROW : SYM_TRICOL) : g.sym;
+        a.pair_n = g.pair_n;
+        a.alpha = g.alpha;
+        a.beta = g.beta;
+        a.nsplit = p.nsplit;
+        a.kbs = p.kbs;
+        a.part = part;
+        a.nonfinite = words;
+        a.status = status;
+        a.counter = reinterpret_cast<unsigned int*>(words + 1);
+        a.wait_ns = 2000000000ull;
+        a.ntiles = (int)(((xn + BM - 1) / BM) * (long long)((yn + BN - 1) / BN) * nb * p.nsplit);
+        const unsigned grid = (unsigned)std::min(a.ntiles, 152);
+        GB_LAUNCH(g.tag, s, f64_tc_kernel<<<grid, THREADS, SMEM_BYTES, s>>>(a));
+        if (p.nsplit > 1) {
+          const long long all = (long long)xn * yn * nb;
+          GB_LAUNCH("f64_tc:sum_parts", s, sum_parts_kernel<<<(unsigned)((all + 255) / 256), 256, 0, s>>>(a));
+        }
+      }
+    }
+  }
+  // a NaN or an infinity in an operand: FP64 arithmetic, as before
+  GemmF64 f = g;
+  f.only_if = words;
+  return gemm_f64(f, s);
+}
+
+}  // namespace gb

@@ -1,6 +1,6 @@
 // Generalized Fock matrices, the Lagrangian from them and the electronic
 // energy (FP64): computeF_RC, computeF_RO, computeLagrange, computeE_elec.
-#include "gemm_f64.cuh"
+#include "f64_tc.cuh"
 #include "ri_kernels.cuh"
 
 using namespace gb;
@@ -138,7 +138,7 @@ extern "C" size_t gb_fock_rc_workspace_f64(int nbf, int nbf5) {
   Sizer z;
   z.add<double>((size_t)nbf5 * nbf5);
   z.add<double>((size_t)nbf5 * nbf5);
-  (void)nbf;
+  z.add<char>(gemm_f64_tc_bytes(nbf5, (long long)nbf * nbf, nbf5, 1, true, true));
   return z.used;
 }
 
@@ -169,12 +169,12 @@ extern "C" int gb_fock_rc_f64(const double* J, const double* K, const double* n,
   g.alpha = 1.0; g.beta = 0.0; g.sym = SYM_NONE;
   g.a_kfast = true; g.b_kfast = false;
   g.tag = "gemm_f64:fock";
-  GB_TRY(gemm_f64(g, s));
+  GB_TRY(gemm_f64_tc(g, tc_work(cv), s));
   // F -= ck12' K
   g.A = {ckm, 0, lin(P), lin(1)};
   g.B = {K, 0, lin(NN), lin(1)};
   g.alpha = -1.0; g.beta = 1.0;
-  GB_TRY(gemm_f64(g, s));
+  GB_TRY(gemm_f64_tc(g, tc_work(cv), s));
   GB_LAUNCH("fock_diag_terms", s,
             fock_diag_terms_kernel<<<dim3(cdiv(NN, 256), P), 256, 0, s>>>(F, J, H, n, N, P, ini, nbeta, nalpha));
   return GB_OK;
@@ -188,7 +188,7 @@ extern "C" size_t gb_fock_ro_workspace_f64(int nbf, int nbf5) {
   z.add<double>((size_t)nbf5 * nbf5);
   z.add<double>((size_t)nbf5 * nbf5);
   z.add<double>((size_t)nbf5);
-  (void)nbf;
+  z.add<char>(gemm_f64_tc_bytes(nbf5, (long long)nbf * nbf, nbf5, 1, true, true));
   return z.used;
 }
 
@@ -221,11 +221,11 @@ extern "C" int gb_fock_ro_f64(const double* J, const double* K, const double* n,
   g.alpha = 1.0; g.beta = 0.0; g.sym = SYM_NONE;
   g.a_kfast = true; g.b_kfast = false;
   g.tag = "gemm_f64:fock";
-  GB_TRY(gemm_f64(g, s));
+  GB_TRY(gemm_f64_tc(g, tc_work(cv), s));
   g.A = {B, 0, lin(P), lin(1)};
   g.B = {K, 0, lin(NN), lin(1)};
   g.alpha = -1.0; g.beta = 1.0;
-  GB_TRY(gemm_f64(g, s));
+  GB_TRY(gemm_f64_tc(g, tc_work(cv), s));
   GB_LAUNCH("fock_add_h", s, fock_add_h_kernel<<<dim3(cdiv(NN, 256), P), 256, 0, s>>>(F, H, a, N));
   return GB_OK;
 }

@@ -7,7 +7,7 @@
 //   K_i[(m,s)] = sum_(n,l) D_i[(n,l)] I[m][n][s][l]             (GEMM whose B operand
 //                 is read through the split maps (n,l) -> n N^2 + l, (m,s) -> m N^3 + s N)
 // Both J_i and K_i are symmetric, so only pairs n >= m are computed (mirrored).
-#include "gemm_f64.cuh"
+#include "f64_tc.cuh"
 #include "ri_kernels.cuh"
 
 using namespace gb;
@@ -69,7 +69,14 @@ int make_density(const double* C, double* D, int N, int P, cudaStream_t s) {
   return GB_OK;
 }
 
-int jk_full_core(const double* D, const double* I, int N, int P, double* J, double* K, cudaStream_t s) {
+// Tensor-core scratch of jk_full_core.
+size_t jk_full_tc_bytes(int N, int P) {
+  const long long NN = (long long)N * N;
+  return gemm_f64_tc_bytes(P, NN, NN, 1, true, true, SYM_PAIRCOL, N);
+}
+
+int jk_full_core(const double* D, const double* I, int N, int P, double* J, double* K, const TcWork& tw,
+                 cudaStream_t s) {
   const long long NN = (long long)N * N;
   GemmF64 g{};
   g.M = P; g.N = (int)NN; g.K = (int)NN; g.batch = 1;
@@ -79,11 +86,11 @@ int jk_full_core(const double* D, const double* I, int N, int P, double* J, doub
   g.alpha = 1.0; g.beta = 0.0; g.sym = SYM_PAIRCOL; g.pair_n = N;
   g.a_kfast = true; g.b_kfast = true;
   g.tag = "gemm_f64:J_full";
-  GB_TRY(gemm_f64(g, s));
+  GB_TRY(gemm_f64_tc(g, tw, s));
   g.B = {I, 0, split(N, NN, 1), split(N, NN * N, N)};  // B((n,l), (m,s)) = I[m][n][s][l]
   g.C = {K, 0, lin(NN), lin(1)};
   g.tag = "gemm_f64:K_full";
-  return gemm_f64(g, s);
+  return gemm_f64_tc(g, tw, s);
 }
 
 }  // namespace
@@ -94,6 +101,7 @@ int jk_full_core(const double* D, const double* I, int N, int P, double* J, doub
 extern "C" size_t gb_jkj_full_workspace_f64(int nbf, int nbf5) {
   Sizer z;
   z.add<double>((size_t)nbf5 * nbf * nbf);
+  z.add<char>(jk_full_tc_bytes(nbf, nbf5));
   return z.used;
 }
 
@@ -108,7 +116,7 @@ extern "C" int gb_jkj_full_f64(const double* C, const double* I, int nbf, int nb
   GB_REQUIRE(D, GB_ERR_WORKSPACE, "gb_jkj_full_f64: workspace too small");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   GB_TRY(make_density(C, D, N, P, s));
-  return jk_full_core(D, I, N, P, J, K, s);
+  return jk_full_core(D, I, N, P, J, K, tc_work(cv), s);
 }
 
 // ---------------------------------------------------------------------------
@@ -120,6 +128,7 @@ extern "C" size_t gb_jkh_mo_full_workspace_f64(int nbf, int nbf5) {
   z.add<double>((size_t)nbf5 * nbf * nbf);  // J
   z.add<double>((size_t)nbf5 * nbf * nbf);  // K
   z.add<double>((size_t)nbf * nbf5);        // H C_p
+  z.add<char>(jk_full_tc_bytes(nbf, nbf5));
   return z.used;
 }
 
@@ -139,7 +148,7 @@ extern "C" int gb_jkh_mo_full_f64(const double* C, const double* H, const double
   GB_REQUIRE(D && J && K && X, GB_ERR_WORKSPACE, "gb_jkh_mo_full_f64: workspace too small");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   GB_TRY(make_density(C, D, N, P, s));
-  GB_TRY(jk_full_core(D, I, N, P, J, K, s));
+  GB_TRY(jk_full_core(D, I, N, P, J, K, tc_work(cv), s));
   const long long NN = (long long)N * N;
   GemmF64 g{};
   g.M = P; g.N = P; g.K = (int)NN; g.batch = 1;
@@ -170,17 +179,28 @@ extern "C" int gb_jkh_mo_full_f64(const double* C, const double* H, const double
 // A6  Integrals_MO_Full: Hmat (N x P) and I_MO[p][q][r][t] (p < N; q, r, t < P)
 //     by four quarter transforms (t, then r, then q, then p).
 // ---------------------------------------------------------------------------
+// Tensor-core scratch of the quarter transforms.
+static size_t mo_full_tc_bytes(int nbf, int nbf5) {
+  const long long N = nbf, P = nbf5;
+  size_t b = gemm_f64_tc_bytes(N * N, P, N, nbf, false, true);
+  for (size_t x : {gemm_f64_tc_bytes(P, N * N * P, N, 1, true, true), gemm_f64_tc_bytes(P, N * P * P, N, 1, true, true),
+                   gemm_f64_tc_bytes(N, P * P * P, N, 1, true, true)})
+    b = x > b ? x : b;
+  return b;
+}
+
 extern "C" size_t gb_mo_full_workspace_f64(int nbf, int nbf5) {
   Sizer z;
   const size_t N = nbf, P = nbf5;
   z.add<double>(N * N * N * P);  // X1 [m][n][s][t], later X3 [m][q][r][t]
   z.add<double>(N * N * P * P);  // X2 [m][n][r][t]
   z.add<double>(N * P);          // H C_p
+  z.add<char>(mo_full_tc_bytes(nbf, nbf5));
   return z.used;
 }
 
 static int mo_full_core(const double* C, const double* H, const double* I, int N, int P, double* Hmat,
-                        double* imo, double* X1, double* X2, double* X, cudaStream_t s) {
+                        double* imo, double* X1, double* X2, double* X, const TcWork& tw, cudaStream_t s) {
   const long long NP = (long long)N * P, P2 = (long long)P * P, P3 = P2 * P, NN = (long long)N * N;
   GemmF64 g{};
   g.alpha = 1.0; g.beta = 0.0; g.sym = SYM_NONE;
@@ -191,27 +211,27 @@ static int mo_full_core(const double* C, const double* H, const double* I, int N
   g.C = {X1, NN * P, lin(P), lin(1)};
   g.a_kfast = true; g.b_kfast = false;
   g.tag = "gemm_f64:quarter";
-  GB_TRY(gemm_f64(g, s));
+  GB_TRY(gemm_f64_tc(g, tw, s));
   // X2[(m,n)][r][t] = sum_s C[s][r] X1[(m,n)][s][t]   columns j = (mn, t)
   g.M = P; g.N = (int)(NN * P); g.K = N; g.batch = 1;
   g.A = {C, 0, lin(1), lin(N)};
   g.B = {X1, 0, lin(P), split(P, NP, 1)};
   g.C = {X2, 0, lin(P), split(P, P2, 1)};
   g.a_kfast = false; g.b_kfast = false;
-  GB_TRY(gemm_f64(g, s));
+  GB_TRY(gemm_f64_tc(g, tw, s));
   // X3[m][q][(r,t)] = sum_n C[n][q] X2[m][n][(r,t)]    columns j = (m, rt); stored over X1
   double* X3 = X1;
   g.M = P; g.N = (int)(N * P2); g.K = N; g.batch = 1;
   g.A = {C, 0, lin(1), lin(N)};
   g.B = {X2, 0, lin(P2), split(P2, N * P2, 1)};
   g.C = {X3, 0, lin(P2), split(P2, P3, 1)};
-  GB_TRY(gemm_f64(g, s));
+  GB_TRY(gemm_f64_tc(g, tw, s));
   // I_MO[p][(q,r,t)] = sum_m C[m][p] X3[m][(q,r,t)]
   g.M = N; g.N = (int)P3; g.K = N; g.batch = 1;
   g.A = {C, 0, lin(1), lin(N)};
   g.B = {X3, 0, lin(P3), lin(1)};
   g.C = {imo, 0, lin(P3), lin(1)};
-  GB_TRY(gemm_f64(g, s));
+  GB_TRY(gemm_f64_tc(g, tw, s));
   // Hmat = C^T (H C_p)
   GemmF64 gh{};
   gh.M = N; gh.N = P; gh.K = N; gh.batch = 1;
@@ -242,7 +262,7 @@ extern "C" int gb_mo_full_f64(const double* C, const double* H, const double* I,
   double* X2 = cv.take<double>((size_t)N * N * P * P);
   double* X = cv.take<double>((size_t)N * P);
   GB_REQUIRE(X1 && X2 && X, GB_ERR_WORKSPACE, "gb_mo_full_f64: workspace too small");
-  return mo_full_core(C, H, I, N, P, Hmat, I_MO, X1, X2, X, static_cast<cudaStream_t>(stream));
+  return mo_full_core(C, H, I, N, P, Hmat, I_MO, X1, X2, X, tc_work(cv), static_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------------------
@@ -255,6 +275,7 @@ extern "C" size_t gb_lagrange2_full_workspace_f64(int nbf, int nbf5) {
   z.add<double>(N * N * P * P);
   z.add<double>(N * P);
   z.add<double>(N * P * P * P);  // I_MO
+  z.add<char>(mo_full_tc_bytes(nbf, nbf5));
   return z.used;
 }
 
@@ -277,7 +298,7 @@ extern "C" int gb_lagrange2_full_f64(const double* C, const double* H, const dou
   double* imo = cv.take<double>((size_t)N * P * P * P);
   GB_REQUIRE(X1 && X2 && X && imo, GB_ERR_WORKSPACE, "gb_lagrange2_full_f64: workspace too small");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  GB_TRY(mo_full_core(C, H, I, N, P, Hmat, imo, X1, X2, X, s));
+  GB_TRY(mo_full_core(C, H, I, N, P, Hmat, imo, X1, X2, X, tc_work(cv), s));
   GB_LAUNCH("lagrange2_full", s,
             lagrange2_full_kernel<<<cdiv((long long)N * P, 8), 256, 0, s>>>(imo, Hmat, n, cj12, ck12, elag, N, P,
                                                                            nbeta, nalpha));
@@ -323,7 +344,7 @@ extern "C" int gb_jk_hf_full_f64(const double* D, const double* I, int nbf, doub
   clear_error();
   GB_TRY(check_full(nbf, 1));
   GB_REQUIRE(D && I && J && K, GB_ERR_INVALID_ARG, "gb_jk_hf_full_f64: null pointer");
-  return jk_full_core(D, I, nbf, 1, J, K, static_cast<cudaStream_t>(stream));
+  return jk_full_core(D, I, nbf, 1, J, K, TcWork{}, static_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------------------
@@ -331,13 +352,29 @@ extern "C" int gb_jk_hf_full_f64(const double* D, const double* I, int nbf, doub
 // integrals.py:601-662): out[p][q][r][t] = sum_{m n s l} C[m][p0+p] C[n][q0+q]
 // I[m][n][s][l] C[s][r0+r] C[l][t0+t], as four quarter transforms.
 // ---------------------------------------------------------------------------
-extern "C" size_t gb_mo4_full_workspace_f64(int nbf, int nq, int nr, int nt) {
+// Tensor-core scratch of the quarter transforms (the first range, p, does not
+// size the workspace: its GEMM takes what the others need, or runs without).
+static size_t mo4_full_tc_bytes(int nbf, int nq, int nr, int nt) {
+  const long long N = nbf, q = nq, r = nr, t = nt;
+  size_t b = gemm_f64_tc_bytes(N * N * N, t, N, 1, true, true);
+  for (size_t x : {gemm_f64_tc_bytes(r, N * N * t, N, 1, true, true), gemm_f64_tc_bytes(q, N * r * t, N, 1, true, true),
+                   gemm_f64_tc_bytes(N, q * r * t, N, 1, true, true)})
+    b = x > b ? x : b;
+  return b;
+}
+
+// Without the tensor-core scratch.
+static size_t mo4_full_base_bytes(int nbf, int nq, int nr, int nt) {
   Sizer z;
   const size_t N = nbf;
   const size_t x1 = N * N * N * nt, x3 = N * (size_t)nq * nr * nt;
   z.add<double>(x1 > x3 ? x1 : x3);  // X1 [m][n][s][t], later X3 [m][q][r][t]
   z.add<double>(N * N * nr * nt);    // X2 [m][n][r][t]
   return z.used;
+}
+
+extern "C" size_t gb_mo4_full_workspace_f64(int nbf, int nq, int nr, int nt) {
+  return mo4_full_base_bytes(nbf, nq, nr, nt) + align256(mo4_full_tc_bytes(nbf, nq, nr, nt));
 }
 
 extern "C" int gb_mo4_full_f64(const double* C, const double* I, int nbf, int p0, int np, int q0, int nq, int r0,
@@ -353,7 +390,7 @@ extern "C" int gb_mo4_full_f64(const double* C, const double* I, int nbf, int p0
                  (long long)N * N * nr * nt <= 2147483647LL,
              GB_ERR_BAD_SHAPE, "gb_mo4_full_f64: sizes too large");
   GB_REQUIRE(C && I && out, GB_ERR_INVALID_ARG, "gb_mo4_full_f64: null pointer");
-  GB_REQUIRE(workspace_bytes >= gb_mo4_full_workspace_f64(N, nq, nr, nt), GB_ERR_WORKSPACE,
+  GB_REQUIRE(workspace_bytes >= mo4_full_base_bytes(N, nq, nr, nt), GB_ERR_WORKSPACE,
              "gb_mo4_full_f64: workspace too small");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (np == 0 || nq == 0 || nr == 0 || nt == 0) return GB_OK;
@@ -361,6 +398,7 @@ extern "C" int gb_mo4_full_f64(const double* C, const double* I, int nbf, int p0
   const size_t x1 = (size_t)N * N * N * nt, x3 = (size_t)N * nq * nr * nt;
   double* X1 = cv.take<double>(x1 > x3 ? x1 : x3);
   double* X2 = cv.take<double>((size_t)N * N * nr * nt);
+  const TcWork tw = tc_work(cv);
   const long long NN = (long long)N * N, RT = (long long)nr * nt, QRT = (long long)nq * RT;
   GemmF64 g{};
   g.alpha = 1.0; g.beta = 0.0; g.sym = SYM_NONE; g.batch = 1;
@@ -371,26 +409,26 @@ extern "C" int gb_mo4_full_f64(const double* C, const double* I, int nbf, int p0
   g.B = {C + t0, 0, lin(N), lin(1)};
   g.C = {X1, 0, lin(nt), lin(1)};
   g.a_kfast = true; g.b_kfast = false;
-  GB_TRY(gemm_f64(g, s));
+  GB_TRY(gemm_f64_tc(g, tw, s));
   // X2[(m,n)][r][t] = sum_s C[s][r0+r] X1[(m,n)][s][t]     columns j = ((m,n), t)
   g.M = nr; g.N = (int)(NN * nt); g.K = N;
   g.A = {C + r0, 0, lin(1), lin(N)};
   g.B = {X1, 0, lin(nt), split(nt, (long long)N * nt, 1)};
   g.C = {X2, 0, lin(nt), split(nt, RT, 1)};
   g.a_kfast = false; g.b_kfast = false;
-  GB_TRY(gemm_f64(g, s));
+  GB_TRY(gemm_f64_tc(g, tw, s));
   // X3[m][q][(r,t)] = sum_n C[n][q0+q] X2[m][n][(r,t)]     columns j = (m, (r,t)); over X1
   double* X3 = X1;
   g.M = nq; g.N = (int)(N * RT); g.K = N;
   g.A = {C + q0, 0, lin(1), lin(N)};
   g.B = {X2, 0, lin(RT), split(RT, N * RT, 1)};
   g.C = {X3, 0, lin(RT), split(RT, QRT, 1)};
-  GB_TRY(gemm_f64(g, s));
+  GB_TRY(gemm_f64_tc(g, tw, s));
   // out[p][(q,r,t)] = sum_m C[m][p0+p] X3[m][(q,r,t)]
   g.M = np; g.N = (int)QRT; g.K = N;
   g.A = {C + p0, 0, lin(1), lin(N)};
   g.B = {X3, 0, lin(QRT), lin(1)};
   g.C = {out, 0, lin(QRT), lin(1)};
-  return gemm_f64(g, s);
+  return gemm_f64_tc(g, tw, s);
 }
 

@@ -84,6 +84,7 @@ __global__ void __launch_bounds__(THREADS) gemm_f64_kernel(const GemmF64 g) {
   __shared__ double As[2][BKT][BM + PAD];
   __shared__ double Bs[2][BKT][BN + PAD];
 
+  if (g.only_if && *g.only_if == 0) return;
   const int m0 = blockIdx.y * BM;
   const int n0 = blockIdx.x * BN;
   const long long bz = blockIdx.z;
@@ -186,6 +187,7 @@ __global__ void __launch_bounds__(THREADS) gemm_f64_kernel(const GemmF64 g) {
 // blocks spread it over the whole GPU.
 template <int UNR>
 __global__ void __launch_bounds__(32) gemm_f64_small_kernel(const GemmF64 g) {
+  if (g.only_if && *g.only_if == 0) return;
   const int lane = threadIdx.x;
   const int m0 = blockIdx.y * 8, n0 = blockIdx.x * 8;
   const long long bz = blockIdx.z;

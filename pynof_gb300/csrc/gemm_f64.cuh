@@ -76,6 +76,7 @@ struct GemmF64 {
   bool a_kfast;  // A's K index is the unit-stride one (coalesced along k)
   bool b_kfast;  // B's K index is the unit-stride one
   const char* tag = "gemm_f64";  // profiler label
+  const int* only_if = nullptr;  // run only if this device word is not zero (null: always)
 };
 
 // Plain strided helpers ---------------------------------------------------

@@ -4,7 +4,7 @@
 // Sizes: N = nbf, P = nbf5, Q = naux.  All matrices are row-major (numpy
 // C order) device arrays: C[m * N + p], b[(m * N + n) * Q + l],
 // J/K[(q * N + m) * N + n], bMO[(a * P + q) * Q + l].
-#include "gemm_f64.cuh"
+#include "f64_tc.cuh"
 #include "ri_kernels.cuh"
 
 using namespace gb;
@@ -26,7 +26,7 @@ int half_transform_first(const double* C, const double* b, int N, int P, int Q, 
 }
 
 // T[q][m][l] = sum_n C[n][q] b[m][n][l]   (contracts b's second index; batch over m)
-int half_transform_second(const double* C, const double* b, int N, int P, int Q, double* T,
+int half_transform_second(const double* C, const double* b, int N, int P, int Q, double* T, const TcWork& tw,
                           cudaStream_t s) {
   GemmF64 g{};
   g.M = P; g.N = Q; g.K = N; g.batch = N;
@@ -36,7 +36,7 @@ int half_transform_second(const double* C, const double* b, int N, int P, int Q,
   g.alpha = 1.0; g.beta = 0.0; g.sym = SYM_NONE;
   g.a_kfast = false; g.b_kfast = false;
   g.tag = "gemm_f64:half_transform2";
-  return gemm_f64(g, s);
+  return gemm_f64_tc(g, tw, s);
 }
 
 // X[m][p] = sum_n H[m][n] C[n][p]  (N x P)
@@ -180,9 +180,15 @@ extern "C" int gb_jkh_mo_ri_f64(const double* C, const double* H, const double* 
 // ---------------------------------------------------------------------------
 // A5  Integrals_MO_RI:  Hmat (N x P) and bMO (N, P, Q)
 // ---------------------------------------------------------------------------
+// Tensor-core scratch of mo_ri_core's GEMMs.
+static size_t mo_ri_tc_bytes(int N, int P, int Q) {
+  const size_t a = gemm_f64_tc_bytes(P, Q, N, N, true, false), b = gemm_f64_tc_bytes(N, Q, N, P, true, false);
+  return a > b ? a : b;
+}
+
 static int mo_ri_core(const double* C, const double* H, const double* b, int N, int P, int Q, double* Hmat,
-                      double* bMO, double* T, double* X, cudaStream_t s) {
-  GB_TRY(half_transform_second(C, b, N, P, Q, T, s));
+                      double* bMO, double* T, double* X, const TcWork& tw, cudaStream_t s) {
+  GB_TRY(half_transform_second(C, b, N, P, Q, T, tw, s));
   // bMO[a][q][l] = sum_m C[m][a] T[q][m][l]   (batch q)
   GemmF64 g{};
   g.M = N; g.N = Q; g.K = N; g.batch = P;
@@ -192,7 +198,7 @@ static int mo_ri_core(const double* C, const double* H, const double* b, int N, 
   g.alpha = 1.0; g.beta = 0.0; g.sym = SYM_NONE;
   g.a_kfast = false; g.b_kfast = false;
   g.tag = "gemm_f64:bMO";
-  GB_TRY(gemm_f64(g, s));
+  GB_TRY(gemm_f64_tc(g, tw, s));
   // Hmat = C^T (H Cp)
   GB_TRY(h_times_cp(H, C, N, P, X, s));
   GemmF64 gh{};
@@ -209,6 +215,7 @@ static int mo_ri_core(const double* C, const double* H, const double* b, int N, 
 static void mo_ri_layout(Sizer& z, int N, int P, int Q) {
   z.add<double>((size_t)P * N * Q);  // T (second-index half transform)
   z.add<double>((size_t)N * P);      // X
+  z.add<char>(mo_ri_tc_bytes(N, P, Q));
 }
 
 extern "C" size_t gb_mo_ri_workspace_f64(int nbf, int nbf5, int naux) {
@@ -228,7 +235,7 @@ extern "C" int gb_mo_ri_f64(const double* C, const double* H, const double* b, i
   double* X = cv.take<double>((size_t)N * P);
   GB_REQUIRE(T && X, GB_ERR_WORKSPACE, "gb_mo_ri_f64: workspace too small (%zu < %zu)", workspace_bytes,
              gb_mo_ri_workspace_f64(N, P, Q));
-  return mo_ri_core(C, H, b, N, P, Q, Hmat, bMO, T, X, static_cast<cudaStream_t>(stream));
+  return mo_ri_core(C, H, b, N, P, Q, Hmat, bMO, T, X, tc_work(cv), static_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------------------
@@ -241,6 +248,8 @@ static void lagrange2_ri_layout(Sizer& z, int N, int P, int Q) {
   z.add<double>((size_t)P * Q);      // d
   z.add<double>((size_t)P * Q);      // w
   z.add<double>((size_t)P * P);      // cj12 with zero diagonal
+  const size_t a = mo_ri_tc_bytes(N, P, Q), b = gemm_f64_tc_bytes(N, P, (long long)P * Q, 1, true, true);
+  z.add<char>(a > b ? a : b);
 }
 
 extern "C" size_t gb_lagrange2_ri_workspace_f64(int nbf, int nbf5, int naux) {
@@ -272,7 +281,8 @@ extern "C" int gb_lagrange2_ri_f64(const double* C, const double* H, const doubl
              gb_lagrange2_ri_workspace_f64(N, P, Q));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 
-  GB_TRY(mo_ri_core(C, H, b, N, P, Q, Hmat, bMO, T, X, s));
+  const TcWork tw = tc_work(cv);
+  GB_TRY(mo_ri_core(C, H, b, N, P, Q, Hmat, bMO, T, X, tw, s));
   // d[b][k] = bMO[b][b][k]
   GB_TRY(launch_gather_diag(bMO, d, P, Q, (long long)P * Q + Q, s));
   // w = cj12' d + coef_b d   (cj12' has a zero diagonal; coef_b = n_b for b in doc or vir)
@@ -299,7 +309,7 @@ extern "C" int gb_lagrange2_ri_f64(const double* C, const double* H, const doubl
   ge.alpha = -1.0; ge.beta = 0.0; ge.sym = SYM_NONE;
   ge.a_kfast = true; ge.b_kfast = true;
   ge.tag = "gemm_f64:ck_exchange";
-  GB_TRY(gemm_f64(ge, s));
+  GB_TRY(gemm_f64_tc(ge, tw, s));
   // elag[a][b] += n_b Hmat[a][b] + sum_k bMO[a][b][k] w[b][k];  elag[:, P:] = 0
   GB_TRY(launch_lagrange2_finish(bMO, w, Hmat, n, elag, N, P, Q, s));
   return GB_OK;

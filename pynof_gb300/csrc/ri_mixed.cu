@@ -7,7 +7,7 @@
 //                      in (m, n), so only the packed upper triangle of the
 //                      pairs is kept and J's GEMM writes each pair twice)
 // and stays resident across builds, like b itself in PyNOF's GPU path.
-#include "gemm_f64.cuh"
+#include "f64_tc.cuh"
 #include "ozaki_tc.cuh"
 #include "ri_kernels.cuh"
 #include "slice.cuh"

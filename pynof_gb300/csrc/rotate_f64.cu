@@ -12,7 +12,7 @@
 #include <cmath>
 #include <cstring>
 
-#include "gemm_f64.cuh"
+#include "f64_tc.cuh"
 
 using namespace gb;
 
@@ -69,7 +69,8 @@ __global__ void scale_kernel(const double* __restrict__ src, double* __restrict_
 inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
 
 // C = A B (+ C when accumulate), square row-major N x N
-int matmul(const double* A, const double* B, double* C, int N, bool accumulate, cudaStream_t s, const char* tag) {
+int matmul(const double* A, const double* B, double* C, int N, bool accumulate, const TcWork& tw, cudaStream_t s,
+           const char* tag) {
   GemmF64 g{};
   g.M = N; g.N = N; g.K = N; g.batch = 1;
   g.A = {A, 0, lin(N), lin(1)};
@@ -78,7 +79,7 @@ int matmul(const double* A, const double* B, double* C, int N, bool accumulate, 
   g.alpha = 1.0; g.beta = accumulate ? 1.0 : 0.0; g.sym = SYM_NONE;
   g.a_kfast = true; g.b_kfast = false;
   g.tag = tag;
-  return gemm_f64(g, s);
+  return gemm_f64_tc(g, tw, s);
 }
 
 template <class Cv>
@@ -96,7 +97,7 @@ void rotate_layout(Cv& c, int N, double** bufs, unsigned long long** norm) {
 extern "C" size_t gb_rotate_orbital_workspace_f64(int nbf) {
   SizeCarve c;
   rotate_layout(c, nbf, nullptr, nullptr);
-  return c.used;
+  return c.used + align256(gemm_f64_tc_bytes(nbf, nbf, nbf, 1, true, true));
 }
 
 extern "C" int gb_rotate_orbital_f64(const double* y, const double* C, int nbf, int nbf5, double norm1,
@@ -106,13 +107,16 @@ extern "C" int gb_rotate_orbital_f64(const double* y, const double* C, int nbf, 
   GB_REQUIRE(N > 0 && P > 0 && P <= N, GB_ERR_BAD_SHAPE, "gb_rotate_orbital_f64: need 0 < nbf5 <= nbf");
   GB_REQUIRE(y && C && Cout, GB_ERR_INVALID_ARG, "gb_rotate_orbital_f64: null pointer");
   GB_REQUIRE(C != Cout, GB_ERR_INVALID_ARG, "gb_rotate_orbital_f64: C and Cout must not alias");
-  GB_REQUIRE(workspace_bytes >= gb_rotate_orbital_workspace_f64(N), GB_ERR_WORKSPACE,
+  SizeCarve base;
+  rotate_layout(base, N, nullptr, nullptr);
+  GB_REQUIRE(workspace_bytes >= base.used, GB_ERR_WORKSPACE,
              "gb_rotate_orbital_f64: workspace too small");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   Carve wc(workspace, workspace_bytes);
   double* buf[6];
   unsigned long long* dnorm = nullptr;
   rotate_layout(wc, N, buf, &dnorm);
+  const TcWork tw = tc_work(wc);
   double *Y = buf[0], *X2 = buf[1], *X3 = buf[2], *X4 = buf[3], *R0 = buf[4], *R1 = buf[5];
   const long long NN = (long long)N * N;
 
@@ -141,9 +145,9 @@ extern "C" int gb_rotate_orbital_f64(const double* y, const double* C, int nbf, 
   double c[TAYLOR_DEG + 1];
   c[0] = 1.0;
   for (int k = 1; k <= TAYLOR_DEG; ++k) c[k] = c[k - 1] / k;
-  GB_TRY(matmul(X, X, X2, N, false, s, "gemm_f64:expm"));
-  GB_TRY(matmul(X2, X, X3, N, false, s, "gemm_f64:expm"));
-  GB_TRY(matmul(X2, X2, X4, N, false, s, "gemm_f64:expm"));
+  GB_TRY(matmul(X, X, X2, N, false, tw, s, "gemm_f64:expm"));
+  GB_TRY(matmul(X2, X, X3, N, false, tw, s, "gemm_f64:expm"));
+  GB_TRY(matmul(X2, X2, X4, N, false, tw, s, "gemm_f64:expm"));
   // R = B3 + c16 X^4
   GB_LAUNCH("rotate_poly", s,
             poly_block_kernel<<<cdiv(NN, 256), 256, 0, s>>>(R0, X, X2, X3, X4, N, c[12], c[13], c[14], c[15],
@@ -154,7 +158,7 @@ extern "C" int gb_rotate_orbital_f64(const double* y, const double* C, int nbf, 
     GB_LAUNCH("rotate_poly", s,
               poly_block_kernel<<<cdiv(NN, 256), 256, 0, s>>>(Rn, X, X2, X3, nullptr, N, c[4 * j], c[4 * j + 1],
                                                                 c[4 * j + 2], c[4 * j + 3], 0.0));
-    GB_TRY(matmul(X4, R, Rn, N, true, s, "gemm_f64:expm"));
+    GB_TRY(matmul(X4, R, Rn, N, true, tw, s, "gemm_f64:expm"));
     double* t = R;
     R = Rn;
     Rn = t;
@@ -162,10 +166,10 @@ extern "C" int gb_rotate_orbital_f64(const double* y, const double* C, int nbf, 
   // s squarings, ping-ponging between R and a free buffer
   double* spare = X2;
   for (int k = 0; k < sq; ++k) {
-    GB_TRY(matmul(R, R, spare, N, false, s, "gemm_f64:expm"));
+    GB_TRY(matmul(R, R, spare, N, false, tw, s, "gemm_f64:expm"));
     double* t = R;
     R = spare;
     spare = t;
   }
-  return matmul(C, R, Cout, N, false, s, "gemm_f64:rotate");
+  return matmul(C, R, Cout, N, false, tw, s, "gemm_f64:rotate");
 }

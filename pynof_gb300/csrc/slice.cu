@@ -27,29 +27,35 @@ __device__ __forceinline__ void make_digits(double x, int E, uint32_t* out) {
   int ex = (int)((bits >> 52) & 0x7FF);
   unsigned long long m = bits & 0xFFFFFFFFFFFFFull;
   if (ex) m |= 1ull << 52; else ex = 1;
-  const int r = 1075 + E - ex - digit_exp(W, S);  // right shift of the 53-bit mantissa (>= 9 for e_S <= 44)
+  // right shift of the 53-bit mantissa (>= 9 for e_S <= 44, a left shift of at most 9 for 62)
+  const int r = 1075 + E - ex - digit_exp(W, S);
   long long xi;
-  if (r >= 64) xi = 0;
+  if (digit_exp(W, S) > 52 && r <= 0) xi = (long long)(m << -r);
+  else if (r >= 64) xi = 0;
   else xi = (long long)((m + (1ull << (r - 1))) >> r);
   if (bits >> 63) xi = -xi;
   constexpr int NL = S - 1 < 3 ? S - 1 : 3, HALF = 1 << (W - 1), MASK = (1 << W) - 1;
-  int L = (int)(xi & ((1ll << (W * NL)) - 1));
-  int H = (int)(xi >> (W * NL));
-#pragma unroll
-  for (int s = S; s > S - NL; --s) {
-    const int d = ((L + HALF) & MASK) - HALF;
-    L = (L - d) >> W;
+  // the three middle digits of seven go through 32 bits of their own
+  constexpr int NM = S == 7 ? 3 : 0;
+  auto digit = [&](int s, int& rest) {
+    const int d = ((rest + HALF) & MASK) - HALF;
+    rest = (rest - d) >> W;
     const float w = __int_as_float((127 - digit_exp(W, s)) << 23);
     out[s - 1] = __float_as_uint(fmaf(__int_as_float(0x4B400000 + d), w, -12582912.0f * w));
+  };
+  int L = (int)(xi & ((1ll << (W * NL)) - 1));
+#pragma unroll
+  for (int s = S; s > S - NL; --s) digit(s, L);
+  int H = (int)(xi >> (W * (NL + NM)));
+  if (NM > 0) {
+    int M = (int)((xi >> (W * NL)) & ((1ll << (W * NM)) - 1)) + L;
+#pragma unroll
+    for (int s = S - NL; s > S - NL - NM; --s) digit(s, M);
+    L = M;
   }
   H += L;
 #pragma unroll
-  for (int s = S - NL; s >= 2; --s) {
-    const int d = ((H + HALF) & MASK) - HALF;
-    H = (H - d) >> W;
-    const float w = __int_as_float((127 - digit_exp(W, s)) << 23);
-    out[s - 1] = __float_as_uint(fmaf(__int_as_float(0x4B400000 + d), w, -12582912.0f * w));
-  }
+  for (int s = S - NL - NM; s >= 2; --s) digit(s, H);
   const float w1 = __int_as_float((127 - digit_exp(W, 1)) << 23);
   out[0] = __float_as_uint(fmaf(__int_as_float(0x4B400000 + H), w1, -12582912.0f * w1));
 }
@@ -68,7 +74,10 @@ __device__ __forceinline__ void clear_norms(int* norms, long long b, long long r
     norms[(b * ((rows + SL_ROWS - 1) / SL_ROWS) + row / SL_ROWS) * SL_NORMS + lane] = 0;
 }
 
-// One warp per row; K is the unit-stride index.
+// One warp per row; K is the unit-stride index.  (One launch for exponents and
+// digits, a CTA reading its 32 rows twice, was slower: 1093 us against 903 for
+// the nine slicings of an orbital step at nbf=300.  So were four and eight
+// explicit loads in flight here and below: 430 us of 285.)
 __global__ void rowexp_kfast_kernel(SliceSrc src, int rows, int K, int* __restrict__ exps, int* __restrict__ norms,
                                     int* status) {
   const long long b = blockIdx.y;
@@ -102,6 +111,33 @@ __global__ void rowexp_kfast_kernel(SliceSrc src, int rows, int K, int* __restri
   }
   if (lane == 0) {
     exps[b * rows + row] = exponent_of(mx);
+    note_nonfinite(mx, status);
+  }
+}
+
+// The same with a row's K cut into gridDim.z ranges, for few long rows (300
+// rows of 180000 took 0.6 ms on 300 warps): every warp folds its range's
+// exponent in with atomicMax; exps and norms are preset below any value.
+__global__ void rowexp_kfast_split_kernel(SliceSrc src, int rows, int K, int* __restrict__ exps, int* status) {
+  const long long b = blockIdx.y;
+  const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const int per = (K + gridDim.z - 1) / gridDim.z, k0 = blockIdx.z * per, k1 = min(K, k0 + per);
+  if (k0 >= k1) return;
+  const double* base = src.p + b * src.sb + src.row_at(row);
+  unsigned long long mx = 0;
+  for (int k = k0 + lane; k < k1; k += 32) {
+    const unsigned long long v = abs_bits(base[src.k.at(k)]);
+    mx = v > mx ? v : mx;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long v = __shfl_xor_sync(0xffffffffu, mx, o);
+    mx = v > mx ? v : mx;
+  }
+  if (lane == 0) {
+    atomicMax(exps + b * rows + row, exponent_of(mx));
     note_nonfinite(mx, status);
   }
 }
@@ -173,7 +209,7 @@ __device__ __forceinline__ void store_group(const double (&xs)[8], int e, unsign
 #pragma unroll
     for (int s = 0; s < S; ++s) pk[s][u >> 1] = __byte_perm(d0[s], d1[s], 0x7632);
 #pragma unroll
-    for (int s = 0; s < (W == 9 ? SL_NORMS : 0); ++s) {
+    for (int s = 0; s < (W != 9 ? 0 : S == 7 ? SL_NORMS : 3); ++s) {
       const float a = __uint_as_float(d0[s]), b = __uint_as_float(d1[s]);
       nq[s] = fmaf(a, a, fmaf(b, b, nq[s]));
     }
@@ -194,7 +230,7 @@ __device__ __forceinline__ void store_group(const double (&xs)[8], int e, unsign
 // k block into registers did (measured: 1.62 ms against 1.87-1.93 ms for the
 // T of one nbf=600 build, 8.64 GB).
 template <int S, int W>
-__global__ void __launch_bounds__(256, 4) digits_blocked_kernel(SliceSrc src, SlicedDesc dst) {
+__global__ void __launch_bounds__(256, S == 7 ? 3 : 4) digits_blocked_kernel(SliceSrc src, SlicedDesc dst) {
   const long long b = blockIdx.y;
   const int kbn = dst.kblocks();
   const int runs = (kbn + SL_KPC - 1) / SL_KPC;
@@ -218,7 +254,7 @@ __global__ void __launch_bounds__(256, 4) digits_blocked_kernel(SliceSrc src, Sl
     // non-negative floats order as their bits
     int* nb = dst.norms + (b * dst.rblocks() + rb) * SL_NORMS;
 #pragma unroll
-    for (int s = 0; s < SL_NORMS; ++s) {
+    for (int s = 0; s < (S == 7 ? SL_NORMS : 3); ++s) {
       const float scale = __int_as_float((127 + 2 * digit_exp(W, s + 1)) << 23);  // back to squares of the digits
       const unsigned int mx = __reduce_max_sync(0xffffffffu, __float_as_uint(nq[s] * scale));
       if (lane == 0) atomicMax(nb + s, (int)mx);
@@ -299,8 +335,8 @@ inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) /
 
 }  // namespace
 
-int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bool exps_ready) {
-  GB_REQUIRE((dst.kind == 0 && dst.S >= 1 && dst.S <= 5) || (dst.kind == 1 && dst.S == 2), GB_ERR_INVALID_ARG,
+int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bool exps_ready, int* status) {
+  GB_REQUIRE((dst.kind == 0 && ((dst.S >= 1 && dst.S <= 5) || dst.S == 7)) || (dst.kind == 1 && dst.S == 2), GB_ERR_INVALID_ARG,
              "slice_operand: bad split form (planes %d, kind %d)", dst.S, dst.kind);
   GB_REQUIRE(dst.batch >= 1 && dst.batch <= 65535 && dst.rows >= 0, GB_ERR_BAD_SHAPE, "slice_operand: bad batch");
   GB_REQUIRE((reinterpret_cast<uintptr_t>(dst.planes) & 15) == 0, GB_ERR_INVALID_ARG,
@@ -308,18 +344,28 @@ int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bo
   if (dst.rows == 0 || dst.K == 0) return GB_OK;
   int* norms = dst.kind == 0 ? dst.norms : nullptr;
   GB_REQUIRE(dst.kind != 0 || norms, GB_ERR_INVALID_ARG, "slice_operand: no norms");
+  int* st = status ? status : device_status_word();
+  const long long warps = (long long)dst.rows * dst.batch;
   if (exps_ready) {
     GB_REQUIRE(dst.kind == 0, GB_ERR_INVALID_ARG, "slice_operand: recorded exponents are for digit slices");
+  } else if (src.kfast && dst.kind == 0 && dst.K >= 8192 && warps <= 4096 &&
+             dst.norms == dst.exps + (size_t)dst.batch * dst.rows) {
+    // fewer warps than the SMs hold: ranges of K of at least 2048
+    long long z = 8192 / warps + 1;
+    z = z < dst.K / 2048 ? z : dst.K / 2048;
+    GB_TRY(cuda_status(cudaMemsetAsync(dst.exps, 0x80, sizeof(int) * sliced_meta_ints(dst.batch, dst.rows), s),
+                       "slice_operand: exponents"));
+    GB_LAUNCH("slice_rowexp", s,
+              rowexp_kfast_split_kernel<<<dim3(cdiv(dst.rows, 8), dst.batch, (unsigned)z), 256, 0, s>>>(
+                  src, dst.rows, dst.K, dst.exps, st));
   } else if (src.kfast) {
-    int* st = device_status_word();
     GB_LAUNCH("slice_rowexp", s,
               rowexp_kfast_kernel<<<dim3(cdiv(dst.rows, 8), dst.batch), 256, 0, s>>>(src, dst.rows, dst.K, dst.exps,
                                                                                     norms, st));
   } else {
-    int* st = device_status_word();
     GB_LAUNCH("slice_rowexp", s,
-              rowexp_rfast_kernel<<<dim3(cdiv(dst.rows, 32), dst.batch), 256, 0, s>>>(src, dst.rows, dst.K,
-                                                                                     dst.exps, norms, st));
+              rowexp_rfast_kernel<<<dim3(cdiv(dst.rows, 32), dst.batch), 256, 0, s>>>(src, dst.rows, dst.K, dst.exps,
+                                                                                     norms, st));
   }
   const long long blocks = (long long)dst.rblocks() * dst.kblocks();
   GB_REQUIRE(blocks <= 2147483647LL, GB_ERR_BAD_SHAPE, "slice_operand: too many blocks");
@@ -329,8 +375,11 @@ int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bo
   }
   const dim3 grid((unsigned)((long long)dst.rblocks() * ((dst.kblocks() + SL_KPC - 1) / SL_KPC)), dst.batch);
   if (dst.W == 9) {
-    GB_REQUIRE(dst.S == 5, GB_ERR_INVALID_ARG, "slice_operand: nine-bit digits come in five planes");
-    GB_LAUNCH("slice_digits", s, digits_blocked_kernel<5, 9><<<grid, 256, 0, s>>>(src, dst));
+    GB_REQUIRE(dst.S == 5 || dst.S == 7, GB_ERR_INVALID_ARG, "slice_operand: nine-bit digits come in five or seven planes");
+    if (dst.S == 5)
+      GB_LAUNCH("slice_digits", s, digits_blocked_kernel<5, 9><<<grid, 256, 0, s>>>(src, dst));
+    else
+      GB_LAUNCH("slice_digits7", s, digits_blocked_kernel<7, 9><<<grid, 256, 0, s>>>(src, dst));
     return GB_OK;
   }
   switch (dst.S) {

@@ -29,10 +29,10 @@
 // Blocks are ordered [batch][rb][kb].  Rows and K are zero-padded to whole
 // blocks.  Exponents: exps[b][r] (int32).
 //
-// Norms: norms[b][rb][s - 1], s <= 3, is the FP32 bit pattern of an upper bound
-// of sum d_s^2 over one k group parity (8 of every 16 k) of any run of 128 k of
-// any row of the block; a run's sum of products of two digits is then at most
-// 2 sqrt(norm_a norm_b) (Cauchy-Schwarz).
+// Norms: norms[b][rb][s - 1], s <= 3 (five planes) or 5 (seven), is the FP32 bit
+// pattern of an upper bound of sum d_s^2 over one k group parity (8 of every 16 k)
+// of any run of 128 k of any row of the block; a run's sum of products of two
+// digits is then at most 2 sqrt(norm_a norm_b) (Cauchy-Schwarz).
 //
 // TF32x3 form (split code SPLIT_TF32X3): two planes, hi = tf32(x 2^-E) and
 // lo = tf32(x 2^-E - hi) (each rounded to nearest even, 11 significant bits,
@@ -55,18 +55,23 @@ constexpr int SL_TILE_BYTES = SL_ROWS * SL_K * 2;  // one slice of one block: 4 
 
 constexpr int SL_SLICE_STEP = SL_ROWS * 16;  // from one slice of a k group to the next
 constexpr int SL_KPC = 8;                  // k blocks per slicer CTA, and per run of the norms
-constexpr int SL_NORMS = 3;                // digits whose norms are recorded
+constexpr int SL_NORMS = 5;                // digits whose norms are recorded (three of five planes, five of seven)
 
 // Split codes ("nslices" in the C ABI): 1..5 seven-bit digit slices, 6 (42 bits,
 // 21 products of s + t <= 7 if they were seven-bit ones) is five nine-bit slices
 // (45 bits, 15 products of s + t <= 6), or the TF32x3 split.
-constexpr int SPLIT_TF32X3 = 32;
+// SPLIT_F64 (inside the library only): seven nine-bit slices, 62 bits, for
+// products that are as accurate as FP64 arithmetic (f64_tc.cuh).
+constexpr int SPLIT_TF32X3 = 32, SPLIT_F64 = 64;
 struct SliceForm {
   int S, kind, W;  // planes; 0 = bf16 digits, 1 = tf32 hi/lo; bits per digit
 };
 __host__ __device__ constexpr bool valid_split(int code) { return (code >= 1 && code <= 6) || code == SPLIT_TF32X3; }
 __host__ __device__ constexpr SliceForm form_of(int code) {
-  return code == SPLIT_TF32X3 ? SliceForm{2, 1, 0} : code == 6 ? SliceForm{5, 0, 9} : SliceForm{code, 0, 7};
+  return code == SPLIT_TF32X3 ? SliceForm{2, 1, 0}
+         : code == SPLIT_F64  ? SliceForm{7, 0, 9}
+         : code == 6          ? SliceForm{5, 0, 9}
+                              : SliceForm{code, 0, 7};
 }
 // e_s of W-bit digits
 __host__ __device__ constexpr int digit_exp(int W, int s) { return W == 9 ? 9 * s - 1 : W * s; }
@@ -79,10 +84,11 @@ struct SliceSrc {
   // > 0: the rows are the packed upper triangle of tri_n x tri_n index
   // pairs (tri_pair); row r reads r.at(m * tri_n + n)
   int tri_n = 0;
+  long long row0 = 0;  // row 0 of the slices is row row0 of the source (a panel of its rows)
   __host__ __device__ __forceinline__ long long row_at(long long row) const {
-    if (tri_n <= 0) return r.at(row);
+    if (tri_n <= 0) return r.at(row0 + row);
     int m, n;
-    tri_pair(row, tri_n, m, n);
+    tri_pair(row0 + row, tri_n, m, n);
     return r.at((long long)m * tri_n + n);
   }
 };
@@ -95,12 +101,20 @@ struct SlicedDesc {
   int W = 7;     // bits per digit (kind 0)
   int* norms = nullptr;  // [batch][row block][SL_NORMS], directly behind exps where it is carved (kind 0)
   __host__ __device__ int kper() const { return kind ? SL_K / 2 : SL_K; }
-  __host__ __device__ int code() const { return kind ? SPLIT_TF32X3 : W == 9 ? 6 : S; }  // the split code it was cut with
+  __host__ __device__ int code() const { return kind ? SPLIT_TF32X3 : W == 9 ? (S == 7 ? SPLIT_F64 : 6) : S; }  // the split code it was cut with
   __host__ __device__ int rblocks() const { return (rows + SL_ROWS - 1) / SL_ROWS; }
   __host__ __device__ int kblocks() const { return (K + kper() - 1) / kper(); }
   __host__ __device__ long long block_bytes() const { return (long long)S * SL_TILE_BYTES; }
   __host__ __device__ long long batch_bytes() const { return (long long)rblocks() * kblocks() * block_bytes(); }
 };
+
+// sqrt of the norms of digits 1..n of the row block that holds row r0 of batch entry b.
+template <int n>
+__device__ __forceinline__ void block_norms(const SlicedDesc& d, int b, int r0, float (&x)[n]) {
+  const int* p = d.norms + ((long long)(d.batch == 1 ? 0 : b) * d.rblocks() + r0 / SL_ROWS) * SL_NORMS;
+#pragma unroll
+  for (int i = 0; i < n; ++i) x[i] = sqrtf(__int_as_float(__ldg(p + i)));
+}
 
 // `code` is a split code (1..6 or SPLIT_TF32X3).
 inline size_t sliced_plane_bytes(int batch, int rows, int K, int code) {
@@ -123,10 +137,12 @@ SlicedDesc take_sliced(Cv& c, int batch, int rows, int K, int code) {
                     e ? e + (size_t)batch * rows : nullptr};
 }
 
-// Exponents then digits; both kernels read the source once.  With
-// exps_ready the row exponents are already in dst.exps (recorded by the
-// kernel that read the source before) and only the digits are formed; the
-// norms then hold a value below every float's bits (memset with 0x80 bytes).
-int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bool exps_ready = false);
+// Exponents and digits.  With exps_ready the row exponents are already in
+// dst.exps (recorded by the kernel that read the source before) and only the
+// digits are formed; the norms then hold a value below every float's bits
+// (memset with 0x80 bytes).  A NaN or an infinity is recorded in *status, the
+// device's status word when null.
+int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bool exps_ready = false,
+                  int* status = nullptr);
 
 }  // namespace gb
