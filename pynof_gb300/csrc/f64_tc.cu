@@ -132,6 +132,7 @@ __device__ __forceinline__ long long exact_sum(float x2, float x3, float x4, flo
 }
 
 __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArgs a) {
+  chain_wait();
   extern __shared__ unsigned char smem_raw[];
   if (*a.nonfinite != 0) return;  // gemm_f64's kernel does this one
   unsigned char* smem =
@@ -461,6 +462,7 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
 
 // Partial sums of the K splits, in order, into the output.
 __global__ void __launch_bounds__(256) sum_parts_kernel(const __grid_constant__ DArgs a) {
+  chain_wait();
   if (*a.nonfinite != 0) return;
   const long long MN = (long long)a.M * a.N, all = MN * a.batch;
   const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
@@ -685,10 +687,11 @@ int gemm_f64_tc(const GemmF64& g, const TcWork& w, cudaStream_t s) {
         a.wait_ns = 2000000000ull;
         a.ntiles = (int)(((xn + BM - 1) / BM) * (long long)((yn + BN - 1) / BN) * nb * p.nsplit);
         const unsigned grid = (unsigned)std::min(a.ntiles, 152);
-        GB_LAUNCH(g.tag, s, f64_tc_kernel<<<grid, THREADS, SMEM_BYTES, s>>>(a));
+        GB_LAUNCH_CHAIN(g.tag, s, f64_tc_kernel, dim3(grid), dim3(THREADS), SMEM_BYTES, a);
         if (p.nsplit > 1) {
           const long long all = (long long)xn * yn * nb;
-          GB_LAUNCH("f64_tc:sum_parts", s, sum_parts_kernel<<<(unsigned)((all + 255) / 256), 256, 0, s>>>(a));
+          GB_LAUNCH_CHAIN("f64_tc:sum_parts", s, sum_parts_kernel, dim3((unsigned)((all + 255) / 256)), dim3(256), 0,
+                          a);
         }
       }
     }

@@ -9,6 +9,7 @@ namespace {
 
 // dst = src with the diagonal entries (i, i), i >= ini, set to zero.
 __global__ void zero_diag_from_kernel(const double* __restrict__ src, double* __restrict__ dst, int P, int ini) {
+  chain_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)P * P) return;
   const int r = (int)(idx / P), c = (int)(idx % P);
@@ -19,6 +20,7 @@ __global__ void zero_diag_from_kernel(const double* __restrict__ src, double* __
 __global__ void fock_diag_terms_kernel(double* __restrict__ F, const double* __restrict__ J,
                                        const double* __restrict__ H, const double* __restrict__ n, int N, int P,
                                        int ini, int nbeta, int nalpha) {
+  chain_wait();
   const long long mn = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int i = blockIdx.y;
   const long long NN = (long long)N * N;
@@ -45,6 +47,7 @@ __global__ void fock_diag_terms_kernel(double* __restrict__ F, const double* __r
 __global__ void fock_ro_coef_kernel(const double* __restrict__ n, const double* __restrict__ cj12,
                                     const double* __restrict__ ck12, double* __restrict__ A, double* __restrict__ B,
                                     double* __restrict__ a, int P, int ini, int nbeta, int nalpha) {
+  chain_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)P * P) return;
   const int i = (int)(idx / P), j = (int)(idx % P);
@@ -73,6 +76,7 @@ __global__ void fock_ro_coef_kernel(const double* __restrict__ n, const double* 
 // F[i] += a_i H
 __global__ void fock_add_h_kernel(double* __restrict__ F, const double* __restrict__ H, const double* __restrict__ a,
                                   int N) {
+  chain_wait();
   const long long mn = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int i = blockIdx.y;
   const long long NN = (long long)N * N;
@@ -84,6 +88,7 @@ __global__ void fock_add_h_kernel(double* __restrict__ F, const double* __restri
 // G[i][m] = sum_n F[i][m][n] C[n][i]   (one warp per (i, m))
 __global__ void fock_times_orbital_kernel(const double* __restrict__ F, const double* __restrict__ C,
                                           double* __restrict__ G, int N, int P) {
+  chain_wait();
   const long long w = (long long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (w >= (long long)P * N) return;
@@ -97,6 +102,7 @@ __global__ void fock_times_orbital_kernel(const double* __restrict__ F, const do
 }
 
 __global__ void zero_outside_kernel(double* __restrict__ elag, int N, int rows, int cols) {
+  chain_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)N * N) return;
   const int r = (int)(idx / N), c = (int)(idx % N);
@@ -108,6 +114,7 @@ __global__ void zero_outside_kernel(double* __restrict__ elag, int N, int rows, 
 __global__ void energy_elec_kernel(const double* __restrict__ elag, const double* __restrict__ Hd,
                                    const double* __restrict__ n, int N, int P, int nbeta, int nalpha, int high_spin,
                                    double* __restrict__ E) {
+  chain_wait();
   __shared__ double red[32];
   double acc = 0.0;
   for (int i = threadIdx.x; i < P; i += blockDim.x) {
@@ -157,8 +164,10 @@ extern "C" int gb_fock_rc_f64(const double* J, const double* K, const double* n,
   GB_REQUIRE(cjm && ckm, GB_ERR_WORKSPACE, "gb_fock_rc_f64: workspace too small");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int ini = no1 > 1 ? no1 : 0;
-  GB_LAUNCH("zero_diag_from", s, zero_diag_from_kernel<<<cdiv((long long)P * P, 256), 256, 0, s>>>(cj12, cjm, P, ini));
-  GB_LAUNCH("zero_diag_from", s, zero_diag_from_kernel<<<cdiv((long long)P * P, 256), 256, 0, s>>>(ck12, ckm, P, ini));
+  GB_LAUNCH_CHAIN("zero_diag_from", s, zero_diag_from_kernel, dim3(cdiv((long long)P * P, 256)), dim3(256), 0, cj12,
+                  cjm, P, ini);
+  GB_LAUNCH_CHAIN("zero_diag_from", s, zero_diag_from_kernel, dim3(cdiv((long long)P * P, 256)), dim3(256), 0, ck12,
+                  ckm, P, ini);
   const long long NN = (long long)N * N;
   // F = cj12' J
   GemmF64 g{};
@@ -175,8 +184,8 @@ extern "C" int gb_fock_rc_f64(const double* J, const double* K, const double* n,
   g.B = {K, 0, lin(NN), lin(1)};
   g.alpha = -1.0; g.beta = 1.0;
   GB_TRY(gemm_f64_tc(g, tc_work(cv), s));
-  GB_LAUNCH("fock_diag_terms", s,
-            fock_diag_terms_kernel<<<dim3(cdiv(NN, 256), P), 256, 0, s>>>(F, J, H, n, N, P, ini, nbeta, nalpha));
+  GB_LAUNCH_CHAIN("fock_diag_terms", s, fock_diag_terms_kernel, dim3(dim3(cdiv(NN, 256), P)), dim3(256), 0, F, J, H,
+                  n, N, P, ini, nbeta, nalpha);
   return GB_OK;
 }
 
@@ -208,9 +217,8 @@ extern "C" int gb_fock_ro_f64(const double* J, const double* K, const double* n,
   GB_REQUIRE(A && B && a, GB_ERR_WORKSPACE, "gb_fock_ro_f64: workspace too small");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int ini = no1 > 1 ? no1 : 0;
-  GB_LAUNCH("fock_ro_coef", s,
-            fock_ro_coef_kernel<<<cdiv((long long)P * P, 256), 256, 0, s>>>(n, cj12, ck12, A, B, a, P, ini, nbeta,
-                                                                             nalpha));
+  GB_LAUNCH_CHAIN("fock_ro_coef", s, fock_ro_coef_kernel, dim3(cdiv((long long)P * P, 256)), dim3(256), 0, n, cj12,
+                  ck12, A, B, a, P, ini, nbeta, nalpha);
   const long long NN = (long long)N * N;
   // F = A J - B K
   GemmF64 g{};
@@ -226,7 +234,7 @@ extern "C" int gb_fock_ro_f64(const double* J, const double* K, const double* n,
   g.B = {K, 0, lin(NN), lin(1)};
   g.alpha = -1.0; g.beta = 1.0;
   GB_TRY(gemm_f64_tc(g, tc_work(cv), s));
-  GB_LAUNCH("fock_add_h", s, fock_add_h_kernel<<<dim3(cdiv(NN, 256), P), 256, 0, s>>>(F, H, a, N));
+  GB_LAUNCH_CHAIN("fock_add_h", s, fock_add_h_kernel, dim3(dim3(cdiv(NN, 256), P)), dim3(256), 0, F, H, a, N);
   return GB_OK;
 }
 
@@ -250,8 +258,8 @@ extern "C" int gb_lagrange_f64(const double* F, const double* C, int nbf, int nb
   double* G = cv.take<double>((size_t)P * N);  // G[i][m]
   GB_REQUIRE(G, GB_ERR_WORKSPACE, "gb_lagrange_f64: workspace too small");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  GB_LAUNCH("fock_times_orbital", s,
-            fock_times_orbital_kernel<<<cdiv((long long)P * N, 8), 256, 0, s>>>(F, C, G, N, P));
+  GB_LAUNCH_CHAIN("fock_times_orbital", s, fock_times_orbital_kernel, dim3(cdiv((long long)P * N, 8)), dim3(256), 0,
+                  F, C, G, N, P);
   GemmF64 g{};
   g.M = noptorb; g.N = P; g.K = N; g.batch = 1;
   g.A = {C, 0, lin(1), lin(N)};   // A(k, m) = C[m][k]
@@ -262,8 +270,8 @@ extern "C" int gb_lagrange_f64(const double* F, const double* C, int nbf, int nb
   g.tag = "gemm_f64:small";
   GB_TRY(gemm_f64(g, s));
   if (noptorb < N || P < N) {
-    GB_LAUNCH("zero_outside", s,
-              zero_outside_kernel<<<cdiv((long long)N * N, 256), 256, 0, s>>>(elag, N, noptorb, P));
+    GB_LAUNCH_CHAIN("zero_outside", s, zero_outside_kernel, dim3(cdiv((long long)N * N, 256)), dim3(256), 0, elag, N,
+                    noptorb, P);
   }
   return GB_OK;
 }
@@ -301,7 +309,7 @@ extern "C" int gb_energy_elec_f64(const double* elag, const double* C, const dou
   g.tag = "gemm_f64:small";
   GB_TRY(gemm_f64(g, s));
   GB_TRY(launch_col_dot(C, N, X, P, Hd, N, P, s));
-  GB_LAUNCH("energy_elec", s,
-            energy_elec_kernel<<<1, 256, 0, s>>>(elag, Hd, n, N, P, nbeta, nalpha, high_spin, E));
+  GB_LAUNCH_CHAIN("energy_elec", s, energy_elec_kernel, dim3(1), dim3(256), 0, elag, Hd, n, N, P, nbeta, nalpha,
+                  high_spin, E);
   return GB_OK;
 }

@@ -15,6 +15,7 @@ using namespace gb;
 namespace {
 
 __global__ void density_kernel(const double* __restrict__ C, double* __restrict__ D, int N, int P) {
+  chain_wait();
   const long long sl = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int i = blockIdx.y;
   if (sl >= (long long)N * N) return;
@@ -28,6 +29,7 @@ __global__ void lagrange2_full_kernel(const double* __restrict__ imo, const doub
                                       const double* __restrict__ n, const double* __restrict__ cj,
                                       const double* __restrict__ ck, double* __restrict__ elag, int N, int P,
                                       int nbeta, int nalpha) {
+  chain_wait();
   const long long w = (long long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (w >= (long long)N * P) return;
@@ -50,6 +52,7 @@ __global__ void lagrange2_full_kernel(const double* __restrict__ imo, const doub
 }
 
 __global__ void zero_cols_from_kernel(double* __restrict__ elag, int N, int P) {
+  chain_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int W = N - P;
   if (idx >= (long long)N * W) return;
@@ -65,7 +68,7 @@ int check_full(int N, int P) {
 }
 
 int make_density(const double* C, double* D, int N, int P, cudaStream_t s) {
-  GB_LAUNCH("density", s, density_kernel<<<dim3(cdiv((long long)N * N, 256), P), 256, 0, s>>>(C, D, N, P));
+  GB_LAUNCH_CHAIN("density", s, density_kernel, dim3(dim3(cdiv((long long)N * N, 256), P)), dim3(256), 0, C, D, N, P);
   return GB_OK;
 }
 
@@ -299,12 +302,11 @@ extern "C" int gb_lagrange2_full_f64(const double* C, const double* H, const dou
   GB_REQUIRE(X1 && X2 && X && imo, GB_ERR_WORKSPACE, "gb_lagrange2_full_f64: workspace too small");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   GB_TRY(mo_full_core(C, H, I, N, P, Hmat, imo, X1, X2, X, tc_work(cv), s));
-  GB_LAUNCH("lagrange2_full", s,
-            lagrange2_full_kernel<<<cdiv((long long)N * P, 8), 256, 0, s>>>(imo, Hmat, n, cj12, ck12, elag, N, P,
-                                                                           nbeta, nalpha));
+  GB_LAUNCH_CHAIN("lagrange2_full", s, lagrange2_full_kernel, dim3(cdiv((long long)N * P, 8)), dim3(256), 0, imo,
+                  Hmat, n, cj12, ck12, elag, N, P, nbeta, nalpha);
   if (N > P) {
-    GB_LAUNCH("zero_tail_cols", s,
-              zero_cols_from_kernel<<<cdiv((long long)N * (N - P), 256), 256, 0, s>>>(elag, N, P));
+    GB_LAUNCH_CHAIN("zero_tail_cols", s, zero_cols_from_kernel, dim3(cdiv((long long)N * (N - P), 256)), dim3(256), 0,
+                    elag, N, P);
   }
   return GB_OK;
 }

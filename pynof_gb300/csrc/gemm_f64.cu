@@ -81,6 +81,7 @@ struct TileLoader {
 
 template <bool AK, bool BKF>
 __global__ void __launch_bounds__(THREADS) gemm_f64_kernel(const GemmF64 g) {
+  chain_wait();
   __shared__ double As[2][BKT][BM + PAD];
   __shared__ double Bs[2][BKT][BN + PAD];
 
@@ -187,6 +188,7 @@ __global__ void __launch_bounds__(THREADS) gemm_f64_kernel(const GemmF64 g) {
 // blocks spread it over the whole GPU.
 template <int UNR>
 __global__ void __launch_bounds__(32) gemm_f64_small_kernel(const GemmF64 g) {
+  chain_wait();
   if (g.only_if && *g.only_if == 0) return;
   const int lane = threadIdx.x;
   const int m0 = blockIdx.y * 8, n0 = blockIdx.x * 8;
@@ -255,18 +257,18 @@ int gemm_f64(const GemmF64& g, cudaStream_t stream) {
   if (gx * gy * g.batch < 152 && g.M <= 65535 * 8) {
     // fewer 64 x 64 tiles than SMs: spread 8 x 8 blocks over the GPU instead
     const dim3 sgrid((unsigned)((g.N + 7) / 8), (unsigned)((g.M + 7) / 8), (unsigned)g.batch);
-    GB_LAUNCH(g.tag, stream, gemm_f64_small_kernel<4><<<sgrid, 32, 0, stream>>>(g));
+    GB_LAUNCH_CHAIN(g.tag, stream, gemm_f64_small_kernel<4>, dim3(sgrid), dim3(32), 0, g);
     return GB_OK;
   }
   dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)g.batch);
   if (g.a_kfast && g.b_kfast)
-    GB_LAUNCH(g.tag, stream, gemm_f64_kernel<true, true><<<grid, THREADS, 0, stream>>>(g));
+    GB_LAUNCH_CHAIN(g.tag, stream, (gemm_f64_kernel<true, true>), dim3(grid), dim3(THREADS), 0, g);
   else if (g.a_kfast)
-    GB_LAUNCH(g.tag, stream, gemm_f64_kernel<true, false><<<grid, THREADS, 0, stream>>>(g));
+    GB_LAUNCH_CHAIN(g.tag, stream, (gemm_f64_kernel<true, false>), dim3(grid), dim3(THREADS), 0, g);
   else if (g.b_kfast)
-    GB_LAUNCH(g.tag, stream, gemm_f64_kernel<false, true><<<grid, THREADS, 0, stream>>>(g));
+    GB_LAUNCH_CHAIN(g.tag, stream, (gemm_f64_kernel<false, true>), dim3(grid), dim3(THREADS), 0, g);
   else
-    GB_LAUNCH(g.tag, stream, gemm_f64_kernel<false, false><<<grid, THREADS, 0, stream>>>(g));
+    GB_LAUNCH_CHAIN(g.tag, stream, (gemm_f64_kernel<false, false>), dim3(grid), dim3(THREADS), 0, g);
   return GB_OK;
 }
 

@@ -813,7 +813,6 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-
   int gkb_issued = 0;  // stages the producer handled, all tiles (its lane 0)
   if (warp == 0) {
     // ---------------- producer ----------------
@@ -1163,6 +1162,7 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
 template <int CODE, int BN, bool FD>
 __global__ void __maxnreg__(MAX_REGS) ozaki_persistent_kernel(const __grid_constant__ KArgs a, int ntiles) {
   extern __shared__ unsigned char smem_raw[];
+  chain_wait();
   if (*(volatile int*)&g_tc_status != 0) return;
   cta_persistent<CODE, BN, false, FD>(a, nullptr, nullptr, 1, ntiles, a.g.tile_counter, smem_raw);
 }
@@ -1175,12 +1175,14 @@ __global__ void __maxnreg__(MAX_REGS)
     ozaki_persistent_grouped_kernel(const KArgs* __restrict__ probs, const long long* __restrict__ starts, int nprob,
                                     int ntiles, unsigned int* counter) {
   extern __shared__ unsigned char smem_raw[];
+  chain_wait();
   if (*(volatile int*)&g_tc_status != 0) return;
   cta_persistent<CODE, BN, true, FD>(probs[0], probs, starts, nprob, ntiles, counter, smem_raw);
 }
 
 template <int CODE, int BN>
 __global__ void __maxnreg__(MAX_REGS) ozaki_kernel(const __grid_constant__ KArgs a) {
+  chain_wait();
   extern __shared__ unsigned char smem_raw[];
   // a CTA of this or an earlier launch gave up: do not start (the host sees the status word)
   if (*(volatile int*)&g_tc_status != 0) return;
@@ -1193,6 +1195,7 @@ __global__ void __maxnreg__(MAX_REGS) ozaki_kernel(const __grid_constant__ KArgs
 template <int CODE, int BN>
 __global__ void __maxnreg__(MAX_REGS)
     ozaki_grouped_kernel(const KArgs* __restrict__ probs, const long long* __restrict__ starts, int nprob) {
+  chain_wait();
   extern __shared__ unsigned char smem_raw[];
   if (*(volatile int*)&g_tc_status != 0) return;
   const long long t = (long long)blockIdx.x + (long long)blockIdx.y * gridDim.x;
@@ -1412,12 +1415,22 @@ int ozaki_gemm(const SlicedDesc& A, const SlicedDesc& B, const OzGemm& g, cudaSt
       kp.g.tile_counter = nullptr;  // one tile per CTA, or the static walk
     }
     const int pi = prof_begin(g.tag, stream);
-    persistent_for(g.S, ka.g.fdrain)<<<(unsigned)grid, THREADS, smem_bytes(g.S, 128), stream>>>(kp, (int)tiles);
+    const cudaError_t e = launch_chain(persistent_for(g.S, ka.g.fdrain), dim3((unsigned)grid), dim3(THREADS),
+                                       smem_bytes(g.S, 128), stream, kp, (int)tiles);
     prof_end(pi, stream);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return launch_error(g.tag, e, g.S, g.bn);
+    }
   } else {
     const int pi = prof_begin(g.tag, stream);
-    kernel_for(g.S, g.bn)<<<grid_for(tiles), THREADS, smem_bytes(g.S, g.bn), stream>>>(ka);
+    const cudaError_t e =
+        launch_chain(kernel_for(g.S, g.bn), grid_for(tiles), dim3(THREADS), smem_bytes(g.S, g.bn), stream, ka);
     prof_end(pi, stream);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return launch_error(g.tag, e, g.S, g.bn);
+    }
   }
   const cudaError_t le = cudaGetLastError();
   if (le != cudaSuccess) return launch_error(g.tag, le, g.S, g.bn);

@@ -42,6 +42,19 @@ void prof_end(int idx, cudaStream_t s) {
   if (idx < (int)g_recs.size()) cudaEventRecord(g_recs[idx].b, s);
 }
 
+int launch_chain_attr(cudaStream_t s, cudaLaunchAttribute* attr) {
+  if (g_on.load(std::memory_order_relaxed)) return 0;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  if (st != cudaStreamCaptureStatusNone) return 0;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  return 1;
+}
+
 }  // namespace gb
 
 extern "C" int gb_profile_start(void) {

@@ -12,6 +12,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 __global__ void contract_diag_kernel(const double* __restrict__ C, const double* __restrict__ T,
                                      double* __restrict__ d, int N, int P, int Q) {
+  chain_wait();
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   const int q = blockIdx.y;
   if (l >= Q) return;
@@ -29,9 +30,14 @@ __global__ void contract_diag_kernel(const double* __restrict__ C, const double*
 // every 32 n.
 // A NaN or an infinity in T (exponent field 0x7FF) is reported in the status
 // word, as the slicer does for the rows it measures.
+// Two rows of T are loaded before either is used: 783 us against 869 at nbf=600
+// (FP64 arithmetic alone ~790), 62 against 73 at nbf=171; with eight it was 1054
+// and 57.
 __global__ void contract_diag_exps_kernel(const double* __restrict__ C, const double* __restrict__ T,
                                           double* __restrict__ d, int* __restrict__ texps, int N, int P, int Q,
                                           int* status) {
+  constexpr int U = 2;
+  chain_wait();
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   const int q = blockIdx.y;
   const int lane = threadIdx.x & 31;
@@ -42,13 +48,22 @@ __global__ void contract_diag_exps_kernel(const double* __restrict__ C, const do
   unsigned int mine = 0;  // exponent field maximum of row n0 + lane
   for (int n0 = 0; n0 < N; n0 += 32) {
     const int nn = min(32, N - n0);
-    for (int j = 0; j < nn; ++j) {
-      const int n = n0 + j;
-      const double t = in ? __ldg(Tq + (long long)n * Q) : 0.0;
-      acc = fma(__ldg(C + (long long)n * N + q), t, acc);
-      const unsigned int ex = (unsigned int)((unsigned long long)__double_as_longlong(t) >> 52) & 0x7FFu;
-      const unsigned int mx = __reduce_max_sync(0xffffffffu, ex);
-      if (lane == j) mine = mx;
+    for (int j0 = 0; j0 < nn; j0 += U) {
+      double t[U], c[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int n = n0 + j0 + u;
+        const bool ok = n < N;
+        t[u] = in && ok ? __ldg(Tq + (long long)n * Q) : 0.0;
+        c[u] = ok ? __ldg(C + (long long)n * N + q) : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (j0 + u < nn) acc = fma(c[u], t[u], acc);
+        const unsigned int ex = (unsigned int)((unsigned long long)__double_as_longlong(t[u]) >> 52) & 0x7FFu;
+        const unsigned int mx = __reduce_max_sync(0xffffffffu, ex);
+        if (lane == j0 + u) mine = mx;
+      }
     }
     if (lane < nn) {
       atomicMax(eq + n0 + lane, (int)(mine > 1u ? mine : 1u) - 1022);
@@ -60,6 +75,7 @@ __global__ void contract_diag_exps_kernel(const double* __restrict__ C, const do
 
 __global__ void gather_diag_kernel(const double* __restrict__ src, double* __restrict__ d, int Q,
                                    long long stride_pp) {
+  chain_wait();
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   const int p = blockIdx.y;
   if (l < Q) d[(long long)p * Q + l] = src[(long long)p * stride_pp + l];
@@ -68,6 +84,7 @@ __global__ void gather_diag_kernel(const double* __restrict__ src, double* __res
 // one warp per row
 __global__ void row_sumsq_kernel(const double* __restrict__ src, double* __restrict__ out, long long rows,
                                  int Q) {
+  chain_wait();
   const long long r = (long long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (r >= rows) return;
@@ -83,6 +100,7 @@ __global__ void row_sumsq_kernel(const double* __restrict__ src, double* __restr
 
 __global__ void col_dot_kernel(const double* __restrict__ C, int ldc, const double* __restrict__ X, int ldx,
                                double* __restrict__ out, int N, int P) {
+  chain_wait();
   const int p = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (p >= P) return;
@@ -93,6 +111,7 @@ __global__ void col_dot_kernel(const double* __restrict__ C, int ldc, const doub
 }
 
 __global__ void copy_zero_diag_kernel(const double* __restrict__ src, double* __restrict__ dst, int P) {
+  chain_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long long)P * P) return;
   const int r = (int)(i / P), c = (int)(i % P);
@@ -101,6 +120,7 @@ __global__ void copy_zero_diag_kernel(const double* __restrict__ src, double* __
 
 __global__ void add_scaled_rows_kernel(double* __restrict__ w, const double* __restrict__ d,
                                        const double* __restrict__ n, int P, int Q, int nbeta, int nalpha) {
+  chain_wait();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
   if (k >= Q) return;
@@ -112,6 +132,7 @@ __global__ void add_scaled_rows_kernel(double* __restrict__ w, const double* __r
 
 __global__ void make_ck_weighted_kernel(const double* __restrict__ bMO, const double* __restrict__ ck12,
                                         double* __restrict__ Y, int P, int Q) {
+  chain_wait();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   const int q = blockIdx.y;
   const int b = blockIdx.z;
@@ -125,6 +146,7 @@ __global__ void make_ck_weighted_kernel(const double* __restrict__ bMO, const do
 __global__ void lagrange2_finish_kernel(const double* __restrict__ bMO, const double* __restrict__ w,
                                         const double* __restrict__ Hmat, const double* __restrict__ n,
                                         double* __restrict__ elag, int N, int P, int Q) {
+  chain_wait();
   const long long pair = (long long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (pair >= (long long)N * P) return;
@@ -147,6 +169,7 @@ __global__ void lagrange2_finish_kernel(const double* __restrict__ bMO, const do
 // (16-byte accesses when Q is even).
 __global__ void make_exchange_operand_kernel(const double* __restrict__ bMO, const double* __restrict__ ck12,
                                              const double* __restrict__ w, double* __restrict__ Y, int P, int Q) {
+  chain_wait();
   const long long rows = (long long)P * P;
   const int half = Q >> 1;
   const bool even = (Q & 1) == 0;
@@ -170,6 +193,7 @@ __global__ void make_exchange_operand_kernel(const double* __restrict__ bMO, con
 // elag[a][b] += n[b] Hmat[a][b] for b < P; elag[a][b] = 0 for b >= P
 __global__ void lagrange2_hterm_kernel(const double* __restrict__ Hmat, const double* __restrict__ n,
                                        double* __restrict__ elag, int N, int P) {
+  chain_wait();
   const long long total = (long long)N * N;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -179,6 +203,7 @@ __global__ void lagrange2_hterm_kernel(const double* __restrict__ Hmat, const do
 }
 
 __global__ void zero_tail_cols_kernel(double* __restrict__ elag, int N, int P) {
+  chain_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int W = N - P;
   if (i >= (long long)N * W) return;
@@ -196,45 +221,49 @@ int launch_contract_diag(const double* C, const double* T, double* d, int N, int
     // every entry below any exponent folded in (0x80808080 < -1021), and below
     // any norm's bits
     GB_TRY(cuda_status(cudaMemsetAsync(texps, 0x80, sizeof(int) * texps_ints, s), "contract_diag exponents"));
-    GB_LAUNCH("contract_diag", s,
-              contract_diag_exps_kernel<<<dim3(cdiv(Q, 128), P), 128, 0, s>>>(C, T, d, texps, N, P, Q,
-                                                                               device_status_word()));
+    GB_LAUNCH_CHAIN("contract_diag", s, contract_diag_exps_kernel, dim3(cdiv(Q, 128), P), dim3(128), 0, C, T, d, texps,
+                    N, P, Q, device_status_word());
     return GB_OK;
   }
-  GB_LAUNCH("contract_diag", s, contract_diag_kernel<<<dim3(cdiv(Q, 128), P), 128, 0, s>>>(C, T, d, N, P, Q));
+  GB_LAUNCH_CHAIN("contract_diag", s, contract_diag_kernel, dim3(dim3(cdiv(Q, 128), P)), dim3(128), 0, C, T, d, N, P,
+                  Q);
   return GB_OK;
 }
 
 int launch_gather_diag(const double* src, double* d, int P, int Q, long long stride_pp, cudaStream_t s) {
-  GB_LAUNCH("gather_diag", s, gather_diag_kernel<<<dim3(cdiv(Q, 128), P), 128, 0, s>>>(src, d, Q, stride_pp));
+  GB_LAUNCH_CHAIN("gather_diag", s, gather_diag_kernel, dim3(dim3(cdiv(Q, 128), P)), dim3(128), 0, src, d, Q,
+                  stride_pp);
   return GB_OK;
 }
 
 int launch_row_sumsq(const double* src, double* out, long long rows, int Q, cudaStream_t s) {
   if (rows <= 0) return GB_OK;
-  GB_LAUNCH("row_sumsq", s, row_sumsq_kernel<<<cdiv(rows, 8), 256, 0, s>>>(src, out, rows, Q));
+  GB_LAUNCH_CHAIN("row_sumsq", s, row_sumsq_kernel, dim3(cdiv(rows, 8)), dim3(256), 0, src, out, rows, Q);
   return GB_OK;
 }
 
 int launch_col_dot(const double* C, int ldc, const double* X, int ldx, double* out, int N, int P,
                    cudaStream_t s) {
-  GB_LAUNCH("col_dot", s, col_dot_kernel<<<cdiv(P, 8), 256, 0, s>>>(C, ldc, X, ldx, out, N, P));
+  GB_LAUNCH_CHAIN("col_dot", s, col_dot_kernel, dim3(cdiv(P, 8)), dim3(256), 0, C, ldc, X, ldx, out, N, P);
   return GB_OK;
 }
 
 int launch_copy_zero_diag(const double* src, double* dst, int P, cudaStream_t s) {
-  GB_LAUNCH("copy_zero_diag", s, copy_zero_diag_kernel<<<cdiv((long long)P * P, 256), 256, 0, s>>>(src, dst, P));
+  GB_LAUNCH_CHAIN("copy_zero_diag", s, copy_zero_diag_kernel, dim3(cdiv((long long)P * P, 256)), dim3(256), 0, src,
+                  dst, P);
   return GB_OK;
 }
 
 int launch_add_scaled_rows(double* w, const double* d, const double* n, int P, int Q, int nbeta, int nalpha,
                            cudaStream_t s) {
-  GB_LAUNCH("add_scaled_rows", s, add_scaled_rows_kernel<<<dim3(cdiv(Q, 128), P), 128, 0, s>>>(w, d, n, P, Q, nbeta, nalpha));
+  GB_LAUNCH_CHAIN("add_scaled_rows", s, add_scaled_rows_kernel, dim3(dim3(cdiv(Q, 128), P)), dim3(128), 0, w, d, n, P,
+                  Q, nbeta, nalpha);
   return GB_OK;
 }
 
 int launch_make_ck_weighted(const double* bMO, const double* ck12, double* Y, int P, int Q, cudaStream_t s) {
-  GB_LAUNCH("make_ck_weighted", s, make_ck_weighted_kernel<<<dim3(cdiv(Q, 128), P, P), 128, 0, s>>>(bMO, ck12, Y, P, Q));
+  GB_LAUNCH_CHAIN("make_ck_weighted", s, make_ck_weighted_kernel, dim3(dim3(cdiv(Q, 128), P, P)), dim3(128), 0, bMO,
+                  ck12, Y, P, Q);
   return GB_OK;
 }
 
@@ -243,8 +272,8 @@ int launch_make_exchange_operand(const double* bMO, const double* ck12, const do
   const long long rows = (long long)P * P;
   if (rows == 0 || Q == 0) return GB_OK;
   const unsigned grid = (unsigned)(rows < 152LL * 16 ? rows : 152LL * 16);
-  GB_LAUNCH("make_exchange_operand", s,
-            make_exchange_operand_kernel<<<grid, 256, 0, s>>>(bMO, ck12, w, Y, P, Q));
+  GB_LAUNCH_CHAIN("make_exchange_operand", s, make_exchange_operand_kernel, dim3(grid), dim3(256), 0, bMO, ck12, w, Y,
+                  P, Q);
   return GB_OK;
 }
 
@@ -252,15 +281,17 @@ int launch_lagrange2_hterm(const double* Hmat, const double* n, double* elag, in
   const long long total = (long long)N * N;
   if (total == 0) return GB_OK;
   const unsigned grid = (unsigned)(cdiv(total, 256) < 152u * 8 ? cdiv(total, 256) : 152u * 8);
-  GB_LAUNCH("lagrange2_hterm", s, lagrange2_hterm_kernel<<<grid, 256, 0, s>>>(Hmat, n, elag, N, P));
+  GB_LAUNCH_CHAIN("lagrange2_hterm", s, lagrange2_hterm_kernel, dim3(grid), dim3(256), 0, Hmat, n, elag, N, P);
   return GB_OK;
 }
 
 int launch_lagrange2_finish(const double* bMO, const double* w, const double* Hmat, const double* n,
                             double* elag, int N, int P, int Q, cudaStream_t s) {
-  GB_LAUNCH("lagrange2_finish", s, lagrange2_finish_kernel<<<cdiv((long long)N * P, 8), 256, 0, s>>>(bMO, w, Hmat, n, elag, N, P, Q));
+  GB_LAUNCH_CHAIN("lagrange2_finish", s, lagrange2_finish_kernel, dim3(cdiv((long long)N * P, 8)), dim3(256), 0, bMO,
+                  w, Hmat, n, elag, N, P, Q);
   if (N > P) {
-    GB_LAUNCH("zero_tail_cols", s, zero_tail_cols_kernel<<<cdiv((long long)N * (N - P), 256), 256, 0, s>>>(elag, N, P));
+    GB_LAUNCH_CHAIN("zero_tail_cols", s, zero_tail_cols_kernel, dim3(cdiv((long long)N * (N - P), 256)), dim3(256), 0,
+                    elag, N, P);
   }
   return GB_OK;
 }

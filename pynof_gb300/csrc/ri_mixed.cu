@@ -476,6 +476,7 @@ int exchange_splits(int N, int P, int Q) {
 
 // out[i] = sum_s part[s][i], i < n
 __global__ void sum_splits_kernel(const double* __restrict__ part, int ns, long long n, double* __restrict__ out) {
+  chain_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double v = 0.0;
@@ -594,8 +595,8 @@ int lagrange2_mixed_body(const double* C, const double* H, const void* prep, con
   GB_TRY(ozaki_gemm(w.Sx, w.Sy, ge, s));
   if (w.ns > 1) {
     const long long np = (long long)N * P;
-    GB_LAUNCH("sum_splits", s,
-              sum_splits_kernel<<<(unsigned)((np + 127) / 128), 128, 0, s>>>(w.part, w.ns, np, w.Z));
+    GB_LAUNCH_CHAIN("sum_splits", s, sum_splits_kernel, dim3((unsigned)((np + 127) / 128)), dim3(128), 0, w.part,
+                    w.ns, np, w.Z);
   }
   // elag[a][b] = -sum_m C[m][a] Z[m][b] (b < nbf5), then the n_b Hmat term; rows b are the unit stride
   GB_TRY(slice_operand(SliceSrc{C, 0, lin(1), lin(N), false}, w.Ct, s));

@@ -22,6 +22,7 @@ constexpr int TAYLOR_DEG = 16;
 
 // Y[i][j] from the packed step: +y for i < j (i < P), -y for i > j (j < P).
 __global__ void build_antisym_kernel(const double* __restrict__ y, int N, int P, double* __restrict__ Y) {
+  chain_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)N * N) return;
   const int i = (int)(idx / N), j = (int)(idx % N);
@@ -50,6 +51,7 @@ __global__ void poly_block_kernel(double* __restrict__ dst, const double* __rest
                                   const double* __restrict__ X2, const double* __restrict__ X3,
                                   const double* __restrict__ X4, int N, double c0, double c1, double c2, double c3,
                                   double c4) {
+  chain_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)N * N) return;
   const int i = (int)(idx / N), j = (int)(idx % N);
@@ -62,6 +64,7 @@ __global__ void poly_block_kernel(double* __restrict__ dst, const double* __rest
 }
 
 __global__ void scale_kernel(const double* __restrict__ src, double* __restrict__ dst, long long n, double f) {
+  chain_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx < n) dst[idx] = src[idx] * f;
 }
@@ -120,7 +123,7 @@ extern "C" int gb_rotate_orbital_f64(const double* y, const double* C, int nbf, 
   double *Y = buf[0], *X2 = buf[1], *X3 = buf[2], *X4 = buf[3], *R0 = buf[4], *R1 = buf[5];
   const long long NN = (long long)N * N;
 
-  GB_LAUNCH("rotate_build", s, build_antisym_kernel<<<cdiv(NN, 256), 256, 0, s>>>(y, N, P, Y));
+  GB_LAUNCH_CHAIN("rotate_build", s, build_antisym_kernel, dim3(cdiv(NN, 256)), dim3(256), 0, y, N, P, Y);
   double norm = norm1;
   if (!(norm1 >= 0.0)) {
     // no bound from the caller: measure ||Y||_1 on the device (one synchronisation)
@@ -140,7 +143,8 @@ extern "C" int gb_rotate_orbital_f64(const double* y, const double* C, int nbf, 
   }
   // X = Y / 2^sq in place
   if (sq > 0)
-    GB_LAUNCH("rotate_scale", s, scale_kernel<<<cdiv(NN, 256), 256, 0, s>>>(Y, Y, NN, std::ldexp(1.0, -sq)));
+    GB_LAUNCH_CHAIN("rotate_scale", s, scale_kernel, dim3(cdiv(NN, 256)), dim3(256), 0, Y, Y, NN, std::ldexp(1.0,
+                    -sq));
   const double* X = Y;
   double c[TAYLOR_DEG + 1];
   c[0] = 1.0;
@@ -149,15 +153,13 @@ extern "C" int gb_rotate_orbital_f64(const double* y, const double* C, int nbf, 
   GB_TRY(matmul(X2, X, X3, N, false, tw, s, "gemm_f64:expm"));
   GB_TRY(matmul(X2, X2, X4, N, false, tw, s, "gemm_f64:expm"));
   // R = B3 + c16 X^4
-  GB_LAUNCH("rotate_poly", s,
-            poly_block_kernel<<<cdiv(NN, 256), 256, 0, s>>>(R0, X, X2, X3, X4, N, c[12], c[13], c[14], c[15],
-                                                              c[16]));
+  GB_LAUNCH_CHAIN("rotate_poly", s, poly_block_kernel, dim3(cdiv(NN, 256)), dim3(256), 0, R0, X, X2, X3, X4, N, c[12],
+                  c[13], c[14], c[15], c[16]);
   double *R = R0, *Rn = R1;
   for (int j = 2; j >= 0; --j) {
     // Rn = Bj + X^4 R
-    GB_LAUNCH("rotate_poly", s,
-              poly_block_kernel<<<cdiv(NN, 256), 256, 0, s>>>(Rn, X, X2, X3, nullptr, N, c[4 * j], c[4 * j + 1],
-                                                                c[4 * j + 2], c[4 * j + 3], 0.0));
+    GB_LAUNCH_CHAIN("rotate_poly", s, poly_block_kernel, dim3(cdiv(NN, 256)), dim3(256), 0, Rn, X, X2, X3, nullptr, N,
+                    c[4 * j], c[4 * j + 1], c[4 * j + 2], c[4 * j + 3], 0.0);
     GB_TRY(matmul(X4, R, Rn, N, true, tw, s, "gemm_f64:expm"));
     double* t = R;
     R = Rn;

@@ -80,6 +80,7 @@ __device__ __forceinline__ void clear_norms(int* norms, long long b, long long r
 // explicit loads in flight here and below: 430 us of 285.)
 __global__ void rowexp_kfast_kernel(SliceSrc src, int rows, int K, int* __restrict__ exps, int* __restrict__ norms,
                                     int* status) {
+  chain_wait();
   const long long b = blockIdx.y;
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -119,6 +120,7 @@ __global__ void rowexp_kfast_kernel(SliceSrc src, int rows, int K, int* __restri
 // rows of 180000 took 0.6 ms on 300 warps): every warp folds its range's
 // exponent in with atomicMax; exps and norms are preset below any value.
 __global__ void rowexp_kfast_split_kernel(SliceSrc src, int rows, int K, int* __restrict__ exps, int* status) {
+  chain_wait();
   const long long b = blockIdx.y;
   const long long row = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -148,6 +150,7 @@ __global__ void rowexp_kfast_split_kernel(SliceSrc src, int rows, int K, int* __
 __global__ void __launch_bounds__(256) rowexp_rfast_kernel(SliceSrc src, int rows, int K, int* __restrict__ exps,
                                                            int* __restrict__ norms, int* status) {
   __shared__ unsigned long long part[8][32];
+  chain_wait();
   const long long b = blockIdx.y;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long long row = (long long)blockIdx.x * 32 + lane;
@@ -219,24 +222,34 @@ __device__ __forceinline__ void store_group(const double (&xs)[8], int e, unsign
     *reinterpret_cast<uint4*>(out + s * SL_SLICE_STEP) = make_uint4(pk[s][0], pk[s][1], pk[s][2], pk[s][3]);
 }
 
-// One CTA of 256 threads per (row block, run of SL_KPC consecutive k blocks):
-// thread -> (row r, k group of 8).  Lanes 0..7 take consecutive rows of one
-// core matrix and a warp covers 32 consecutive rows of one k group, i.e. four
-// whole consecutive core matrices (512 contiguous bytes) per slice, written
-// with 16-byte stores; it reads 64 contiguous source bytes per row and k block
-// (K-fast sources: the run reads SL_KPC x 128 contiguous bytes of each row) or
-// 256 contiguous bytes per k (row-fast sources).  At most 64 registers (four
-// CTAs per SM): occupancy keeps more loads in flight than prefetching the next
-// k block into registers did (measured: 1.62 ms against 1.87-1.93 ms for the
-// T of one nbf=600 build, 8.64 GB).
+// One CTA of G 256-thread groups per (row block, kpc consecutive k blocks, a run
+// of the norms); group g takes the run's k blocks g, g + G, ..: thread -> (row r, k group
+// of 8).  Lanes 0..7 take consecutive rows of one core matrix and a warp covers 32
+// consecutive rows of one k group, i.e. four whole consecutive core matrices (512
+// contiguous bytes) per slice, written with 16-byte stores; it reads 64
+// contiguous source bytes per row and k block (K-fast sources: the run reads
+// SL_KPC x 128 contiguous bytes of each row) or 256 contiguous bytes per k
+// (row-fast sources).  At most 64 registers (four CTAs per SM): occupancy keeps
+// more loads in flight than prefetching the next k block into registers did
+// (measured: 1.62 ms against 1.87-1.93 ms for the T of one nbf=600 build, 8.64 GB).
+// Where the grid has fewer CTAs than two per SM (a thread's k blocks follow each
+// other, ~1 us each): a CTA per k block for K up to one run (its norms times the
+// eight blocks of a run bound the run's), G = 4 for longer ones, whose chunks need
+// the tighter norms (half transform at nbf=600 6.20 ms, 6.89 with the looser).
+// Three slicings of an nbf=24 build: 41 us with runs of eight, 33 with G = 4, 20.
 template <int S, int W>
-__global__ void __launch_bounds__(256, S == 7 ? 3 : 4) digits_blocked_kernel(SliceSrc src, SlicedDesc dst) {
+__global__ void __launch_bounds__(S == 7 ? 256 : 1024, S == 7 ? 3 : 1) digits_blocked_kernel(SliceSrc src, SlicedDesc dst,
+                                                                                                   int kpc) {
+  constexpr int ND = W != 9 ? 0 : S == 7 ? SL_NORMS : 3;  // digits with norms
+  __shared__ float s_nq[S == 7 || W != 9 ? 1 : 3 * 256 * 3];
+  chain_wait();
   const long long b = blockIdx.y;
   const int kbn = dst.kblocks();
-  const int runs = (kbn + SL_KPC - 1) / SL_KPC;
-  const int rb = blockIdx.x / runs, kb0 = (blockIdx.x % runs) * SL_KPC;
-  const int kb1 = min(kb0 + SL_KPC, kbn);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int runs = (kbn + kpc - 1) / kpc;
+  const int rb = blockIdx.x / runs, kb0 = (blockIdx.x % runs) * kpc;
+  const int kb1 = min(kb0 + kpc, kbn);
+  const int G = blockDim.x >> 8, grp = threadIdx.x >> 8;
+  const int warp = (threadIdx.x >> 5) & 7, lane = threadIdx.x & 31;
   const int ri = lane & 7, kg = warp >> 2, rg = (warp & 3) * 4 + (lane >> 3);
   const int r = rb * SL_ROWS + rg * 8 + ri;
   const bool rok = r < dst.rows;
@@ -246,16 +259,29 @@ __global__ void __launch_bounds__(256, S == 7 ? 3 : 4) digits_blocked_kernel(Sli
                         ((long long)rb * kbn * S) * SL_TILE_BYTES + (kg * S * 16 + rg) * 128 + ri * 16;
   double xa[8];
   float nq[SL_NORMS] = {};
-  for (int kb = kb0; kb < kb1; ++kb) {
+  for (int kb = kb0 + grp; kb < kb1; kb += G) {
     load_group(src, base, rok, kb * SL_K + kg * 8, dst.K, xa);
     store_group<S, W>(xa, e, out0 + (long long)kb * S * SL_TILE_BYTES, nq);
+  }
+  if (S != 7 && ND > 0 && G > 1) {
+    // the run's sums of squares over the groups
+    const int t = threadIdx.x & 255;
+    if (grp > 0)
+#pragma unroll
+      for (int s = 0; s < ND; ++s) s_nq[((grp - 1) * ND + s) * 256 + t] = nq[s];
+    __syncthreads();
+    if (grp > 0) return;
+    for (int g = 0; g < G - 1; ++g)
+#pragma unroll
+      for (int s = 0; s < ND; ++s) nq[s] += s_nq[(g * ND + s) * 256 + t];
   }
   if constexpr (W == 9) {
     // non-negative floats order as their bits
     int* nb = dst.norms + (b * dst.rblocks() + rb) * SL_NORMS;
 #pragma unroll
-    for (int s = 0; s < (S == 7 ? SL_NORMS : 3); ++s) {
-      const float scale = __int_as_float((127 + 2 * digit_exp(W, s + 1)) << 23);  // back to squares of the digits
+    for (int s = 0; s < ND; ++s) {
+      // back to squares of the digits, for a whole run
+      const float scale = __int_as_float((127 + 2 * digit_exp(W, s + 1)) << 23) * (float)(SL_KPC / kpc);
       const unsigned int mx = __reduce_max_sync(0xffffffffu, __float_as_uint(nq[s] * scale));
       if (lane == 0) atomicMax(nb + s, (int)mx);
     }
@@ -309,6 +335,7 @@ __device__ __forceinline__ void tf32_split(double x, int E, uint32_t& hi, uint32
 // -> (row r, k group of 4), 16-byte stores per plane (same thread map as the
 // bf16 digits).
 __global__ void __launch_bounds__(256) tf32_blocked_kernel(SliceSrc src, SlicedDesc dst) {
+  chain_wait();
   const long long b = blockIdx.y;
   const int kbn = dst.kblocks();
   const int rb = blockIdx.x / kbn, kb = blockIdx.x % kbn;
@@ -355,39 +382,41 @@ int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bo
     z = z < dst.K / 2048 ? z : dst.K / 2048;
     GB_TRY(cuda_status(cudaMemsetAsync(dst.exps, 0x80, sizeof(int) * sliced_meta_ints(dst.batch, dst.rows), s),
                        "slice_operand: exponents"));
-    GB_LAUNCH("slice_rowexp", s,
-              rowexp_kfast_split_kernel<<<dim3(cdiv(dst.rows, 8), dst.batch, (unsigned)z), 256, 0, s>>>(
-                  src, dst.rows, dst.K, dst.exps, st));
+    GB_LAUNCH_CHAIN("slice_rowexp", s, rowexp_kfast_split_kernel, dim3(dim3(cdiv(dst.rows, 8), dst.batch,
+                    (unsigned)z)), dim3(256), 0,  src, dst.rows, dst.K, dst.exps, st);
   } else if (src.kfast) {
-    GB_LAUNCH("slice_rowexp", s,
-              rowexp_kfast_kernel<<<dim3(cdiv(dst.rows, 8), dst.batch), 256, 0, s>>>(src, dst.rows, dst.K, dst.exps,
-                                                                                    norms, st));
+    GB_LAUNCH_CHAIN("slice_rowexp", s, rowexp_kfast_kernel, dim3(cdiv(dst.rows, 8), dst.batch), dim3(256), 0, src,
+                    dst.rows, dst.K, dst.exps, norms, st);
   } else {
-    GB_LAUNCH("slice_rowexp", s,
-              rowexp_rfast_kernel<<<dim3(cdiv(dst.rows, 32), dst.batch), 256, 0, s>>>(src, dst.rows, dst.K, dst.exps,
-                                                                                     norms, st));
+    GB_LAUNCH_CHAIN("slice_rowexp", s, rowexp_rfast_kernel, dim3(cdiv(dst.rows, 32), dst.batch), dim3(256), 0, src,
+                    dst.rows, dst.K, dst.exps, norms, st);
   }
   const long long blocks = (long long)dst.rblocks() * dst.kblocks();
   GB_REQUIRE(blocks <= 2147483647LL, GB_ERR_BAD_SHAPE, "slice_operand: too many blocks");
   if (dst.kind == 1) {
-    GB_LAUNCH("slice_tf32", s, tf32_blocked_kernel<<<dim3((unsigned)blocks, dst.batch), 256, 0, s>>>(src, dst));
+    GB_LAUNCH_CHAIN("slice_tf32", s, tf32_blocked_kernel, dim3(dim3((unsigned)blocks, dst.batch)), dim3(256), 0, src,
+                    dst);
     return GB_OK;
   }
-  const dim3 grid((unsigned)((long long)dst.rblocks() * ((dst.kblocks() + SL_KPC - 1) / SL_KPC)), dst.batch);
+  const long long runs = (dst.kblocks() + SL_KPC - 1) / SL_KPC;
+  const bool few = (long long)dst.rblocks() * runs * dst.batch < 304;
+  const int kpc = few && runs == 1 ? 1 : SL_KPC;
+  const dim3 grid((unsigned)((long long)dst.rblocks() * ((dst.kblocks() + kpc - 1) / kpc)), dst.batch);
+  const dim3 block(few && runs > 1 && dst.S != 7 ? 1024 : 256);
   if (dst.W == 9) {
     GB_REQUIRE(dst.S == 5 || dst.S == 7, GB_ERR_INVALID_ARG, "slice_operand: nine-bit digits come in five or seven planes");
     if (dst.S == 5)
-      GB_LAUNCH("slice_digits", s, digits_blocked_kernel<5, 9><<<grid, 256, 0, s>>>(src, dst));
+      GB_LAUNCH_CHAIN("slice_digits", s, (digits_blocked_kernel<5, 9>), grid, block, 0, src, dst, kpc);
     else
-      GB_LAUNCH("slice_digits7", s, digits_blocked_kernel<7, 9><<<grid, 256, 0, s>>>(src, dst));
+      GB_LAUNCH_CHAIN("slice_digits7", s, (digits_blocked_kernel<7, 9>), grid, block, 0, src, dst, kpc);
     return GB_OK;
   }
   switch (dst.S) {
-    case 1: GB_LAUNCH("slice_digits", s, digits_blocked_kernel<1, 7><<<grid, 256, 0, s>>>(src, dst)); break;
-    case 2: GB_LAUNCH("slice_digits", s, digits_blocked_kernel<2, 7><<<grid, 256, 0, s>>>(src, dst)); break;
-    case 3: GB_LAUNCH("slice_digits", s, digits_blocked_kernel<3, 7><<<grid, 256, 0, s>>>(src, dst)); break;
-    case 4: GB_LAUNCH("slice_digits", s, digits_blocked_kernel<4, 7><<<grid, 256, 0, s>>>(src, dst)); break;
-    default: GB_LAUNCH("slice_digits", s, digits_blocked_kernel<5, 7><<<grid, 256, 0, s>>>(src, dst)); break;
+    case 1: GB_LAUNCH_CHAIN("slice_digits", s, (digits_blocked_kernel<1, 7>), grid, block, 0, src, dst, kpc); break;
+    case 2: GB_LAUNCH_CHAIN("slice_digits", s, (digits_blocked_kernel<2, 7>), grid, block, 0, src, dst, kpc); break;
+    case 3: GB_LAUNCH_CHAIN("slice_digits", s, (digits_blocked_kernel<3, 7>), grid, block, 0, src, dst, kpc); break;
+    case 4: GB_LAUNCH_CHAIN("slice_digits", s, (digits_blocked_kernel<4, 7>), grid, block, 0, src, dst, kpc); break;
+    default: GB_LAUNCH_CHAIN("slice_digits", s, (digits_blocked_kernel<5, 7>), grid, block, 0, src, dst, kpc); break;
   }
   return GB_OK;
 }
