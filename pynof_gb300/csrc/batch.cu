@@ -189,12 +189,19 @@ extern "C" int gb_jkj_batch_create_mixed(int nmol, const double* const* C, const
     }));
     GB_TRY(ozaki_gemm_grouped(tabT, nmol, tilesT, S, pt[0].g.bn, s, "ozaki_tc:batch_half_transform", persT, fdT));
     GB_TRY(branches([&](int i, cudaStream_t b) {
-      GB_TRY(launch_contract_diag(C[i], ws[i].Tf, ws[i].dv, nbf[i], nbf5[i], naux[i], b));
+      // the contraction records the row exponents of T's slicing, as in the single build
+      const SlicedDesc& T = ws[i].T;
+      if (T.kind == 0)
+        GB_TRY(cuda_status(cudaMemsetAsync(T.exps, META_PRESET_BYTE, sizeof(int) * sliced_meta_ints(T.batch, T.rows), b),
+                           "batch exponents"));
+      GB_TRY(launch_contract_diag(C[i], ws[i].Tf, ws[i].dv, nbf[i], nbf5[i], naux[i], b,
+                                  T.kind == 0 ? T.exps : nullptr));
       return slice_operand(SliceSrc{ws[i].dv, 0, lin(naux[i]), lin(1), true}, ws[i].d, b);
     }));
     GB_TRY(ozaki_gemm_grouped(tabJ, nmol, tilesJ, S, pj[0].g.bn, s, "ozaki_tc:batch_J", persJ, fdJ));
     GB_TRY(branches([&](int i, cudaStream_t b) {
-      return slice_operand(SliceSrc{ws[i].Tf, (long long)nbf[i] * naux[i], lin(naux[i]), lin(1), true}, ws[i].T, b);
+      return slice_operand(SliceSrc{ws[i].Tf, (long long)nbf[i] * naux[i], lin(naux[i]), lin(1), true}, ws[i].T, b,
+                           ws[i].T.kind == 0);
     }));
     GB_TRY(ozaki_gemm_grouped(tabK, nmol, tilesK, S, 128, s, "ozaki_tc:batch_K", persK, fdK));
     return GB_OK;

@@ -44,7 +44,10 @@ struct OutF64 {
 // r -> (m, n) with m <= n (tri_pair), pair_n (pair_n + 1) / 2 of them; the
 // output at pair m * pair_n + n is written, and for n > m also its mirror
 // n * pair_n + m.
-enum SymMode { SYM_NONE = 0, SYM_ROWCOL = 1, SYM_PAIRCOL = 2, SYM_TRIROW = 4, SYM_TRICOL = 5 };
+// SYM_BATCHCOL (persistent tensor-core kernel only): the batch index and the
+// column are one symmetric pair (batch == N): columns up to the batch index are
+// computed, each also written as column `batch` of batch entry `column`.
+enum SymMode { SYM_NONE = 0, SYM_ROWCOL = 1, SYM_PAIRCOL = 2, SYM_TRIROW = 4, SYM_TRICOL = 5, SYM_BATCHCOL = 6 };
 
 // Packed upper-triangle index r = m N - m (m - 1) / 2 + (n - m), 0 <= m <= n < N,
 // back to (m, n) (rows of the triangle in order, each from its diagonal on).

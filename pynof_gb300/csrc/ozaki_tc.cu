@@ -323,7 +323,12 @@ __device__ __forceinline__ bool decode_tile(const OzGemm& g, long long t, int& b
     n0 = (int)(r % ntiles) * BN;
     m0 = (int)(r / ntiles) * BM;
   }
-  return !(g.sym == SYM_ROWCOL && m0 > n0);
+  return !(g.sym == SYM_ROWCOL && m0 > n0) && !(g.sym == SYM_BATCHCOL && n0 > bz);
+}
+
+// Columns a tile needs (from n0 on; more than BN: all).
+__device__ __forceinline__ int tile_cols(const OzGemm& g, int bz, int n0) {
+  return (g.sym == SYM_BATCHCOL && bz + 1 < g.N ? bz + 1 : g.N) - n0;
 }
 
 // One output tile, all roles.
@@ -831,7 +836,7 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
         for (;;) {
           unsigned int u;
           if (counter) {
-            u = atomicAdd(counter, 1u);
+            u = atomicAdd(counter, 1u) - a0.g.counter_start;
           } else {
             u = next;
             next += gridDim.x;
@@ -909,7 +914,7 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
         const int nkb = (g.K + BK - 1) / BK;
         int bz, m0, n0;
         decode_tile<BN>(g, t, bz, m0, n0);
-        const int n_valid = min(BN, g.N - n0);
+        const int n_valid = min(BN, tile_cols(g, bz, n0));
         const int n_mma = (n_valid + 15) & ~15;
         const uint32_t idesc = (T::IDESC & ~(0x3Fu << 17)) | ((uint32_t)(n_mma >> 3) << 17);
         const bool wide = wide_tile<BN>(n_mma);
@@ -1019,13 +1024,14 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
           const bool in = jj < g.N;
           long long mc = -1;
           if (in && g.sym == SYM_ROWCOL) mc = g.c_r.at(jj);
+          if (in && g.sym == SYM_BATCHCOL) mc = (long long)jj * g.c_sb + g.c_c.at(bz);
           e_coff[c] = in ? g.c_c.at(jj) : 0;
           e_mc[c] = mc;
           e_scol[c] = in ? a.B.exps[bbz * g.N + jj] - group_exp(W, gE) - a.frac : 0;
         }
       }
       epi_barrier_any(false);  // tables visible
-      const int n_valid = min(BN, g.N - n0);
+      const int n_valid = min(BN, tile_cols(g, bz, n0));
       const bool cols_live = cg * CW < n_valid;  // warp-uniform
       long long R[CW];
 #pragma unroll
@@ -1087,12 +1093,13 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
       }
       // convert and store from registers (rows are the output's unit stride)
       double* Cb = g.C + (long long)bz * g.c_sb;
-      const int rlim = min(BM, g.M - m0), cw = min(CW, g.N - n0 - cg * CW);  // this warp's columns
+      const int rlim = min(BM, g.M - m0), cw = min(CW, tile_cols(g, bz, n0) - cg * CW);  // this warp's columns
       if (row < rlim && cw > 0) {
         const uint32_t flip = g.negate ? 0x80000000u : 0u;
         const int c0 = cg * CW, srow = e_srow[row];
         // a mirror image: none, of an off-diagonal tile (SYM_ROWCOL; the row's
-        // columns are consecutive there), or of a pair (SYM_TRIROW)
+        // columns are consecutive there), of a pair (SYM_TRIROW), or the batch
+        // entry of each column below the batch index (SYM_BATCHCOL)
         const bool mirror_rc = g.sym == SYM_ROWCOL && m0 != n0;
         const long long ro = e_roff[row], mr = g.sym == SYM_TRIROW || mirror_rc ? e_mr[row] : -1;
         double* mir = mirror_rc ? Cb + mr + e_mc[c0] : nullptr;
@@ -1113,6 +1120,7 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
               const long long co = e_coff[c0 + j + u];
               Cb[ro + co] = v[u];
               if (mr >= 0 && !mirror_rc) Cb[mr + co] = v[u];
+              if (g.sym == SYM_BATCHCOL && n0 + c0 + j + u < bz) g.C[ro + e_mc[c0 + j + u]] = v[u];
             }
           if (mirror_rc) {
             if (vec == 4) {
@@ -1140,6 +1148,7 @@ __device__ __forceinline__ void cta_persistent(const KArgs& a0, const KArgs* __r
             Cb[ro + co] = val;
             if (mirror_rc) mir[j] = val;
             else if (mr >= 0) Cb[mr + co] = val;
+            if (g.sym == SYM_BATCHCOL && n0 + c0 + j < bz) g.C[ro + e_mc[c0 + j]] = val;
           }
         }
       }
@@ -1355,6 +1364,9 @@ int check_problem(const SlicedDesc& A, const SlicedDesc& B, const OzGemm& g) {
              "ozaki_gemm: SYM_ROWCOL needs M == N and 128-wide tiles");
   GB_REQUIRE(g.sym != SYM_PAIRCOL, GB_ERR_INVALID_ARG,
              "ozaki_gemm: pair symmetry runs over the packed pair triangle here (SYM_TRIROW / SYM_TRICOL)");
+  GB_REQUIRE(g.sym != SYM_BATCHCOL || (g.batch == g.N && g.S <= 6 && g.bn == 128 && g.c_r.div == 0 && g.c_r.s0 == 1 &&
+                                       !(g.c_c.div == 0 && g.c_c.s0 == 1)),
+             GB_ERR_BAD_SHAPE, "ozaki_gemm: SYM_BATCHCOL needs batch == N and the persistent form");
   GB_REQUIRE(g.sym != SYM_TRIROW || (long long)g.pair_n * (g.pair_n + 1) / 2 == g.M, GB_ERR_BAD_SHAPE,
              "ozaki_gemm: SYM_TRIROW needs M == pair_n (pair_n + 1) / 2");
   GB_REQUIRE(g.sym != SYM_TRICOL || (long long)g.pair_n * (g.pair_n + 1) / 2 == g.N, GB_ERR_BAD_SHAPE,
@@ -1410,7 +1422,8 @@ int ozaki_gemm(const SlicedDesc& A, const SlicedDesc& B, const OzGemm& g, cudaSt
     const long long grid = tiles < nsm ? tiles : nsm;
     KArgs kp = ka;
     if (g.tile_counter && tiles > grid) {
-      GB_TRY(cuda_status(cudaMemsetAsync(g.tile_counter, 0, sizeof(unsigned int), stream), "tile counter"));
+      if (g.counter_start == 0)
+        GB_TRY(cuda_status(cudaMemsetAsync(g.tile_counter, 0, sizeof(unsigned int), stream), "tile counter"));
     } else {
       kp.g.tile_counter = nullptr;  // one tile per CTA, or the static walk
     }

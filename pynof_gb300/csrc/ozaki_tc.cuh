@@ -43,6 +43,8 @@ struct OzGemm {
   // from which the persistent form hands out tiles in order; null = a static
   // round-robin walk.  Launches that share it must be ordered (one stream).
   unsigned int* tile_counter = nullptr;
+  // Not zero: the counter is already at this value (no memset before the launch).
+  unsigned int counter_start = 0;
   const char* tag = "ozaki_tc";
 };
 

@@ -73,6 +73,107 @@ __global__ void contract_diag_exps_kernel(const double* __restrict__ C, const do
   if (in) d[(long long)q * Q + l] = acc;
 }
 
+// Exponent E of |x| < 2^E from the exponent field (or the bits) of the largest |x|.
+__device__ __forceinline__ int field_exponent(unsigned int field) { return (int)(field > 1u ? field : 1u) - 1022; }
+__device__ __forceinline__ unsigned int exp_field(double x) {
+  return ((unsigned int)__double2hiint(x) >> 20) & 0x7FFu;
+}
+
+// A thread's l keeps its maximum over m; a warp's 32 l share one reduction per m,
+// which lands in lane m % 32 and is folded in with atomicMax every 32 m.  One read
+// of T, where two exponent passes read it twice.
+__global__ void __launch_bounds__(128) t_exponents_kernel(const double* __restrict__ T, int* __restrict__ et,
+                                                          int* __restrict__ ex, int N, int Q, int qps, int* status) {
+  constexpr int U = 4;
+  chain_wait();
+  const int l = blockIdx.x * blockDim.x + threadIdx.x;
+  const int q = blockIdx.y;
+  const int lane = threadIdx.x & 31;
+  const bool in = l < Q;  // the whole warp stays for the reductions
+  const double* Tq = T + (long long)q * N * Q + (in ? l : 0);
+  int* e = ex + (long long)(q / qps) * N;
+  unsigned int over_m = 0, mine = 0;
+  for (int m0 = 0; m0 < N; m0 += 32) {
+    const int nm = min(32, N - m0);
+    for (int j0 = 0; j0 < nm; j0 += U) {
+      double t[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) t[u] = in && j0 + u < nm ? __ldg(Tq + (long long)(m0 + j0 + u) * Q) : 0.0;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const unsigned int f = exp_field(t[u]);
+        over_m = max(over_m, f);
+        const unsigned int mx = __reduce_max_sync(0xffffffffu, f);
+        if (lane == j0 + u) mine = mx;
+      }
+    }
+    if (lane < nm) atomicMax(e + m0 + lane, field_exponent(mine));
+  }
+  if (in) {
+    et[(long long)q * Q + l] = field_exponent(over_m);
+    if (over_m == 0x7FFu && status) atomicCAS(status, 0, GB_ERR_NONFINITE);
+  }
+}
+
+// One warp per pair q <= b: the largest |bMO[b][q][l]|, whose scaled value bounds
+// both rows' operands (the product is rounded monotonically), and the square sum.
+__global__ void __launch_bounds__(256) mo_rows_kernel(const double* __restrict__ bMO, const double* __restrict__ ck12,
+                                                      const double* __restrict__ w, int* __restrict__ ey,
+                                                      double* __restrict__ K_MO, int P, int Q, int qps, int* status) {
+  chain_wait();
+  const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (r >= (long long)P * P) return;
+  const int b = (int)(r / P), q = (int)(r % P);
+  if (q > b) return;
+  const double* x = bMO + r * Q;
+  const double* y = w + (long long)b * Q;
+  double sum = 0.0;
+  unsigned long long mx = 0;
+  auto largest = [&](double v) {
+    const unsigned long long a = (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+    mx = a > mx ? a : mx;
+  };
+  // four loads and four sums in flight (an FP64 FMA's latency is 64 clocks here)
+  double part[4] = {};
+  for (int l0 = lane; l0 < Q; l0 += 128) {
+    double v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = l0 + 32 * u < Q ? __ldg(x + l0 + 32 * u) : 0.0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (K_MO) part[u] = fma(v[u], v[u], part[u]);
+      if (q < b) largest(v[u]);
+    }
+  }
+  sum = (part[0] + part[1]) + (part[2] + part[3]);
+  if (q == b)
+    for (int l = lane; l < Q; l += 32) largest(y[l]);
+  if (K_MO) sum = warp_sum(sum);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long v = __shfl_xor_sync(0xffffffffu, mx, o);
+    mx = v > mx ? v : mx;
+  }
+  if (lane != 0) return;
+  if (K_MO) {
+    K_MO[r] = sum;
+    K_MO[(long long)q * P + b] = sum;
+  }
+  auto record = [&](int row, int orb, double v) {
+    const unsigned int f = exp_field(v);
+    atomicMax(ey + (long long)(orb / qps) * P + row, field_exponent(f));
+    if (f == 0x7FFu && status) atomicCAS(status, 0, GB_ERR_NONFINITE);
+  };
+  const double m = __longlong_as_double((long long)mx);
+  if (q == b) {
+    record(b, b, m);
+  } else {
+    record(b, q, ck12[(long long)b * P + q] * m);
+    record(q, b, ck12[(long long)q * P + b] * m);
+  }
+}
+
 __global__ void gather_diag_kernel(const double* __restrict__ src, double* __restrict__ d, int Q,
                                    long long stride_pp) {
   chain_wait();
@@ -83,11 +184,14 @@ __global__ void gather_diag_kernel(const double* __restrict__ src, double* __res
 
 // one warp per row
 __global__ void row_sumsq_kernel(const double* __restrict__ src, double* __restrict__ out, long long rows,
-                                 int Q) {
+                                 int Q,
+                                 int sym_p) {
   chain_wait();
   const long long r = (long long)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (r >= rows) return;
+  const long long p = sym_p > 0 ? r / sym_p : 0, q = sym_p > 0 ? r % sym_p : 0;
+  if (q > p) return;
   const double* s = src + r * Q;
   double acc = 0.0;
   for (int l = lane; l < Q; l += 32) {
@@ -95,7 +199,10 @@ __global__ void row_sumsq_kernel(const double* __restrict__ src, double* __restr
     acc = fma(v, v, acc);
   }
   acc = warp_sum(acc);
-  if (lane == 0) out[r] = acc;
+  if (lane == 0) {
+    out[r] = acc;
+    if (sym_p > 0) out[q * sym_p + p] = acc;
+  }
 }
 
 __global__ void col_dot_kernel(const double* __restrict__ C, int ldc, const double* __restrict__ X, int ldx,
@@ -216,11 +323,8 @@ inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) /
 }  // namespace
 
 int launch_contract_diag(const double* C, const double* T, double* d, int N, int P, int Q, cudaStream_t s,
-                         int* texps, size_t texps_ints) {
+                         int* texps) {
   if (texps) {
-    // every entry below any exponent folded in (0x80808080 < -1021), and below
-    // any norm's bits
-    GB_TRY(cuda_status(cudaMemsetAsync(texps, 0x80, sizeof(int) * texps_ints, s), "contract_diag exponents"));
     GB_LAUNCH_CHAIN("contract_diag", s, contract_diag_exps_kernel, dim3(cdiv(Q, 128), P), dim3(128), 0, C, T, d, texps,
                     N, P, Q, device_status_word());
     return GB_OK;
@@ -236,9 +340,22 @@ int launch_gather_diag(const double* src, double* d, int P, int Q, long long str
   return GB_OK;
 }
 
-int launch_row_sumsq(const double* src, double* out, long long rows, int Q, cudaStream_t s) {
+int launch_row_sumsq(const double* src, double* out, long long rows, int Q, cudaStream_t s, int sym_p) {
   if (rows <= 0) return GB_OK;
-  GB_LAUNCH_CHAIN("row_sumsq", s, row_sumsq_kernel, dim3(cdiv(rows, 8)), dim3(256), 0, src, out, rows, Q);
+  GB_LAUNCH_CHAIN("row_sumsq", s, row_sumsq_kernel, dim3(cdiv(rows, 8)), dim3(256), 0, src, out, rows, Q, sym_p);
+  return GB_OK;
+}
+
+int launch_t_exponents(const double* T, int* et, int* ex, int N, int P, int Q, int qps, cudaStream_t s) {
+  GB_LAUNCH_CHAIN("t_exponents", s, t_exponents_kernel, dim3(cdiv(Q, 128), P), dim3(128), 0, T, et, ex, N, Q, qps,
+                  device_status_word());
+  return GB_OK;
+}
+
+int launch_mo_rows(const double* bMO, const double* ck12, const double* w, int* ey, double* K_MO, int P, int Q, int qps,
+                   cudaStream_t s) {
+  GB_LAUNCH_CHAIN("mo_rows", s, mo_rows_kernel, dim3(cdiv((long long)P * P, 8)), dim3(256), 0, bMO, ck12, w, ey, K_MO, P,
+                  Q, qps, device_status_word());
   return GB_OK;
 }
 

@@ -28,10 +28,10 @@ bool orbitals_on_n(long long P, long long rows) {
 
 // T[q][(n,l)] = sum_m C[m][q] b[m][(n,l)] from the sliced C^T (A, rows q) and b (bT)
 int half_transform_gemm(const SlicedDesc& A, const SlicedDesc& bT, int N, int P, int Q, double* Tf,
-                        unsigned int* ctr, cudaStream_t s) {
+                        unsigned int* ctr, cudaStream_t s, unsigned int ctr_start = 0) {
   OzGemm gt{};
   gt.K = N; gt.batch = 1; gt.S = A.code(); gt.C = Tf; gt.c_sb = 0; gt.sym = SYM_NONE; gt.tag = "ozaki_tc:half_transform";
-  gt.tile_counter = ctr;
+  gt.tile_counter = ctr; gt.counter_start = ctr_start;
   if (orbitals_on_n(P, (long long)N * Q)) {
     gt.M = N * Q; gt.N = P; gt.c_r = lin(1); gt.c_c = lin((long long)N * Q);
     return ozaki_gemm(bT, A, gt, s);
@@ -68,24 +68,30 @@ struct JkjMixedWs {
   SlicedDesc A, d, T;
   double* Tf;
   double* dv;
-  unsigned int* ctr;  // tile counter of the persistent GEMMs
+  unsigned int* ctr;  // tile counters of the half transform, J and K GEMMs
+  int* meta;          // T's exponents and norms, then the counters: preset together
+  size_t meta_bytes;
 };
 
 template <class C>
 void jkj_mixed_layout(C& c, int N, int P, int Q, int S, JkjMixedWs* w) {
+  const size_t ints = sliced_meta_ints(P, N);
+  int* meta = c.template take<int>(ints + 4);
+  int* next = meta;
   SlicedDesc A = take_sliced(c, 1, P, N, S);
   auto* tf = c.template take<double>((size_t)P * N * Q);
   auto* dv = c.template take<double>((size_t)P * Q);
   SlicedDesc d = take_sliced(c, 1, P, Q, S);
-  SlicedDesc T = take_sliced(c, P, N, Q, S);
-  auto* ctr = c.template take<unsigned int>(1);
+  SlicedDesc T = take_planes(c, P, N, Q, S, next);
   if (w) {
     w->A = A;
     w->Tf = tf;
     w->dv = dv;
     w->d = d;
     w->T = T;
-    w->ctr = ctr;
+    w->meta = meta;
+    w->meta_bytes = sizeof(int) * (ints + 4);
+    w->ctr = reinterpret_cast<unsigned int*>(next);
   }
 }
 
@@ -128,21 +134,23 @@ namespace {
 // Leaves T, d's slices and the row exponents of T's slicing in the
 // workspace for jkj_mixed_jr and jkj_mixed_k.
 int jkj_mixed_t(const double* C, const Prepared& pr, const JkjMixedWs& w, int N, int P, int Q, cudaStream_t s) {
+  // first, so that the kernels after it follow each other closely
+  GB_TRY(cuda_status(cudaMemsetAsync(w.meta, META_PRESET_BYTE, w.meta_bytes, s), "JK build: exponents and counters"));
   // A rows q over K = m: element C[m][q]
   GB_TRY(slice_operand(SliceSrc{C, 0, lin(1), lin(N), false}, w.A, s));
   // T[q][(n,l)] = sum_m C[m][q] b[m][(n,l)]
-  GB_TRY(half_transform_gemm(w.A, pr.bT, N, P, Q, w.Tf, w.ctr, s));
+  GB_TRY(half_transform_gemm(w.A, pr.bT, N, P, Q, w.Tf, w.ctr, s, META_PRESET));
   // the contraction also records the row exponents of T's slicing (jkj_mixed_k)
-  GB_TRY(launch_contract_diag(C, w.Tf, w.dv, N, P, Q, s, w.T.kind == 0 ? w.T.exps : nullptr,
-                              sliced_meta_ints(P, N)));
+  GB_TRY(launch_contract_diag(C, w.Tf, w.dv, N, P, Q, s, w.T.kind == 0 ? w.T.exps : nullptr));
   return slice_operand(SliceSrc{w.dv, 0, lin(Q), lin(1), true}, w.d, s);
 }
 
 // J[q][(m,n)] = sum_l d[q][l] b[(m,n)][l] for orbitals q0 <= q < q1 (q0 a
 // multiple of the 128-row slice block, so the range starts a block of d's
 // slices).  bJ's rows are the pairs m <= n; each result is also written to (n, m).
+// whole: the one J GEMM after jkj_mixed_t (its preset counter).
 int jkj_mixed_jr(const Prepared& pr, const JkjMixedWs& w, int N, int P, int Q, int S, int q0, int q1, double* J,
-                 cudaStream_t s) {
+                 cudaStream_t s, bool whole = false) {
   if (q1 <= q0) return GB_OK;
   SlicedDesc d = w.d;
   d.planes = reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<unsigned char*>(w.d.planes) +
@@ -152,7 +160,7 @@ int jkj_mixed_jr(const Prepared& pr, const JkjMixedWs& w, int N, int P, int Q, i
   d.rows = q1 - q0;
   OzGemm gj{};
   gj.K = Q; gj.batch = 1; gj.S = S; gj.C = J + (size_t)q0 * N * N; gj.c_sb = 0; gj.pair_n = N; gj.tag = "ozaki_tc:J";
-  gj.tile_counter = w.ctr;
+  gj.tile_counter = w.ctr + (whole ? 1 : 3); gj.counter_start = whole ? META_PRESET : 0;
   const int npairs = N * (N + 1) / 2;
   if (orbitals_on_n(P, npairs)) {
     gj.M = npairs; gj.N = q1 - q0; gj.c_r = lin(1); gj.c_c = lin((long long)N * N); gj.sym = SYM_TRIROW;
@@ -166,12 +174,13 @@ int jkj_mixed_jr(const Prepared& pr, const JkjMixedWs& w, int N, int P, int Q, i
 int jkj_mixed_j(const double* C, const Prepared& pr, const JkjMixedWs& w, int N, int P, int Q, int S, double* J,
                 cudaStream_t s) {
   GB_TRY(jkj_mixed_t(C, pr, w, N, P, Q, s));
-  return jkj_mixed_jr(pr, w, N, P, Q, S, 0, P, J, s);
+  return jkj_mixed_jr(pr, w, N, P, Q, S, 0, P, J, s, true);
 }
 
 // The K half for orbitals q0 <= q < q1: K[q] = T_q T_q^T from the T that
 // jkj_mixed_j left in the workspace.
-int jkj_mixed_k(const JkjMixedWs& w, int N, int Q, int S, int q0, int q1, double* K, cudaStream_t s) {
+int jkj_mixed_k(const JkjMixedWs& w, int N, int Q, int S, int q0, int q1, double* K, cudaStream_t s,
+                bool whole = false) {
   if (q1 <= q0) return GB_OK;
   SlicedDesc T = w.T;
   T.planes = reinterpret_cast<__nv_bfloat16*>(reinterpret_cast<unsigned char*>(w.T.planes) +
@@ -186,7 +195,8 @@ int jkj_mixed_k(const JkjMixedWs& w, int N, int Q, int S, int q0, int q1, double
   // K_q is symmetric: the tile is stored transposed (rows on the unit stride),
   // which lets the epilogue store straight from its TMEM-lane layout
   gk.C = K + (size_t)q0 * N * N; gk.c_sb = (long long)N * N; gk.c_r = lin(1); gk.c_c = lin(N);
-  gk.sym = SYM_ROWCOL; gk.tag = "ozaki_tc:K"; gk.tile_counter = w.ctr;
+  gk.sym = SYM_ROWCOL; gk.tag = "ozaki_tc:K";
+  gk.tile_counter = w.ctr + (whole ? 2 : 3); gk.counter_start = whole ? META_PRESET : 0;
   return ozaki_gemm(T, T, gk, s);
 }
 
@@ -212,7 +222,7 @@ extern "C" int gb_jkj_ri_mixed(const double* C, const void* prep, int nbf, int n
   jkj_mixed_layout(wc, N, P, Q, S, &w);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   GB_TRY(jkj_mixed_j(C, pr, w, N, P, Q, S, J, s));
-  return jkj_mixed_k(w, N, Q, S, 0, P, K, s);
+  return jkj_mixed_k(w, N, Q, S, 0, P, K, s, true);
 }
 
 extern "C" int gb_jkj_ri_mixed_j(const double* C, const void* prep, int nbf, int nbf5, int naux, int nslices,
@@ -335,10 +345,49 @@ extern "C" int gb_dgemm_mixed(const double* A, const double* B, int M, int N, in
 //   J_MO = d d^T (d[p] = bpq[p][p]),  K_MO[p][q] = sum_l bpq[p][q][l]^2,  H_core
 // ---------------------------------------------------------------------------
 namespace {
+// K splits of J_MO = d d^T (P x P, K = naux): its one to six tiles would run on as
+// many SMs (72 us at nbf=300), so K is cut in equal ranges of at least 256 that run
+// as a batch, summed in order.  1 where naux has no such divisor.
+int jmo_splits(int P, int Q) {
+  const int t = (P + 127) / 128;
+  for (int s = 152 / (t * (t + 1) / 2); s > 1; --s)
+    if (Q % s == 0 && Q / s >= 256) return s;
+  return 1;
+}
+
+// out[i] = sum_s part[s][i], i < n
+__global__ void sum_splits_kernel(const double* __restrict__ part, int ns, long long n, double* __restrict__ out) {
+  chain_wait();
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double v = 0.0;
+#pragma unroll 4
+  for (int s = 0; s < ns; ++s) v += part[s * n + i];
+  out[i] = v;
+}
+
+// J_MO = d d^T (symmetric: the SYRK form, stored transposed) from d's slices, one
+// batch entry per K range; part: the ranges' products.
+int jmo_gemm(const SlicedDesc& dS, double* part, double* J_MO, int S, unsigned int* ctr, cudaStream_t s) {
+  const int P = dS.rows;
+  OzGemm gj{};
+  gj.M = P; gj.N = P; gj.K = dS.K; gj.batch = dS.batch; gj.S = S;
+  gj.C = dS.batch > 1 ? part : J_MO; gj.c_sb = (long long)P * P; gj.c_r = lin(1); gj.c_c = lin(P);
+  gj.sym = SYM_ROWCOL; gj.tag = "ozaki_tc:J_MO";
+  gj.tile_counter = ctr; gj.counter_start = META_PRESET;
+  GB_TRY(ozaki_gemm(dS, dS, gj, s));
+  if (dS.batch > 1) {
+    const long long n = (long long)P * P;
+    GB_LAUNCH_CHAIN("sum_splits", s, sum_splits_kernel, dim3((unsigned)((n + 127) / 128)), dim3(128), 0, part, dS.batch,
+                    n, J_MO);
+  }
+  return GB_OK;
+}
+
 struct JkhMixedWs {
   SlicedDesc A, Tt, dS;
-  double *Tf, *bpq, *d, *X;
-  unsigned int* ctr;  // tile counter of the persistent GEMMs
+  double *Tf, *bpq, *d, *X, *jpart;
+  unsigned int* ctr;  // tile counters of the half transform, bpq and J_MO GEMMs
 };
 
 template <class Cv>
@@ -349,9 +398,11 @@ void jkh_mixed_layout(Cv& c, int N, int P, int Q, int S, JkhMixedWs* w) {
   auto* bpq = c.template take<double>((size_t)P * P * Q);
   auto* d = c.template take<double>((size_t)P * Q);
   auto* X = c.template take<double>((size_t)N * P);
-  auto* ctr = c.template take<unsigned int>(1);
-  SlicedDesc dS = take_sliced(c, 1, P, Q, S);  // d rows p, K = l (J_MO)
-  if (w) *w = JkhMixedWs{A, Tt, dS, tf, bpq, d, X, ctr};
+  auto* ctr = c.template take<unsigned int>(3);
+  const int js = jmo_splits(P, Q);
+  SlicedDesc dS = take_sliced(c, js, P, Q / js, S);  // d rows p, K = l (J_MO)
+  auto* jpart = js > 1 ? c.template take<double>((size_t)js * P * P) : nullptr;
+  if (w) *w = JkhMixedWs{A, Tt, dS, tf, bpq, d, X, jpart, ctr};
 }
 
 // H_core[p] = C_p^T H C_p and (optionally) Hmat = C^T H C_p in FP64
@@ -377,10 +428,17 @@ int hcore_f64(const double* C, const double* H, int N, int P, double* X, double*
   return GB_OK;
 }
 
+// (pq|l) = (qp|l), p, q < nbf5: the batched MO transform computes q <= p and writes
+// both (its tiles past the diagonal are skipped: 4.7 ms of MMAs at nbf=600, nbf5=300
+// become 2.7).  Six digits only: with fewer, (pq|l) and (qp|l) differ by the split's
+// error and both are the form's results.  Nor where the rows are not alone the
+// unit stride.
+int mo_symmetry(int P, int Q, int S) { return S == 6 && Q > 1 && P > 1 ? SYM_BATCHCOL : SYM_NONE; }
+
 int half_transform_mixed(const double* C, const SlicedDesc& A, const SlicedDesc& bT, int N, int P, int Q,
                          double* Tf, unsigned int* ctr, cudaStream_t s) {
   GB_TRY(slice_operand(SliceSrc{C, 0, lin(1), lin(N), false}, A, s));
-  return half_transform_gemm(A, bT, N, P, Q, Tf, ctr, s);
+  return half_transform_gemm(A, bT, N, P, Q, Tf, ctr, s, META_PRESET);
 }
 }  // namespace
 
@@ -406,28 +464,20 @@ extern "C" int gb_jkh_mo_ri_mixed(const double* C, const double* H, const void* 
   JkhMixedWs w;
   jkh_mixed_layout(wc, N, P, Q, S, &w);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  GB_TRY(cuda_status(cudaMemsetAsync(w.ctr, META_PRESET_BYTE, 3 * sizeof(int), s), "tile counters"));
   GB_TRY(half_transform_mixed(C, w.A, pr.bT, N, P, Q, w.Tf, w.ctr, s));
   // T read with rows l and K = n: element T[p][n][l]
   GB_TRY(slice_operand(SliceSrc{w.Tf, (long long)N * Q, lin(1), lin(Q), false}, w.Tt, s));
   OzGemm gq{};
-  gq.K = N; gq.batch = P; gq.S = S; gq.C = w.bpq; gq.c_sb = (long long)P * Q; gq.sym = SYM_NONE; gq.tag = "ozaki_tc:bpq";
-  gq.tile_counter = w.ctr;
-  if (orbitals_on_n(P, Q)) {
-    gq.M = Q; gq.N = P; gq.c_r = lin(1); gq.c_c = lin(Q);
-    GB_TRY(ozaki_gemm(w.Tt, w.A, gq, s));
-  } else {
-    gq.M = P; gq.N = Q; gq.c_r = lin(Q); gq.c_c = lin(1);
-    GB_TRY(ozaki_gemm(w.A, w.Tt, gq, s));
-  }
+  gq.M = Q; gq.N = P; gq.K = N; gq.batch = P; gq.S = S;
+  gq.C = w.bpq; gq.c_sb = (long long)P * Q; gq.c_r = lin(1); gq.c_c = lin(Q);
+  gq.sym = mo_symmetry(P, Q, S); gq.tag = "ozaki_tc:bpq";
+  gq.tile_counter = w.ctr + 1; gq.counter_start = META_PRESET;
+  GB_TRY(ozaki_gemm(w.Tt, w.A, gq, s));
   GB_TRY(launch_gather_diag(w.bpq, w.d, P, Q, (long long)P * Q + Q, s));
-  // J_MO = d d^T (symmetric: the SYRK form, stored transposed)
-  GB_TRY(slice_operand(SliceSrc{w.d, 0, lin(Q), lin(1), true}, w.dS, s));
-  OzGemm gj{};
-  gj.M = P; gj.N = P; gj.K = Q; gj.batch = 1; gj.S = S;
-  gj.C = J_MO; gj.c_sb = 0; gj.c_r = lin(1); gj.c_c = lin(P);
-  gj.sym = SYM_ROWCOL; gj.tag = "ozaki_tc:J_MO"; gj.tile_counter = w.ctr;
-  GB_TRY(ozaki_gemm(w.dS, w.dS, gj, s));
-  GB_TRY(launch_row_sumsq(w.bpq, K_MO, (long long)P * P, Q, s));
+  GB_TRY(slice_operand(SliceSrc{w.d, w.dS.K, lin(Q), lin(1), true}, w.dS, s));
+  GB_TRY(jmo_gemm(w.dS, w.jpart, J_MO, S, w.ctr + 2, s));
+  GB_TRY(launch_row_sumsq(w.bpq, K_MO, (long long)P * P, Q, s, mo_symmetry(P, Q, S) == SYM_BATCHCOL ? P : 0));
   return hcore_f64(C, H, N, P, w.X, H_core, nullptr, s);
 }
 
@@ -443,9 +493,12 @@ struct Lag2MixedWs {
   SlicedDesc dS, dT, cjS, Ct, Zt;  // the small GEMMs' operands (w, J_MO, elag = -C^T Z)
   double *Tf, *bMO, *Y, *X, *d, *w, *cjm;
   double* part;  // ns partial exchange products (ns > 1)
+  double* jpart;  // partial products of J_MO
   double* Z;     // Z^T: Z[b][m] = sum_(q,l) T[q][m][l] Y[b][q][l]
   int ns, kc;    // K splits of the exchange GEMM (whole ranges of orbitals q) and K per split
-  unsigned int* ctr;  // tile counter of the persistent GEMMs
+  unsigned int* ctr;  // tile counters of the GEMMs, in order
+  int* meta;          // Tt's, Sx's and Sy's exponents and norms, then the counters: preset together
+  size_t meta_bytes;
 };
 
 // K splits of the exchange GEMM (M = nbf, N = nbf5, K = nbf5 naux): with few
@@ -474,41 +527,35 @@ int exchange_splits(int N, int P, int Q) {
   return (int)s;
 }
 
-// out[i] = sum_s part[s][i], i < n
-__global__ void sum_splits_kernel(const double* __restrict__ part, int ns, long long n, double* __restrict__ out) {
-  chain_wait();
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double v = 0.0;
-#pragma unroll 4
-  for (int s = 0; s < ns; ++s) v += part[s * n + i];
-  out[i] = v;
-}
-
 template <class Cv>
 void lag2_mixed_layout(Cv& c, int N, int P, int Q, int S, Lag2MixedWs* w) {
-  SlicedDesc Ap = take_sliced(c, 1, P, N, S);
-  auto* tf = c.template take<double>((size_t)P * N * Q);
-  SlicedDesc Tt = take_sliced(c, P, Q, N, S);
-  auto* bmo = c.template take<double>((size_t)P * P * Q);
-  auto* Y = c.template take<double>((size_t)P * P * Q);
   const int ns = exchange_splits(N, P, Q);
   const int kc = (P / ns) * Q;  // K per split: P / ns whole orbitals
-  SlicedDesc Sx = take_sliced(c, ns, N, kc, S);
-  SlicedDesc Sy = take_sliced(c, ns, P, kc, S);
+  const size_t ints = sliced_meta_ints(P, Q) + sliced_meta_ints(ns, N) + sliced_meta_ints(ns, P);
+  int* meta = c.template take<int>(ints + 8);
+  int* next = meta;
+  SlicedDesc Ap = take_sliced(c, 1, P, N, S);
+  auto* tf = c.template take<double>((size_t)P * N * Q);
+  SlicedDesc Tt = take_planes(c, P, Q, N, S, next);
+  auto* bmo = c.template take<double>((size_t)P * P * Q);
+  auto* Y = S == 6 && (Q > 1 || P == 1) ? nullptr : c.template take<double>((size_t)P * P * Q);  // (six digits: cut from bMO directly)
+  SlicedDesc Sx = take_planes(c, ns, N, kc, S, next);
+  SlicedDesc Sy = take_planes(c, ns, P, kc, S, next);
   auto* part = ns > 1 ? c.template take<double>((size_t)ns * N * P) : nullptr;
   auto* Z = c.template take<double>((size_t)N * P);
   auto* X = c.template take<double>((size_t)N * P);
   auto* d = c.template take<double>((size_t)P * Q);
   auto* wv = c.template take<double>((size_t)P * Q);
   auto* cjm = c.template take<double>((size_t)P * P);
-  auto* ctr = c.template take<unsigned int>(1);
-  SlicedDesc dS = take_sliced(c, 1, P, Q, S);  // d rows p, K = l
+  const int js = jmo_splits(P, Q);
+  SlicedDesc dS = take_sliced(c, js, P, Q / js, S);  // d rows p, K = l
+  auto* jpart = js > 1 ? c.template take<double>((size_t)js * P * P) : nullptr;
   SlicedDesc dT = take_sliced(c, 1, Q, P, S);  // d^T rows l, K = q
   SlicedDesc cjS = take_sliced(c, 1, P, P, S);  // cj12 (zero diagonal) rows b, K = q
   SlicedDesc Ct = take_sliced(c, 1, N, N, S);  // C^T rows a, K = m
   SlicedDesc Zt = take_sliced(c, 1, P, N, S);  // Z^T rows b, K = m
-  if (w) *w = Lag2MixedWs{Ap, Tt, Sx, Sy, dS, dT, cjS, Ct, Zt, tf, bmo, Y, X, d, wv, cjm, part, Z, ns, kc, ctr};
+  if (w) *w = Lag2MixedWs{Ap, Tt, Sx, Sy, dS, dT, cjS, Ct, Zt, tf, bmo, Y, X, d, wv, cjm, part, jpart, Z, ns, kc,
+                        reinterpret_cast<unsigned int*>(next), meta, sizeof(int) * (ints + 8)};
 }
 }  // namespace
 
@@ -543,31 +590,37 @@ int lagrange2_mixed_body(const double* C, const double* H, const void* prep, con
   Lag2MixedWs w;
   lag2_mixed_layout(wc, N, P, Q, S, &w);
 
+  // first, so that the kernels after it follow each other closely
+  GB_TRY(cuda_status(cudaMemsetAsync(w.meta, META_PRESET_BYTE, w.meta_bytes, s), "lagrange2: exponents and counters"));
   // C^T rows a < nbf5 (K = m): the half transform's and the MO transform's A
   GB_TRY(slice_operand(SliceSrc{C, 0, lin(1), lin(N), false}, w.Ap, s));
-  GB_TRY(half_transform_gemm(w.Ap, pr.bT, N, P, Q, w.Tf, w.ctr, s));
-  GB_TRY(slice_operand(SliceSrc{w.Tf, (long long)N * Q, lin(1), lin(Q), false}, w.Tt, s));
+  GB_TRY(half_transform_gemm(w.Ap, pr.bT, N, P, Q, w.Tf, w.ctr, s, META_PRESET));
+  const int qps = P / w.ns;  // orbitals per K range of the exchange GEMM
+  const bool digits = w.Tt.kind == 0;
+  const bool from_bmo = S == 6 && (P == 1 || mo_symmetry(P, Q, S) == SYM_BATCHCOL);  // bMO exactly symmetric
+  if (digits) {
+    // T's two slicings (rows l over K = m, rows m over K = (q, l)) take their row
+    // exponents from one read of it
+    GB_TRY(launch_t_exponents(w.Tf, w.Tt.exps, w.Sx.exps, N, P, Q, qps, s));
+  }
+  GB_TRY(slice_operand(SliceSrc{w.Tf, (long long)N * Q, lin(1), lin(Q), false}, w.Tt, s, digits));
   // bMO[a][q][l], a < nbf5 (batch q): rows l (the output's unit stride, the
   // persistent form) x orbitals a on the N tile (a ragged orbital count pads
   // less there)
   OzGemm gm{};
   gm.M = Q; gm.N = P; gm.K = N; gm.batch = P; gm.S = S;
   gm.C = w.bMO; gm.c_sb = Q; gm.c_r = lin(1); gm.c_c = lin((long long)P * Q);
-  gm.sym = SYM_NONE; gm.tag = "ozaki_tc:bMO"; gm.tile_counter = w.ctr;
+  gm.sym = mo_symmetry(P, Q, S); gm.tag = "ozaki_tc:bMO";
+  gm.tile_counter = w.ctr + 1; gm.counter_start = META_PRESET;
   GB_TRY(ozaki_gemm(w.Tt, w.Ap, gm, s));
   GB_TRY(hcore_f64(C, H, N, P, w.X, H_core, Hmat, s));
   GB_TRY(launch_gather_diag(w.bMO, w.d, P, Q, (long long)P * Q + Q, s));
   // d's slices: rows p over K = l (J_MO) and rows l over K = q (w)
-  GB_TRY(slice_operand(SliceSrc{w.d, 0, lin(Q), lin(1), true}, w.dS, s));
+  if (J_MO) GB_TRY(slice_operand(SliceSrc{w.d, w.dS.K, lin(Q), lin(1), true}, w.dS, s));
   GB_TRY(slice_operand(SliceSrc{w.d, 0, lin(1), lin(Q), false}, w.dT, s));
   if (J_MO) {
-    // J_MO = d d^T (symmetric: the SYRK form, stored transposed)
-    OzGemm gj{};
-    gj.M = P; gj.N = P; gj.K = Q; gj.batch = 1; gj.S = S;
-    gj.C = J_MO; gj.c_sb = 0; gj.c_r = lin(1); gj.c_c = lin(P);
-    gj.sym = SYM_ROWCOL; gj.tag = "ozaki_tc:J_MO"; gj.tile_counter = w.ctr;
-    GB_TRY(ozaki_gemm(w.dS, w.dS, gj, s));
-    GB_TRY(launch_row_sumsq(w.bMO, K_MO, (long long)P * P, Q, s));
+    GB_TRY(jmo_gemm(w.dS, w.jpart, J_MO, S, w.ctr + 2, s));
+    if (!from_bmo) GB_TRY(launch_row_sumsq(w.bMO, K_MO, (long long)P * P, Q, s));
   }
   // w[b][l] = sum_q cj12[b][q] d[q][l] (diagonal of cj12 zero): rows l x orbitals b
   GB_TRY(launch_copy_zero_diag(cj12, w.cjm, P, s));
@@ -575,21 +628,32 @@ int lagrange2_mixed_body(const double* C, const double* H, const void* prep, con
   OzGemm gw{};
   gw.M = Q; gw.N = P; gw.K = P; gw.batch = 1; gw.S = S;
   gw.C = w.w; gw.c_sb = 0; gw.c_r = lin(1); gw.c_c = lin(Q);
-  gw.sym = SYM_NONE; gw.tag = "ozaki_tc:w"; gw.tile_counter = w.ctr;
+  gw.sym = SYM_NONE; gw.tag = "ozaki_tc:w";
+  gw.tile_counter = w.ctr + 3; gw.counter_start = META_PRESET;
   GB_TRY(ozaki_gemm(w.dT, w.cjS, gw, s));
   GB_TRY(launch_add_scaled_rows(w.w, w.d, n, P, Q, nbeta, nalpha, s));
-  // the w term rides in the diagonal blocks of the exchange operand
-  GB_TRY(launch_make_exchange_operand(w.bMO, ck12, w.w, w.Y, P, Q, s));
   // Z[m][b] = sum_(q,l) T[q][m][l] Y[b][q][l]; K = (q, l) cut into w.ns ranges
   // of whole orbitals (split s = batch s: its T block starts at orbital
   // s P / ns, element (m, k) at k / Q * N Q + m Q + k % Q; Y row b at b P Q + s kc + k)
-  const long long qps = P / w.ns;  // orbitals per split
-  GB_TRY(slice_operand(SliceSrc{w.Tf, qps * N * Q, lin(Q), split(Q, (long long)N * Q, 1), true}, w.Sx, s));
-  GB_TRY(slice_operand(SliceSrc{w.Y, w.kc, lin((long long)P * Q), lin(1), true}, w.Sy, s));
+  const Index2 runs = split(Q, (long long)N * Q, 1);
+  GB_TRY(slice_operand(SliceSrc{w.Tf, (long long)qps * N * Q, lin(Q), runs, true}, w.Sx, s, digits));
+  // the w term rides in the diagonal blocks of the exchange operand
+  if (from_bmo) {
+    // Y is cut from bMO while it is scaled: not written, and bMO read once for the
+    // exponents and K_MO (q <= b) and once for the digits
+    GB_TRY(launch_mo_rows(w.bMO, ck12, w.w, w.Sy.exps, J_MO ? K_MO : nullptr, P, Q, qps, s));
+    SliceSrc y{w.bMO, w.kc, lin((long long)P * Q), split(Q, Q, 1), true};
+    y.ex_scale = ck12; y.ex_diag = w.w; y.ex_n = P; y.ex_runs = qps;
+    GB_TRY(slice_operand(y, w.Sy, s, true));
+  } else {
+    GB_TRY(launch_make_exchange_operand(w.bMO, ck12, w.w, w.Y, P, Q, s));
+    GB_TRY(slice_operand(SliceSrc{w.Y, w.kc, lin((long long)P * Q), lin(1), true}, w.Sy, s));
+  }
   // rows m x orbitals b on the N tile (a ragged orbital count pads less there)
   OzGemm ge{};
   ge.M = N; ge.N = P; ge.K = w.kc; ge.batch = w.ns; ge.S = S;
-  ge.sym = SYM_NONE; ge.tag = "ozaki_tc:ck_exchange"; ge.tile_counter = w.ctr;
+  ge.sym = SYM_NONE; ge.tag = "ozaki_tc:ck_exchange";
+  ge.tile_counter = w.ctr + 4; ge.counter_start = META_PRESET;
   // stored transposed, [b][m]: the tile rows are then the unit stride (the persistent kernel)
   ge.C = w.ns > 1 ? w.part : w.Z; ge.c_sb = (long long)N * P; ge.c_r = lin(1); ge.c_c = lin(N);
   GB_TRY(ozaki_gemm(w.Sx, w.Sy, ge, s));
@@ -604,7 +668,8 @@ int lagrange2_mixed_body(const double* C, const double* H, const void* prep, con
   OzGemm gz{};
   gz.M = P; gz.N = N; gz.K = N; gz.batch = 1; gz.S = S; gz.negate = 1;
   gz.C = elag; gz.c_sb = 0; gz.c_r = lin(1); gz.c_c = lin(N);
-  gz.sym = SYM_NONE; gz.tag = "ozaki_tc:elag"; gz.tile_counter = w.ctr;
+  gz.sym = SYM_NONE; gz.tag = "ozaki_tc:elag";
+  gz.tile_counter = w.ctr + 5; gz.counter_start = META_PRESET;
   GB_TRY(ozaki_gemm(w.Zt, w.Ct, gz, s));
   return launch_lagrange2_hterm(Hmat, n, elag, N, P, s);
 }

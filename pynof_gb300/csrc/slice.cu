@@ -16,11 +16,12 @@ __device__ __forceinline__ int exponent_of(unsigned long long maxbits) {
 
 // Balanced W-bit digits of round(x 2^(e_S - E)), pre-weighted: digit s as the
 // FP32 bits of d 2^-e_s (exact in bf16, so the upper half of those bits is the
-// bf16 pattern; the lower half is zero).  The 64-bit integer xi = H 2^(W NL) + L
-// (0 <= L < 2^(W NL)) is taken apart in 32-bit pieces: the NL lowest digits come
-// from L (its carry, 0 or 1, goes to H), the others from H.  Each digit's FP32
-// value comes from the 1.5 * 2^23 magic number (exact for |d| < 2^22), scaled
-// by its weight in the same (exact) fused multiply-add.
+// bf16 pattern; the lower half is zero).  Half a digit's range added at every
+// place makes the balanced digits plain fields of a non-negative integer, with no
+// carries between them.  A field's FP32 value comes from the 1.5 * 2^23 magic
+// number (the field or-ed into its low bits), its bias and weight from one exact
+// fused multiply-add: three instructions a digit (with carries from digit to digit
+// five; the slicer, at 87 % of the copy rate at nbf=600, takes the same time).
 template <int S, int W>
 __device__ __forceinline__ void make_digits(double x, int E, uint32_t* out) {
   const unsigned long long bits = (unsigned long long)__double_as_longlong(x);
@@ -29,35 +30,25 @@ __device__ __forceinline__ void make_digits(double x, int E, uint32_t* out) {
   if (ex) m |= 1ull << 52; else ex = 1;
   // right shift of the 53-bit mantissa (>= 9 for e_S <= 44, a left shift of at most 9 for 62)
   const int r = 1075 + E - ex - digit_exp(W, S);
-  long long xi;
-  if (digit_exp(W, S) > 52 && r <= 0) xi = (long long)(m << -r);
-  else if (r >= 64) xi = 0;
-  else xi = (long long)((m + (1ull << (r - 1))) >> r);
-  if (bits >> 63) xi = -xi;
-  constexpr int NL = S - 1 < 3 ? S - 1 : 3, HALF = 1 << (W - 1), MASK = (1 << W) - 1;
-  // the three middle digits of seven go through 32 bits of their own
-  constexpr int NM = S == 7 ? 3 : 0;
-  auto digit = [&](int s, int& rest) {
-    const int d = ((rest + HALF) & MASK) - HALF;
-    rest = (rest - d) >> W;
+  unsigned long long mag;
+  if (digit_exp(W, S) > 52 && r <= 0) mag = m << -r;
+  else if (r >= 64) mag = 0;
+  else mag = (m + (1ull << (r - 1))) >> r;
+  // half a digit's range at every place, the leading digit's bound 2^e_1 at its own
+  constexpr int E1 = digit_exp(W, 1);
+  constexpr unsigned long long ONES = ((1ull << (W * S)) - 1) / ((1ull << W) - 1);
+  constexpr unsigned long long BIAS =
+      (ONES << (W - 1)) + (((1ull << E1) - (1ull << (W - 1))) << (W * (S - 1)));
+  const unsigned long long sg = (unsigned long long)((long long)bits >> 63);
+  const unsigned long long u = (mag ^ sg) + (BIAS - sg);
+#pragma unroll
+  for (int s = S; s >= 1; --s) {
+    // the leading digit's field is 0 .. 2^(e_1 + 1)
+    const uint32_t f = (uint32_t)(u >> (W * (S - s))) & ((1u << (s == 1 ? E1 + 2 : W)) - 1u);
     const float w = __int_as_float((127 - digit_exp(W, s)) << 23);
-    out[s - 1] = __float_as_uint(fmaf(__int_as_float(0x4B400000 + d), w, -12582912.0f * w));
-  };
-  int L = (int)(xi & ((1ll << (W * NL)) - 1));
-#pragma unroll
-  for (int s = S; s > S - NL; --s) digit(s, L);
-  int H = (int)(xi >> (W * (NL + NM)));
-  if (NM > 0) {
-    int M = (int)((xi >> (W * NL)) & ((1ll << (W * NM)) - 1)) + L;
-#pragma unroll
-    for (int s = S - NL; s > S - NL - NM; --s) digit(s, M);
-    L = M;
+    const float zero = 12582912.0f + (float)(1 << (s == 1 ? E1 : W - 1));
+    out[s - 1] = __float_as_uint(fmaf(__uint_as_float(0x4B400000u | f), w, -zero * w));
   }
-  H += L;
-#pragma unroll
-  for (int s = S - NL - NM; s >= 2; --s) digit(s, H);
-  const float w1 = __int_as_float((127 - digit_exp(W, 1)) << 23);
-  out[0] = __float_as_uint(fmaf(__int_as_float(0x4B400000 + H), w1, -12582912.0f * w1));
 }
 
 // A NaN or an infinity has the largest magnitude bits of all; it has no digits,
@@ -197,6 +188,40 @@ __device__ __forceinline__ void load_group(const SliceSrc& src, const double* ba
   }
 }
 
+// The same of an exchange operand (SliceSrc::ex_scale); r: the row, b: the batch entry.
+__device__ __forceinline__ void load_group_exchange(const SliceSrc& src, const double* base, bool rok, int r, int b,
+                                                    int k0, int K, double (&xs)[8]) {
+  const int div = (int)src.k.div;
+  int q = k0 / div, l = k0 - q * div;
+  q += b * src.ex_runs;
+  const double* p8 = base + k0;
+  if (rok && div % 8 == 0 && k0 + 8 <= K && q != r && (reinterpret_cast<uintptr_t>(p8) & 15) == 0) {
+    const double c = __ldg(src.ex_scale + (long long)r * src.ex_n + q);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const double2 v = __ldg(reinterpret_cast<const double2*>(p8) + u);
+      xs[2 * u] = c * v.x;
+      xs[2 * u + 1] = c * v.y;
+    }
+    return;
+  }
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    double v = 0.0;
+    if (rok && k0 + u < K) {
+      if (q == r)
+        v = -src.ex_diag[(long long)r * div + l];
+      else
+        v = src.ex_scale[(long long)r * src.ex_n + q] * p8[u];
+    }
+    xs[u] = v;
+    if (++l == div) {
+      l = 0;
+      ++q;
+    }
+  }
+}
+
 // Digits of the 8 values, packed per slice as 8 bf16 (one 16-byte store each);
 // nq[s] += the sum of the squares of the weighted digits of slice s < SL_NORMS
 // (nine-bit digits).
@@ -237,7 +262,7 @@ __device__ __forceinline__ void store_group(const double (&xs)[8], int e, unsign
 // eight blocks of a run bound the run's), G = 4 for longer ones, whose chunks need
 // the tighter norms (half transform at nbf=600 6.20 ms, 6.89 with the looser).
 // Three slicings of an nbf=24 build: 41 us with runs of eight, 33 with G = 4, 20.
-template <int S, int W>
+template <int S, int W, bool EX = false>
 __global__ void __launch_bounds__(S == 7 ? 256 : 1024, S == 7 ? 3 : 1) digits_blocked_kernel(SliceSrc src, SlicedDesc dst,
                                                                                                    int kpc) {
   constexpr int ND = W != 9 ? 0 : S == 7 ? SL_NORMS : 3;  // digits with norms
@@ -260,7 +285,10 @@ __global__ void __launch_bounds__(S == 7 ? 256 : 1024, S == 7 ? 3 : 1) digits_bl
   double xa[8];
   float nq[SL_NORMS] = {};
   for (int kb = kb0 + grp; kb < kb1; kb += G) {
-    load_group(src, base, rok, kb * SL_K + kg * 8, dst.K, xa);
+    if (EX)
+      load_group_exchange(src, base, rok, r, (int)b, kb * SL_K + kg * 8, dst.K, xa);
+    else
+      load_group(src, base, rok, kb * SL_K + kg * 8, dst.K, xa);
     store_group<S, W>(xa, e, out0 + (long long)kb * S * SL_TILE_BYTES, nq);
   }
   if (S != 7 && ND > 0 && G > 1) {
@@ -403,6 +431,12 @@ int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bo
   const int kpc = few && runs == 1 ? 1 : SL_KPC;
   const dim3 grid((unsigned)((long long)dst.rblocks() * ((dst.kblocks() + kpc - 1) / kpc)), dst.batch);
   const dim3 block(few && runs > 1 && dst.S != 7 ? 1024 : 256);
+  if (src.ex_scale) {
+    GB_REQUIRE(exps_ready && src.kfast && src.k.div > 0 && dst.S == 5 && dst.W == 9, GB_ERR_INVALID_ARG,
+               "slice_operand: an exchange operand takes six digits and recorded exponents");
+    GB_LAUNCH_CHAIN("slice_digits", s, (digits_blocked_kernel<5, 9, true>), grid, block, 0, src, dst, kpc);
+    return GB_OK;
+  }
   if (dst.W == 9) {
     GB_REQUIRE(dst.S == 5 || dst.S == 7, GB_ERR_INVALID_ARG, "slice_operand: nine-bit digits come in five or seven planes");
     if (dst.S == 5)

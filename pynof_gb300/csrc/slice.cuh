@@ -85,6 +85,12 @@ struct SliceSrc {
   // pairs (tri_pair); row r reads r.at(m * tri_n + n)
   int tri_n = 0;
   long long row0 = 0;  // row 0 of the slices is row row0 of the source (a panel of its rows)
+  // The exchange operand (six digits, recorded exponents; its k runs of k.div
+  // follow each other): with ex_scale the element of row r in k run q = batch ex_runs + k / k.div is ex_scale[r ex_n + q]
+  // times the source's, and -ex_diag[r k.div + k % k.div] in run q == r.
+  const double* ex_scale = nullptr;
+  const double* ex_diag = nullptr;
+  int ex_n = 0, ex_runs = 0;
   __host__ __device__ __forceinline__ long long row_at(long long row) const {
     if (tri_n <= 0) return r.at(row0 + row);
     int m, n;
@@ -132,6 +138,20 @@ template <class Cv>
 SlicedDesc take_sliced(Cv& c, int batch, int rows, int K, int code) {
   auto* p = c.template take<unsigned char>(sliced_plane_bytes(batch, rows, K, code));
   auto* e = c.template take<int>(sliced_meta_ints(batch, rows));
+  const SliceForm f = form_of(code);
+  return SlicedDesc{reinterpret_cast<__nv_bfloat16*>(p), e, batch, rows, K, f.S, f.kind, f.W,
+                    e ? e + (size_t)batch * rows : nullptr};
+}
+
+// The same with the exponents and norms in `meta`, which is moved past them: several
+// operands' that one memset presets (META_PRESET below any exponent and any norm).
+constexpr int META_PRESET_BYTE = 0x80;
+constexpr unsigned int META_PRESET = 0x80808080u;
+template <class Cv>
+SlicedDesc take_planes(Cv& c, int batch, int rows, int K, int code, int*& meta) {
+  auto* p = c.template take<unsigned char>(sliced_plane_bytes(batch, rows, K, code));
+  int* e = meta;
+  if (meta) meta += sliced_meta_ints(batch, rows);
   const SliceForm f = form_of(code);
   return SlicedDesc{reinterpret_cast<__nv_bfloat16*>(p), e, batch, rows, K, f.S, f.kind, f.W,
                     e ? e + (size_t)batch * rows : nullptr};

@@ -69,3 +69,26 @@ def test_build_with_equal_orbitals(ops, nbf, naux, nbf5):
     ops.check_device_status()
     for got, ref in ((dJ, J), (dK, K)):
         assert np.max(np.abs(got.cpu().numpy() - ref)) / np.max(np.abs(ref)) < 3 * TOL
+
+
+@pytest.mark.parametrize("nbf,naux,nbf5", [(20, 41, 1), (40, 70, 17), (150, 130, 128), (140, 90, 129), (210, 60, 207)])
+def test_symmetric_mo_transform(ops, nbf, naux, nbf5):
+    """(pq|l) computed for q <= p: J_MO, K_MO and the Lagrangian around the edges
+    of the 128- and 16-column steps, against the FP64 path.  The split's error
+    is a few 2^-45 of the row bounds per k (TOL above); K_MO and the Lagrangian
+    square or contract (pq|l), which doubles it."""
+    rng = np.random.default_rng(nbf5)
+    b = rng.standard_normal((nbf, nbf, naux))
+    b = ops.to_device(0.5 * (b + b.transpose(1, 0, 2)))
+    C = ops.to_device(np.linalg.qr(rng.standard_normal((nbf, nbf)))[0])
+    H = rng.standard_normal((nbf, nbf))
+    H, n = ops.to_device(H + H.T), rng.random(nbf5)
+    cj, ck = ops.to_device(2 * np.outer(n, n)), ops.to_device(np.outer(n, n))
+    n, prep = ops.to_device(n), ops.PreparedRI(b, 6)
+    ref = ops.jkh_mo_ri(C, H, b, nbf5) + ops.lagrange2_ri(C, H, b, n, cj, ck, nbf5, 1, 1)
+    got = ops.jkh_lagrange2_ri_mixed(C, H, prep, n, cj, ck, nbf5, 1, 1)
+    mo = ops.jkh_mo_ri_mixed(C, H, prep, nbf5)
+    ops.check_device_status()
+    for x, r in zip(got + mo, ref + ref[:3]):
+        x, r = x.cpu().numpy(), r.cpu().numpy()
+        assert np.max(np.abs(x - r)) / np.max(np.abs(r)) < 4 * TOL
