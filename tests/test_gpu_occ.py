@@ -97,6 +97,31 @@ def test_energy_grad_matches_host(torch_cuda, case):
         assert r[4] == np.max(np.abs(gd))
 
 
+@pytest.mark.parametrize("P,no1,ndoc,ncwo", [
+    (2, 0, 1, 1),      # one pair
+    (33, 1, 8, 3),     # a group of one orbital
+    (64, 0, 16, 3),    # whole groups and blocks
+    (450, 0, 3, 149),  # a pair per CTA
+    (700, 0, 2, 349),  # pairs whose roots are kept in the workspace
+    (711, 1, 142, 4),  # the largest whose step works in shared memory
+    (712, 0, 178, 3),  # and the smallest that works in the workspace
+])
+def test_energy_grad_shapes(torch_cuda, P, no1, ndoc, ncwo):
+    """Edges of the evaluation's split, held to test_energy_grad_matches_host's bounds."""
+    from pynof_gb300 import nof, ops, synthetic
+
+    p = synthetic.Structure(nbf=P, nbfaux=4 * P, ndoc=ndoc, ncwo=ncwo, no1=no1)
+    rng = np.random.default_rng(P)
+    A, B = (0.01 * rng.standard_normal((P, P)) for _ in range(2))
+    J, K, Hc = np.abs(A + A.T) + np.eye(P), np.abs(B + B.T) + np.eye(P), -np.linspace(5.0, 0.1, P)
+    assert p.nbf5 == P
+    x = 0.5 * rng.standard_normal(ndoc * ncwo)
+    E, g = nof.OccFunction(J, K, Hc, p)(x)
+    res, grad = ops.OccMinimizer(P, no1, ndoc, ncwo).energy_grad(*_dev(x, J, K, Hc))
+    assert abs(res.cpu().numpy()[0] - E) <= 1e-13 * abs(E)
+    assert nrel(grad.cpu().numpy(), g) < 1e-11
+
+
 @pytest.mark.parametrize("case", CASES)
 def test_minimize_matches_scipy(torch_cuda, case):
     import scipy.optimize
