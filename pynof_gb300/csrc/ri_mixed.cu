@@ -40,6 +40,25 @@ int half_transform_gemm(const SlicedDesc& A, const SlicedDesc& bT, int N, int P,
   return ozaki_gemm(A, bT, gt, s);
 }
 
+// The slices of the orbitals C^T (rows q over K = m: element C[m][q]), the first
+// launch of a chain that begins with the exponents and counters in `meta` preset.
+// Few of them are preset by the slicing's exponent kernel: a memset ahead of the
+// chain is one more launch that nothing overlaps (a JK build at nbf=24 68.7 us with
+// it, 63.3 without, an orbital step at nbf=53 307 and 303, a build at nbf=171 373 and
+// 370).  Many (64 a
+// thread of one CTA and up) take the memset: the kernel has a CTA per 32 orbitals.
+int slice_orbitals(const double* C, int N, const SlicedDesc& A, void* meta, size_t meta_bytes, cudaStream_t s) {
+  constexpr size_t kKernelWords = 16384;
+  SliceSrc src{C, 0, lin(1), lin(N), false};
+  if (meta_bytes / sizeof(int) <= kKernelWords) {
+    src.preset = static_cast<unsigned int*>(meta);
+    src.preset_n = (int)(meta_bytes / sizeof(int));
+  } else {
+    GB_TRY(cuda_status(cudaMemsetAsync(meta, META_PRESET_BYTE, meta_bytes, s), "exponents and counters"));
+  }
+  return slice_operand(src, A, s);
+}
+
 struct Prepared {
   SlicedDesc bT, bJ;
 };
@@ -134,10 +153,7 @@ namespace {
 // Leaves T, d's slices and the row exponents of T's slicing in the
 // workspace for jkj_mixed_jr and jkj_mixed_k.
 int jkj_mixed_t(const double* C, const Prepared& pr, const JkjMixedWs& w, int N, int P, int Q, cudaStream_t s) {
-  // first, so that the kernels after it follow each other closely
-  GB_TRY(cuda_status(cudaMemsetAsync(w.meta, META_PRESET_BYTE, w.meta_bytes, s), "JK build: exponents and counters"));
-  // A rows q over K = m: element C[m][q]
-  GB_TRY(slice_operand(SliceSrc{C, 0, lin(1), lin(N), false}, w.A, s));
+  GB_TRY(slice_orbitals(C, N, w.A, w.meta, w.meta_bytes, s));
   // T[q][(n,l)] = sum_m C[m][q] b[m][(n,l)]
   GB_TRY(half_transform_gemm(w.A, pr.bT, N, P, Q, w.Tf, w.ctr, s, META_PRESET));
   // the contraction also records the row exponents of T's slicing (jkj_mixed_k)
@@ -434,12 +450,6 @@ int hcore_f64(const double* C, const double* H, int N, int P, double* X, double*
 // error and both are the form's results.  Nor where the rows are not alone the
 // unit stride.
 int mo_symmetry(int P, int Q, int S) { return S == 6 && Q > 1 && P > 1 ? SYM_BATCHCOL : SYM_NONE; }
-
-int half_transform_mixed(const double* C, const SlicedDesc& A, const SlicedDesc& bT, int N, int P, int Q,
-                         double* Tf, unsigned int* ctr, cudaStream_t s) {
-  GB_TRY(slice_operand(SliceSrc{C, 0, lin(1), lin(N), false}, A, s));
-  return half_transform_gemm(A, bT, N, P, Q, Tf, ctr, s, META_PRESET);
-}
 }  // namespace
 
 extern "C" size_t gb_jkh_mo_ri_workspace_mixed(int nbf, int nbf5, int naux, int nslices) {
@@ -464,8 +474,8 @@ extern "C" int gb_jkh_mo_ri_mixed(const double* C, const double* H, const void* 
   JkhMixedWs w;
   jkh_mixed_layout(wc, N, P, Q, S, &w);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  GB_TRY(cuda_status(cudaMemsetAsync(w.ctr, META_PRESET_BYTE, 3 * sizeof(int), s), "tile counters"));
-  GB_TRY(half_transform_mixed(C, w.A, pr.bT, N, P, Q, w.Tf, w.ctr, s));
+  GB_TRY(slice_orbitals(C, N, w.A, w.ctr, 3 * sizeof(int), s));
+  GB_TRY(half_transform_gemm(w.A, pr.bT, N, P, Q, w.Tf, w.ctr, s, META_PRESET));
   // T read with rows l and K = n: element T[p][n][l]
   GB_TRY(slice_operand(SliceSrc{w.Tf, (long long)N * Q, lin(1), lin(Q), false}, w.Tt, s));
   OzGemm gq{};
@@ -590,10 +600,8 @@ int lagrange2_mixed_body(const double* C, const double* H, const void* prep, con
   Lag2MixedWs w;
   lag2_mixed_layout(wc, N, P, Q, S, &w);
 
-  // first, so that the kernels after it follow each other closely
-  GB_TRY(cuda_status(cudaMemsetAsync(w.meta, META_PRESET_BYTE, w.meta_bytes, s), "lagrange2: exponents and counters"));
   // C^T rows a < nbf5 (K = m): the half transform's and the MO transform's A
-  GB_TRY(slice_operand(SliceSrc{C, 0, lin(1), lin(N), false}, w.Ap, s));
+  GB_TRY(slice_orbitals(C, N, w.Ap, w.meta, w.meta_bytes, s));
   GB_TRY(half_transform_gemm(w.Ap, pr.bT, N, P, Q, w.Tf, w.ctr, s, META_PRESET));
   const int qps = P / w.ns;  // orbitals per K range of the exchange GEMM
   const bool digits = w.Tt.kind == 0;

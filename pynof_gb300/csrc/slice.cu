@@ -146,6 +146,9 @@ __global__ void __launch_bounds__(256) rowexp_rfast_kernel(SliceSrc src, int row
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const long long row = (long long)blockIdx.x * 32 + lane;
   if (w == 0) clear_norms(norms, b, (long long)blockIdx.x * 32, rows, lane);
+  if (b == 0)
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < src.preset_n; i += gridDim.x * blockDim.x)
+      src.preset[i] = META_PRESET;
   unsigned long long mx = 0;
   if (row < rows) {
     const double* base = src.p + b * src.sb + src.row_at(row);
@@ -397,6 +400,8 @@ int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bo
   GB_REQUIRE((reinterpret_cast<uintptr_t>(dst.planes) & 15) == 0, GB_ERR_INVALID_ARG,
              "slice_operand: planes not 16-byte aligned");
   if (dst.rows == 0 || dst.K == 0) return GB_OK;
+  GB_REQUIRE(!src.preset || (!src.kfast && !exps_ready), GB_ERR_INVALID_ARG,
+             "slice_operand: words are preset by the exponent kernel of unit-stride rows");
   int* norms = dst.kind == 0 ? dst.norms : nullptr;
   GB_REQUIRE(dst.kind != 0 || norms, GB_ERR_INVALID_ARG, "slice_operand: no norms");
   int* st = status ? status : device_status_word();
@@ -410,8 +415,8 @@ int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bo
     z = z < dst.K / 2048 ? z : dst.K / 2048;
     GB_TRY(cuda_status(cudaMemsetAsync(dst.exps, 0x80, sizeof(int) * sliced_meta_ints(dst.batch, dst.rows), s),
                        "slice_operand: exponents"));
-    GB_LAUNCH_CHAIN("slice_rowexp", s, rowexp_kfast_split_kernel, dim3(dim3(cdiv(dst.rows, 8), dst.batch,
-                    (unsigned)z)), dim3(256), 0,  src, dst.rows, dst.K, dst.exps, st);
+    GB_LAUNCH_CHAIN("slice_rowexp", s, rowexp_kfast_split_kernel,
+                    dim3(cdiv(dst.rows, 8), dst.batch, (unsigned)z), dim3(256), 0, src, dst.rows, dst.K, dst.exps, st);
   } else if (src.kfast) {
     GB_LAUNCH_CHAIN("slice_rowexp", s, rowexp_kfast_kernel, dim3(cdiv(dst.rows, 8), dst.batch), dim3(256), 0, src,
                     dst.rows, dst.K, dst.exps, norms, st);
@@ -422,7 +427,7 @@ int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bo
   const long long blocks = (long long)dst.rblocks() * dst.kblocks();
   GB_REQUIRE(blocks <= 2147483647LL, GB_ERR_BAD_SHAPE, "slice_operand: too many blocks");
   if (dst.kind == 1) {
-    GB_LAUNCH_CHAIN("slice_tf32", s, tf32_blocked_kernel, dim3(dim3((unsigned)blocks, dst.batch)), dim3(256), 0, src,
+    GB_LAUNCH_CHAIN("slice_tf32", s, tf32_blocked_kernel, dim3((unsigned)blocks, dst.batch), dim3(256), 0, src,
                     dst);
     return GB_OK;
   }

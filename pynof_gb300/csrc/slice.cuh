@@ -86,11 +86,16 @@ struct SliceSrc {
   int tri_n = 0;
   long long row0 = 0;  // row 0 of the slices is row row0 of the source (a panel of its rows)
   // The exchange operand (six digits, recorded exponents; its k runs of k.div
-  // follow each other): with ex_scale the element of row r in k run q = batch ex_runs + k / k.div is ex_scale[r ex_n + q]
-  // times the source's, and -ex_diag[r k.div + k % k.div] in run q == r.
+  // follow each other): with ex_scale the element of row r in k run q = batch
+  // ex_runs + k / k.div is ex_scale[r ex_n + q] times the source's, and
+  // -ex_diag[r k.div + k % k.div] in run q == r.
   const double* ex_scale = nullptr;
   const double* ex_diag = nullptr;
   int ex_n = 0, ex_runs = 0;
+  // words that the exponent kernel of unit-stride rows presets to META_PRESET for
+  // the kernels after it
+  unsigned int* preset = nullptr;
+  int preset_n = 0;
   __host__ __device__ __forceinline__ long long row_at(long long row) const {
     if (tri_n <= 0) return r.at(row0 + row);
     int m, n;
