@@ -16,28 +16,17 @@ using namespace gb;
 
 namespace {
 
-// Orbitals on the N side of the tiles (the ragged last tile is only as wide as
-// it needs) when that pads less than 128-row tiles of orbitals: e.g. 300
-// orbitals take 304 columns instead of 384 rows.
-bool orbitals_on_n(long long P, long long rows) {
-  const long long rows128 = (rows + 127) / 128 * 128;
-  const long long normal = (P + 127) / 128 * 128 * rows128;
-  const long long swapped = rows128 * (P / 128 * 128 + ((P % 128) + 15) / 16 * 16);
-  return swapped <= normal;  // equal: the rows-fast form, which runs persistent
-}
-
-// T[q][(n,l)] = sum_m C[m][q] b[m][(n,l)] from the sliced C^T (A, rows q) and b (bT)
+// T[q][(n,l)] = sum_m C[m][q] b[m][(n,l)] from the sliced C^T (A, rows q) and b (bT).
+// Orbitals are on the N side of the tiles here and in J: the ragged last tile is only
+// as wide as it needs (300 orbitals take 304 columns instead of 384 rows), and the
+// rows are the unit stride, which runs persistent.
 int half_transform_gemm(const SlicedDesc& A, const SlicedDesc& bT, int N, int P, int Q, double* Tf,
                         unsigned int* ctr, cudaStream_t s, unsigned int ctr_start = 0) {
   OzGemm gt{};
   gt.K = N; gt.batch = 1; gt.S = A.code(); gt.C = Tf; gt.c_sb = 0; gt.sym = SYM_NONE; gt.tag = "ozaki_tc:half_transform";
   gt.tile_counter = ctr; gt.counter_start = ctr_start;
-  if (orbitals_on_n(P, (long long)N * Q)) {
-    gt.M = N * Q; gt.N = P; gt.c_r = lin(1); gt.c_c = lin((long long)N * Q);
-    return ozaki_gemm(bT, A, gt, s);
-  }
-  gt.M = P; gt.N = N * Q; gt.c_r = lin((long long)N * Q); gt.c_c = lin(1);
-  return ozaki_gemm(A, bT, gt, s);
+  gt.M = N * Q; gt.N = P; gt.c_r = lin(1); gt.c_c = lin((long long)N * Q);
+  return ozaki_gemm(bT, A, gt, s);
 }
 
 // The slices of the orbitals C^T (rows q over K = m: element C[m][q]), the first
@@ -46,7 +35,7 @@ int half_transform_gemm(const SlicedDesc& A, const SlicedDesc& bT, int N, int P,
 // chain is one more launch that nothing overlaps (a JK build at nbf=24 68.7 us with
 // it, 63.3 without, an orbital step at nbf=53 307 and 303, a build at nbf=171 373 and
 // 370).  Many (64 a
-// thread of one CTA and up) take the memset: the kernel has a CTA per 32 orbitals.
+// thread of one CTA) take the memset: the kernel has a CTA per 32 orbitals.
 int slice_orbitals(const double* C, int N, const SlicedDesc& A, void* meta, size_t meta_bytes, cudaStream_t s) {
   constexpr size_t kKernelWords = 16384;
   SliceSrc src{C, 0, lin(1), lin(N), false};
@@ -72,7 +61,6 @@ void prepared_layout(C& c, int N, int Q, int S, Prepared* out) {
     out->bJ = j;
   }
 }
-
 
 int check_mixed(int N, int P, int Q, int S) {
   GB_REQUIRE(N > 0 && P > 0 && Q > 0 && P <= N, GB_ERR_BAD_SHAPE,
@@ -178,12 +166,8 @@ int jkj_mixed_jr(const Prepared& pr, const JkjMixedWs& w, int N, int P, int Q, i
   gj.K = Q; gj.batch = 1; gj.S = S; gj.C = J + (size_t)q0 * N * N; gj.c_sb = 0; gj.pair_n = N; gj.tag = "ozaki_tc:J";
   gj.tile_counter = w.ctr + (whole ? 1 : 3); gj.counter_start = whole ? META_PRESET : 0;
   const int npairs = N * (N + 1) / 2;
-  if (orbitals_on_n(P, npairs)) {
-    gj.M = npairs; gj.N = q1 - q0; gj.c_r = lin(1); gj.c_c = lin((long long)N * N); gj.sym = SYM_TRIROW;
-    return ozaki_gemm(pr.bJ, d, gj, s);
-  }
-  gj.M = q1 - q0; gj.N = npairs; gj.c_r = lin((long long)N * N); gj.c_c = lin(1); gj.sym = SYM_TRICOL;
-  return ozaki_gemm(d, pr.bJ, gj, s);
+  gj.M = npairs; gj.N = q1 - q0; gj.c_r = lin(1); gj.c_c = lin((long long)N * N); gj.sym = SYM_TRIROW;
+  return ozaki_gemm(pr.bJ, d, gj, s);
 }
 
 // The J half of the build: the prelude, then J for every orbital.
@@ -548,7 +532,8 @@ void lag2_mixed_layout(Cv& c, int N, int P, int Q, int S, Lag2MixedWs* w) {
   auto* tf = c.template take<double>((size_t)P * N * Q);
   SlicedDesc Tt = take_planes(c, P, Q, N, S, next);
   auto* bmo = c.template take<double>((size_t)P * P * Q);
-  auto* Y = S == 6 && (Q > 1 || P == 1) ? nullptr : c.template take<double>((size_t)P * P * Q);  // (six digits: cut from bMO directly)
+  // (six digits: cut from bMO directly)
+  auto* Y = S == 6 && (Q > 1 || P == 1) ? nullptr : c.template take<double>((size_t)P * P * Q);
   SlicedDesc Sx = take_planes(c, ns, N, kc, S, next);
   SlicedDesc Sy = take_planes(c, ns, P, kc, S, next);
   auto* part = ns > 1 ? c.template take<double>((size_t)ns * N * P) : nullptr;

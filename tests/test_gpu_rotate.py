@@ -45,6 +45,20 @@ def test_rotate_matches_scipy(torch_cuda, N, P, scale):
     assert err < 1e-12
 
 
+@pytest.mark.parametrize("N,P", [(2, 1), (7, 7), (8, 4), (9, 9), (65, 33), (371, 200), (449, 100)])
+def test_rotate_symmetric_products(torch_cuda, N, P):
+    """The half-computed products' edges (8 x 8 blocks of the triangle, and the sizes
+    that take the tensor cores), held to test_rotate_matches_scipy's bound."""
+    from oracle import pynof_oracle as orc
+    from pynof_gb300 import ops
+
+    rng = np.random.default_rng(N)
+    y = rng.standard_normal(_nvar(N, P)) * 0.1
+    C, _ = np.linalg.qr(rng.standard_normal((N, N)))
+    out = ops.rotate_orbital(ops.to_device(y), ops.to_device(C), P).cpu().numpy()
+    assert nrel(out, orc.rotate_orbital(y, C, _p(N, P))) < 1e-12
+
+
 def test_rotate_identity_and_orthogonality(torch_cuda):
     from pynof_gb300 import ops
 
