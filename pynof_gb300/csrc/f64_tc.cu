@@ -531,8 +531,9 @@ Plan make_plan(long long M, long long N, long long K, int batch, bool a_shared, 
   const double all_tiles = (double)tiles(p.xr, p.yr) * batch * (sym == SYM_ROWCOL ? 0.55 : 1.0);
   // Rule: the estimated time against gemm_f64's.  Measured on GB300: a stage of a
   // tile takes ~1300 clocks at ~2 GHz, slicing moves 30 bytes an element at ~5 TB/s,
-  // the seven launches of a GEMM ~60 us (at 300^3, 62 us of FP64 arithmetic, this took 85); the FP64 pipe gives 1.0 TFLOP/s when its
-  // 64 x 64 tiles fill the SMs (gemm_f64's other kernel less).
+  // the seven launches of a GEMM ~60 us (at 300^3, 62 us of FP64 arithmetic, this
+  // took 80); the FP64 pipe gives 1.0 TFLOP/s when its 64 x 64 tiles fill the SMs
+  // (gemm_f64's other kernel less).
   const double el = (double)M * K * (a_shared ? 1 : batch) + (double)n * K * (b_shared ? 1 : batch);
   const double ctas = std::min(152.0, all_tiles * (double)std::max(1ll, nkb / 16));
   const double t_tc = 60e-6 + el * 30.0 / 5e12 + all_tiles * nkb * 1300.0 / 2e9 / ctas;

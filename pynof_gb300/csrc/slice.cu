@@ -136,11 +136,14 @@ __global__ void rowexp_kfast_split_kernel(SliceSrc src, int rows, int K, int* __
 }
 
 // Rows are the unit-stride index: 32 consecutive rows per CTA (lane = row,
-// each warp reads 256 contiguous bytes per k) and its 8 warps split K; the
-// partial maxima meet in shared memory.
-__global__ void __launch_bounds__(256) rowexp_rfast_kernel(SliceSrc src, int rows, int K, int* __restrict__ exps,
-                                                           int* __restrict__ norms, int* status) {
-  __shared__ unsigned long long part[8][32];
+// each warp reads 256 contiguous bytes per k) and its 8 warps split K, or 32 warps
+// where the grid has fewer CTAs than two per SM (a warp's loads follow each other,
+// ~0.3 us each: C^T's pass at nbf=600 21 us with 8, 14 with 32); the partial maxima
+// meet in shared memory.
+template <int NW>
+__global__ void __launch_bounds__(32 * NW) rowexp_rfast_kernel(SliceSrc src, int rows, int K, int* __restrict__ exps,
+                                                               int* __restrict__ norms, int* status) {
+  __shared__ unsigned long long part[NW][32];
   chain_wait();
   const long long b = blockIdx.y;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -152,7 +155,7 @@ __global__ void __launch_bounds__(256) rowexp_rfast_kernel(SliceSrc src, int row
   unsigned long long mx = 0;
   if (row < rows) {
     const double* base = src.p + b * src.sb + src.row_at(row);
-    for (int k = w; k < K; k += 8) {
+    for (int k = w; k < K; k += NW) {
       const unsigned long long v = abs_bits(base[src.k.at(k)]);
       mx = v > mx ? v : mx;
     }
@@ -161,7 +164,7 @@ __global__ void __launch_bounds__(256) rowexp_rfast_kernel(SliceSrc src, int row
   __syncthreads();
   if (w == 0 && row < rows) {
 #pragma unroll
-    for (int j = 1; j < 8; ++j) mx = part[j][lane] > mx ? part[j][lane] : mx;
+    for (int j = 1; j < NW; ++j) mx = part[j][lane] > mx ? part[j][lane] : mx;
     exps[b * rows + row] = exponent_of(mx);
     note_nonfinite(mx, status);
   }
@@ -421,8 +424,13 @@ int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bo
     GB_LAUNCH_CHAIN("slice_rowexp", s, rowexp_kfast_kernel, dim3(cdiv(dst.rows, 8), dst.batch), dim3(256), 0, src,
                     dst.rows, dst.K, dst.exps, norms, st);
   } else {
-    GB_LAUNCH_CHAIN("slice_rowexp", s, rowexp_rfast_kernel, dim3(cdiv(dst.rows, 32), dst.batch), dim3(256), 0, src,
-                    dst.rows, dst.K, dst.exps, norms, st);
+    const dim3 grid(cdiv(dst.rows, 32), dst.batch);
+    if ((long long)grid.x * dst.batch < 304)
+      GB_LAUNCH_CHAIN("slice_rowexp", s, rowexp_rfast_kernel<32>, grid, dim3(1024), 0, src, dst.rows, dst.K, dst.exps,
+                      norms, st);
+    else
+      GB_LAUNCH_CHAIN("slice_rowexp", s, rowexp_rfast_kernel<8>, grid, dim3(256), 0, src, dst.rows, dst.K, dst.exps,
+                      norms, st);
   }
   const long long blocks = (long long)dst.rblocks() * dst.kblocks();
   GB_REQUIRE(blocks <= 2147483647LL, GB_ERR_BAD_SHAPE, "slice_operand: too many blocks");
