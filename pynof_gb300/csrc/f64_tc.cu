@@ -1,19 +1,31 @@
 // FP64-accurate GEMM on the tensor cores: see f64_tc.cuh.
 //
 // One persistent CTA per SM, 18 warps as in ozaki_tc.cu: a producer (one bulk
-// copy of A's slices and two per slice of B's per 16-k stage, five stages), the
-// MMA issuer, and 16 epilogue warps.  CTA tile 128 x 64: five exact accumulators
-// and the FP32 one take 384 TMEM columns (a 128-wide tile's six would need 768),
-// and an epilogue thread keeps 16 elements, each as a 64-bit integer and an FP64
+// copy of A's planes and two per plane of B's per 16-k stage, four stages), the
+// MMA issuer, and 16 epilogue warps.  CTA tile 128 x 64: five exact accumulators,
+// the FP32 one and the sizes' take 448 TMEM columns (a 128-wide tile's would need
+// 896), and an epilogue thread keeps 16 elements, each as a 64-bit integer and an FP64
 // sum, in registers.
 //
-// What bounds it: per 16-k stage 28 products of 128 x 64, of which the exact ones
-// run as MMAs up to 256 columns wide (consecutive B slices into consecutive
-// accumulators); a 64-column MMA takes 53 clocks, 83 % of a 128-column one, so a
-// stage is ~1100 clocks of MMAs.
+// What bounds it: per 16-k stage 28 products of 128 x 64 and the one of the sizes, of
+// which the exact ones run as MMAs up to 256 columns wide (consecutive B slices into
+// consecutive accumulators); a 64-column MMA takes 53 clocks, 83 % of a 128-column
+// one, so a stage is ~1150 clocks of MMAs.
+//
+// Which tiles are done: an element is held to FP64's bound by its sum of sizes P,
+// about S = sum_k |a_k b_k| over the product of its two row bounds.  The dropped
+// digits and digit products leave 2^-63.2 sqrt(K) of the row bounds (exact emulation of
+// Gaussian, graded and decaying rows, K = 40 .. 2000; 2^-60 K with every digit at its
+// largest), FP64 arithmetic up to 2^-53 K S and typically ~2^-54.5 sqrt(K) S where a
+// few terms dominate.  P >= 2^-6 keeps the first an order of magnitude below the second.
+// Gaussian rows, also ones that fall off by e^-0.05 per k, have P of 0.04 and more.  A
+// tile with an element below (P > 0: an element whose products are all zero is exact) is
+// not stored: gemm_f64's kernel, launched behind this one, computes the 64 x 64
+// tiles that are not marked done.
 #include "f64_tc.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "tc_prims.cuh"
@@ -21,15 +33,16 @@
 namespace gb {
 namespace {
 
-constexpr int S = 7, GE = 6, GMAX = 8;
-constexpr int BM = TC_BM, BN = 64, STAGES = 5, CW = BN / 4;
+constexpr int S = F64_DIGITS, PL = F64_PLANES, GE = 6, GMAX = 8;
+constexpr int BM = TC_BM, BN = 64, STAGES = 4, CW = BN / 4;
 constexpr int THREADS = 32 * (2 + NUM_EPI_WARPS), MAX_REGS = 96;
-constexpr uint32_t A_BYTES = S * SL_TILE_BYTES, B_BYTES = S * BN * SL_K * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+constexpr uint32_t A_BYTES = PL * SL_TILE_BYTES, B_BYTES = PL * BN * SL_K * 2, STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t TABLE_BYTES = 20u * (BM + BN);
 constexpr size_t SMEM_BYTES = (size_t)STAGES * STAGE_BYTES + TABLE_BYTES + 256 + 1024;
 constexpr int SUPER = 64;   // stages (1024 k) an element's 64-bit sum covers: |sum| < 1024 * 1.01 * 2^52 < 2^63
 constexpr int CH_MIN = 3;   // stages per chunk whatever the digits are: 5 * 2^16 * 48 < 2^24 - 2^16 units of group 6
+constexpr float SIZE_MIN = 0x1p-6f;  // smallest sum of sizes of an element stored here
 constexpr float LIM_TOP = 4194304.0f - 65536.0f, LIM = 16777216.0f - 65536.0f;
 
 struct DArgs {
@@ -43,9 +56,13 @@ struct DArgs {
   double alpha, beta;
   int nsplit, kbs;  // K splits and stages per split; partial sums go to part
   double* part;     // [split][batch][j][i]
+  float* psize;     // the splits' sums of sizes, as part
+  int* done;        // gemm_f64's tiles (GemmF64::done): splits stored, then DONE_TILE
+  int b_off, done_i, done_j;  // batch entry 0's; tiles of 64 over all rows / columns
+  int swap;         // the rows are the GEMM's columns
   const int* nonfinite;
-  int* status;  // the device's status word (timeouts)
   unsigned int* counter;
+  int* status;  // the device's status word (timeouts)
   unsigned long long wait_ns;
   int ntiles;
 };
@@ -53,6 +70,13 @@ struct DArgs {
 __device__ __forceinline__ void give_up(volatile int* abort_flag, int* status) {
   *abort_flag = 1;
   if (status) atomicCAS(status, 0, GB_ERR_TIMEOUT);
+}
+
+// gemm_f64's word of the 64 x 64 tile of rows from i, columns from j of batch entry b.
+__device__ __forceinline__ int* done_word(const DArgs& a, int b, int i, int j) {
+  const int ti = (a.m_off + i) / 64, tj = (a.n_off + j) / 64;
+  const long long r = a.swap ? tj : ti, c = a.swap ? ti : tj;
+  return a.done + ((a.b_off + b) * (long long)(a.swap ? a.done_j : a.done_i) + r) * (a.swap ? a.done_i : a.done_j) + c;
 }
 
 // Tile -> (split, batch, m0, n0); false for tiles a symmetric output does not
@@ -131,10 +155,22 @@ __device__ __forceinline__ long long exact_sum(float x2, float x3, float x4, flo
   return (long long)magic_int(x2, U2) * (1ll << 36) + (long long)magic_int(mid, U4) * (1ll << 18) + magic_int(low, U6);
 }
 
+// R plus the FP32 group f (units of 2^-52; |f| < 2^20 of them) as a double: where R
+// leaves room the fraction of f is kept to 2^-7 units.
+__device__ __forceinline__ double with_rest(long long R, float f) {
+  const int m = magic_int(f, 0x1p52f);
+  const int rest = magic_int(fmaf(f, 0x1p52f, -(float)m), 128.0f);
+  R += m;
+  const bool room = (unsigned long long)(R + (1ll << 55)) < (1ull << 56);
+  const double d = __ll2double_rn(room ? R * 128 + rest : R);
+  const int h = __double2hiint(d);
+  return room && h != 0 ? __hiloint2double(h - (7 << 20), __double2loint(d)) : d;
+}
+
 __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArgs a) {
   chain_wait();
   extern __shared__ unsigned char smem_raw[];
-  if (*a.nonfinite != 0) return;  // gemm_f64's kernel does this one
+  if (*a.nonfinite != 0) return;  // gemm_f64's kernel computes every tile
   unsigned char* smem =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   long long* e_roff = reinterpret_cast<long long*>(smem + STAGES * STAGE_BYTES);
@@ -148,7 +184,7 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 14);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 15);
   constexpr int RING = 4;
-  static_assert(2 * STAGES + 4 <= 14 && 24 * 8 + 2 * RING * 4 <= 256, "barrier block");
+  static_assert(2 * STAGES <= 10 && 24 * 8 + 2 * RING * 4 <= 256, "barrier block");
   volatile int* ring = reinterpret_cast<volatile int*>(bars + 24);
   volatile int* ringc = ring + RING;
   const uint32_t sbase = smem_u32(smem), bar0 = smem_u32(bars);
@@ -216,7 +252,7 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
         const unsigned char* ga = reinterpret_cast<const unsigned char*>(a.A.planes) + abz * a.A.batch_bytes() +
                                   (long long)(m0 / BM) * nkb * A_BYTES;
         const unsigned char* gbp = reinterpret_cast<const unsigned char*>(a.B.planes) + bbz * a.B.batch_bytes() +
-                                   (long long)(n0 / SL_ROWS) * nkb * (S * SL_TILE_BYTES) + ((n0 % SL_ROWS) / 8) * 128;
+                                   (long long)(n0 / SL_ROWS) * nkb * (PL * SL_TILE_BYTES) + ((n0 % SL_ROWS) / 8) * 128;
         for (int kb = kb0; kb < kb1; ++kb) {
           const int st = gkb % STAGES;
           if (!mbar_wait(empty_bar(st), (uint32_t)(((gkb / STAGES) & 1) ^ 1), abort_flag, a.wait_ns)) {
@@ -227,9 +263,9 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
           mbar_expect_tx(full_bar(st), STAGE_BYTES);
           const uint32_t sa = sbase + st * STAGE_BYTES;
           bulk_load(sa, ga + (long long)kb * A_BYTES, A_BYTES, full_bar(st));
-          const unsigned char* gblk = gbp + (long long)kb * (S * SL_TILE_BYTES);
+          const unsigned char* gblk = gbp + (long long)kb * (PL * SL_TILE_BYTES);
 #pragma unroll
-          for (int x = 0; x < 2 * S; ++x)  // 64 rows of each slice of each k group
+          for (int x = 0; x < 2 * PL; ++x)  // 64 rows of each plane of each k group
             bulk_load(sa + A_BYTES + x * (BN * 16), gblk + x * SL_SLICE_STEP, BN * 16, full_bar(st));
           ++gkb;
         }
@@ -264,7 +300,7 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
           if (ok) {
             tc_fence_after();
             const uint32_t sa = sbase + st * STAGE_BYTES;
-            const uint64_t da = desc_tile(sa, S * BM), db = desc_tile(sa + A_BYTES, S * BN);
+            const uint64_t da = desc_tile(sa, PL * BM), db = desc_tile(sa + A_BYTES, PL * BN);
             if (kc > 0 || gch == 0) {
               issue_products<S, GE, GMAX, BN, 0, true>(tmem, da, db, 0, kc == 0, kc == 0);
             } else if (ks == 0) {
@@ -278,6 +314,10 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
               ok = drained(accempty_bar, gch);
               if (ok) issue_products<S, GE, GMAX, BN, 2, true>(tmem, da, db, 0, true, false);
             }
+            // the sizes, over the whole tile (read with its last FP32 group)
+            if (ok)
+              mma_bf16(tmem + GE * BN, da + (uint64_t)(S * (SL_SLICE_STEP >> 4)), db + (uint64_t)(S * BN), mma_idesc(BN),
+                       kb > kb0);
           }
           if (!ok) {
             give_up(abort_flag, a.status);
@@ -364,7 +404,7 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
       epi_barrier_any(false);  // tables visible
       double acc[CW];
       long long R[CW];
-      bool ok = true;
+      bool ok = true, graded = false;
       for (int s0 = kb0; s0 < kb1 && ok; s0 += SUPER) {
         const int s1 = min(s0 + SUPER, kb1);
 #pragma unroll
@@ -394,30 +434,56 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
           if (lane == 0) mbar_arrive(accempty_bar);
         }
         if (!ok) break;
-        // the FP32 group's whole units (below 2^20; what is below half a unit, 2^-53
-        // of the row bounds, is less than FP64 arithmetic loses from ~50 k on)
+        // the FP32 group (below 2^20 units), and into FP64: one conversion an element
+        // (the FP64 pipe takes ~2 a clock and SM), one addition more from the second
+        // 1024 k on
 #pragma unroll
         for (int h = 0; h < CW / 4; ++h) {
           uint32_t f[4];
           tmem_ld4_async(lbase + (uint32_t)((GE - 1) * BN + h * 4), f);
           tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 4; ++j) R[h * 4 + j] += magic_int(__uint_as_float(f[j]), 0x1p52f);
+          for (int j = 0; j < 4; ++j) {
+            const double d = with_rest(R[h * 4 + j], __uint_as_float(f[j]));
+            acc[h * 4 + j] = s0 == kb0 ? d : acc[h * 4 + j] + d;
+          }
+          asm volatile("" ::: "memory");  // four columns at a time: R and the sums hold 64 of the 96 registers
+        }
+        if (s1 == kb1) {
+          // the tile's sums of sizes
+          float* ps = nullptr;
+          int pn = 0;  // columns to keep
+          if (parts && m0 + row < a.M) {
+            pn = a.N - n0 - cg * CW;
+            ps = a.psize + (((long long)sp * a.batch + bz) * a.N + n0 + cg * CW) * a.M + m0 + row;
+          }
+#pragma unroll
+          for (int h = 0; h < CW / 4; ++h) {
+            uint32_t p[4];
+            tmem_ld4_async(lbase + (uint32_t)(GE * BN + h * 4), p);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float v = __uint_as_float(p[j]);
+              graded |= !parts && v > 0.0f && v < SIZE_MIN;
+              if (h * 4 + j < pn) *ps = v;
+              ps += a.M;
+            }
+          }
         }
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(fempty_bar);
-        // into FP64: one conversion an element (the FP64 pipe takes ~2 a clock and
-        // SM), one addition more from the second 1024 k on
-        if (s0 == kb0) {
-#pragma unroll
-          for (int j = 0; j < CW; ++j) acc[j] = __ll2double_rn(R[j]);
-        } else {
-#pragma unroll
-          for (int j = 0; j < CW; ++j) acc[j] += __ll2double_rn(R[j]);
-        }
       }
-      if (!ok) continue;  // the next tile's barrier sees the abort flag in every warp
+      // stored by all warps or by none (after an abort the next tile's barrier ends them)
+      if (epi_barrier_any(!ok || graded)) continue;
+      if (et < 2 && m0 + 64 * et < a.M) {
+        int* d = done_word(a, bz, m0 + 64 * et, n0);
+        if (parts)
+          atomicAdd(d, 1);
+        else
+          *d = DONE_TILE;
+      }
       const int gi = m0 + row;
       if (gi < a.M) {
         double* Cb = parts ? a.part + ((long long)sp * a.batch + bz) * (long long)a.M * a.N : a.C + (long long)bz * a.c_sb;
@@ -460,35 +526,47 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
   }
 }
 
-// Partial sums of the K splits, in order, into the output.
+// Partial sums of the K splits, in order, into the output: a CTA per 64 x 64 tile that
+// every split has stored and none of whose elements' sums of sizes is too small.
 __global__ void __launch_bounds__(256) sum_parts_kernel(const __grid_constant__ DArgs a) {
   chain_wait();
-  if (*a.nonfinite != 0) return;
+  const int bz = blockIdx.z, i0 = blockIdx.x * 64, j0 = blockIdx.y * 64;
+  if (a.sym == SYM_ROWCOL && i0 > j0) return;
+  int* done = done_word(a, bz, i0, j0);
+  if (*done != a.nsplit) return;
   const long long MN = (long long)a.M * a.N, all = MN * a.batch;
-  const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
-  if (idx >= all) return;
-  const int bz = (int)(idx / MN);
-  const long long r = idx % MN;
-  const int i = (int)(r % a.M), j = (int)(r / a.M);
-  if (a.sym == SYM_ROWCOL && j < i) return;
-  double v = 0.0;
-  for (int s = 0; s < a.nsplit; ++s) v += a.part[s * all + idx];
-  const long long gi = (long long)a.m_off + i, gj = (long long)a.n_off + j;
-  long long off, moff = -1;
-  int mm, nn;
-  if (a.sym == SYM_TRIROW) {
-    tri_pair(gi, a.pair_n, mm, nn);
-    off = a.c_r.at((long long)mm * a.pair_n + nn) + a.c_c.at(gj);
-    if (nn > mm) moff = a.c_r.at((long long)nn * a.pair_n + mm) + a.c_c.at(gj);
-  } else if (a.sym == SYM_TRICOL) {
-    tri_pair(gj, a.pair_n, mm, nn);
-    off = a.c_r.at(gi) + a.c_c.at((long long)mm * a.pair_n + nn);
-    if (nn > mm) moff = a.c_r.at(gi) + a.c_c.at((long long)nn * a.pair_n + mm);
-  } else {
-    off = a.c_r.at(gi) + a.c_c.at(gj);
-    if (a.sym == SYM_ROWCOL && j > i) moff = a.c_r.at(gj) + a.c_c.at(gi);
+  const int i = i0 + (threadIdx.x & 63), jb = j0 + (threadIdx.x >> 6);
+  const bool row = i < a.M;
+  bool graded = false;
+  for (int j = jb; row && j < min(j0 + 64, a.N); j += 4) {
+    float p = 0.0f;
+    for (int s = 0; s < a.nsplit; ++s) p += a.psize[s * all + bz * MN + (long long)j * a.M + i];
+    graded |= p > 0.0f && p < SIZE_MIN;
   }
-  put(a, a.C + (long long)bz * a.c_sb, off, moff, v);
+  if (__syncthreads_or(graded)) return;
+  if (threadIdx.x == 0) *done = DONE_TILE;
+  for (int j = jb; row && j < min(j0 + 64, a.N); j += 4) {
+    if (a.sym == SYM_ROWCOL && j < i) continue;
+    const long long idx = bz * MN + (long long)j * a.M + i;
+    double v = 0.0;
+    for (int s = 0; s < a.nsplit; ++s) v += a.part[s * all + idx];
+    const long long gi = (long long)a.m_off + i, gj = (long long)a.n_off + j;
+    long long off, moff = -1;
+    int mm, nn;
+    if (a.sym == SYM_TRIROW) {
+      tri_pair(gi, a.pair_n, mm, nn);
+      off = a.c_r.at((long long)mm * a.pair_n + nn) + a.c_c.at(gj);
+      if (nn > mm) moff = a.c_r.at((long long)nn * a.pair_n + mm) + a.c_c.at(gj);
+    } else if (a.sym == SYM_TRICOL) {
+      tri_pair(gj, a.pair_n, mm, nn);
+      off = a.c_r.at(gi) + a.c_c.at((long long)mm * a.pair_n + nn);
+      if (nn > mm) moff = a.c_r.at(gi) + a.c_c.at((long long)nn * a.pair_n + mm);
+    } else {
+      off = a.c_r.at(gi) + a.c_c.at(gj);
+      if (a.sym == SYM_ROWCOL && j > i) moff = a.c_r.at(gj) + a.c_c.at(gi);
+    }
+    put(a, a.C + (long long)bz * a.c_sb, off, moff, v);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -511,9 +589,13 @@ struct Plan {
   int pb = 1;                // batch entries per panel
   long long px = 0, py = 0;  // rows of X, Y per panel
   int nsplit = 1, kbs = 0;   // K splits per panel, stages each
-  size_t xb = 0, yb = 0, partb = 0;
-  size_t bytes() const { return 256 + xb + yb + partb; }
+  size_t xb = 0, yb = 0, partb = 0, doneb = 0;
+  size_t bytes() const { return doneb + xb + yb + partb; }
 };
+
+// Words in front of the done tiles: [0] non-finite operand, [1] tile counter.
+constexpr size_t WORDS = 2;
+size_t done_words(long long M, long long N, int batch) { return (size_t)((M + 63) / 64 * ((N + 63) / 64) * batch); }
 
 Plan make_plan(long long M, long long N, long long K, int batch, bool a_shared, bool b_shared, int sym, int pair_n) {
   Plan p;
@@ -530,13 +612,13 @@ Plan make_plan(long long M, long long N, long long K, int batch, bool a_shared, 
   if (p.xr > (1 << 30) || p.yr > (1 << 30) || K > (1 << 30) || K >= (1ll << 31) - 16) return p;
   const double all_tiles = (double)tiles(p.xr, p.yr) * batch * (sym == SYM_ROWCOL ? 0.55 : 1.0);
   // Rule: the estimated time against gemm_f64's.  Measured on GB300: a stage of a
-  // tile takes ~1300 clocks at ~2 GHz, slicing moves 30 bytes an element at ~5 TB/s,
+  // tile takes ~1300 clocks at ~2 GHz, slicing moves 32 bytes an element at ~5 TB/s,
   // the seven launches of a GEMM ~60 us (at 300^3, 62 us of FP64 arithmetic, this
   // took 80); the FP64 pipe gives 1.0 TFLOP/s when its 64 x 64 tiles fill the SMs
   // (gemm_f64's other kernel less).
   const double el = (double)M * K * (a_shared ? 1 : batch) + (double)n * K * (b_shared ? 1 : batch);
   const double ctas = std::min(152.0, all_tiles * (double)std::max(1ll, nkb / 16));
-  const double t_tc = 60e-6 + el * 30.0 / 5e12 + all_tiles * nkb * 1300.0 / 2e9 / ctas;
+  const double t_tc = 60e-6 + el * 32.0 / 5e12 + all_tiles * nkb * 1300.0 / 2e9 / ctas;
   const double t_f64 = 2.0 * M * N * K * batch * (sym == SYM_NONE ? 1.0 : 0.5) / 1.0e12;
   p.use = t_tc < 0.7 * t_f64;
   if (!p.use) return p;
@@ -585,7 +667,9 @@ Plan make_plan(long long M, long long N, long long K, int batch, bool a_shared, 
   }
   p.kbs = (int)kbs;
   p.nsplit = (int)((nkb + kbs - 1) / kbs);
-  p.partb = p.nsplit > 1 ? align256(sizeof(double) * (size_t)p.nsplit * p.pb * p.px * p.py) : 0;
+  const size_t parts = p.nsplit > 1 ? (size_t)p.nsplit * p.pb * p.px * p.py : 0;
+  p.partb = align256(sizeof(double) * parts) + align256(sizeof(float) * parts);
+  p.doneb = align256(sizeof(int) * (WORDS + done_words(M, n, batch)));
   return p;
 }
 
@@ -623,7 +707,9 @@ int gemm_f64_tc(const GemmF64& g, const TcWork& w, cudaStream_t s) {
   if (!p.use || !w.p || w.bytes < p.bytes() || (g.beta != 0.0 && panels)) return gemm_f64(g, s);
   GB_TRY(configure());
   Carve cv(w.p, w.bytes);
-  int* words = cv.take<int>(2);  // [0] non-finite operand, [1] tile counter
+  const long long n = p.tri ? (long long)g.pair_n * (g.pair_n + 1) / 2 : g.N;
+  const size_t nwords = WORDS + done_words(g.M, n, g.batch);
+  int* words = cv.take<int>(nwords);
   auto sliced = [&](long long batch, long long rows) { return take_sliced(cv, (int)batch, (int)rows, g.K, SPLIT_F64); };
   const bool xs = p.swap ? b_shared : a_shared, ys = p.swap ? a_shared : b_shared;
   // the sources: A's rows are the M index, B's the N index
@@ -633,9 +719,10 @@ int gemm_f64_tc(const GemmF64& g, const TcWork& w, cudaStream_t s) {
   const bool one = !p.tri && g.M == g.N && g.A.p == g.B.p && g.A.sb == g.B.sb && same_index(g.A.r, g.B.c) &&
                    same_index(g.A.c, g.B.r) && p.px == p.xr && p.py == p.yr;
   SlicedDesc X = sliced(xs ? 1 : p.pb, p.px), Y = one ? X : sliced(ys ? 1 : p.pb, p.py);
-  double* part = p.nsplit > 1 ? cv.take<double>((size_t)p.nsplit * p.pb * p.px * p.py) : nullptr;
-  int* status = device_status_word();
-  GB_TRY(cuda_status(cudaMemsetAsync(words, 0, 2 * sizeof(int), s), "f64_tc: words"));
+  const size_t parts = p.nsplit > 1 ? (size_t)p.nsplit * p.pb * p.px * p.py : 0;
+  double* part = parts ? cv.take<double>(parts) : nullptr;
+  float* psize = parts ? cv.take<float>(parts) : nullptr;
+  GB_TRY(cuda_status(cudaMemsetAsync(words, 0, nwords * sizeof(int), s), "f64_tc: words"));
   bool first = true;
   for (int b0 = 0; b0 < g.batch; b0 += p.pb) {
     const int nb = std::min(p.pb, g.batch - b0);
@@ -682,24 +769,34 @@ int gemm_f64_tc(const GemmF64& g, const TcWork& w, cudaStream_t s) {
         a.nsplit = p.nsplit;
         a.kbs = p.kbs;
         a.part = part;
+        a.psize = psize;
+        a.done = words + WORDS;
+        a.b_off = b0;
+        a.done_i = (int)((p.xr + 63) / 64);
+        a.done_j = (int)((p.yr + 63) / 64);
+        a.swap = p.swap;
         a.nonfinite = words;
-        a.status = status;
         a.counter = reinterpret_cast<unsigned int*>(words + 1);
+        a.status = device_status_word();
         a.wait_ns = 2000000000ull;
         a.ntiles = (int)(((xn + BM - 1) / BM) * (long long)((yn + BN - 1) / BN) * nb * p.nsplit);
         const unsigned grid = (unsigned)std::min(a.ntiles, 152);
         GB_LAUNCH_CHAIN(g.tag, s, f64_tc_kernel, dim3(grid), dim3(THREADS), SMEM_BYTES, a);
         if (p.nsplit > 1) {
-          const long long all = (long long)xn * yn * nb;
-          GB_LAUNCH_CHAIN("f64_tc:sum_parts", s, sum_parts_kernel, dim3((unsigned)((all + 255) / 256)), dim3(256), 0,
-                          a);
+          GB_LAUNCH_CHAIN("f64_tc:sum_parts", s, sum_parts_kernel,
+                          dim3((unsigned)((xn + 63) / 64), (unsigned)((yn + 63) / 64), (unsigned)nb), dim3(256), 0, a);
         }
       }
     }
   }
-  // a NaN or an infinity in an operand: FP64 arithmetic, as before
+  // FP64 arithmetic for the tiles that are not done: graded rows, and every tile where
+  // an operand holds a NaN or an infinity
   GemmF64 f = g;
-  f.only_if = words;
+  f.done = words + WORDS;
+  if (p.tri) {
+    f.sym = SYM_TRICOL;
+    f.N = (int)n;
+  }
   return gemm_f64(f, s);
 }
 

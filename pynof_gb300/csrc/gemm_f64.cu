@@ -18,6 +18,13 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
                : "d"(a), "d"(b));
 }
 
+// Packed pair r -> m * n + n' of its pair (m, n').
+__device__ __forceinline__ long long pair_index(long long r, int n) {
+  int a, b;
+  tri_pair(r, n, a, b);
+  return (long long)a * n + b;
+}
+
 // Loader for one operand tile of R rows (the non-K index) x BKT (the K index).
 // KFAST: consecutive threads take consecutive k (16 k x 8 rows per pass);
 // otherwise consecutive threads take consecutive rows (64 rows x 2 k per pass).
@@ -27,7 +34,9 @@ struct TileLoader {
   bool ok[8];
   int lane_k, lane_r;
 
-  __device__ void init(const Index2& rmap, int r0, int rlim) {
+  // tri_n > 0: the rows are the packed pairs of tri_n (SYM_TRICOL)
+  __device__ void init(const Index2& rmap, int r0, int rlim, int tri_n = 0) {
+    auto at = [&](int r) { return rmap.at(tri_n > 0 ? pair_index(r, tri_n) : r); };
     const int tid = threadIdx.x;
     if (KFAST) {
       lane_k = tid & 15;
@@ -36,14 +45,14 @@ struct TileLoader {
       for (int i = 0; i < 8; ++i) {
         int r = r0 + lane_r + 8 * i;
         ok[i] = r < rlim;
-        off[i] = ok[i] ? rmap.at(r) : 0;
+        off[i] = ok[i] ? at(r) : 0;
       }
     } else {
       lane_r = tid & 63;
       lane_k = tid >> 6;
       int r = r0 + lane_r;
       ok[0] = r < rlim;
-      off[0] = ok[0] ? rmap.at(r) : 0;
+      off[0] = ok[0] ? at(r) : 0;
     }
   }
 
@@ -79,16 +88,22 @@ struct TileLoader {
   }
 };
 
+__device__ __forceinline__ bool tile_done(const GemmF64& g, int m0, int n0, long long bz) {
+  if (!g.done) return false;
+  const long long mt = (g.M + BM - 1) / BM, nt = (g.N + BN - 1) / BN;
+  return g.done[(bz * mt + m0 / BM) * nt + n0 / BN] == DONE_TILE;
+}
+
 template <bool AK, bool BKF>
 __global__ void __launch_bounds__(THREADS) gemm_f64_kernel(const GemmF64 g) {
   chain_wait();
   __shared__ double As[2][BKT][BM + PAD];
   __shared__ double Bs[2][BKT][BN + PAD];
 
-  if (g.only_if && *g.only_if == 0) return;
   const int m0 = blockIdx.y * BM;
   const int n0 = blockIdx.x * BN;
   const long long bz = blockIdx.z;
+  if (tile_done(g, m0, n0, bz)) return;
 
   if (g.sym == SYM_ROWCOL && m0 > n0) return;
   if (g.sym == SYM_PAIRCOL) {
@@ -103,7 +118,7 @@ __global__ void __launch_bounds__(THREADS) gemm_f64_kernel(const GemmF64 g) {
   TileLoader<AK> la;
   TileLoader<BKF> lb;
   la.init(g.A.r, m0, g.M);   // A rows are the M index, A columns the K index
-  lb.init(g.B.c, n0, g.N);   // B columns are the N index, B rows the K index
+  lb.init(g.B.c, n0, g.N, g.sym == SYM_TRICOL ? g.pair_n : 0);   // B columns are the N index, B rows the K index
 
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -167,13 +182,17 @@ __global__ void __launch_bounds__(THREADS) gemm_f64_kernel(const GemmF64 g) {
         const int j = n0 + wn * 32 + b * 8 + 2 * tq + e;
         if (j >= g.N) continue;
         double v = g.alpha * acc[a][b][e];
-        double* dst = Cb + ri + g.C.c.at(j);
+        double* dst = Cb + ri + g.C.c.at(g.sym == SYM_TRICOL ? pair_index(j, g.pair_n) : j);
         if (g.beta != 0.0) v += g.beta * *dst;
         *dst = v;
         if (mirror_rc) {
           Cb[g.C.r.at(j) + g.C.c.at(i)] = v;
         } else if (g.sym == SYM_PAIRCOL) {
           const int mm = j / g.pair_n, nn = j % g.pair_n;
+          if (nn > mm) Cb[ri + g.C.c.at((long long)nn * g.pair_n + mm)] = v;
+        } else if (g.sym == SYM_TRICOL) {
+          int mm, nn;
+          tri_pair(j, g.pair_n, mm, nn);
           if (nn > mm) Cb[ri + g.C.c.at((long long)nn * g.pair_n + mm)] = v;
         }
       }
@@ -189,7 +208,6 @@ __global__ void __launch_bounds__(THREADS) gemm_f64_kernel(const GemmF64 g) {
 template <int UNR>
 __global__ void __launch_bounds__(32) gemm_f64_small_kernel(const GemmF64 g) {
   chain_wait();
-  if (g.only_if && *g.only_if == 0) return;
   const int lane = threadIdx.x;
   int m0 = blockIdx.y * 8, n0 = blockIdx.x * 8;
   const long long bz = blockIdx.z;
@@ -201,6 +219,7 @@ __global__ void __launch_bounds__(32) gemm_f64_small_kernel(const GemmF64 g) {
     m0 *= 8;
     n0 *= 8;
   }
+  if (tile_done(g, m0, n0, bz)) return;
   if (g.sym == SYM_PAIRCOL) {
     const int j1 = min(n0 + 8, g.N) - 1;
     const int ma = n0 / g.pair_n, mb = j1 / g.pair_n;
@@ -210,7 +229,8 @@ __global__ void __launch_bounds__(32) gemm_f64_small_kernel(const GemmF64 g) {
   const int ia = m0 + gq, jb = n0 + gq;  // A row / B column of this lane's fragments
   const bool iok = ia < g.M, jok = jb < g.N;
   const double* __restrict__ Ab = g.A.p + bz * g.A.sb + (iok ? g.A.r.at(ia) : 0);
-  const double* __restrict__ Bb = g.B.p + bz * g.B.sb + (jok ? g.B.c.at(jb) : 0);
+  const double* __restrict__ Bb =
+      g.B.p + bz * g.B.sb + (jok ? g.B.c.at(g.sym == SYM_TRICOL ? pair_index(jb, g.pair_n) : jb) : 0);
   double c0 = 0.0, c1 = 0.0;
   for (int k0 = 0; k0 < g.K; k0 += 4 * UNR) {
     double a[UNR], b[UNR];
@@ -235,13 +255,17 @@ __global__ void __launch_bounds__(32) gemm_f64_small_kernel(const GemmF64 g) {
     if (j >= g.N) continue;
     if (g.sym == SYM_ROWCOL && m0 == n0 && j < i) continue;  // the diagonal block's mirror writes these
     double v = g.alpha * (e ? c1 : c0);
-    double* dst = Cb + ri + g.C.c.at(j);
+    double* dst = Cb + ri + g.C.c.at(g.sym == SYM_TRICOL ? pair_index(j, g.pair_n) : j);
     if (g.beta != 0.0) v += g.beta * *dst;
     *dst = v;
     if (g.sym == SYM_ROWCOL && (mirror_rc || j > i)) {
       Cb[g.C.r.at(j) + g.C.c.at(i)] = v;
     } else if (g.sym == SYM_PAIRCOL) {
       const int mm = j / g.pair_n, nn = j % g.pair_n;
+      if (nn > mm) Cb[ri + g.C.c.at((long long)nn * g.pair_n + mm)] = v;
+    } else if (g.sym == SYM_TRICOL) {
+      int mm, nn;
+      tri_pair(j, g.pair_n, mm, nn);
       if (nn > mm) Cb[ri + g.C.c.at((long long)nn * g.pair_n + mm)] = v;
     }
   }
@@ -257,6 +281,8 @@ int gemm_f64(const GemmF64& g, cudaStream_t stream) {
   GB_REQUIRE(g.sym != SYM_ROWCOL || g.M == g.N, GB_ERR_BAD_SHAPE, "gemm_f64: SYM_ROWCOL needs M == N");
   GB_REQUIRE(g.sym != SYM_PAIRCOL || (g.pair_n > 0 && (long long)g.pair_n * g.pair_n == g.N),
              GB_ERR_BAD_SHAPE, "gemm_f64: SYM_PAIRCOL needs N == pair_n^2");
+  GB_REQUIRE(g.sym != SYM_TRICOL || (g.pair_n > 0 && (long long)g.pair_n * (g.pair_n + 1) / 2 == g.N),
+             GB_ERR_BAD_SHAPE, "gemm_f64: SYM_TRICOL needs N == pair_n (pair_n + 1) / 2");
   const long long gy = (g.M + BM - 1) / BM;
   const long long gx = (g.N + BN - 1) / BN;
   GB_REQUIRE(gy <= 65535 && g.batch <= 65535 && gx <= 2147483647LL, GB_ERR_BAD_SHAPE,

@@ -13,7 +13,9 @@
 //   SYM_PAIRCOL  columns encode an index pair j = m * pair_n + n and the
 //                output is symmetric in (m, n): tiles whose every column has
 //                n < m are skipped, columns with n > m are also written to
-//                n * pair_n + m.
+//                n * pair_n + m;
+//   SYM_TRICOL   the same with the columns j the packed upper triangle of the
+//                pairs (tri_pair), pair_n (pair_n + 1) / 2 of them.
 #pragma once
 
 #include "gb_common.cuh"
@@ -39,11 +41,10 @@ struct OutF64 {
   Index2 r, c;
 };
 
-// SYM_TRIROW / SYM_TRICOL (tensor-core path only, where they replace
-// SYM_PAIRCOL): rows (columns) are the packed upper triangle of the pairs,
-// r -> (m, n) with m <= n (tri_pair), pair_n (pair_n + 1) / 2 of them; the
-// output at pair m * pair_n + n is written, and for n > m also its mirror
-// n * pair_n + m.
+// SYM_TRIROW (tensor-core paths only, as SYM_PAIRCOL is not for them) / SYM_TRICOL:
+// rows (columns) are the packed upper triangle of the pairs, r -> (m, n) with
+// m <= n (tri_pair), pair_n (pair_n + 1) / 2 of them; the output at pair
+// m * pair_n + n is written, and for n > m also its mirror n * pair_n + m.
 // SYM_BATCHCOL (persistent tensor-core kernel only): the batch index and the
 // column are one symmetric pair (batch == N): columns up to the batch index are
 // computed, each also written as column `batch` of batch entry `column`.
@@ -79,8 +80,11 @@ struct GemmF64 {
   bool a_kfast;  // A's K index is the unit-stride one (coalesced along k)
   bool b_kfast;  // B's K index is the unit-stride one
   const char* tag = "gemm_f64";  // profiler label
-  const int* only_if = nullptr;  // run only if this device word is not zero (null: always)
+  // 64 x 64 tiles of the output that are done already: a word per tile (DONE_TILE: done),
+  // columns' tiles fastest, then rows', then the batch.  Null: none.
+  const int* done = nullptr;
 };
+constexpr int DONE_TILE = 1 << 30;
 
 // Plain strided helpers ---------------------------------------------------
 inline Index2 lin(long long s) { return Index2{0, 0, s}; }

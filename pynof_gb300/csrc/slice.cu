@@ -228,12 +228,20 @@ __device__ __forceinline__ void load_group_exchange(const SliceSrc& src, const d
   }
 }
 
-// Digits of the 8 values, packed per slice as 8 bf16 (one 16-byte store each);
+// The size plane's value of an element whose leading digit's FP32 bits are d1.
+__device__ __forceinline__ uint32_t size_bits(double x, uint32_t d1) {
+  const uint32_t a = d1 & 0x7FFFFFFFu;
+  return a != 0 || abs_bits(x) == 0 ? a : (127u - 30u) << 23;
+}
+
+// Digits of the 8 values, packed per slice as 8 bf16 (one 16-byte store each), and
+// the size plane behind seven of them;
 // nq[s] += the sum of the squares of the weighted digits of slice s < SL_NORMS
 // (nine-bit digits).
 template <int S, int W>
 __device__ __forceinline__ void store_group(const double (&xs)[8], int e, unsigned char* out, float (&nq)[SL_NORMS]) {
-  uint32_t pk[S][4];
+  constexpr bool SIZES = S == F64_DIGITS;
+  uint32_t pk[S + SIZES][4];
 #pragma unroll
   for (int u = 0; u < 8; u += 2) {
     uint32_t d0[S], d1[S];
@@ -242,14 +250,15 @@ __device__ __forceinline__ void store_group(const double (&xs)[8], int e, unsign
     // the two bf16 patterns (upper halves) side by side
 #pragma unroll
     for (int s = 0; s < S; ++s) pk[s][u >> 1] = __byte_perm(d0[s], d1[s], 0x7632);
+    if constexpr (SIZES) pk[S][u >> 1] = __byte_perm(size_bits(xs[u], d0[0]), size_bits(xs[u + 1], d1[0]), 0x7632);
 #pragma unroll
-    for (int s = 0; s < (W != 9 ? 0 : S == 7 ? SL_NORMS : 3); ++s) {
+    for (int s = 0; s < (W != 9 ? 0 : SIZES ? SL_NORMS : 3); ++s) {
       const float a = __uint_as_float(d0[s]), b = __uint_as_float(d1[s]);
       nq[s] = fmaf(a, a, fmaf(b, b, nq[s]));
     }
   }
 #pragma unroll
-  for (int s = 0; s < S; ++s)
+  for (int s = 0; s < S + SIZES; ++s)
     *reinterpret_cast<uint4*>(out + s * SL_SLICE_STEP) = make_uint4(pk[s][0], pk[s][1], pk[s][2], pk[s][3]);
 }
 
@@ -269,10 +278,11 @@ __device__ __forceinline__ void store_group(const double (&xs)[8], int e, unsign
 // the tighter norms (half transform at nbf=600 6.20 ms, 6.89 with the looser).
 // Three slicings of an nbf=24 build: 41 us with runs of eight, 33 with G = 4, 20.
 template <int S, int W, bool EX = false>
-__global__ void __launch_bounds__(S == 7 ? 256 : 1024, S == 7 ? 3 : 1) digits_blocked_kernel(SliceSrc src, SlicedDesc dst,
-                                                                                                   int kpc) {
-  constexpr int ND = W != 9 ? 0 : S == 7 ? SL_NORMS : 3;  // digits with norms
-  __shared__ float s_nq[S == 7 || W != 9 ? 1 : 3 * 256 * 3];
+__global__ void __launch_bounds__(S == F64_DIGITS ? 256 : 1024, S == F64_DIGITS ? 3 : 1)
+    digits_blocked_kernel(SliceSrc src, SlicedDesc dst, int kpc) {
+  constexpr int ND = W != 9 ? 0 : S == F64_DIGITS ? SL_NORMS : 3;  // digits with norms
+  constexpr int PL = S == F64_DIGITS ? F64_PLANES : S;
+  __shared__ float s_nq[S == F64_DIGITS || W != 9 ? 1 : 3 * 256 * 3];
   chain_wait();
   const long long b = blockIdx.y;
   const int kbn = dst.kblocks();
@@ -287,7 +297,7 @@ __global__ void __launch_bounds__(S == 7 ? 256 : 1024, S == 7 ? 3 : 1) digits_bl
   const double* base = src.p + b * src.sb + (rok ? src.row_at(r) : 0);
   const int e = rok ? dst.exps[b * dst.rows + r] : 0;
   unsigned char* out0 = reinterpret_cast<unsigned char*>(dst.planes) + b * dst.batch_bytes() +
-                        ((long long)rb * kbn * S) * SL_TILE_BYTES + (kg * S * 16 + rg) * 128 + ri * 16;
+                        ((long long)rb * kbn * PL) * SL_TILE_BYTES + (kg * PL * 16 + rg) * 128 + ri * 16;
   double xa[8];
   float nq[SL_NORMS] = {};
   for (int kb = kb0 + grp; kb < kb1; kb += G) {
@@ -295,9 +305,9 @@ __global__ void __launch_bounds__(S == 7 ? 256 : 1024, S == 7 ? 3 : 1) digits_bl
       load_group_exchange(src, base, rok, r, (int)b, kb * SL_K + kg * 8, dst.K, xa);
     else
       load_group(src, base, rok, kb * SL_K + kg * 8, dst.K, xa);
-    store_group<S, W>(xa, e, out0 + (long long)kb * S * SL_TILE_BYTES, nq);
+    store_group<S, W>(xa, e, out0 + (long long)kb * PL * SL_TILE_BYTES, nq);
   }
-  if (S != 7 && ND > 0 && G > 1) {
+  if (S != F64_DIGITS && ND > 0 && G > 1) {
     // the run's sums of squares over the groups
     const int t = threadIdx.x & 255;
     if (grp > 0)
@@ -397,7 +407,7 @@ inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) /
 }  // namespace
 
 int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bool exps_ready, int* status) {
-  GB_REQUIRE((dst.kind == 0 && ((dst.S >= 1 && dst.S <= 5) || dst.S == 7)) || (dst.kind == 1 && dst.S == 2), GB_ERR_INVALID_ARG,
+  GB_REQUIRE((dst.kind == 0 && ((dst.S >= 1 && dst.S <= 5) || dst.S == F64_PLANES)) || (dst.kind == 1 && dst.S == 2), GB_ERR_INVALID_ARG,
              "slice_operand: bad split form (planes %d, kind %d)", dst.S, dst.kind);
   GB_REQUIRE(dst.batch >= 1 && dst.batch <= 65535 && dst.rows >= 0, GB_ERR_BAD_SHAPE, "slice_operand: bad batch");
   GB_REQUIRE((reinterpret_cast<uintptr_t>(dst.planes) & 15) == 0, GB_ERR_INVALID_ARG,
@@ -443,7 +453,7 @@ int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bo
   const bool few = (long long)dst.rblocks() * runs * dst.batch < 304;
   const int kpc = few && runs == 1 ? 1 : SL_KPC;
   const dim3 grid((unsigned)((long long)dst.rblocks() * ((dst.kblocks() + kpc - 1) / kpc)), dst.batch);
-  const dim3 block(few && runs > 1 && dst.S != 7 ? 1024 : 256);
+  const dim3 block(few && runs > 1 && dst.S != F64_PLANES ? 1024 : 256);
   if (src.ex_scale) {
     GB_REQUIRE(exps_ready && src.kfast && src.k.div > 0 && dst.S == 5 && dst.W == 9, GB_ERR_INVALID_ARG,
                "slice_operand: an exchange operand takes six digits and recorded exponents");
@@ -451,11 +461,12 @@ int slice_operand(const SliceSrc& src, const SlicedDesc& dst, cudaStream_t s, bo
     return GB_OK;
   }
   if (dst.W == 9) {
-    GB_REQUIRE(dst.S == 5 || dst.S == 7, GB_ERR_INVALID_ARG, "slice_operand: nine-bit digits come in five or seven planes");
+    GB_REQUIRE(dst.S == 5 || dst.S == F64_PLANES, GB_ERR_INVALID_ARG,
+               "slice_operand: nine-bit digits come in five planes or eight");
     if (dst.S == 5)
       GB_LAUNCH_CHAIN("slice_digits", s, (digits_blocked_kernel<5, 9>), grid, block, 0, src, dst, kpc);
     else
-      GB_LAUNCH_CHAIN("slice_digits7", s, (digits_blocked_kernel<7, 9>), grid, block, 0, src, dst, kpc);
+      GB_LAUNCH_CHAIN("slice_digits7", s, (digits_blocked_kernel<F64_DIGITS, 9>), grid, block, 0, src, dst, kpc);
     return GB_OK;
   }
   switch (dst.S) {

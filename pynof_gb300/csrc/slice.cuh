@@ -29,10 +29,15 @@
 // Blocks are ordered [batch][rb][kb].  Rows and K are zero-padded to whole
 // blocks.  Exponents: exps[b][r] (int32).
 //
-// Norms: norms[b][rb][s - 1], s <= 3 (five planes) or 5 (seven), is the FP32 bit
+// Norms: norms[b][rb][s - 1], s <= 3 (five digits) or 5 (seven), is the FP32 bit
 // pattern of an upper bound of sum d_s^2 over one k group parity (8 of every 16 k)
 // of any run of 128 k of any row of the block; a run's sum of products of two
 // digits is then at most 2 sqrt(norm_a norm_b) (Cauchy-Schwarz).
+//
+// Size plane (the eighth plane of SPLIT_F64): |d_1| 2^-e_1, or 2^-30 where d_1 is zero
+// and the element is not, 0 for a zero.  A sum of products of two size planes is zero
+// only where every product of the elements is, and otherwise sum |a b| over the
+// two row bounds, to the accuracy of the leading digits (below four times it).
 //
 // TF32x3 form (split code SPLIT_TF32X3): two planes, hi = tf32(x 2^-E) and
 // lo = tf32(x 2^-E - hi) (each rounded to nearest even, 11 significant bits,
@@ -55,21 +60,22 @@ constexpr int SL_TILE_BYTES = SL_ROWS * SL_K * 2;  // one slice of one block: 4 
 
 constexpr int SL_SLICE_STEP = SL_ROWS * 16;  // from one slice of a k group to the next
 constexpr int SL_KPC = 8;                  // k blocks per slicer CTA, and per run of the norms
-constexpr int SL_NORMS = 5;                // digits whose norms are recorded (three of five planes, five of seven)
+constexpr int SL_NORMS = 5;                // digits whose norms are recorded (three of five, five of seven)
 
 // Split codes ("nslices" in the C ABI): 1..5 seven-bit digit slices, 6 (42 bits,
 // 21 products of s + t <= 7 if they were seven-bit ones) is five nine-bit slices
 // (45 bits, 15 products of s + t <= 6), or the TF32x3 split.
-// SPLIT_F64 (inside the library only): seven nine-bit slices, 62 bits, for
-// products that are as accurate as FP64 arithmetic (f64_tc.cuh).
+// SPLIT_F64 (inside the library only): seven nine-bit slices, 62 bits, and the size
+// plane, for products that are as accurate as FP64 arithmetic (f64_tc.cuh).
 constexpr int SPLIT_TF32X3 = 32, SPLIT_F64 = 64;
+constexpr int F64_DIGITS = 7, F64_PLANES = 8;
 struct SliceForm {
   int S, kind, W;  // planes; 0 = bf16 digits, 1 = tf32 hi/lo; bits per digit
 };
 __host__ __device__ constexpr bool valid_split(int code) { return (code >= 1 && code <= 6) || code == SPLIT_TF32X3; }
 __host__ __device__ constexpr SliceForm form_of(int code) {
   return code == SPLIT_TF32X3 ? SliceForm{2, 1, 0}
-         : code == SPLIT_F64  ? SliceForm{7, 0, 9}
+         : code == SPLIT_F64  ? SliceForm{F64_PLANES, 0, 9}
          : code == 6          ? SliceForm{5, 0, 9}
                               : SliceForm{code, 0, 7};
 }
@@ -112,7 +118,7 @@ struct SlicedDesc {
   int W = 7;     // bits per digit (kind 0)
   int* norms = nullptr;  // [batch][row block][SL_NORMS], directly behind exps where it is carved (kind 0)
   __host__ __device__ int kper() const { return kind ? SL_K / 2 : SL_K; }
-  __host__ __device__ int code() const { return kind ? SPLIT_TF32X3 : W == 9 ? (S == 7 ? SPLIT_F64 : 6) : S; }  // the split code it was cut with
+  __host__ __device__ int code() const { return kind ? SPLIT_TF32X3 : W == 9 ? (S == F64_PLANES ? SPLIT_F64 : 6) : S; }  // the split code it was cut with
   __host__ __device__ int rblocks() const { return (rows + SL_ROWS - 1) / SL_ROWS; }
   __host__ __device__ int kblocks() const { return (K + kper() - 1) / kper(); }
   __host__ __device__ long long block_bytes() const { return (long long)S * SL_TILE_BYTES; }

@@ -109,3 +109,79 @@ def test_nonfinite_operands_take_fp64_arithmetic(ops, bad):
         assert nrel(got[others], ref[others]) < TOL
     again = _host(*ops.jkj_full(ops.to_device(C), ops.to_device(I), P))
     assert all(np.array_equal(x, y) for x, y in zip(again, good))
+
+
+def _product(ops, A, B):
+    """A B for A (K, K) without a diagonal and B (K, N^2) through fock_rc, whose
+    other terms are zero here (n = 0, H = 0, ck12 = 0)."""
+    K, N = A.shape[0], int(round(B.shape[1] ** 0.5))
+    J, z = ops.to_device(B.reshape(K, N, N)), ops.to_device(np.zeros((K, K)))
+    F = ops.fock_rc(J, J, ops.to_device(np.zeros(K)), ops.to_device(np.zeros((N, N))), ops.to_device(A), z, 1, 1)
+    return F.cpu().numpy().reshape(K, N * N)
+
+
+def _element_error(got, A, B, rows=slice(None), cols=slice(None)):
+    """Largest |got - A B| over sum_k |a_k b_k|, in units of 2^-53, in extended precision."""
+    a, b = A[rows].astype(np.longdouble), B[:, cols].astype(np.longdouble)
+    ref = np.zeros((a.shape[0], b.shape[1]), dtype=np.longdouble)
+    size = ref.copy()
+    for k in range(a.shape[1]):
+        t = a[:, k, None] * b[None, k]
+        ref += t
+        size += np.abs(t)
+    err = np.abs(got[rows][:, cols] - ref)
+    assert (err[size == 0] == 0).all()
+    return float((err[size > 0] / size[size > 0]).max() * 2.0**53)
+
+
+# An FP64 sum of K products is off by at most K 2^-53 sum |a b|, and by ~sqrt(K) of it
+# where the roundings are independent: 2 sqrt(K) for every element holds a product to
+# what FP64 arithmetic gives element by element (a lost bit per factor of two beyond).
+@pytest.mark.parametrize("spread", [0, 10, 20, 40, 200])
+@pytest.mark.parametrize("P,N", [(40, 230), (150, 150)])
+def test_graded_operands_keep_fp64_accuracy(ops, P, N, spread):
+    """Columns of A scaled by d_k and rows of B by 1 / d_k, d_k over 2^spread: every
+    element's leading terms are far below the product of its row bounds."""
+    rng = np.random.default_rng(P + spread)
+    A, B = rng.standard_normal((P, P)), rng.standard_normal((P, N * N))
+    np.fill_diagonal(A, 0.0)
+    d = np.exp2(np.rint(spread * rng.random(P)))
+    assert _element_error(_product(ops, A * d, B / d[:, None]), A * d, B / d[:, None], cols=slice(0, N * N, 37)) < \
+        2 * np.sqrt(P)
+
+
+def test_one_graded_row_among_ungraded(ops):
+    """Row 77 alone meets one column alone badly; the rest of the output is as it was,
+    and products that are all zero give zero."""
+    P, N = 150, 150
+    rng = np.random.default_rng(5)
+    A, B = rng.standard_normal((P, P)), rng.standard_normal((P, N * N))
+    np.fill_diagonal(A, 0.0)
+    plain = _product(ops, A, B)
+    A[77, 0], B[0, 5000] = 1e9, 1e-9  # the row's bound is in k = 0, the column has nothing there
+    A[3], B[:, 200] = 0.0, 0.0
+    A[3, ::2], B[1::2, 200] = 1.0, 1.0
+    A[3, 3] = 0.0
+    got = _product(ops, A, B)
+    assert _element_error(got, A, B, rows=[3, 77, 78], cols=slice(4900, 5100)) < 2 * np.sqrt(P)
+    assert _element_error(got, A, B, rows=slice(0, P, 9), cols=slice(0, N * N, 101)) < 2 * np.sqrt(P)
+    assert got[3, 200] == 0.0
+    keep = np.ones_like(got, dtype=bool)
+    keep[[3, 77]], keep[:, [200, 5000]] = False, False
+    assert nrel(got[keep], (A @ B)[keep]) < TOL and nrel(plain[keep], got[keep]) < 1e-8
+
+
+@pytest.mark.parametrize("spread", [0, 20, 60])
+def test_graded_k_splits(ops, spread):
+    """The same through a long K in splits and packed output pairs (J of the four-index
+    route; D is rounded once more on the way)."""
+    N, P = 60, 40
+    rng = np.random.default_rng(spread)
+    I, C = rng.standard_normal((N, N, N, N)), rng.standard_normal((N, N))
+    I = I + I.transpose(1, 0, 2, 3)
+    d = np.exp2(np.rint(0.5 * spread * rng.random(N)))
+    C, I = C * d[:, None], I / d[:, None] / d
+    J, _ = ops.jkj_full(ops.to_device(C), ops.to_device(I), P)
+    D = np.einsum("si,li->isl", C[:, :P], C[:, :P]).reshape(P, N * N)
+    assert _element_error(J.cpu().numpy().reshape(P, N * N), D, I.reshape(N * N, N * N).T,
+                          rows=slice(0, P, 7), cols=slice(0, N * N, 61)) < 2 * N + 1
