@@ -57,7 +57,7 @@ struct DArgs {
   int nsplit, kbs;  // K splits and stages per split; partial sums go to part
   double* part;     // [split][batch][j][i]
   float* psize;     // the splits' sums of sizes, as part
-  int* done;        // gemm_f64's tiles (GemmF64::done): splits stored, then DONE_TILE
+  int* done;        // gemm_f64's tiles (GemmF64::done): splits stored, GRADED with an element too small
   int b_off, done_i, done_j;  // batch entry 0's; tiles of 64 over all rows / columns
   int swap;         // the rows are the GEMM's columns
   const int* nonfinite;
@@ -71,6 +71,8 @@ __device__ __forceinline__ void give_up(volatile int* abort_flag, int* status) {
   *abort_flag = 1;
   if (status) atomicCAS(status, 0, GB_ERR_TIMEOUT);
 }
+
+constexpr int GRADED = 1 << 20;
 
 // gemm_f64's word of the 64 x 64 tile of rows from i, columns from j of batch entry b.
 __device__ __forceinline__ int* done_word(const DArgs& a, int b, int i, int j) {
@@ -155,16 +157,22 @@ __device__ __forceinline__ long long exact_sum(float x2, float x3, float x4, flo
   return (long long)magic_int(x2, U2) * (1ll << 36) + (long long)magic_int(mid, U4) * (1ll << 18) + magic_int(low, U6);
 }
 
-// R plus the FP32 group f (units of 2^-52; |f| < 2^20 of them) as a double: where R
-// leaves room the fraction of f is kept to 2^-7 units.
-__device__ __forceinline__ double with_rest(long long R, float f) {
+// R plus the FP32 group f (units of 2^-52; |f| < 2^20 of them).  Where R leaves room the
+// result is in units of 2^-59, which keeps f's fraction: true then.
+__device__ __forceinline__ bool add_rest(long long& R, float f) {
   const int m = magic_int(f, 0x1p52f);
   const int rest = magic_int(fmaf(f, 0x1p52f, -(float)m), 128.0f);
   R += m;
   const bool room = (unsigned long long)(R + (1ll << 55)) < (1ull << 56);
-  const double d = __ll2double_rn(room ? R * 128 + rest : R);
+  if (room) R = R * 128 + rest;
+  return room;
+}
+
+// R as a double in units of 2^-52.
+__device__ __forceinline__ double from_units(long long R, bool fine) {
+  const double d = __ll2double_rn(R);
   const int h = __double2hiint(d);
-  return room && h != 0 ? __hiloint2double(h - (7 << 20), __double2loint(d)) : d;
+  return fine && h != 0 ? __hiloint2double(h - (7 << 20), __double2loint(d)) : d;
 }
 
 __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArgs a) {
@@ -434,20 +442,15 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
           if (lane == 0) mbar_arrive(accempty_bar);
         }
         if (!ok) break;
-        // the FP32 group (below 2^20 units), and into FP64: one conversion an element
-        // (the FP64 pipe takes ~2 a clock and SM), one addition more from the second
-        // 1024 k on
+        // the FP32 group
+        uint32_t fine = 0;  // elements in units of 2^-59
 #pragma unroll
         for (int h = 0; h < CW / 4; ++h) {
           uint32_t f[4];
           tmem_ld4_async(lbase + (uint32_t)((GE - 1) * BN + h * 4), f);
           tmem_wait_ld();
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const double d = with_rest(R[h * 4 + j], __uint_as_float(f[j]));
-            acc[h * 4 + j] = s0 == kb0 ? d : acc[h * 4 + j] + d;
-          }
-          asm volatile("" ::: "memory");  // four columns at a time: R and the sums hold 64 of the 96 registers
+          for (int j = 0; j < 4; ++j) fine |= (uint32_t)add_rest(R[h * 4 + j], __uint_as_float(f[j])) << (h * 4 + j);
         }
         if (s1 == kb1) {
           // the tile's sums of sizes
@@ -474,6 +477,13 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(fempty_bar);
+        // into FP64: one conversion an element (the FP64 pipe takes ~2 a clock and SM),
+        // one addition more from the second 1024 k on
+#pragma unroll
+        for (int j = 0; j < CW; ++j) {
+          const double d = from_units(R[j], (fine >> j) & 1u);
+          acc[j] = s0 == kb0 ? d : acc[j] + d;
+        }
       }
       // stored by all warps or by none (after an abort the next tile's barrier ends them)
       if (epi_barrier_any(!ok || graded)) continue;
@@ -482,7 +492,7 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
         if (parts)
           atomicAdd(d, 1);
         else
-          *d = DONE_TILE;
+          *d = 1;
       }
       const int gi = m0 + row;
       if (gi < a.M) {
@@ -526,47 +536,43 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
   }
 }
 
-// Partial sums of the K splits, in order, into the output: a CTA per 64 x 64 tile that
-// every split has stored and none of whose elements' sums of sizes is too small.
+// Partial sums of the K splits, in order, into the output, where every split has stored
+// its tile.  An element whose sum of sizes is too small leaves the tile to gemm_f64's
+// kernel, which writes all of it again.
 __global__ void __launch_bounds__(256) sum_parts_kernel(const __grid_constant__ DArgs a) {
   chain_wait();
-  const int bz = blockIdx.z, i0 = blockIdx.x * 64, j0 = blockIdx.y * 64;
-  if (a.sym == SYM_ROWCOL && i0 > j0) return;
-  int* done = done_word(a, bz, i0, j0);
-  if (*done != a.nsplit) return;
   const long long MN = (long long)a.M * a.N, all = MN * a.batch;
-  const int i = i0 + (threadIdx.x & 63), jb = j0 + (threadIdx.x >> 6);
-  const bool row = i < a.M;
-  bool graded = false;
-  for (int j = jb; row && j < min(j0 + 64, a.N); j += 4) {
-    float p = 0.0f;
-    for (int s = 0; s < a.nsplit; ++s) p += a.psize[s * all + bz * MN + (long long)j * a.M + i];
-    graded |= p > 0.0f && p < SIZE_MIN;
+  const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
+  if (idx >= all) return;
+  const int bz = (int)(idx / MN);
+  const long long r = idx % MN;
+  const int i = (int)(r % a.M), j = (int)(r / a.M);
+  if (a.sym == SYM_ROWCOL && j < i) return;
+  int* done = done_word(a, bz, i, j);
+  if ((*(volatile int*)done & (GRADED - 1)) != a.nsplit) return;
+  double v = 0.0;
+  float p = 0.0f;
+  for (int s = 0; s < a.nsplit; ++s) {
+    v += a.part[s * all + idx];
+    p += a.psize[s * all + idx];
   }
-  if (__syncthreads_or(graded)) return;
-  if (threadIdx.x == 0) *done = DONE_TILE;
-  for (int j = jb; row && j < min(j0 + 64, a.N); j += 4) {
-    if (a.sym == SYM_ROWCOL && j < i) continue;
-    const long long idx = bz * MN + (long long)j * a.M + i;
-    double v = 0.0;
-    for (int s = 0; s < a.nsplit; ++s) v += a.part[s * all + idx];
-    const long long gi = (long long)a.m_off + i, gj = (long long)a.n_off + j;
-    long long off, moff = -1;
-    int mm, nn;
-    if (a.sym == SYM_TRIROW) {
-      tri_pair(gi, a.pair_n, mm, nn);
-      off = a.c_r.at((long long)mm * a.pair_n + nn) + a.c_c.at(gj);
-      if (nn > mm) moff = a.c_r.at((long long)nn * a.pair_n + mm) + a.c_c.at(gj);
-    } else if (a.sym == SYM_TRICOL) {
-      tri_pair(gj, a.pair_n, mm, nn);
-      off = a.c_r.at(gi) + a.c_c.at((long long)mm * a.pair_n + nn);
-      if (nn > mm) moff = a.c_r.at(gi) + a.c_c.at((long long)nn * a.pair_n + mm);
-    } else {
-      off = a.c_r.at(gi) + a.c_c.at(gj);
-      if (a.sym == SYM_ROWCOL && j > i) moff = a.c_r.at(gj) + a.c_c.at(gi);
-    }
-    put(a, a.C + (long long)bz * a.c_sb, off, moff, v);
+  if (p > 0.0f && p < SIZE_MIN) atomicOr(done, GRADED);
+  const long long gi = (long long)a.m_off + i, gj = (long long)a.n_off + j;
+  long long off, moff = -1;
+  int mm, nn;
+  if (a.sym == SYM_TRIROW) {
+    tri_pair(gi, a.pair_n, mm, nn);
+    off = a.c_r.at((long long)mm * a.pair_n + nn) + a.c_c.at(gj);
+    if (nn > mm) moff = a.c_r.at((long long)nn * a.pair_n + mm) + a.c_c.at(gj);
+  } else if (a.sym == SYM_TRICOL) {
+    tri_pair(gj, a.pair_n, mm, nn);
+    off = a.c_r.at(gi) + a.c_c.at((long long)mm * a.pair_n + nn);
+    if (nn > mm) moff = a.c_r.at(gi) + a.c_c.at((long long)nn * a.pair_n + mm);
+  } else {
+    off = a.c_r.at(gi) + a.c_c.at(gj);
+    if (a.sym == SYM_ROWCOL && j > i) moff = a.c_r.at(gj) + a.c_c.at(gi);
   }
+  put(a, a.C + (long long)bz * a.c_sb, off, moff, v);
 }
 
 // ---------------------------------------------------------------------------
@@ -701,10 +707,9 @@ size_t gemm_f64_tc_bytes(long long M, long long N, long long K, int batch, bool 
 int gemm_f64_tc(const GemmF64& g, const TcWork& w, cudaStream_t s) {
   const bool a_shared = g.batch == 1 || g.A.sb == 0, b_shared = g.batch == 1 || g.B.sb == 0;
   const Plan p = make_plan(g.M, g.N, g.K, g.batch, a_shared, b_shared, g.sym, g.pair_n);
-  // a second panel cannot follow a first that already added into the output
-  // (a NaN in its rows would have gemm_f64 add again)
-  const bool panels = p.use && (p.pb < g.batch || p.px < p.xr || p.py < p.yr);
-  if (!p.use || !w.p || w.bytes < p.bytes() || (g.beta != 0.0 && panels)) return gemm_f64(g, s);
+  // where the output is added to, no element of a tile is stored before all are known
+  // to be kept, which sum_parts_kernel does not see
+  if (!p.use || !w.p || w.bytes < p.bytes() || (g.beta != 0.0 && p.nsplit > 1)) return gemm_f64(g, s);
   GB_TRY(configure());
   Carve cv(w.p, w.bytes);
   const long long n = p.tri ? (long long)g.pair_n * (g.pair_n + 1) / 2 : g.N;
@@ -783,8 +788,9 @@ int gemm_f64_tc(const GemmF64& g, const TcWork& w, cudaStream_t s) {
         const unsigned grid = (unsigned)std::min(a.ntiles, 152);
         GB_LAUNCH_CHAIN(g.tag, s, f64_tc_kernel, dim3(grid), dim3(THREADS), SMEM_BYTES, a);
         if (p.nsplit > 1) {
-          GB_LAUNCH_CHAIN("f64_tc:sum_parts", s, sum_parts_kernel,
-                          dim3((unsigned)((xn + 63) / 64), (unsigned)((yn + 63) / 64), (unsigned)nb), dim3(256), 0, a);
+          const long long all = (long long)xn * yn * nb;
+          GB_LAUNCH_CHAIN("f64_tc:sum_parts", s, sum_parts_kernel, dim3((unsigned)((all + 255) / 256)), dim3(256), 0,
+                          a);
         }
       }
     }
@@ -793,6 +799,7 @@ int gemm_f64_tc(const GemmF64& g, const TcWork& w, cudaStream_t s) {
   // an operand holds a NaN or an infinity
   GemmF64 f = g;
   f.done = words + WORDS;
+  f.done_value = p.nsplit;
   if (p.tri) {
     f.sym = SYM_TRICOL;
     f.N = (int)n;

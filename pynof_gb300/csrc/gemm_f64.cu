@@ -91,7 +91,7 @@ struct TileLoader {
 __device__ __forceinline__ bool tile_done(const GemmF64& g, int m0, int n0, long long bz) {
   if (!g.done) return false;
   const long long mt = (g.M + BM - 1) / BM, nt = (g.N + BN - 1) / BN;
-  return g.done[(bz * mt + m0 / BM) * nt + n0 / BN] == DONE_TILE;
+  return g.done[(bz * mt + m0 / BM) * nt + n0 / BN] == g.done_value;
 }
 
 template <bool AK, bool BKF>

@@ -80,11 +80,11 @@ struct GemmF64 {
   bool a_kfast;  // A's K index is the unit-stride one (coalesced along k)
   bool b_kfast;  // B's K index is the unit-stride one
   const char* tag = "gemm_f64";  // profiler label
-  // 64 x 64 tiles of the output that are done already: a word per tile (DONE_TILE: done),
-  // columns' tiles fastest, then rows', then the batch.  Null: none.
+  // 64 x 64 tiles of the output that are done already: a word per tile (done_value where
+  // it is), columns' tiles fastest, then rows', then the batch.  Null: none.
   const int* done = nullptr;
+  int done_value = 0;
 };
-constexpr int DONE_TILE = 1 << 30;
 
 // Plain strided helpers ---------------------------------------------------
 inline Index2 lin(long long s) { return Index2{0, 0, s}; }
