@@ -54,6 +54,7 @@ struct DArgs {
   Index2 c_r, c_c;
   int sym, pair_n;  // SYM_NONE, SYM_ROWCOL, SYM_TRIROW, SYM_TRICOL
   double alpha, beta;
+  const double* C0;  // what beta multiplies (C itself where it is added in place)
   int nsplit, kbs;  // K splits and stages per split; partial sums go to part
   double* part;     // [split][batch][j][i]
   float* psize;     // the splits' sums of sizes, as part
@@ -127,12 +128,12 @@ __device__ __forceinline__ double scaled(double v, int scale) {
   return v == 0.0 ? 0.0 : scalbn(v, scale);
 }
 
-// Where element (i, j) of a finished result goes, with its mirror image.
-__device__ __forceinline__ void put(const DArgs& a, double* C, long long off, long long moff, double v) {
+// Element off of batch entry bz's finished result, with its mirror image.
+__device__ __forceinline__ void put(const DArgs& a, int bz, long long off, long long moff, double v) {
+  double* C = a.C + (long long)bz * a.c_sb;
   if (a.alpha != 1.0) v *= a.alpha;
-  double* p = C + off;
-  if (a.beta != 0.0) v = fma(a.beta, *p, v);
-  *p = v;
+  if (a.beta != 0.0) v = fma(a.beta, a.C0[(long long)bz * a.c_sb + off], v);
+  C[off] = v;
   if (moff >= 0) C[moff] = v;
 }
 
@@ -496,7 +497,7 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
       }
       const int gi = m0 + row;
       if (gi < a.M) {
-        double* Cb = parts ? a.part + ((long long)sp * a.batch + bz) * (long long)a.M * a.N : a.C + (long long)bz * a.c_sb;
+        double* Cb = parts ? a.part + ((long long)sp * a.batch + bz) * (long long)a.M * a.N : nullptr;
         const long long ro = e_roff[row], mr = e_mr[row];
         const int srow = e_srow[row];
 #pragma unroll
@@ -508,14 +509,14 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
             if (parts) {
               Cb[ro + co] = v;
             } else if (a.sym == SYM_ROWCOL) {
-              if (gj >= gi) put(a, Cb, ro + co, gj > gi ? mr + e_mc[c] : -1, v);
+              if (gj >= gi) put(a, bz, ro + co, gj > gi ? mr + e_mc[c] : -1, v);
             } else if (a.sym == SYM_TRIROW) {
-              put(a, Cb, ro + co, mr >= 0 ? mr + co : -1, v);
+              put(a, bz, ro + co, mr >= 0 ? mr + co : -1, v);
             } else if (a.sym == SYM_TRICOL) {
               const long long mc = e_mc[c];
-              put(a, Cb, ro + co, mc >= 0 ? ro + mc : -1, v);
+              put(a, bz, ro + co, mc >= 0 ? ro + mc : -1, v);
             } else {
-              put(a, Cb, ro + co, -1, v);
+              put(a, bz, ro + co, -1, v);
             }
           }
           asm volatile("" ::: "memory");
@@ -572,7 +573,7 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const __grid_constant__ 
     off = a.c_r.at(gi) + a.c_c.at(gj);
     if (a.sym == SYM_ROWCOL && j > i) moff = a.c_r.at(gj) + a.c_c.at(gi);
   }
-  put(a, a.C + (long long)bz * a.c_sb, off, moff, v);
+  put(a, bz, off, moff, v);
 }
 
 // ---------------------------------------------------------------------------
@@ -603,7 +604,8 @@ struct Plan {
 constexpr size_t WORDS = 2;
 size_t done_words(long long M, long long N, int batch) { return (size_t)((M + 63) / 64 * ((N + 63) / 64) * batch); }
 
-Plan make_plan(long long M, long long N, long long K, int batch, bool a_shared, bool b_shared, int sym, int pair_n) {
+Plan make_plan(long long M, long long N, long long K, int batch, bool a_shared, bool b_shared, int sym, int pair_n,
+               bool in_place) {
   Plan p;
   if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return p;
   p.tri = sym == SYM_PAIRCOL;
@@ -662,7 +664,9 @@ Plan make_plan(long long M, long long N, long long K, int batch, bool a_shared, 
   const long long pt = tiles(p.px, p.py) * p.pb;
   long long kbs = nkb;
   double best = 1e300;
-  for (long long ns = 1; ns <= 64 && (ns == 1 || nkb / ns >= 16) && (ns == 1 || pt * ns <= 152 * 8); ++ns) {
+  // (none where the output is added to in place: no element of a tile is stored before
+  // all are known to be kept, which sum_parts_kernel does not see)
+  for (long long ns = 1; ns <= (in_place ? 1 : 64) && (ns == 1 || nkb / ns >= 16) && (ns == 1 || pt * ns <= 152 * 8); ++ns) {
     long long k = (nkb + ns - 1) / ns;
     if (ns > 1) k = (k + SL_KPC - 1) / SL_KPC * SL_KPC;
     const double cost = (double)((pt * ((nkb + k - 1) / k) + 151) / 152) * (double)(k + 12);
@@ -699,17 +703,17 @@ bool same_index(const Index2& a, const Index2& b) { return a.div == b.div && a.s
 }  // namespace
 
 size_t gemm_f64_tc_bytes(long long M, long long N, long long K, int batch, bool a_shared, bool b_shared, int sym,
-                         int pair_n) {
-  const Plan p = make_plan(M, N, K, batch, a_shared, b_shared, sym, pair_n);
+                         int pair_n, bool in_place) {
+  const Plan p = make_plan(M, N, K, batch, a_shared, b_shared, sym, pair_n, in_place);
   return p.use ? p.bytes() : 0;
 }
 
 int gemm_f64_tc(const GemmF64& g, const TcWork& w, cudaStream_t s) {
   const bool a_shared = g.batch == 1 || g.A.sb == 0, b_shared = g.batch == 1 || g.B.sb == 0;
-  const Plan p = make_plan(g.M, g.N, g.K, g.batch, a_shared, b_shared, g.sym, g.pair_n);
-  // where the output is added to, no element of a tile is stored before all are known
-  // to be kept, which sum_parts_kernel does not see
-  if (!p.use || !w.p || w.bytes < p.bytes() || (g.beta != 0.0 && p.nsplit > 1)) return gemm_f64(g, s);
+  const double* C0 = g.C0 ? g.C0 : g.C.p;
+  const Plan p = make_plan(g.M, g.N, g.K, g.batch, a_shared, b_shared, g.sym, g.pair_n,
+                           g.beta != 0.0 && C0 == g.C.p);
+  if (!p.use || !w.p || w.bytes < p.bytes()) return gemm_f64(g, s);
   GB_TRY(configure());
   Carve cv(w.p, w.bytes);
   const long long n = p.tri ? (long long)g.pair_n * (g.pair_n + 1) / 2 : g.N;
@@ -771,6 +775,7 @@ int gemm_f64_tc(const GemmF64& g, const TcWork& w, cudaStream_t s) {
         a.pair_n = g.pair_n;
         a.alpha = g.alpha;
         a.beta = g.beta;
+        a.C0 = C0 + (long long)b0 * g.C.sb;
         a.nsplit = p.nsplit;
         a.kbs = p.kbs;
         a.part = part;

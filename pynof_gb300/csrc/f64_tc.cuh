@@ -42,9 +42,10 @@ inline TcWork tc_work(const Carve& c) {
 }
 
 // Bytes gemm_f64_tc takes for a GEMM of these sizes (0: it runs on gemm_f64).
-// a_shared / b_shared: the operand's batch stride is 0.  sym: SYM_PAIRCOL counts the N = pair_n^2 columns.
+// a_shared / b_shared: the operand's batch stride is 0; in_place: beta is not 0 and
+// multiplies C itself.  sym: SYM_PAIRCOL counts the N = pair_n^2 columns.
 size_t gemm_f64_tc_bytes(long long M, long long N, long long K, int batch, bool a_shared, bool b_shared,
-                         int sym = SYM_NONE, int pair_n = 0);
+                         int sym = SYM_NONE, int pair_n = 0, bool in_place = false);
 
 // gemm_f64 with the tensor cores where they are faster.
 int gemm_f64_tc(const GemmF64& g, const TcWork& w, cudaStream_t stream);

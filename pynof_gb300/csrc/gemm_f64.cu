@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(THREADS) gemm_f64_kernel(const GemmF64 g) {
         if (j >= g.N) continue;
         double v = g.alpha * acc[a][b][e];
         double* dst = Cb + ri + g.C.c.at(g.sym == SYM_TRICOL ? pair_index(j, g.pair_n) : j);
-        if (g.beta != 0.0) v += g.beta * *dst;
+        if (g.beta != 0.0) v += g.beta * (g.C0 ? g.C0[dst - g.C.p] : *dst);
         *dst = v;
         if (mirror_rc) {
           Cb[g.C.r.at(j) + g.C.c.at(i)] = v;
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(32) gemm_f64_small_kernel(const GemmF64 g) {
     if (g.sym == SYM_ROWCOL && m0 == n0 && j < i) continue;  // the diagonal block's mirror writes these
     double v = g.alpha * (e ? c1 : c0);
     double* dst = Cb + ri + g.C.c.at(g.sym == SYM_TRICOL ? pair_index(j, g.pair_n) : j);
-    if (g.beta != 0.0) v += g.beta * *dst;
+    if (g.beta != 0.0) v += g.beta * (g.C0 ? g.C0[dst - g.C.p] : *dst);
     *dst = v;
     if (g.sym == SYM_ROWCOL && (mirror_rc || j > i)) {
       Cb[g.C.r.at(j) + g.C.c.at(i)] = v;
@@ -276,8 +276,8 @@ __global__ void __launch_bounds__(32) gemm_f64_small_kernel(const GemmF64 g) {
 int gemm_f64(const GemmF64& g, cudaStream_t stream) {
   if (g.M <= 0 || g.N <= 0 || g.batch <= 0) return GB_OK;
   GB_REQUIRE(g.K >= 0, GB_ERR_BAD_SHAPE, "gemm_f64: negative K");
-  GB_REQUIRE(g.sym == SYM_NONE || g.beta == 0.0, GB_ERR_INVALID_ARG,
-             "gemm_f64: symmetric modes do not take beta");
+  GB_REQUIRE(g.sym == SYM_NONE || g.sym == SYM_ROWCOL || g.beta == 0.0, GB_ERR_INVALID_ARG,
+             "gemm_f64: pair symmetries do not take beta");
   GB_REQUIRE(g.sym != SYM_ROWCOL || g.M == g.N, GB_ERR_BAD_SHAPE, "gemm_f64: SYM_ROWCOL needs M == N");
   GB_REQUIRE(g.sym != SYM_PAIRCOL || (g.pair_n > 0 && (long long)g.pair_n * g.pair_n == g.N),
              GB_ERR_BAD_SHAPE, "gemm_f64: SYM_PAIRCOL needs N == pair_n^2");

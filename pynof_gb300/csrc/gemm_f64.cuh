@@ -74,12 +74,13 @@ struct GemmF64 {
   MatF64 A;  // M x K
   MatF64 B;  // K x N
   OutF64 C;  // M x N
-  double alpha, beta;
+  double alpha, beta;  // beta with SYM_NONE, or SYM_ROWCOL where what is added is symmetric too
   int sym;
   int pair_n;
   bool a_kfast;  // A's K index is the unit-stride one (coalesced along k)
   bool b_kfast;  // B's K index is the unit-stride one
   const char* tag = "gemm_f64";  // profiler label
+  const double* C0 = nullptr;    // what beta multiplies, at C's strides (null: C)
   // 64 x 64 tiles of the output that are done already: a word per tile (done_value where
   // it is), columns' tiles fastest, then rows', then the batch.  Null: none.
   const int* done = nullptr;

@@ -7,16 +7,19 @@
 // Taylor polynomial of X (truncation < 0.5^17 / 17! ~ 2e-20 relative), then s
 // squarings.  X is antisymmetric, so Z = X^2 and every polynomial in it are
 // symmetric, and half of each such product is computed:
-//   p(X) = E(Z) + X O(Z),  E = sum_k Z^k / (2k)!,  O = sum_k Z^k / (2k+1)!,
-//   E = e0 + e1 Z + e2 Z^2 + e3 Z^3 + Z^4 (e4 + e5 Z + e6 Z^2 + e7 Z^3 + e8 Z^4),
+//   p(X) - I = E(Z) + X + X O(Z),  E = sum_(k>0) Z^k / (2k)!,  O = sum_(k>0) Z^k / (2k+1)!,
+//   E = e1 Z + e2 Z^2 + e3 Z^3 + e4 Z^4 + (e5 Z + e6 Z^2 + e7 Z^3 + e8 Z^4) Z^4,
 // O alike with k <= 7.  Products: Z, Z^2, then Z^3 and Z^4 as one launch, both
 // brackets times Z^4 as one launch, and X O, the only one computed whole: four
-// products' work in five launches, where a Horner scheme in X^4 took six of each.
-// Then s squarings and the final C U.  Bound by the FP64 pipe: at nbf=300 with three
-// squarings 481 us, 586 before (the Horner scheme, nine products and C U of 62 us each).
+// products' work in five launches.  Then s squarings of F = p - I, 2 F + F F, and the
+// final C + C F.  Without the identity in them no operand's rows are near multiples
+// of it, whose products the tensor cores would leave to FP64 arithmetic
+// (f64_tc.cuh): at nbf=600 4.8 ms with it, 0.97 ms without, and an error of 2e-15
+// instead of 2e-14.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <utility>
 
 #include "f64_tc.cuh"
 
@@ -54,29 +57,28 @@ __global__ void col_abs_max_kernel(const double* __restrict__ Y, int N, unsigned
 
 // The coefficients of E and O: 1 / (2k)! and 1 / (2k+1)!
 struct Coefs {
-  double e[9], o[9];
+  double e[9], o[8];
 };
 
-// HIGH: the brackets that Z^4 multiplies, dst = [E's, O's], from Z, Z^2 (z) and Z^3,
-// Z^4 (q).  Otherwise the whole: dst = [E, O], from the products w, Z, Z^2 and Z^3.
-template <bool HIGH>
-__global__ void poly_kernel(double* __restrict__ dst, const double* __restrict__ z, const double* __restrict__ q,
-                            const double* __restrict__ w, int N, const __grid_constant__ Coefs c) {
+// From Z, Z^2, Z^4, Z^3 in s[0..3]: E's and O's first four terms into s[0], s[1], their
+// brackets into s[3], s[4].
+__global__ void poly_kernel(double* __restrict__ s, int N, const __grid_constant__ Coefs c) {
   chain_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x, NN = (long long)N * N;
   if (idx >= NN) return;
-  const bool diag = idx / N == idx % N;
-  const double z1 = z[idx], z2 = z[NN + idx], z3 = q[idx], z4 = HIGH ? q[NN + idx] : 0.0;
-  constexpr int B = HIGH ? 4 : 0;
-  double e = HIGH ? c.e[8] * z4 : w[idx], o = HIGH ? 0.0 : w[NN + idx];
-  if (diag) {
-    e += c.e[B];
-    o += c.o[B];
-  }
-  e = fma(c.e[B + 3], z3, fma(c.e[B + 2], z2, fma(c.e[B + 1], z1, e)));
-  o = fma(c.o[B + 3], z3, fma(c.o[B + 2], z2, fma(c.o[B + 1], z1, o)));
-  dst[idx] = e;
-  dst[NN + idx] = o;
+  double* p = s + idx;
+  const double z1 = p[0], z2 = p[NN], z4 = p[2 * NN], z3 = p[3 * NN];
+  auto poly = [&](const double* k) { return fma(k[0], z1, fma(k[1], z2, fma(k[2], z3, k[3] * z4))); };
+  p[0] = poly(c.e + 1);
+  p[NN] = poly(c.o + 1);
+  p[3 * NN] = poly(c.e + 5);
+  p[4 * NN] = fma(c.o[5], z1, fma(c.o[6], z2, c.o[7] * z3));
+}
+
+__global__ void add_kernel(double* __restrict__ dst, const double* __restrict__ src, long long n) {
+  chain_wait();
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx < n) dst[idx] += src[idx];
 }
 
 __global__ void scale_kernel(const double* __restrict__ src, double* __restrict__ dst, long long n, double f) {
@@ -87,30 +89,29 @@ __global__ void scale_kernel(const double* __restrict__ src, double* __restrict_
 
 inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
 
-// C = A B (+ C when accumulate), square row-major N x N; sym: the product is
-// symmetric.  batch: consecutive A and C, one B.
-int matmul(const double* A, const double* B, double* C, int N, bool accumulate, const TcWork& tw, cudaStream_t s,
-           const char* tag, int sym = SYM_NONE, int batch = 1) {
-  const long long NN = batch > 1 ? (long long)N * N : 0;
+// C = A B + beta C0, square row-major N x N; sym: the product is symmetric (and C0).
+// batch: two consecutive A, C cs apart, one B.
+int matmul(const double* A, const double* B, double* C, int N, double beta, const double* C0, const TcWork& tw,
+           cudaStream_t s, const char* tag, int sym = SYM_NONE, long long cs = 0) {
   GemmF64 g{};
-  g.M = N; g.N = N; g.K = N; g.batch = batch;
-  g.A = {A, NN, lin(N), lin(1)};
+  g.M = N; g.N = N; g.K = N; g.batch = cs ? 2 : 1;
+  g.A = {A, cs ? (long long)N * N : 0, lin(N), lin(1)};
   g.B = {B, 0, lin(N), lin(1)};
-  g.C = {C, NN, lin(N), lin(1)};
-  g.alpha = 1.0; g.beta = accumulate ? 1.0 : 0.0; g.sym = sym;
+  g.C = {C, cs, lin(N), lin(1)};
+  g.alpha = 1.0; g.beta = beta; g.sym = sym; g.C0 = C0;
   g.a_kfast = true; g.b_kfast = false;
   g.tag = tag;
   return gemm_f64_tc(g, tw, s);
 }
 
 template <class Cv>
-void rotate_layout(Cv& c, int N, double** bufs, unsigned long long** norm) {
-  // X, then pairs: Z Z^2, Z^3 Z^4, the brackets (then E, O), their products
-  for (int k = 0; k < 5; ++k) {
-    double* p = c.template take<double>((size_t)(k == 0 ? 1 : 2) * N * N);
-    if (bufs) bufs[k] = p;
-  }
+void rotate_layout(Cv& c, int N, double** X, double** S, unsigned long long** norm) {
+  // X, and five consecutive: Z, Z^2, Z^4, Z^3 and one more (poly_kernel)
+  double* x = c.template take<double>((size_t)N * N);
+  double* z = c.template take<double>((size_t)5 * N * N);
   auto* nm = c.template take<unsigned long long>(1);
+  if (X) *X = x;
+  if (S) *S = z;
   if (norm) *norm = nm;
 }
 
@@ -118,10 +119,11 @@ void rotate_layout(Cv& c, int N, double** bufs, unsigned long long** norm) {
 
 extern "C" size_t gb_rotate_orbital_workspace_f64(int nbf) {
   SizeCarve c;
-  rotate_layout(c, nbf, nullptr, nullptr);
+  rotate_layout(c, nbf, nullptr, nullptr, nullptr);
   size_t tc = gemm_f64_tc_bytes(nbf, nbf, nbf, 1, true, true);
   tc = std::max(tc, gemm_f64_tc_bytes(nbf, nbf, nbf, 1, true, true, SYM_ROWCOL));
   tc = std::max(tc, gemm_f64_tc_bytes(nbf, nbf, nbf, 2, false, true, SYM_ROWCOL));
+  tc = std::max(tc, gemm_f64_tc_bytes(nbf, nbf, nbf, 2, false, true, SYM_ROWCOL, 0, true));
   return c.used + align256(tc);
 }
 
@@ -133,16 +135,15 @@ extern "C" int gb_rotate_orbital_f64(const double* y, const double* C, int nbf, 
   GB_REQUIRE(y && C && Cout, GB_ERR_INVALID_ARG, "gb_rotate_orbital_f64: null pointer");
   GB_REQUIRE(C != Cout, GB_ERR_INVALID_ARG, "gb_rotate_orbital_f64: C and Cout must not alias");
   SizeCarve base;
-  rotate_layout(base, N, nullptr, nullptr);
+  rotate_layout(base, N, nullptr, nullptr, nullptr);
   GB_REQUIRE(workspace_bytes >= base.used, GB_ERR_WORKSPACE,
              "gb_rotate_orbital_f64: workspace too small");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   Carve wc(workspace, workspace_bytes);
-  double* buf[5];
+  double *Y, *S;
   unsigned long long* dnorm = nullptr;
-  rotate_layout(wc, N, buf, &dnorm);
+  rotate_layout(wc, N, &Y, &S, &dnorm);
   const TcWork tw = tc_work(wc);
-  double *Y = buf[0], *Z = buf[1], *Q = buf[2], *B = buf[3], *W = buf[4];
   const long long NN = (long long)N * N;
 
   GB_LAUNCH_CHAIN("rotate_build", s, build_antisym_kernel, dim3(cdiv(NN, 256)), dim3(256), 0, y, N, P, Y);
@@ -175,22 +176,21 @@ extern "C" int gb_rotate_orbital_f64(const double* y, const double* C, int nbf, 
     (k % 2 ? c.o : c.e)[k / 2] = f;
   }
   const char* tag = "gemm_f64:expm";
-  GB_TRY(matmul(X, X, Z, N, false, tw, s, tag, SYM_ROWCOL));
-  GB_TRY(matmul(Z, Z, Z + NN, N, false, tw, s, tag, SYM_ROWCOL));
-  GB_TRY(matmul(Z, Z + NN, Q, N, false, tw, s, tag, SYM_ROWCOL, 2));
-  GB_LAUNCH_CHAIN("rotate_poly", s, poly_kernel<true>, dim3(cdiv(NN, 256)), dim3(256), 0, B, Z, Q, nullptr, N, c);
-  GB_TRY(matmul(B, Q + NN, W, N, false, tw, s, tag, SYM_ROWCOL, 2));
-  GB_LAUNCH_CHAIN("rotate_poly", s, poly_kernel<false>, dim3(cdiv(NN, 256)), dim3(256), 0, B, Z, Q, W, N, c);
-  // R = E + X O
-  double* R = B;
-  GB_TRY(matmul(X, B + NN, R, N, true, tw, s, tag));
-  // s squarings, ping-ponging between R and a free buffer
-  double* spare = W;
+  double *Z = S, *Z2 = S + NN, *Z4 = S + 2 * NN, *Z3 = S + 3 * NN;
+  GB_TRY(matmul(X, X, Z, N, 0.0, nullptr, tw, s, tag, SYM_ROWCOL));
+  GB_TRY(matmul(Z, Z, Z2, N, 0.0, nullptr, tw, s, tag, SYM_ROWCOL));
+  GB_TRY(matmul(Z, Z2, Z3, N, 0.0, nullptr, tw, s, tag, SYM_ROWCOL, -NN));
+  GB_LAUNCH_CHAIN("rotate_poly", s, poly_kernel, dim3(cdiv(NN, 256)), dim3(256), 0, S, N, c);
+  // E, O += their brackets (S + 3 NN and on) times Z^4
+  double *E = S, *O = S + NN;
+  GB_TRY(matmul(S + 3 * NN, Z4, E, N, 1.0, E, tw, s, tag, SYM_ROWCOL, NN));
+  // F = (E + X) + X O
+  GB_LAUNCH_CHAIN("rotate_add", s, add_kernel, dim3(cdiv(NN, 256)), dim3(256), 0, E, X, NN);
+  double *F = S + 3 * NN, *spare = S;
+  GB_TRY(matmul(X, O, F, N, 1.0, E, tw, s, tag));
   for (int k = 0; k < sq; ++k) {
-    GB_TRY(matmul(R, R, spare, N, false, tw, s, "gemm_f64:expm"));
-    double* t = R;
-    R = spare;
-    spare = t;
+    GB_TRY(matmul(F, F, spare, N, 2.0, F, tw, s, tag));
+    std::swap(F, spare);
   }
-  return matmul(C, R, Cout, N, false, tw, s, "gemm_f64:rotate");
+  return matmul(C, F, Cout, N, 1.0, C, tw, s, "gemm_f64:rotate");
 }

@@ -110,3 +110,30 @@ def test_host_norm_bound_matches_device_norm(torch_cuda):
     a = ops.rotate_orbital(dy, dC, P).cpu().numpy()
     b = ops.rotate_orbital(dy, dC, P, norm1=ops.AntisymNorm(N, P)(y)).cpu().numpy()
     assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("N,P", [(24, 12), (53, 53), (400, 200)])
+def test_rotate_in_six_matrices_of_workspace(torch_cuda, N, P):
+    """Six N x N matrices and one word (each rounded up to 256 bytes) are workspace
+    enough; what the query asks for beyond is the tensor cores'.  Bound as in
+    test_rotate_matches_scipy."""
+    from oracle import pynof_oracle as orc
+    from pynof_gb300 import _lib, ops
+
+    torch = torch_cuda
+    rng = np.random.default_rng(N)
+    y = rng.standard_normal(_nvar(N, P)) * 0.1
+    C, _ = np.linalg.qr(rng.standard_normal((N, N)))
+    dy, dC = ops.to_device(y), ops.to_device(C)
+    nbytes = 6 * ((8 * N * N + 255) // 256 * 256) + 256
+    ws = torch.empty(nbytes + 256, dtype=torch.uint8, device=dC.device)
+    ws[nbytes:] = 0xA5
+    out = torch.empty_like(dC)
+    _lib.call("gb_rotate_orbital_f64", dy.data_ptr(), dC.data_ptr(), N, P, -1.0, out.data_ptr(), ws.data_ptr(), nbytes,
+              torch.cuda.current_stream().cuda_stream)
+    assert nrel(out.cpu().numpy(), orc.rotate_orbital(y, C, _p(N, P))) < 1e-12
+    assert bool((ws[nbytes:] == 0xA5).all())
+    with pytest.raises(_lib.GBError) as ei:
+        _lib.call("gb_rotate_orbital_f64", dy.data_ptr(), dC.data_ptr(), N, P, -1.0, out.data_ptr(), ws.data_ptr(),
+                  6 * 8 * N * N - 256, torch.cuda.current_stream().cuda_stream)
+    assert ei.value.status == 3
