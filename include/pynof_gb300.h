@@ -341,19 +341,24 @@ int gb_graph_destroy(gb_graph* graph);
  * launch on the device returns without work until the word is cleared
  * (reset != 0), so every caller that reads it after its own work sees the
  * failure.  Synchronises the device.  No counterpart in the reference, which
- * has no device-side failure reporting. */
+ * has no device-side failure reporting.
+ *
+ * The FP64 calls (gb_*_f64) neither read nor set it: what a tensor-core kernel of
+ * theirs leaves undone -- after a wait that ran out, or where an operand holds a
+ * NaN or an infinity -- is computed by FP64 arithmetic behind it. */
 int gb_device_status(int reset, int* status);
 
-/* Limit of every bounded wait inside the split-product kernels launched after
+/* Limit of every bounded wait inside the tensor-core kernels launched after
  * this call, in nanoseconds (0 restores the default of 2 s).  No counterpart
  * in the reference. */
 int gb_set_wait_limit_ns(unsigned long long limit_ns);
 
 /* Test hook for the timeout path, no counterpart in the reference: while
- * stage >= 0, the first CTA of every split-product GEMM launched afterwards
+ * stage >= 0, the first CTA of every tensor-core GEMM launched afterwards
  * never issues the copy of that pipeline stage, so its wait for the stage
  * runs out (after the wait limit), the kernel gives up cleanly and
- * GB_ERR_TIMEOUT is recorded.  stage < 0 turns it off. */
+ * GB_ERR_TIMEOUT is recorded (not by the FP64 calls' kernels).  stage < 0 turns it
+ * off. */
 int gb_test_withhold_stage(int stage);
 
 /* Generic FP64-accurate GEMM on the tensor cores: C = A B^T with row-major

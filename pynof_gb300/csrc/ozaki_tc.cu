@@ -1382,7 +1382,7 @@ std::atomic<unsigned long long> g_wait_limit_ns{kDefaultWaitNs};
 std::atomic<int> g_withhold_stage{-1};
 
 KArgs make_args(const SlicedDesc& A, const SlicedDesc& B, const OzGemm& g) {
-  KArgs ka{g, A, B, frac_bits(g.S, g.K), g_wait_limit_ns.load(), g_withhold_stage.load()};
+  KArgs ka{g, A, B, frac_bits(g.S, g.K), wait_limit_ns(), withheld_stage()};
   if (g.K > FDRAIN_K && g.S != SPLIT_TF32X3) ka.g.fdrain = 1;
   return ka;
 }
@@ -1402,6 +1402,9 @@ int launch_error(const char* tag, cudaError_t le, int S, int BN) {
 }
 
 }  // namespace
+
+unsigned long long wait_limit_ns() { return g_wait_limit_ns.load(); }
+int withheld_stage() { return g_withhold_stage.load(); }
 
 long long ozaki_tiles(const OzGemm& g) {
   return ((long long)(g.M + BM - 1) / BM) * ((g.N + g.bn - 1) / g.bn) * (long long)g.batch;

@@ -74,6 +74,11 @@ int ozaki_gemm_grouped(const void* table, int nprob, long long total_tiles, int 
 // Tiles of one problem (for building the grouped tile ranges).
 long long ozaki_tiles(const OzGemm& g);
 
+// Limit of every bounded wait of the tensor-core kernels, and the stage withheld by
+// the test hook (-1: none), for the launches from now on.
+unsigned long long wait_limit_ns();
+int withheld_stage();
+
 // Device status word of the tensor-core kernels (0 = ok, GB_ERR_TIMEOUT when a
 // bounded wait gave up).  Reading synchronises the current device.
 int ozaki_status(int reset, int* out);

@@ -150,3 +150,50 @@ def test_nonfinite_operand_reported(torch_cuda, clean_status):
     # finite inputs go through again
     ops.jkj_ri_mixed(ops.to_device(C), prep, st.nbf5)
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("stage", [0, 3, 12])
+def test_fp64_gemms_finish_what_a_cta_gave_up_on(torch_cuda, clean_status, stage):
+    """The FP64 calls' tensor-core kernel gives up on a withheld stage (K splits and
+    packed pairs in J, K; accumulation in place in the Fock matrices): FP64 arithmetic
+    behind it computes the tiles that are left, nothing is recorded, and a set status
+    word does not concern them.
+
+    Bound: both runs' elements are within ~sqrt(K) 2^-53 of sum |a b|, which is at most
+    ~sqrt(K) times the largest result for these operands (K <= 4096)."""
+    from pynof_gb300 import _lib, ops
+
+    rng = np.random.default_rng(8)
+    N, P = 64, 60
+    C, I = rng.standard_normal((N, N)), rng.standard_normal((N, N, N, N))
+    I = I + I.transpose(1, 0, 2, 3)
+    n, H, cj, ck = rng.random(P), rng.standard_normal((N, N)), rng.standard_normal((P, P)), rng.standard_normal((P, P))
+    M = 150
+    Jf, Kf = rng.standard_normal((2, P, M, M))
+    Hf = rng.standard_normal((M, M))
+    dC, dI = ops.to_device(C), ops.to_device(I)
+    fock = [ops.to_device(x) for x in (Jf, Kf, n, Hf, cj, ck)]
+
+    def run():
+        J, K = ops.jkj_full(dC, dI, P)
+        F = ops.fock_rc(*fock, 6, 6)
+        torch_cuda.cuda.synchronize()
+        return [x.cpu().numpy() for x in (J, K, F)]
+
+    plain = run()
+    _withheld(stage)
+    try:
+        got = run()
+    finally:
+        _restore()
+    assert _lib.device_status(reset=False) == 0
+    for a, b in zip(got, plain):
+        assert nrel(a, b) < 4096 * 2.0**-52
+    # FP64 arithmetic rounds otherwise: the stage was withheld (the Fock GEMMs have four)
+    assert not np.array_equal(got[0], plain[0]) and not np.array_equal(got[1], plain[1])
+    assert stage > 3 or not np.array_equal(got[2], plain[2])
+    assert all(np.array_equal(a, b) for a, b in zip(run(), plain))
+    # a failure of a split-product call leaves the FP64 calls alone
+    ops.dgemm_mixed(ops.to_device(np.full((128, 64), np.nan)), ops.to_device(np.ones((128, 64))), 6)
+    assert all(np.array_equal(a, b) for a, b in zip(run(), plain))
+    assert ops.reset_device_status() == 6
