@@ -361,6 +361,11 @@ int gb_set_wait_limit_ns(unsigned long long limit_ns);
  * off. */
 int gb_test_withhold_stage(int stage);
 
+/* Test hook, no counterpart in the reference: the FP64 calls' tensor-core GEMMs
+ * hold at most this many bytes of operand slices at a time (0 restores the default
+ * of 3 GB), running larger ones in panels.  Query workspaces after it. */
+int gb_test_panel_bytes(size_t bytes);
+
 /* Generic FP64-accurate GEMM on the tensor cores: C = A B^T with row-major
  * A [M][K], B [N][K], C [M][N].  No counterpart in the reference (PyNOF's
  * GEMMs go through numpy / cupy). */

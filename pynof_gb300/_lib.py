@@ -85,6 +85,7 @@ SIGNATURES = {
     "gb_device_status": (_I, [_I, _c.POINTER(_I)]),
     "gb_set_wait_limit_ns": (_I, [_c.c_ulonglong]),
     "gb_test_withhold_stage": (_I, [_I]),
+    "gb_test_panel_bytes": (_I, [_Z]),
     "gb_dgemm_mixed_workspace": (_Z, [_I, _I, _I, _I]),
     "gb_dgemm_mixed": (_I, [_P, _P, _I, _I, _I, _I, _P, _P, _Z, _P]),
     "gb_ri_prepare_bytes_mixed": (_Z, [_I, _I, _I]),

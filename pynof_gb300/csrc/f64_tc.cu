@@ -27,6 +27,7 @@
 #include "f64_tc.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <mutex>
 
@@ -581,7 +582,9 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const __grid_constant__ 
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-constexpr size_t PANEL_BYTES = (size_t)3 << 30;  // slices held at a time, where an operand is cut into panels
+// Slices held at a time, where an operand is cut into panels (3 GB; less by the test hook).
+constexpr size_t PANEL_BYTES = (size_t)3 << 30;
+std::atomic<size_t> g_panel_bytes{PANEL_BYTES};
 
 long long up128(long long x) { return (x + 127) / 128 * 128; }
 size_t slice_bytes(long long batch, long long rows, long long K) {
@@ -641,15 +644,16 @@ Plan make_plan(long long M, long long N, long long K, int batch, bool a_shared, 
     p.yb = slice_bytes(ys ? 1 : p.pb, p.py, K);
   };
   size();
-  if (p.xb + p.yb > PANEL_BYTES) {
+  const size_t most = g_panel_bytes.load();
+  if (p.xb + p.yb > most) {
     if (batch > 1) {
-      while (p.pb > 1 && p.xb + p.yb > PANEL_BYTES) {
+      while (p.pb > 1 && p.xb + p.yb > most) {
         p.pb = (p.pb + 1) / 2;
         size();
       }
     } else {
       long long& big = p.px >= p.py ? p.px : p.py;
-      while (big > 128 && p.xb + p.yb > PANEL_BYTES) {
+      while (big > 128 && p.xb + p.yb > most) {
         big = up128((big + 1) / 2);
         size();
       }
@@ -815,3 +819,9 @@ int gemm_f64_tc(const GemmF64& g, const TcWork& w, cudaStream_t s) {
 }
 
 }  // namespace gb
+
+extern "C" int gb_test_panel_bytes(size_t bytes) {
+  gb::clear_error();
+  gb::g_panel_bytes.store(bytes ? bytes : gb::PANEL_BYTES);
+  return GB_OK;
+}

@@ -185,3 +185,54 @@ def test_graded_k_splits(ops, spread):
     D = np.einsum("si,li->isl", C[:, :P], C[:, :P]).reshape(P, N * N)
     assert _element_error(J.cpu().numpy().reshape(P, N * N), D, I.reshape(N * N, N * N).T,
                           rows=slice(0, P, 7), cols=slice(0, N * N, 61)) < 2 * N + 1
+
+
+@pytest.fixture
+def small_panels(ops):
+    """2 MB of slices at a time: what takes several GB of them otherwise runs in panels."""
+    from pynof_gb300 import _lib
+
+    _lib.call("gb_test_panel_bytes", 2 << 20)
+    yield
+    _lib.call("gb_test_panel_bytes", 0)
+
+
+@pytest.mark.parametrize("N,P", [(64, 60), (66, 66), (53, 33)])
+def test_panels_of_packed_pairs(ops, small_panels, N, P):
+    """Row panels on either side (the pairs are the tiles' rows at P = 60, their columns
+    at P = 66) with K splits, graded rows in one panel, and a NaN in the last one only."""
+    rng = np.random.default_rng(N)
+    I, C = _eri(N, rng), np.linalg.qr(rng.standard_normal((N, N)))[0]
+    D = np.einsum("si,li->isl", C[:, :P], C[:, :P])
+    Jr, Kr = np.einsum("isl,mnsl->imn", D, I, optimize=True), np.einsum("inl,mnsl->ims", D, I, optimize=True)
+    J, K = _host(*ops.jkj_full(ops.to_device(C), ops.to_device(I), P))
+    assert nrel(J, Jr) < TOL and nrel(K, Kr) < TOL
+    m = N - 1
+    I2 = I.copy()
+    I2[m, m, 0, 0] = np.nan  # the last pair of J; K of row m and column 0
+    J, _ = _host(*ops.jkj_full(ops.to_device(C), ops.to_device(I2), P))
+    assert np.isnan(J[:, m, m]).all()
+    J[:, m, m] = Jr[:, m, m]
+    assert nrel(J, Jr) < TOL
+    I3 = I.copy()
+    I3[m, m] = 1e-12 * rng.standard_normal((N, N))
+    I3[m, m, 0, 0] = 1.0 / max(abs(D[0, 0, 0]), 1e-3)
+    C3 = C.copy()
+    C3[0] *= 1e-10  # what meets the bound of pair (m, m) is far below it
+    J, _ = _host(*ops.jkj_full(ops.to_device(C3), ops.to_device(I3), P))
+    D3 = np.einsum("si,li->isl", C3[:, :P], C3[:, :P]).reshape(P, N * N)
+    assert _element_error(J.reshape(P, N * N), D3, I3.reshape(N * N, N * N).T, rows=slice(0, P, 5),
+                          cols=[0, N + 1, m * N, m * N + m]) < 2 * N + 1
+
+
+def test_panels_of_a_batch_and_in_place(ops, small_panels):
+    """Batch panels with one shared operand and a ragged last one (the MO transforms),
+    row panels of a GEMM that adds to its output (the Fock matrices)."""
+    test_lagrangian(ops, 97, 305, 40)
+    test_fock_accumulates(ops, 131, 70, 14)
+    test_graded_operands_keep_fp64_accuracy(ops, 40, 230, 20)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_panels_with_nonfinite_operands(ops, small_panels, bad):
+    test_nonfinite_operands_take_fp64_arithmetic(ops, bad)
