@@ -18,7 +18,8 @@
  *   asynchronous with respect to the host; results are valid once the stream
  *   has been synchronised.
  * - Scratch memory comes from the caller: `workspace` must hold at least the
- *   number of bytes the matching *_workspace_* query returns.  The library
+ *   number of bytes the matching *_workspace_* query returns (the FP64 calls run
+ *   with less, more slowly: gb_query_minimum).  The library
  *   allocates no device memory and never frees caller memory.
  * - The return value is a GB_* status; gb_last_error() returns the message of
  *   the last failing call on the calling thread.
@@ -49,6 +50,12 @@ extern "C" {
 const char* gb_last_error(void);
 /* Library version, major * 10000 + minor * 100 + patch. */
 int gb_version(void);
+
+/* While on (for the calling thread), the *_workspace_f64 queries return the least
+ * that a call takes, without the scratch of its tensor-core GEMMs; with less than
+ * a GEMM's scratch that GEMM runs on the FP64 units.  For callers short of device
+ * memory. */
+int gb_query_minimum(int on);
 
 /* Launch profiler.  While enabled, every kernel the library launches is
  * bracketed by two CUDA events on its stream.  gb_profile_stop synchronises on

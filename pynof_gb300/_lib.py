@@ -33,6 +33,7 @@ _Z = _c.c_size_t
 SIGNATURES = {
     "gb_last_error": (_c.c_char_p, []),
     "gb_version": (_I, []),
+    "gb_query_minimum": (_I, [_I]),
     "gb_profile_start": (_I, []),
     "gb_profile_stop": (_I, [_c.c_char_p, _Z]),
     "gb_check_symmetric_f64": (_I, [_P, _I, _I, _P, _P]),
@@ -155,6 +156,15 @@ def call(name: str, *args) -> None:
 
 def query(name: str, *args) -> int:
     return int(getattr(load(), name)(*args))
+
+
+def query_minimum(name: str, *args) -> int:
+    """The least workspace an FP64 call takes (without its tensor-core scratch)."""
+    call("gb_query_minimum", 1)
+    try:
+        return query(name, *args)
+    finally:
+        call("gb_query_minimum", 0)
 
 
 def device_status(reset: bool = True) -> int:

@@ -585,6 +585,7 @@ __global__ void __launch_bounds__(256) sum_parts_kernel(const __grid_constant__ 
 // Slices held at a time, where an operand is cut into panels (3 GB; less by the test hook).
 constexpr size_t PANEL_BYTES = (size_t)3 << 30;
 std::atomic<size_t> g_panel_bytes{PANEL_BYTES};
+thread_local bool t_query_minimum = false;  // this thread's queries leave the scratch out
 
 long long up128(long long x) { return (x + 127) / 128 * 128; }
 size_t slice_bytes(long long batch, long long rows, long long K) {
@@ -710,6 +711,7 @@ bool same_index(const Index2& a, const Index2& b) { return a.div == b.div && a.s
 
 size_t gemm_f64_tc_bytes(long long M, long long N, long long K, int batch, bool a_shared, bool b_shared, int sym,
                          int pair_n, bool in_place) {
+  if (t_query_minimum) return 0;
   const Plan p = make_plan(M, N, K, batch, a_shared, b_shared, sym, pair_n, in_place);
   return p.use ? p.bytes() : 0;
 }
@@ -819,6 +821,12 @@ int gemm_f64_tc(const GemmF64& g, const TcWork& w, cudaStream_t s) {
 }
 
 }  // namespace gb
+
+extern "C" int gb_query_minimum(int on) {
+  gb::clear_error();
+  gb::t_query_minimum = on != 0;
+  return GB_OK;
+}
 
 extern "C" int gb_test_panel_bytes(size_t bytes) {
   gb::clear_error();

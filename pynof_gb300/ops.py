@@ -77,8 +77,16 @@ POOL = WorkspacePool()
 
 
 def _ws(query: str, *sizes, device) -> tuple[int, int]:
+    """Workspace of a call: what its query asks for or, where device memory does
+    not hold the FP64 calls' tensor-core scratch, the least that it takes."""
     n = _lib.query(query, *sizes)
-    buf = POOL.get(n, device)
+    try:
+        buf = POOL.get(n, device)
+    except torch.OutOfMemoryError:
+        least = _lib.query_minimum(query, *sizes)
+        if least >= n:
+            raise
+        buf = POOL.get(least, device)
     return buf.data_ptr(), buf.numel()
 
 

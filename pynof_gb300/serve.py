@@ -67,8 +67,10 @@ def reservation_bytes(st, precision: str, nslices: int) -> int:
                  _lib.query("gb_lagrange2_ri_workspace_mixed", N, P, Q, nslices))
     else:
         prep = 0
-    # the FP64 path is also used after the precision switch
-    ws64 = max(_lib.query("gb_jkh_mo_ri_workspace_f64", N, P, Q), _lib.query("gb_lagrange2_ri_workspace_f64", N, P, Q))
+    # the FP64 path is also used after the precision switch; its tensor-core scratch
+    # is left out where memory is short, so it is not reserved
+    ws64 = max(_lib.query_minimum("gb_jkh_mo_ri_workspace_f64", N, P, Q),
+               _lib.query_minimum("gb_lagrange2_ri_workspace_f64", N, P, Q))
     ws = max(ws64, ws if precision == "mixed" else 0)
     out = 2 * N * N * 8 + N * P * 8 + 4 * P * P * 8
     return int(b + prep + ws + out)

@@ -236,3 +236,27 @@ def test_panels_of_a_batch_and_in_place(ops, small_panels):
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
 def test_panels_with_nonfinite_operands(ops, small_panels, bad):
     test_nonfinite_operands_take_fp64_arithmetic(ops, bad)
+
+
+def test_without_scratch(ops, monkeypatch):
+    """Where the pool has no room for the scratch, the calls run on what they needed
+    before (on the FP64 units)."""
+    from pynof_gb300 import _lib
+
+    torch = pytest.importorskip("torch")
+    N, P = 53, 33
+    rng = np.random.default_rng(N)
+    I, C = _eri(N, rng), np.linalg.qr(rng.standard_normal((N, N)))[0]
+    real, least = ops.WorkspacePool(), _lib.query_minimum("gb_jkj_full_workspace_f64", N, P)
+
+    class Pool:
+        def get(self, nbytes, device):
+            if nbytes > least:
+                raise torch.OutOfMemoryError("no room")
+            return real.get(nbytes, device)
+
+    monkeypatch.setattr(ops, "POOL", Pool())
+    J, K = _host(*ops.jkj_full(ops.to_device(C), ops.to_device(I), P))
+    D = np.einsum("si,li->isl", C[:, :P], C[:, :P])
+    assert nrel(J, np.einsum("isl,mnsl->imn", D, I, optimize=True)) < TOL
+    assert nrel(K, np.einsum("inl,mnsl->ims", D, I, optimize=True)) < TOL
