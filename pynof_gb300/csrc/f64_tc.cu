@@ -45,6 +45,7 @@ constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t TABLE_BYTES = 20u * (BM + BN);
 constexpr size_t SMEM_BYTES = (size_t)STAGES * STAGE_BYTES + TABLE_BYTES + 256 + 1024;
 constexpr int SUPER = 64;   // stages (1024 k) an element's 64-bit sum covers: |sum| < 1024 * 1.01 * 2^52 < 2^63
+constexpr int SMS = 152;    // GB300's, for estimates and splits (the launch asks the device)
 constexpr int CH_MIN = 3;   // stages per chunk whatever the digits are: 5 * 2^16 * 48 < 2^24 - 2^16 units of group 6
 constexpr float SIZE_MIN = 0x1p-6f;  // smallest sum of sizes of an element stored here
 constexpr float LIM_TOP = 4194304.0f - 65536.0f, LIM = 16777216.0f - 65536.0f;
@@ -610,6 +611,34 @@ struct Plan {
 constexpr size_t WORDS = 2;
 size_t done_words(long long M, long long N, int batch) { return (size_t)((M + 63) / 64 * ((N + 63) / 64) * batch); }
 
+// The two kernels' estimated times, from these measured on GB300 (whole calls, each
+// GEMM forced one way, us FP64 units / us tensor cores): Fock matrices of nbf5, nbf
+// (two GEMMs) 20, 80 39/90; 20, 160 268/129; 40, 110 286/97; 60, 60 74/107; 60, 90
+// 151/115; 150, 150 2650/368; four-index J, K of nbf 24 134/170; 30 209/183; 53 917/293;
+// FP64 Lagrangian of nbf 24 151/182; 32 238/184; 60 969/244; rotation of nbf 300
+// 492/773; 371 877/818; 450 1785/964.
+//
+// gemm_f64: 64 x 64 tiles at ~1.0 TFLOP/s in whole rounds of the SMs, or 8 x 8 blocks at
+// 0.8, at least 0.115 us per k (one warp's chain); of the skipped blocks of a square grid
+// half are paid for.
+double time_f64(long long M, long long N, long long K, int batch, int sym) {
+  auto up = [](long long x, long long to) { return (double)((x + to - 1) / to * to); };
+  const double t64 = up(M, 64) / 64 * up(N, 64) / 64 * batch;
+  const double half = sym == SYM_NONE ? 1.0 : 0.5;
+  if (t64 >= SMS) return std::ceil(t64 * half / SMS) * SMS * 8192.0 * up(K, 16) / 1.0e12;
+  const double part = sym == SYM_PAIRCOL ? 0.75 : half;
+  return 4e-6 + std::max(0.115e-6 * K, 2.0 * up(M, 8) * up(N, 8) * K * batch * part / 0.8e12);
+}
+
+// The tensor cores: seven launches, 32 bytes of slicing an element, and a stage of a
+// tile 1.1 (long K) to 1.5 us with ~7 us a tile, in whole rounds of the SMs.
+double time_tc(double tiles, long long nkb, double el, bool in_place) {
+  const double fixed = 50e-6 + el * 32.0 / 3.5e12, stage = 1.4e-6, tile = 7e-6;
+  if (tiles >= SMS) return fixed + std::ceil(tiles / SMS) * (nkb * stage + tile);
+  const double ctas = in_place ? tiles : std::min((double)SMS, tiles * (double)std::max(1ll, nkb / 16));
+  return fixed + tiles * nkb * stage / ctas + tile + (ctas > tiles ? 5e-6 : 0.0);
+}
+
 Plan make_plan(long long M, long long N, long long K, int batch, bool a_shared, bool b_shared, int sym, int pair_n,
                bool in_place) {
   Plan p;
@@ -623,18 +652,11 @@ Plan make_plan(long long M, long long N, long long K, int batch, bool a_shared, 
   p.yr = p.swap ? M : n;
   const bool xs = batch == 1 || (p.swap ? b_shared : a_shared), ys = batch == 1 || (p.swap ? a_shared : b_shared);
   const long long nkb = (K + SL_K - 1) / SL_K;
-  if (p.xr > (1 << 30) || p.yr > (1 << 30) || K > (1 << 30) || K >= (1ll << 31) - 16) return p;
+  if (p.xr > (1 << 30) || p.yr > (1 << 30) || K > (1 << 30)) return p;
   const double all_tiles = (double)tiles(p.xr, p.yr) * batch * (sym == SYM_ROWCOL ? 0.55 : 1.0);
-  // Rule: the estimated time against gemm_f64's.  Measured on GB300: a stage of a
-  // tile takes ~1300 clocks at ~2 GHz, slicing moves 32 bytes an element at ~5 TB/s,
-  // the seven launches of a GEMM ~60 us (at 300^3, 62 us of FP64 arithmetic, this
-  // took 80); the FP64 pipe gives 1.0 TFLOP/s when its 64 x 64 tiles fill the SMs
-  // (gemm_f64's other kernel less).
-  const double el = (double)M * K * (a_shared ? 1 : batch) + (double)n * K * (b_shared ? 1 : batch);
-  const double ctas = std::min(152.0, all_tiles * (double)std::max(1ll, nkb / 16));
-  const double t_tc = 60e-6 + el * 32.0 / 5e12 + all_tiles * nkb * 1300.0 / 2e9 / ctas;
-  const double t_f64 = 2.0 * M * N * K * batch * (sym == SYM_NONE ? 1.0 : 0.5) / 1.0e12;
-  p.use = t_tc < 0.7 * t_f64;
+  const double el = ((double)M * (a_shared ? 1 : batch) + (double)n * (b_shared ? 1 : batch)) * (double)(nkb * SL_K);
+  // (0.7: graded rows pay for both)
+  p.use = time_tc(all_tiles, nkb, el, in_place) < 0.7 * time_f64(M, N, K, batch, sym);
   if (!p.use) return p;
   // panels: over the batch, or over the rows of the operand with more of them
   p.px = p.xr;
@@ -666,17 +688,17 @@ Plan make_plan(long long M, long long N, long long K, int batch, bool a_shared, 
     return p;
   }
   // K splits of at least 16 stages, whole norm runs: the split count whose tiles
-  // take the fewest stages in a row on 152 SMs (a tile more costs an SM its
+  // take the fewest stages in a row on the SMs (a tile more costs an SM its
   // epilogue, ~12 stages' time)
   const long long pt = tiles(p.px, p.py) * p.pb;
   long long kbs = nkb;
   double best = 1e300;
   // (none where the output is added to in place: no element of a tile is stored before
   // all are known to be kept, which sum_parts_kernel does not see)
-  for (long long ns = 1; ns <= (in_place ? 1 : 64) && (ns == 1 || nkb / ns >= 16) && (ns == 1 || pt * ns <= 152 * 8); ++ns) {
+  for (long long ns = 1; ns <= (in_place ? 1 : 64) && (ns == 1 || nkb / ns >= 16) && (ns == 1 || pt * ns <= SMS * 8); ++ns) {
     long long k = (nkb + ns - 1) / ns;
     if (ns > 1) k = (k + SL_KPC - 1) / SL_KPC * SL_KPC;
-    const double cost = (double)((pt * ((nkb + k - 1) / k) + 151) / 152) * (double)(k + 12);
+    const double cost = (double)((pt * ((nkb + k - 1) / k) + SMS - 1) / SMS) * (double)(k + 12);
     if (cost < best) {
       best = cost;
       kbs = k;
@@ -690,17 +712,26 @@ Plan make_plan(long long M, long long N, long long K, int batch, bool a_shared, 
   return p;
 }
 
-int configure() {
+// Once per device context; *sms: the device's SMs.
+int configure(int* sms) {
   static std::mutex mu;
   static unsigned long long done[64] = {0};
+  static int count[64] = {0};
   int dev = 0;
   GB_TRY(cuda_status(cudaGetDevice(&dev), "cudaGetDevice"));
   const unsigned long long ctx = current_context_id();
   std::lock_guard<std::mutex> lk(mu);
-  if (dev < 0 || dev >= 64 || (ctx != 0 && done[dev] == ctx)) return GB_OK;
+  if (dev < 0 || dev >= 64) return GB_OK;
+  if (ctx != 0 && done[dev] == ctx) {
+    *sms = count[dev];
+    return GB_OK;
+  }
   GB_TRY(cuda_status(
       cudaFuncSetAttribute(f64_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES),
       "f64_tc: cudaFuncSetAttribute"));
+  GB_TRY(cuda_status(cudaDeviceGetAttribute(&count[dev], cudaDevAttrMultiProcessorCount, dev),
+                     "cudaDeviceGetAttribute"));
+  *sms = count[dev];
   done[dev] = current_context_id();
   return GB_OK;
 }
@@ -722,7 +753,8 @@ int gemm_f64_tc(const GemmF64& g, const TcWork& w, cudaStream_t s) {
   const Plan p = make_plan(g.M, g.N, g.K, g.batch, a_shared, b_shared, g.sym, g.pair_n,
                            g.beta != 0.0 && C0 == g.C.p);
   if (!p.use || !w.p || w.bytes < p.bytes()) return gemm_f64(g, s);
-  GB_TRY(configure());
+  int sms = SMS;
+  GB_TRY(configure(&sms));
   Carve cv(w.p, w.bytes);
   const long long n = p.tri ? (long long)g.pair_n * (g.pair_n + 1) / 2 : g.N;
   const size_t nwords = WORDS + done_words(g.M, n, g.batch);
@@ -798,7 +830,7 @@ int gemm_f64_tc(const GemmF64& g, const TcWork& w, cudaStream_t s) {
         a.wait_ns = wait_limit_ns();
         a.withhold = withheld_stage();
         a.ntiles = (int)(((xn + BM - 1) / BM) * (long long)((yn + BN - 1) / BN) * nb * p.nsplit);
-        const unsigned grid = (unsigned)std::min(a.ntiles, 152);
+        const unsigned grid = (unsigned)std::min(a.ntiles, sms);
         GB_LAUNCH_CHAIN(g.tag, s, f64_tc_kernel, dim3(grid), dim3(THREADS), SMEM_BYTES, a);
         if (p.nsplit > 1) {
           const long long all = (long long)xn * yn * nb;

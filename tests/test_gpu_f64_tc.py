@@ -260,3 +260,22 @@ def test_without_scratch(ops, monkeypatch):
     D = np.einsum("si,li->isl", C[:, :P], C[:, :P])
     assert nrel(J, np.einsum("isl,mnsl->imn", D, I, optimize=True)) < TOL
     assert nrel(K, np.einsum("inl,mnsl->ims", D, I, optimize=True)) < TOL
+
+
+@pytest.mark.parametrize("N", [24, 29, 31, 36, 43])
+def test_sizes_where_the_rule_changes_units(ops, N):
+    """Small sizes on both sides of the line between the FP64 units and the tensor cores,
+    through every kind of GEMM that takes them."""
+    P, Q = N // 2, 3 * N + 5
+    test_four_index_jk(ops, N, P)
+    test_lagrangian(ops, N, Q, P)
+    test_fock_accumulates(ops, 4 * N, P, max(1, P // 5))
+    rng = np.random.default_rng(N)
+    I, C, H = _eri(N, rng), np.linalg.qr(rng.standard_normal((N, N)))[0], rng.standard_normal((N, N))
+    dC, dI = ops.to_device(C), ops.to_device(I)
+    hm, imo = _host(*ops.mo_full(dC, ops.to_device(H), dI, P))
+    Cp = C[:, :P]
+    ref = np.einsum("mp,nq,mnsl,sr,lt->pqrt", C, Cp, I, Cp, Cp, optimize=True)
+    assert nrel(imo, ref) < TOL and nrel(hm, C.T @ H @ Cp) < TOL
+    m4, = _host(ops.mo4_full(dC, dI, (1, P), (0, N), (2, N), (0, P)))
+    assert nrel(m4, np.einsum("mp,nq,mnsl,sr,lt->pqrt", C[:, 1:P], C, I, C[:, 2:], Cp, optimize=True)) < TOL
