@@ -92,3 +92,50 @@ def test_symmetric_mo_transform(ops, nbf, naux, nbf5):
     for x, r in zip(got + mo, ref + ref[:3]):
         x, r = x.cpu().numpy(), r.cpu().numpy()
         assert np.max(np.abs(x - r)) / np.max(np.abs(r)) < 4 * TOL
+
+
+def _all_255(places):
+    """The number below 1 whose nine-bit digits are all 255."""
+    return sum(255 * 2.0 ** -(9 * s - 1) for s in range(1, places + 1))
+
+
+@pytest.mark.parametrize("K", [4095, 4096, 4097, 6100])
+def test_full_digits_over_a_long_k(ops, K):
+    """Both drains at their longest: 32-bit pairs up to K = 4096, 64-bit sums and the FP32
+    group per chunk beyond.  The bound of TOL above at this K: 4 (2^-42.9 + 2^-44 +
+    2^-49.8 K)."""
+    tol = 4 * (2.0**-42.9 + 2.0**-44 + 2.0**-49.8 * K)
+    x = _all_255(5)
+    M, N = 130, 104
+    sg = np.where(np.random.default_rng(K).random(K) < 0.5, -x, x)
+    for a, b in ((np.full(K, x), np.full(K, x)), (sg, sg)):
+        C = ops.dgemm_mixed(ops.to_device(np.tile(a, (M, 1))), ops.to_device(np.tile(b, (N, 1))), 6).cpu().numpy()
+        assert np.max(np.abs(C / (K * x * x) - 1.0)) < tol
+    # the persistent kernel: J of a factor and orbitals of that size (K = naux)
+    nbf = 20
+    db = ops.to_device(np.full((nbf, nbf, K), x))
+    J, Km = ops.jkj_ri_mixed(ops.to_device(np.full((nbf, nbf), x)), ops.PreparedRI(db, 6), 3)
+    ops.check_device_status()
+    T = nbf * x * x
+    assert np.max(np.abs(J.cpu().numpy() / (K * nbf * x * T * x) - 1.0)) < 3 * tol
+    assert np.max(np.abs(Km.cpu().numpy() / (K * T * T) - 1.0)) < 3 * tol
+
+
+def test_full_digits_of_the_fp64_engine(ops):
+    """Six planes of 255 (53 bits) in both operands, K past the 1024 of one integer sum,
+    through the Fock matrices' product (n = 0, H = 0, ck12 = 0).  The sum is exact but for
+    two roundings to FP64 and, relative to it, the dropped digit products (6 * 2^-63) and
+    the FP32 group's own roundings (2^-57): 2^-52."""
+    torch = pytest.importorskip("torch")
+    from fractions import Fraction
+
+    P, x = 1030, _all_255(6)
+    exact = float((P - 1) * Fraction(x) ** 2)
+    J = torch.full((P, P, P), x, dtype=torch.float64, device="cuda")
+    cj = torch.full((P, P), x, dtype=torch.float64, device="cuda")
+    z = torch.zeros((P, P), dtype=torch.float64, device="cuda")
+    F = ops.fock_rc(J, J, z[0].contiguous(), z, cj, z, 1, 1)
+    assert float((F / exact - 1.0).abs().max()) <= 2.0**-52
+    sg = torch.where(torch.arange(P, device="cuda") % 3 == 0, -1.0, 1.0).double()
+    F = ops.fock_rc(J * sg[:, None, None], J, z[0].contiguous(), z, cj * sg[None, :], z, 1, 1)
+    assert float((F / exact - 1.0).abs().max()) <= 2.0**-52
