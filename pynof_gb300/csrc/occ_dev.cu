@@ -208,14 +208,10 @@ __device__ __noinline__ double shifted_softmax(const double* x, int nd, int nc, 
 __device__ void prep_point(const OccArgs& a, const OccStage& w, const double* __restrict__ x) {
   const int tid = threadIdx.x, nd = a.ndoc, nc = a.ncwo, nv = a.nv, nvr = (nv + 31) / 32 * 32;
   // one exponential per logit, all at once (a pair with a logit past exp's
-  // range is redone with its largest logit below)
+  // range is redone with its largest logit below; a NaN stays one)
   const int r0 = tid % nd;
   double* ex = w.ew;  // free between a step and the next evaluation
-  for (int t = tid; t < nv; t += blockDim.x) {
-    const double xv = x[t];
-    const bool big = __double_as_longlong(xv) > __double_as_longlong(700.0) || isnan(xv);
-    ex[t] = exp(big ? 700.0 : xv);
-  }
+  for (int t = tid; t < nv; t += blockDim.x) ex[t] = exp(x[t]);
   __syncthreads();
   for (int t = tid; t < nvr + nd; t += blockDim.x) {
     const bool strong = t >= nvr;

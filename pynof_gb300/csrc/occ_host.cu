@@ -80,9 +80,9 @@ extern "C" int gb_occ_energy_grad_f64(const double* gamma, const double* J, cons
       ns[p] = std::exp(-top) / den;
       for (int j = 0; j < ncwo; ++j) nw[(size_t)p * ncwo + j] = std::exp(gamma[L.gam(p, j)] - top) / den;
     } else {
-      for (int j = 0; j < ncwo; ++j) den += std::exp(std::fmin(gamma[L.gam(p, j)], 700.0));
+      for (int j = 0; j < ncwo; ++j) den += std::exp(gamma[L.gam(p, j)]);  // (below 700, or a NaN)
       ns[p] = 1.0 / den;
-      for (int j = 0; j < ncwo; ++j) nw[(size_t)p * ncwo + j] = std::exp(std::fmin(gamma[L.gam(p, j)], 700.0)) / den;
+      for (int j = 0; j < ncwo; ++j) nw[(size_t)p * ncwo + j] = std::exp(gamma[L.gam(p, j)]) / den;
     }
     n[p] = ns[p];
     for (int j = 0; j < ncwo; ++j) n[L.weak(p, j)] = nw[(size_t)p * ncwo + j];

@@ -252,3 +252,24 @@ def test_host_driven_matches_graph(torch_cuda, case):
     assert b[1][3] == 1.0
     for x, y in zip(a, b):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("case", ["c1", "ncwo1", "p300"])
+def test_nan_logit_stays_nan(torch_cuda, case):
+    """A NaN in gamma gives a NaN energy and gradient, and a minimisation that stops at
+    once without success, as scipy's does."""
+    from pynof_gb300 import ops
+
+    p, g0, J, K, Hc = _problem(case)
+    g = g0.copy()
+    g[len(g) // 2] = np.nan
+    om = ops.OccMinimizer(p.nbf5, p.no1, p.ndoc, p.ncwo)
+    dJ, dK, dH = _dev(J, K, Hc)
+    r, grad = om.energy_grad(*_dev(g), dJ, dK, dH)
+    assert np.isnan(r.cpu().numpy()[0]) and np.isnan(grad.cpu().numpy()[len(g) // 2])
+    for host_driven in (False, True):
+        r = om.minimize(*_dev(g), dJ, dK, dH, host_driven=host_driven)[1].cpu().numpy()
+        assert np.isnan(r[0]) and r[2] == 1 and r[3] == 0.0
+    # finite logits again
+    assert np.isfinite(om.energy_grad(*_dev(g0), dJ, dK, dH)[0].cpu().numpy()[0])
+    om.close()

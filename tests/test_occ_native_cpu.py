@@ -103,3 +103,20 @@ def test_calce_sums_with_compensation():
     plain = float(np.sum(cj * J.T))
     print(f"exact {exact:.17g}  compensated {E:.17g}  plain {plain:.17g}")
     assert abs(E - exact) < 1e-10
+
+
+@pytest.mark.parametrize("beside", [1.0, 800.0])
+def test_nan_logit_stays_nan(beside):
+    """A NaN in gamma gives a NaN energy, as the softmax has it in NumPy."""
+    st = Structure(**STRUCTS[0])
+    J, K, H = _mo(st.nbf5, np.random.default_rng(1), 0.0)
+    g = nof.gamma_guess_softmax(st)
+    g[2], g[2 + st.ndoc] = np.nan, beside
+    from pynof_gb300 import _lib
+
+    E, grad = np.zeros(1), np.zeros(st.nv)
+    J, K, H, g = (np.ascontiguousarray(x) for x in (J, K, H, g))
+    _lib.call("gb_occ_energy_grad_f64", g.ctypes.data, J.ctypes.data, K.ctypes.data, H.ctypes.data, st.nbf5, st.no1,
+              st.ndoc, st.ncwo, E.ctypes.data, grad.ctypes.data)
+    assert np.isnan(E[0]) and np.isnan(grad[2])
+    assert np.isnan(nof.calcocce(g, J, K, H, st))
