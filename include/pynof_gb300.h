@@ -24,7 +24,7 @@
  * - The return value is a GB_* status; gb_last_error() returns the message of
  *   the last failing call on the calling thread.
  * - The RI entry points use the (m, n) symmetry of b: J is computed on the
- *   pairs n >= m and mirrored.  PyNOF's b_mnl is symmetric by construction
+ *   pairs n >= m and mirrored, (pq|l) at nslices = 6 on the pairs q <= p.  PyNOF's b_mnl is symmetric by construction
  *   (pynof/integrals.py:39-49 builds it from the (P|mn) integrals);
  *   gb_check_symmetric_f64 verifies a buffer.
  */

@@ -1439,6 +1439,7 @@ int ozaki_gemm(const SlicedDesc& A, const SlicedDesc& B, const OzGemm& g, cudaSt
       return launch_error(g.tag, e, g.S, g.bn);
     }
   } else {
+    GB_REQUIRE(g.sym != SYM_BATCHCOL, GB_ERR_BAD_SHAPE, "%s: SYM_BATCHCOL runs on the persistent kernel alone", g.tag);
     const int pi = prof_begin(g.tag, stream);
     const cudaError_t e =
         launch_chain(kernel_for(g.S, g.bn), grid_for(tiles), dim3(THREADS), smem_bytes(g.S, g.bn), stream, ka);
@@ -1474,6 +1475,8 @@ int ozaki_group_upload(const OzProblem* probs, int nprob, void* table, bool* per
     const OzGemm& g = probs[i].g;
     all_rows_fast = all_rows_fast && !(g.c_c.div == 0 && g.c_c.s0 == 1) && (g.c_r.div == 0 && g.c_r.s0 == 1);
   }
+  for (int i = 0; i < nprob; ++i)
+    GB_REQUIRE(probs[i].g.sym != SYM_BATCHCOL, GB_ERR_INVALID_ARG, "ozaki_group_upload: no SYM_BATCHCOL in a group");
   // one drain form for the group (the fraction bits suit both)
   for (KArgs& ka : args) ka.g.fdrain = fdrain;
   if (group_fdrain) *group_fdrain = fdrain != 0;
