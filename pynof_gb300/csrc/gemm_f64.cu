@@ -231,6 +231,19 @@ __global__ void __launch_bounds__(32) gemm_f64_small_kernel(const GemmF64 g) {
   const double* __restrict__ Ab = g.A.p + bz * g.A.sb + (iok ? g.A.r.at(ia) : 0);
   const double* __restrict__ Bb =
       g.B.p + bz * g.B.sb + (jok ? g.B.c.at(g.sym == SYM_TRICOL ? pair_index(jb, g.pair_n) : jb) : 0);
+  double* __restrict__ Cb = g.C.p + bz * g.C.sb;
+  const int i = m0 + gq;
+  const long long ri = iok ? g.C.r.at(i) : 0;
+  // what beta multiplies is under way while the products run
+  double add[2] = {};
+  if (g.beta != 0.0) {
+    const double* c0 = (g.C0 ? g.C0 + bz * g.C.sb : Cb) + ri;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int j = n0 + 2 * tq + e;
+      if (iok && j < g.N) add[e] = c0[g.C.c.at(j)];
+    }
+  }
   double c0 = 0.0, c1 = 0.0;
   for (int k0 = 0; k0 < g.K; k0 += 4 * UNR) {
     double a[UNR], b[UNR];
@@ -244,11 +257,8 @@ __global__ void __launch_bounds__(32) gemm_f64_small_kernel(const GemmF64 g) {
 #pragma unroll
     for (int u = 0; u < UNR; ++u) dmma(c0, c1, a[u], b[u]);
   }
-  double* __restrict__ Cb = g.C.p + bz * g.C.sb;
-  const int i = m0 + gq;
-  if (i >= g.M) return;
+  if (!iok) return;
   const bool mirror_rc = (g.sym == SYM_ROWCOL) && (m0 != n0);
-  const long long ri = g.C.r.at(i);
 #pragma unroll
   for (int e = 0; e < 2; ++e) {
     const int j = n0 + 2 * tq + e;
@@ -256,7 +266,7 @@ __global__ void __launch_bounds__(32) gemm_f64_small_kernel(const GemmF64 g) {
     if (g.sym == SYM_ROWCOL && m0 == n0 && j < i) continue;  // the diagonal block's mirror writes these
     double v = g.alpha * (e ? c1 : c0);
     double* dst = Cb + ri + g.C.c.at(g.sym == SYM_TRICOL ? pair_index(j, g.pair_n) : j);
-    if (g.beta != 0.0) v += g.beta * (g.C0 ? g.C0[dst - g.C.p] : *dst);
+    if (g.beta != 0.0) v += g.beta * add[e];
     *dst = v;
     if (g.sym == SYM_ROWCOL && (mirror_rc || j > i)) {
       Cb[g.C.r.at(j) + g.C.c.at(i)] = v;

@@ -29,8 +29,9 @@ namespace {
 
 constexpr int TAYLOR_DEG = 16;
 
-// Y[i][j] from the packed step: +y for i < j (i < P), -y for i > j (j < P).
-__global__ void build_antisym_kernel(const double* __restrict__ y, int N, int P, double* __restrict__ Y) {
+// Y[i][j] from the packed step: +y for i < j (i < P), -y for i > j (j < P),
+// scaled by the power of two f.
+__global__ void build_antisym_kernel(const double* __restrict__ y, int N, int P, double f, double* __restrict__ Y) {
   chain_wait();
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)N * N) return;
@@ -40,7 +41,7 @@ __global__ void build_antisym_kernel(const double* __restrict__ y, int N, int P,
   if (lo != hi && lo < P) {
     // offset of row lo in the packed upper triangle: sum_{r < lo} (N - 1 - r)
     const long long off = (long long)lo * (N - 1) - (long long)lo * (lo - 1) / 2;
-    v = y[off + (hi - lo - 1)];
+    v = f * y[off + (hi - lo - 1)];
     if (i > j) v = -v;
   }
   Y[idx] = v;
@@ -146,10 +147,12 @@ extern "C" int gb_rotate_orbital_f64(const double* y, const double* C, int nbf, 
   const TcWork tw = tc_work(wc);
   const long long NN = (long long)N * N;
 
-  GB_LAUNCH_CHAIN("rotate_build", s, build_antisym_kernel, dim3(cdiv(NN, 256)), dim3(256), 0, y, N, P, Y);
+  const dim3 grid(cdiv(NN, 256)), block(256);
   double norm = norm1;
-  if (!(norm1 >= 0.0)) {
+  const bool measure = !(norm1 >= 0.0);
+  if (measure) {
     // no bound from the caller: measure ||Y||_1 on the device (one synchronisation)
+    GB_LAUNCH_CHAIN("rotate_build", s, build_antisym_kernel, grid, block, 0, y, N, P, 1.0, Y);
     GB_TRY(cuda_status(cudaMemsetAsync(dnorm, 0, sizeof(unsigned long long), s), "cudaMemsetAsync"));
     GB_LAUNCH("rotate_norm", s, col_abs_max_kernel<<<cdiv(N, 128), 128, 0, s>>>(Y, N, dnorm));
     unsigned long long nbits = 0;
@@ -164,10 +167,11 @@ extern "C" int gb_rotate_orbital_f64(const double* y, const double* C, int nbf, 
     norm *= 0.5;
     ++sq;
   }
-  // X = Y / 2^sq in place
-  if (sq > 0)
-    GB_LAUNCH_CHAIN("rotate_scale", s, scale_kernel, dim3(cdiv(NN, 256)), dim3(256), 0, Y, Y, NN,
-                    std::ldexp(1.0, -sq));
+  // X = Y / 2^sq
+  if (!measure)
+    GB_LAUNCH_CHAIN("rotate_build", s, build_antisym_kernel, grid, block, 0, y, N, P, std::ldexp(1.0, -sq), Y);
+  else if (sq > 0)
+    GB_LAUNCH_CHAIN("rotate_scale", s, scale_kernel, grid, block, 0, Y, Y, NN, std::ldexp(1.0, -sq));
   const double* X = Y;
   Coefs c{};
   double f = 1.0;
@@ -180,12 +184,12 @@ extern "C" int gb_rotate_orbital_f64(const double* y, const double* C, int nbf, 
   GB_TRY(matmul(X, X, Z, N, 0.0, nullptr, tw, s, tag, SYM_ROWCOL));
   GB_TRY(matmul(Z, Z, Z2, N, 0.0, nullptr, tw, s, tag, SYM_ROWCOL));
   GB_TRY(matmul(Z, Z2, Z3, N, 0.0, nullptr, tw, s, tag, SYM_ROWCOL, -NN));
-  GB_LAUNCH_CHAIN("rotate_poly", s, poly_kernel, dim3(cdiv(NN, 256)), dim3(256), 0, S, N, c);
+  GB_LAUNCH_CHAIN("rotate_poly", s, poly_kernel, grid, block, 0, S, N, c);
   // E, O += their brackets (S + 3 NN and on) times Z^4
   double *E = S, *O = S + NN;
   GB_TRY(matmul(S + 3 * NN, Z4, E, N, 1.0, E, tw, s, tag, SYM_ROWCOL, NN));
   // F = (E + X) + X O
-  GB_LAUNCH_CHAIN("rotate_add", s, add_kernel, dim3(cdiv(NN, 256)), dim3(256), 0, E, X, NN);
+  GB_LAUNCH_CHAIN("rotate_add", s, add_kernel, grid, block, 0, E, X, NN);
   double *F = S + 3 * NN, *spare = S;
   GB_TRY(matmul(X, O, F, N, 1.0, E, tw, s, tag));
   for (int k = 0; k < sq; ++k) {
