@@ -59,6 +59,7 @@ struct DArgs {
   Index2 c_r, c_c;
   int sym, pair_n;  // SYM_NONE, SYM_ROWCOL, SYM_TRIROW, SYM_TRICOL
   double alpha, beta;
+  int times, plus;   // alpha is not 1, beta not 0 (FP64 comparisons cost what additions do)
   const double* C0;  // what beta multiplies (C itself where it is added in place)
   int nsplit, kbs;  // K splits and stages per split; partial sums go to part
   double* part;     // [split][batch][j][i]
@@ -131,8 +132,8 @@ __device__ __forceinline__ double scaled(double v, int scale) {
 // Element off of batch entry bz's finished result, with its mirror image.
 __device__ __forceinline__ void put(const DArgs& a, int bz, long long off, long long moff, double v) {
   double* C = a.C + (long long)bz * a.c_sb;
-  if (a.alpha != 1.0) v *= a.alpha;
-  if (a.beta != 0.0) v = fma(a.beta, a.C0[(long long)bz * a.c_sb + off], v);
+  if (a.times) v *= a.alpha;
+  if (a.plus) v = fma(a.beta, a.C0[(long long)bz * a.c_sb + off], v);
   C[off] = v;
   if (moff >= 0) C[moff] = v;
 }
@@ -487,7 +488,10 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
 #pragma unroll
         for (int j = 0; j < CW; ++j) {
           const double d = from_units(R[j], (fine >> j) & 1u);
-          acc[j] = s0 == kb0 ? d : acc[j] + d;
+          if (s0 == kb0)
+            acc[j] = d;
+          else
+            acc[j] += d;
         }
       }
       // stored by all warps or by none (after an abort the next tile's barrier ends them)
@@ -815,6 +819,8 @@ int gemm_f64_tc(const GemmF64& g, const TcWork& w, cudaStream_t s) {
         a.pair_n = g.pair_n;
         a.alpha = g.alpha;
         a.beta = g.beta;
+        a.times = g.alpha != 1.0;
+        a.plus = g.beta != 0.0;
         a.C0 = C0 + (long long)b0 * g.C.sb;
         a.nsplit = p.nsplit;
         a.kbs = p.kbs;
