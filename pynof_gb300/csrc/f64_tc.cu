@@ -418,7 +418,7 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
       epi_barrier_any(false);  // tables visible
       double acc[CW];
       long long R[CW];
-      bool ok = true, graded = false;
+      bool ok = true, graded = false, skip = false;
       for (int s0 = kb0; s0 < kb1 && ok; s0 += SUPER) {
         const int s1 = min(s0 + SUPER, kb1);
 #pragma unroll
@@ -483,6 +483,8 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(fempty_bar);
+        // a tile is stored by all warps or by none
+        if (s1 == kb1) skip = epi_barrier_any(graded);
         // into FP64: one conversion an element (the FP64 pipe takes ~2 a clock and SM),
         // one addition more from the second 1024 k on
 #pragma unroll
@@ -494,8 +496,8 @@ __global__ void __maxnreg__(MAX_REGS) f64_tc_kernel(const __grid_constant__ DArg
             acc[j] += d;
         }
       }
-      // stored by all warps or by none (after an abort the next tile's barrier ends them)
-      if (epi_barrier_any(!ok || graded)) continue;
+      if (!ok) skip = epi_barrier_any(true);  // (the next tile's barrier ends the walk)
+      if (skip) continue;
       if (et < 2 && m0 + 64 * et < a.M) {
         int* d = done_word(a, bz, m0 + 64 * et, n0);
         if (parts)

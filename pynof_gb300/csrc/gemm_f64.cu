@@ -94,7 +94,9 @@ __device__ __forceinline__ bool tile_done(const GemmF64& g, int m0, int n0, long
   return g.done[(bz * mt + m0 / BM) * nt + n0 / BN] == g.done_value;
 }
 
-template <bool AK, bool BKF>
+// EXT: packed pairs (SYM_TRICOL) or a C0; apart, since their branches in the store loop
+// made the plain form 13 % slower at K = 30.
+template <bool AK, bool BKF, bool EXT>
 __global__ void __launch_bounds__(THREADS) gemm_f64_kernel(const GemmF64 g) {
   chain_wait();
   __shared__ double As[2][BKT][BM + PAD];
@@ -118,7 +120,7 @@ __global__ void __launch_bounds__(THREADS) gemm_f64_kernel(const GemmF64 g) {
   TileLoader<AK> la;
   TileLoader<BKF> lb;
   la.init(g.A.r, m0, g.M);   // A rows are the M index, A columns the K index
-  lb.init(g.B.c, n0, g.N, g.sym == SYM_TRICOL ? g.pair_n : 0);   // B columns are the N index, B rows the K index
+  lb.init(g.B.c, n0, g.N, EXT && g.sym == SYM_TRICOL ? g.pair_n : 0);   // B columns are the N index, B rows the K index
 
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -182,15 +184,15 @@ __global__ void __launch_bounds__(THREADS) gemm_f64_kernel(const GemmF64 g) {
         const int j = n0 + wn * 32 + b * 8 + 2 * tq + e;
         if (j >= g.N) continue;
         double v = g.alpha * acc[a][b][e];
-        double* dst = Cb + ri + g.C.c.at(g.sym == SYM_TRICOL ? pair_index(j, g.pair_n) : j);
-        if (g.beta != 0.0) v += g.beta * (g.C0 ? g.C0[dst - g.C.p] : *dst);
+        double* dst = Cb + ri + g.C.c.at(EXT && g.sym == SYM_TRICOL ? pair_index(j, g.pair_n) : j);
+        if (g.beta != 0.0) v += g.beta * (EXT && g.C0 ? g.C0[dst - g.C.p] : *dst);
         *dst = v;
         if (mirror_rc) {
           Cb[g.C.r.at(j) + g.C.c.at(i)] = v;
         } else if (g.sym == SYM_PAIRCOL) {
           const int mm = j / g.pair_n, nn = j % g.pair_n;
           if (nn > mm) Cb[ri + g.C.c.at((long long)nn * g.pair_n + mm)] = v;
-        } else if (g.sym == SYM_TRICOL) {
+        } else if (EXT && g.sym == SYM_TRICOL) {
           int mm, nn;
           tri_pair(j, g.pair_n, mm, nn);
           if (nn > mm) Cb[ri + g.C.c.at((long long)nn * g.pair_n + mm)] = v;
@@ -205,7 +207,7 @@ __global__ void __launch_bounds__(THREADS) gemm_f64_kernel(const GemmF64 g) {
 // ahead.  GB300's FP64 rate per SM is low (~7 GFLOP/s), so a GEMM that gives
 // the 64 x 64 kernel fewer CTAs than SMs is latency-bound on a few SMs; 8 x 8
 // blocks spread it over the whole GPU.
-template <int UNR>
+template <int UNR, bool EXT>
 __global__ void __launch_bounds__(32) gemm_f64_small_kernel(const GemmF64 g) {
   chain_wait();
   const int lane = threadIdx.x;
@@ -230,13 +232,13 @@ __global__ void __launch_bounds__(32) gemm_f64_small_kernel(const GemmF64 g) {
   const bool iok = ia < g.M, jok = jb < g.N;
   const double* __restrict__ Ab = g.A.p + bz * g.A.sb + (iok ? g.A.r.at(ia) : 0);
   const double* __restrict__ Bb =
-      g.B.p + bz * g.B.sb + (jok ? g.B.c.at(g.sym == SYM_TRICOL ? pair_index(jb, g.pair_n) : jb) : 0);
+      g.B.p + bz * g.B.sb + (jok ? g.B.c.at(EXT && g.sym == SYM_TRICOL ? pair_index(jb, g.pair_n) : jb) : 0);
   double* __restrict__ Cb = g.C.p + bz * g.C.sb;
   const int i = m0 + gq;
   const long long ri = iok ? g.C.r.at(i) : 0;
   // what beta multiplies is under way while the products run
   double add[2] = {};
-  if (g.beta != 0.0) {
+  if (EXT && g.beta != 0.0) {
     const double* c0 = (g.C0 ? g.C0 + bz * g.C.sb : Cb) + ri;
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
@@ -265,15 +267,15 @@ __global__ void __launch_bounds__(32) gemm_f64_small_kernel(const GemmF64 g) {
     if (j >= g.N) continue;
     if (g.sym == SYM_ROWCOL && m0 == n0 && j < i) continue;  // the diagonal block's mirror writes these
     double v = g.alpha * (e ? c1 : c0);
-    double* dst = Cb + ri + g.C.c.at(g.sym == SYM_TRICOL ? pair_index(j, g.pair_n) : j);
-    if (g.beta != 0.0) v += g.beta * add[e];
+    double* dst = Cb + ri + g.C.c.at(EXT && g.sym == SYM_TRICOL ? pair_index(j, g.pair_n) : j);
+    if (g.beta != 0.0) v += g.beta * (EXT ? add[e] : *dst);
     *dst = v;
     if (g.sym == SYM_ROWCOL && (mirror_rc || j > i)) {
       Cb[g.C.r.at(j) + g.C.c.at(i)] = v;
     } else if (g.sym == SYM_PAIRCOL) {
       const int mm = j / g.pair_n, nn = j % g.pair_n;
       if (nn > mm) Cb[ri + g.C.c.at((long long)nn * g.pair_n + mm)] = v;
-    } else if (g.sym == SYM_TRICOL) {
+    } else if (EXT && g.sym == SYM_TRICOL) {
       int mm, nn;
       tri_pair(j, g.pair_n, mm, nn);
       if (nn > mm) Cb[ri + g.C.c.at((long long)nn * g.pair_n + mm)] = v;
@@ -297,23 +299,26 @@ int gemm_f64(const GemmF64& g, cudaStream_t stream) {
   const long long gx = (g.N + BN - 1) / BN;
   GB_REQUIRE(gy <= 65535 && g.batch <= 65535 && gx <= 2147483647LL, GB_ERR_BAD_SHAPE,
              "gemm_f64: grid too large (M=%d N=%d batch=%d)", g.M, g.N, g.batch);
+  const bool ext = g.sym == SYM_TRICOL || g.C0;
   if (gx * gy * g.batch < 152 && g.M <= 65535 * 8) {
     // fewer 64 x 64 tiles than SMs: spread 8 x 8 blocks over the GPU instead
     const unsigned nb = (unsigned)((g.N + 7) / 8);
     const dim3 sgrid = g.sym == SYM_ROWCOL ? dim3(nb * (nb + 1) / 2, 1, (unsigned)g.batch)
                                            : dim3(nb, (unsigned)((g.M + 7) / 8), (unsigned)g.batch);
-    GB_LAUNCH_CHAIN(g.tag, stream, gemm_f64_small_kernel<4>, sgrid, dim3(32), 0, g);
+    if (ext)
+      GB_LAUNCH_CHAIN(g.tag, stream, (gemm_f64_small_kernel<4, true>), sgrid, dim3(32), 0, g);
+    else
+      GB_LAUNCH_CHAIN(g.tag, stream, (gemm_f64_small_kernel<4, false>), sgrid, dim3(32), 0, g);
     return GB_OK;
   }
-  dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)g.batch);
-  if (g.a_kfast && g.b_kfast)
-    GB_LAUNCH_CHAIN(g.tag, stream, (gemm_f64_kernel<true, true>), grid, dim3(THREADS), 0, g);
-  else if (g.a_kfast)
-    GB_LAUNCH_CHAIN(g.tag, stream, (gemm_f64_kernel<true, false>), grid, dim3(THREADS), 0, g);
-  else if (g.b_kfast)
-    GB_LAUNCH_CHAIN(g.tag, stream, (gemm_f64_kernel<false, true>), grid, dim3(THREADS), 0, g);
-  else
-    GB_LAUNCH_CHAIN(g.tag, stream, (gemm_f64_kernel<false, false>), grid, dim3(THREADS), 0, g);
+  using Kernel = void (*)(GemmF64);
+  static const Kernel kernels[2][2][2] = {
+      {{gemm_f64_kernel<false, false, false>, gemm_f64_kernel<false, false, true>},
+       {gemm_f64_kernel<false, true, false>, gemm_f64_kernel<false, true, true>}},
+      {{gemm_f64_kernel<true, false, false>, gemm_f64_kernel<true, false, true>},
+       {gemm_f64_kernel<true, true, false>, gemm_f64_kernel<true, true, true>}}};
+  GB_LAUNCH_CHAIN(g.tag, stream, kernels[g.a_kfast][g.b_kfast][ext], dim3((unsigned)gx, (unsigned)gy, (unsigned)g.batch),
+                  dim3(THREADS), 0, g);
   return GB_OK;
 }
 
