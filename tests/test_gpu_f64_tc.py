@@ -279,3 +279,24 @@ def test_sizes_where_the_rule_changes_units(ops, N):
     assert nrel(imo, ref) < TOL and nrel(hm, C.T @ H @ Cp) < TOL
     m4, = _host(ops.mo4_full(dC, dI, (1, P), (0, N), (2, N), (0, P)))
     assert nrel(m4, np.einsum("mp,nq,mnsl,sr,lt->pqrt", C[:, 1:P], C, I, C[:, 2:], Cp, optimize=True)) < TOL
+
+
+@pytest.mark.parametrize("spread", [0, 40])
+def test_graded_rows_in_place(ops, spread):
+    """F = cj J - ck K adds to its output in place: tiles left to FP64 arithmetic beside
+    tiles that are stored, each added once."""
+    P, N = 150, 150
+    rng = np.random.default_rng(spread)
+    J, K = rng.standard_normal((2, P, N * N))
+    cj, ck = rng.standard_normal((2, P, P))
+    np.fill_diagonal(cj, 0.0)
+    np.fill_diagonal(ck, 0.0)
+    ck[[5, 149], 0], K[0, [70, 10000]] = 2.0**spread, 2.0**-spread
+    z = ops.to_device(np.zeros(P))
+    F, = _host(ops.fock_rc(*(ops.to_device(x.reshape(P, N, N)) for x in (J, K)), z, ops.to_device(np.zeros((N, N))),
+                           ops.to_device(cj), ops.to_device(ck), 1, 1))
+    F, ref = F.reshape(P, N * N), cj @ J - ck @ K
+    rows = np.setdiff1d(np.arange(P), [5, 149])
+    assert nrel(F[rows], ref[rows]) < TOL
+    assert _element_error(-F, np.concatenate([-cj, ck], 1), np.concatenate([J, K], 0), rows=[5, 6, 149],
+                          cols=[0, 70, 71, 9999, 10000]) < 2 * np.sqrt(2 * P)
