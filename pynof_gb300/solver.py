@@ -157,8 +157,6 @@ class Backend:
         if sq >= 0:
             b["Cprev"].copy_(b["C"])
             ops.rotate_orbital(b["y"], b["Cprev"], st.nbf5, out=b["C"], norm1=0.5 * 2.0 ** sq)
-        self.calls["jkh_mo"] += 1
-        self.calls["lagrange2"] += 1
         mo_out, l2_out = (b["J"], b["K"], b["Hc"]), (b["elag"], b["Hmat"])
         if self.precision == "mixed":
             # one call: the half transform and the MO transform serve both
@@ -171,6 +169,8 @@ class Backend:
 
     def _run_step(self, sq):
         b = self._static()
+        self.calls["jkh_mo"] += 1
+        self.calls["lagrange2"] += 1
         with torch.cuda.stream(self.stream):
             if not self.use_graphs:
                 self._step_body(sq)

@@ -63,3 +63,20 @@ def test_solver_converges_and_precision_switch(torch_cuda):
     # level; the arithmetic difference of the mixed path itself is 4e-9 Eh at
     # nbf=600 (bench.py --mode precision)
     assert abs(r64.E_elec - rmx.E_elec) < 1e-5, (r64.E_elec, rmx.E_elec)
+
+
+@pytest.mark.parametrize("use_graphs", [True, False])
+def test_every_orbital_step_is_counted(torch_cuda, use_graphs):
+    """The step count that a server reports: one per step, replayed or not."""
+    from pynof_gb300 import nof, solver, synthetic
+
+    st = synthetic.Structure.for_nbf(30)
+    b, C, H, n = synthetic.make_inputs(st, 3)
+    cj, ck = nof.cjckd8(n, st)
+    np.fill_diagonal(cj, 0.0)
+    np.fill_diagonal(ck, 0.0)
+    be = solver.Backend(st, b, H, "mixed", use_graphs=use_graphs)
+    be.orbital_begin(C, n, cj, ck)
+    for _ in range(5):
+        be.orbital_step(np.full(st.nvar, 1e-3))
+    assert be.calls == {"jkh_mo": 6, "lagrange2": 6}
